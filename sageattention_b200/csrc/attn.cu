@@ -15,35 +15,41 @@
 //
 // O lives in tensor memory and the P.V MMAs accumulate into it (the reference keeps O in registers and adds a
 // fresh product per key tile); like the reference it is multiplied by 2^((m_old - m_new) c) whenever a row's
-// maximum has moved - here in place in tensor memory, and only by the warps in which some row's maximum did move,
-// which after the first few key tiles of a long row is rare.  P, its block scales and the row sum are the
-// reference's value for value (kLazyLog2 = 0).  A build with kLazyLog2 > 0 rescales only after the maximum has
-// grown by more than 2^kLazyLog2 and normalises P to 2688 / 2^kLazyLog2 instead; the E4M3 rounding of the block
-// scales then falls differently than in the reference (same size of error, different realisation), which
-// measured 2.7-3.1 % relative L1 against the restatement of the reference - outside the 2 % parity bar - for a
-// gain of a few percent, so it is not the default.
+// maximum has moved - here in place in tensor memory, and only by the warps in which some row's maximum did move.
+// P, its block scales and the row sum are the reference's value for value.
 //
 // One persistent CTA per SM walks a static list of work items (round r: item r*grid + i, odd rounds in
 // reverse CTA order; causal items sorted by falling cost over all heads);
 // an item is TWO adjacent 128-row query tiles of one head, which share every K / V tile.  All
-// barrier phases keep counting across items, so the loads and the first Q.K^T of the next item are
-// under way while the last softmax and the output store of the current one finish.  12 warps:
+// barrier phases keep counting across items, so the loads, the first Q.K^T and the first softmax of the next item are
+// under way while the output of the current one is stored.  16 warps:
 //   warps 0-3   softmax warpgroup of query tile 0: thread r owns score row r (tensor-memory lane r).  Per key
 //               tile it copies its 128 scores from tensor memory into registers and releases the score buffer at
 //               once (the Q.K^T of the other query tile is issued into it while this tile is worked on), then:
 //               16-key block maxima, block scales, exponentials, E2M1 codes of P^ into tensor memory (the P.V MMA
-//               takes its A operand from there; only the block scales go through shared memory).  It never
-//               waits for the P.V product: the MMA accumulates into the tile's O in tensor memory.  At the end of
-//               an item O / l goes out as bf16 (D=128: through a swizzled staging tile and TMA stores).
-//   warps 4-7   the same for query tile 1; the two warpgroups settle half a period apart
-//   warp  8     TMA producer (Q tiles per item, then a ring of K and V stages; scale factors and the
+//               takes its A operand from there; only the block scales go through shared memory).
+//   warps 4-7   the same for query tile 1
+//   warps 8-11  O: rescale it between two P.V MMAs where a row maximum moved, and at the end of an item write O / l as
+//               bf16 (D=128: through a swizzled staging tile and TMA stores).  One warp per 32 rows, for both query
+//               tiles in turn
+//   warp  12    TMA producer (Q tiles per item, then a ring of K and V stages; scale factors and the
 //               delta_s rows by plain bulk copies)
-//   warp  9     QK issuer (one lane): scale-factor copies, rank-1 delta_s MMA and Q.K^T MMAs, both tiles in turn
+//   warp  13    QK issuer: scale-factor copies, rank-1 delta_s MMA and Q.K^T MMAs, both tiles in turn
 //               into the ONE score buffer
-//   warp 10     turns each delta_s row (128 bf16) into the B operand of a rank-1 bf16 MMA
+//   warp  14    turns each delta_s row (128 bf16) into the B operand of a rank-1 bf16 MMA
 //               (ones x delta_s) that initialises the score accumulator, so the softmax warps never
 //               touch delta_s
-//   warp 11     PV issuer (one lane): scale-factor copies and P.V MMAs, O_t += P^_t V^
+//   warp  15    PV issuer: scale-factor copies and P.V MMAs, O_t += P^_t V^
+//
+// What bounds it: the softmax warps' own instruction stream.  Two of them share a sub-partition (a score row in
+// registers leaves room for no more), so whatever one waits for is idle time unless the other happens to be in its
+// exponentials.  Hence: everything that is not softmax - the rescaling, the output - is other warps' work
+// (B4 Hq32 Hkv8 N8192 D128 causal: 1.79 -> 1.61 ms; B4 H32 N4096 D64: 0.815 -> 0.79 ms); all 32 lanes of a role warp
+// wait and one issues, because a wait executed by a single lane polls instead of parking and answers 40 cycles later;
+// waits for what has usually happened test once before they park (45 cycles instead of 120); the poll loop is a handful
+// of instructions in one asm block (left to the compiler it was unrolled at every wait); and 3 of 16 exponentials run on
+// the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile.  At B1 H10 N32760 D128 the
+// kernel went from 3.86 to 3.63 ms (1560 cycles per key tile and 128 query rows; 61 % of the issue slots used).
 //
 // Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128), 48 columns of scale factors, P^0 and P^1 (16
 // columns each: 128 FP4 codes per row).
@@ -82,33 +88,19 @@ namespace {
 
 constexpr int kBlockM = 128;
 constexpr int kBlockN = 128;
-#ifndef SAGE3_STAGES
-#define SAGE3_STAGES 3
-#endif
-constexpr int kStages = SAGE3_STAGES;                   // K / V ring depth
-constexpr int kAttnThreads = 384;
+constexpr int kStages = 3;                              // K / V ring depth (4 and 5 measured the same or 1 % slower)
+constexpr int kAttnThreads = 512;
 // Register hand-over (setmaxnreg) moves registers inside the pool the CTA was LAUNCHED with; a request beyond
 // it would block forever, so the split is checked here.  kLaunchRegs is what the compiler allocates under
-// __launch_bounds__(384, 1).
-constexpr int kLaunchRegs = 168;
-#ifndef SAGE3_REGS_SOFTMAX
-#define SAGE3_REGS_SOFTMAX 224
-#define SAGE3_REGS_ROLE 56
-#endif
-template <int D> struct RegSplit { static constexpr int softmax = SAGE3_REGS_SOFTMAX, role = SAGE3_REGS_ROLE; };
-static_assert(256 * RegSplit<128>::softmax + 128 * RegSplit<128>::role <= kAttnThreads * kLaunchRegs,
+// __launch_bounds__(512, 1).
+constexpr int kLaunchRegs = 128;
+struct RegSplit { static constexpr int softmax = 192, corr = 80, role = 48; };
+static_assert(256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role) <= kAttnThreads * kLaunchRegs,
               "setmaxnreg split exceeds the CTA's register pool");
+constexpr float kNoMax = -1.0e30f;                     // row maximum where no key has been visible
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLog2Inv2688 = -11.392317422778762f;   // log2(1 / (448 * 6))  softmax_fused.h:33
 constexpr float kLog2Inv6 = -2.584962500721156f;       // log2(1 / 6)          softmax_fused.h:34
-// O in tensor memory is rescaled when a row maximum has grown by more than this (log2 units of P) since the row's
-// reference maximum was set; P is normalised to 2688 / 2^kLazyLog2 at the reference maximum so that it cannot
-// exceed 2688 (block scale 448, the E4M3 maximum) before that happens.  0 = the reference's arithmetic.
-#ifndef SAGE3_LAZY_LOG2
-#define SAGE3_LAZY_LOG2 0
-#endif
-constexpr float kLazyLog2 = (float)SAGE3_LAZY_LOG2;
-constexpr float kLog2InvTop = kLog2Inv2688 + kLazyLog2;
 
 template <int D>
 struct Smem {
@@ -132,11 +124,13 @@ struct Smem {
   static constexpr int lam = dsraw + kStages * 2 * 256;   // [2 * kStages][128] f32: lambda of the key slots (K-packing
                                                           // mode), arrives with the K stage; twice as many slots as
                                                           // stages because the softmax reads it after the stage is freed
-  static constexpr int bars = lam + 2 * kStages * 512;
-  // output staging for the TMA store: [2 tiles][D/64 column halves][128 rows x 128 bytes], 128-byte swizzle
-  static constexpr int kOStage = 128 * 128;
+  static constexpr int alpha = lam + 2 * kStages * 512;   // [2 query tiles][128] f32: factor of O where the row maximum moved
+  static constexpr int lx = alpha + 1024;                 // [2 items][2 query tiles][l, m][128] f32
+  static constexpr int bars = lx + 4096;
+  // output staging for the TMA store: [2 tiles][4 warps][D/64 column halves][32 rows x 128 bytes], 128-byte swizzle
+  static constexpr int kOStage = 32 * 128;
   static constexpr int ostage = (bars + 512 + 1023) / 1024 * 1024;
-  static constexpr int total = ostage + ((!SAGE3_VARLEN_BUILD && D == 128) ? 2 * (D / 64) * kOStage : 0);
+  static constexpr int total = ostage + ((!SAGE3_VARLEN_BUILD && D == 128) ? 8 * (D / 64) * kOStage : 0);
 };
 
 struct Bars {            // byte offsets inside the barrier block
@@ -151,13 +145,13 @@ struct Bars {            // byte offsets inside the barrier block
   static constexpr int s_free = s_full + 16;              // the score buffer has been copied into registers
   static constexpr int p_full = s_free + 8;               // [2] P^ and its scales written (O rescaled if it had to be)
   static constexpr int pv_done = p_full + 16;             // [2] P.V MMAs of tile t complete: P^ may be rewritten, O_t is current
-  static constexpr int o_free = pv_done + 16;             // [2] the epilogue has read O_t out of tensor memory
-  static constexpr int drain = o_free + 16;               // [2] the issuers' last commit when giving up
-  static constexpr int epi = drain + 16;                  // [2] rendezvous of a softmax warpgroup around its output staging
-  static constexpr int tmem_slot = epi + 16;              // u32 written by tcgen05.alloc
+  static constexpr int drain = pv_done + 16;              // [2] the issuers' last commit when giving up
+  static constexpr int corr = drain + 16;                 // [4 row quarters][2] alpha of a key tile is in shared memory, O_t may be rescaled
+  static constexpr int tmem_slot = corr + 64;             // u32 written by tcgen05.alloc
   static constexpr int abort_flag = tmem_slot + 8;
   static constexpr int run_flag = abort_flag + 4;
 };
+static_assert(Bars::run_flag + 4 <= 512, "barrier block");
 
 struct KParams {
   const uint8_t *q_sf, *k_sf, *vt_sf;
@@ -180,6 +174,10 @@ struct KParams {
 #endif
 };
 
+// one arrival per warp: lane 0's, predicated instead of branched around
+__device__ __forceinline__ void mbar_arrive_if(const bool who, const uint32_t bar) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(bar), "r"((uint32_t)who) : "memory");
+}
 // ---- packed fp32x2 arithmetic (one issue slot for two elements) and 3-input max
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -206,7 +204,7 @@ __device__ __forceinline__ float max16(const uint32_t* r) {
   const float c = fmax3(__uint_as_float(r[6]), __uint_as_float(r[7]), __uint_as_float(r[8]));
   const float d = fmax3(__uint_as_float(r[9]), __uint_as_float(r[10]), __uint_as_float(r[11]));
   const float e = fmax3(__uint_as_float(r[12]), __uint_as_float(r[13]), __uint_as_float(r[14]));
-  return fmaxf(fmax3(a, b, c), fmax3(d, e, __uint_as_float(r[15])));
+  return fmax3(fmax3(a, b, c), fmax3(d, e, __uint_as_float(r[15])), kNoMax);
 }
 
 // The softmax of one key tile works on one score row (128 values) held in the registers of one thread; every
@@ -236,6 +234,30 @@ __device__ __forceinline__ void load_scores(const uint32_t tm_S, uint32_t (&s)[1
   tmem_wait_ld();
 }
 
+// 2^x for two values on the FMA pipe (the special-function unit paces the softmax): x = n + r with n the nearest
+// integer, found by adding and subtracting 1.5 * 2^23, |r| <= 1/2; 2^r by a polynomial of degree 5, minimax in the
+// relative error (Remez exchange, computed for this file: 7.5e-8 in exact arithmetic, 2.1e-7 = 2^-22.2 evaluated in
+// fp32, the error bound of ex2.approx being 2^-22); n goes into the exponent bits.  x <= log2(6) here; below -125 (a
+// masked score) the result is 2^-125: code 0, and nothing beside the 6 that the block's largest value adds to its sum.
+__device__ __forceinline__ float2 ex2_poly(float2 x) {
+  const auto both = [](const float v) { return make_float2(v, v); };
+  x.x = fmaxf(x.x, -125.f); x.y = fmaxf(x.y, -125.f);
+  const float2 t = fadd2(x, both(12582912.f));
+  const float2 r = ffma2(fadd2(t, both(-12582912.f)), both(-1.f), x);
+  float2 p = ffma2(r, both(0.0013276472454890609f), both(0.009675540961325169f));
+  p = ffma2(p, r, both(0.05550713092088699f));
+  p = ffma2(p, r, both(0.24022120237350464f));
+  p = ffma2(p, r, both(0.6931469440460205f));
+  p = ffma2(p, r, both(1.0000001192092896f));
+  p.x = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
+  p.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
+  return p;
+}
+// Which of the 8 pairs of a 16-key block take it: 3 in 16.  Measured for 0 / 2 / 3 / 4 of 16 on rows of 256 key tiles
+// (B1 H10 N32760): D=128 3.98 / 3.75 / 3.65 / 3.72 ms, D=64 3.86 / 3.73 / 3.62 / 3.65 ms - more, and the 12
+// instructions per pair cost more issue slots than the unit's cycles they save.
+__device__ constexpr bool on_fma_pipe(const int blk, const int pair) { return pair == 3 || (pair == 6 && (blk & 1)); }
+
 // P / blockscale = 2^(s*c - (bm*c + log2(1/6))) in [0, 6] -> E2M1 codes into this row's 16 tensor-memory columns of
 // P^ (8 codes per column, in key order - the A operand of the P.V MMA is read from there); returns the row sum of the unquantised P = sum over blocks of (sum of P/blockscale) * blockscale
 // (softmax_fused.h:135-153).  neg_e[b] = -(bm_b*c + log2(1/6)), sb[b] = the block's unrounded scale.
@@ -256,8 +278,8 @@ __device__ __forceinline__ float exp_quantise_store(const uint32_t (&s)[128], co
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       e[i] = ffma2(make_float2(__uint_as_float(s[16 * blk + 2 * i]), __uint_as_float(s[16 * blk + 2 * i + 1])), c2, nb2);
-      e[i].x = ex2_approx(e[i].x);
-      e[i].y = ex2_approx(e[i].y);
+      if (on_fma_pipe(blk, i)) e[i] = ex2_poly(e[i]);
+      else { e[i].x = ex2_approx(e[i].x); e[i].y = ex2_approx(e[i].y); }
     }
     const float2 s4 = fadd2(fadd2(fadd2(e[0], e[1]), fadd2(e[2], e[3])), fadd2(fadd2(e[4], e[5]), fadd2(e[6], e[7])));
     float bsum = s4.x + s4.y;
@@ -368,10 +390,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   constexpr uint32_t kSwzQK = (D == 128) ? 4u : 6u;        // 64-byte / 32-byte swizzle
   constexpr uint32_t kSboQK = (D == 128) ? 512u : 256u;
   constexpr bool kTmaStore = !SAGE3_VARLEN_BUILD && D == 128;   // see the epilogue
-  // How the two MMA issuer threads wait (measured, same box): the longer park of a hinted try_wait costs them a
-  // little reaction time per key tile but leaves the sub-partition's issue slots to the softmax warp that shares it:
-  // +9 % on rows of 256 key tiles, -2 to -4 % on rows of 8 to 64 (and D=64 gains at every length).
-  const bool issuer_hint = (D == 64) || P.Tk >= 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled tiles need 1024-byte alignment
   const uint32_t sbase = smem_u32(smem);
@@ -386,10 +404,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       mbar_init(bars + Bars::q_full + 8 * t, 1);
       mbar_init(bars + Bars::q_empty + 8 * t, 1);          // tcgen05.commit after the last QK that reads the tile
       mbar_init(bars + Bars::s_full + 8 * t, 1);           // tcgen05.commit
-      mbar_init(bars + Bars::p_full + 8 * t, 128);
+      mbar_init(bars + Bars::p_full + 8 * t, 8);           // the softmax warps of the tile and the four of O
       mbar_init(bars + Bars::pv_done + 8 * t, 1);          // tcgen05.commit
-      mbar_init(bars + Bars::o_free + 8 * t, 128);
-      mbar_init(bars + Bars::epi + 8 * t, 128);
     }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bars + Bars::k_full + 8 * s, 1);
@@ -398,7 +414,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       mbar_init(bars + Bars::v_empty + 8 * s, 1);          // tcgen05.commit
       mbar_init(bars + Bars::ds_ready + 8 * s, 1);
     }
-    mbar_init(bars + Bars::s_free, 128);
+    mbar_init(bars + Bars::s_free, 4);
+    for (int i = 0; i < 8; ++i) mbar_init(bars + Bars::corr + 8 * i, 1);
     mbar_init(bars + Bars::drain, 1);
     mbar_init(bars + Bars::drain + 8, 1);
     // a failure reported by an earlier CTA (or an earlier launch that shares *status) stops new work
@@ -410,7 +427,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   // rank-1 operands: zero everything, then column 0 of A1 = 1.0
   for (int i = threadIdx.x; i < (L::dsraw - L::a1) / 16; i += kAttnThreads)
     reinterpret_cast<uint4*>(smem + L::a1)[i] = make_uint4(0, 0, 0, 0);
-  if (warp == 9) {
+  if (warp == 13) {
     tmem_alloc(bars + Bars::tmem_slot, 512);
     tmem_relinquish();
   }
@@ -435,15 +452,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   // and all barrier phases simply keep counting across items, so the loads, MMAs and softmax of the
   // next item start while the tail of the current one is still being finished.
   if (run) {
-    if (warp >= 8) {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit<D>::role));
-      if (warp == 8 && lane == 0) {
+    if (warp >= 12) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit::role));
+      if (warp == 12) {
         // ---------------------------------------------------------------- TMA producer
-        prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_o);
+        if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_o); }
         uint32_t g = 0;                       // K/V stages completely issued so far
         uint32_t gk = 0;                      // K stages issued so far (g or g + 1)
         uint32_t qn[2] = {0, 0};              // Q tiles loaded so far per slot
         bool ok = true;
+#pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked>(P, w);
           int64_t ds_row[2];
@@ -456,35 +474,45 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               if (qn[t] > 0 && !(ok = wait_bar<false>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1, abort_s, P.status, 12))) break;
               const int64_t qtile = ((int64_t)wk.b * P.Hq + wk.hq) * P.Tq + qt;
               const uint32_t qb = bars + Bars::q_full + 8 * t;
-              mbar_arrive_expect_tx(qb, L::kQBytes + L::kSfRow);
-              tma_load_2d(sbase + L::q + t * L::kQBytes, &tm_q, 0, (int)(qtile * kBlockM), qb);
-              bulk_load(sbase + L::sfq + t * 1024, P.q_sf + qtile * L::kSfRow, L::kSfRow, qb);
+              if (lane == 0) {
+                mbar_arrive_expect_tx(qb, L::kQBytes + L::kSfRow);
+                tma_load_2d(sbase + L::q + t * L::kQBytes, &tm_q, 0, (int)(qtile * kBlockM), qb);
+                bulk_load(sbase + L::sfq + t * 1024, P.q_sf + qtile * L::kSfRow, L::kSfRow, qb);
+              }
+              __syncwarp();
               ++qn[t];
             }
           }
           const int64_t kvhead = ((int64_t)wk.b * P.Hkv + wk.hkv) * P.Tk;
+#pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             const uint32_t ph = ((g / kStages) & 1) ^ 1;
             if (!(ok = wait_bar<false>(bars + Bars::k_empty + 8 * s, ph, abort_s, P.status, 10))) break;
             const uint32_t kb = bars + Bars::k_full + 8 * s;
             const int nds = has_ds ? (int)(j < wk.n_t[0]) + (int)(j < wk.n_t[1]) : 0;
-            mbar_arrive_expect_tx(kb, L::kKBytes + L::kSfRow + 256 * nds + (kPacked ? 512 : 0));
-            if (kPacked) bulk_load(sbase + L::lam + (g % (2 * kStages)) * 512, P.lam + (kvhead + j) * kBlockN, 512, kb);
-            tma_load_2d(sbase + L::k + s * L::kKBytes, &tm_k, 0, (int)((kvhead + j) * kBlockN), kb);
-            bulk_load(sbase + L::sfk + s * 1024, P.k_sf + (kvhead + j) * L::kSfRow, L::kSfRow, kb);
-            if (has_ds) {
+            if (lane == 0) {
+              mbar_arrive_expect_tx(kb, L::kKBytes + L::kSfRow + 256 * nds + (kPacked ? 512 : 0));
+              if (kPacked) bulk_load(sbase + L::lam + (g % (2 * kStages)) * 512, P.lam + (kvhead + j) * kBlockN, 512, kb);
+              tma_load_2d(sbase + L::k + s * L::kKBytes, &tm_k, 0, (int)((kvhead + j) * kBlockN), kb);
+              bulk_load(sbase + L::sfk + s * 1024, P.k_sf + (kvhead + j) * L::kSfRow, L::kSfRow, kb);
+              if (has_ds) {
 #pragma unroll
-              for (int t = 0; t < 2; ++t)
-                if (j < wk.n_t[t])
-                  bulk_load(sbase + L::dsraw + (s * 2 + t) * 256, P.ds + (ds_row[t] * P.Tk + j) * kBlockN, 256, kb);
+                for (int t = 0; t < 2; ++t)
+                  if (j < wk.n_t[t])
+                    bulk_load(sbase + L::dsraw + (s * 2 + t) * 256, P.ds + (ds_row[t] * P.Tk + j) * kBlockN, 256, kb);
+              }
             }
+            __syncwarp();
             ++gk;
             if (!(ok = wait_bar<false>(bars + Bars::v_empty + 8 * s, ph, abort_s, P.status, 11))) break;
             const uint32_t vb = bars + Bars::v_full + 8 * s;
-            mbar_arrive_expect_tx(vb, L::kVBytes + L::kSfV);
-            tma_load_2d(sbase + L::v + s * L::kVBytes, &tm_v, 0, (int)((kvhead + j) * D), vb);
-            bulk_load(sbase + L::sfv + s * 1024, P.vt_sf + (kvhead + j) * L::kSfV, L::kSfV, vb);
+            if (lane == 0) {
+              mbar_arrive_expect_tx(vb, L::kVBytes + L::kSfV);
+              tma_load_2d(sbase + L::v + s * L::kVBytes, &tm_v, 0, (int)((kvhead + j) * D), vb);
+              bulk_load(sbase + L::sfv + s * 1024, P.vt_sf + (kvhead + j) * L::kSfV, L::kSfV, vb);
+            }
+            __syncwarp();
           }
         }
         if (*abort_s) {
@@ -496,14 +524,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           for (uint32_t i = (g > (uint32_t)kStages ? g - kStages : 0); i < g; ++i)
             mbar_wait(bars + Bars::v_full + 8 * (i % kStages), (i / kStages) & 1, 1u << 16);
         }
-      } else if (warp == 10 && has_ds) {
+      } else if (warp == 14 && has_ds) {
         // ---------------------------------------------------------------- delta_s -> rank-1 B operand
         // B1 is a K-major [128 keys x 16] bf16 operand in 8x16-byte core matrices: key n's first
         // element sits at (n/8)*128 + (n%8)*16; everything else stays zero.
         uint32_t g = 0;
         bool ok = true;
+#pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked>(P, w);
+#pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             if (!(ok = wait_bar<false>(bars + Bars::k_full + 8 * s, (g / kStages) & 1, abort_s, P.status, 40))) break;
@@ -521,11 +551,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             if (lane == 0) mbar_arrive(bars + Bars::ds_ready + 8 * s);
           }
         }
-      } else if (warp == 9 && lane == 0) {
+      } else if (warp == 13) {
         // ---------------------------------------------------------------- QK issuer
-        // This one thread paces the CTA, so its instruction stream is kept minimal: every shared-memory
-        // descriptor is a constant high word (stride / swizzle / version bits) plus a low word
-        // (address >> 4, leading-offset field) that only needs an integer add per use.
+        // Its instruction stream is kept minimal: every shared-memory descriptor is a constant high word (stride /
+        // swizzle / version bits) plus a low word (address >> 4, leading-offset field) that only needs an integer
+        // add per use.  It waits with a suspend-time hint (1 % over all shapes).
         constexpr uint32_t idesc_qk = make_idesc_nvf4(kBlockM, kBlockN);
         constexpr uint32_t idesc_r1 = make_idesc_bf16(kBlockM, kBlockN);
         constexpr uint32_t HI_QK = (kSboQK >> 4) | (1u << 14) | (kSwzQK << 29);
@@ -539,59 +569,64 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t g = 0;                       // K stages consumed so far
         uint32_t nqk = 0;                     // QK groups issued so far (= uses of the score buffer)
         uint32_t qn[2] = {0, 0};              // Q tiles taken so far per slot
+#pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked>(P, w);
+#pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             const uint32_t ph = (g / kStages) & 1;
-            if (!(ok = wait_bar_dyn(bars + Bars::k_full + 8 * s, ph, issuer_hint, abort_s, P.status, 21))) break;
-            if (has_ds && !(ok = wait_bar_dyn(bars + Bars::ds_ready + 8 * s, ph, issuer_hint, abort_s, P.status, 25))) break;
+            if (!(ok = wait_bar<true>(bars + Bars::k_full + 8 * s, ph, abort_s, P.status, 21))) break;
+            if (has_ds && !(ok = wait_bar<true>(bars + Bars::ds_ready + 8 * s, ph, abort_s, P.status, 25))) break;
             bool first = true;
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
               if (!ok || j >= wk.n_t[t]) continue;
               // the one score buffer must be free: the softmax warpgroup that got the previous Q.K^T (the other
               // query tile, or this one in the previous key tile) has copied it into registers
-              if (nqk > 0 && !(ok = wait_bar_dyn(bars + Bars::s_free, (nqk - 1) & 1, issuer_hint, abort_s, P.status, 23))) break;
+              if (nqk > 0 && !(ok = wait_bar<true>(bars + Bars::s_free, (nqk - 1) & 1, abort_s, P.status, 23))) break;
               if (it == wk.n_max - wk.n_t[t]) {                    // first key tile of this query tile
-                if (!(ok = wait_bar_dyn(bars + Bars::q_full + 8 * t, qn[t] & 1, issuer_hint, abort_s, P.status, 20))) break;
+                if (!(ok = wait_bar<true>(bars + Bars::q_full + 8 * t, qn[t] & 1, abort_s, P.status, 20))) break;
                 ++qn[t];
                 tc_fence_after();
+                if (lane == 0)
 #pragma unroll
-                for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfq + 8 * t + 4 * kb, sfq_lo + t * 64 + kb * 32, HI_SF);
+                  for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfq + 8 * t + 4 * kb, sfq_lo + t * 64 + kb * 32, HI_SF);
               }
               tc_fence_after();
-              if (first) {
-                first = false;
+              if (lane == 0) {
+                if (first) {
 #pragma unroll
-                for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfk + 4 * kb, sfk_lo + s * 64 + kb * 32, HI_SF);
-              }
-              if (has_ds) {
-                // buffer i sits i*2048 bytes higher, so its distance to the shared zero chunk is i*2048 smaller
-                const uint32_t i = (uint32_t)(s * 2 + t);
-                tc_mma_bf16(tm_Sbuf, a1_lo, HI_SF, b1_lo + i * 128u - ((i * 128u) << 16), HI_SF, idesc_r1, 0);
-              }
+                  for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfk + 4 * kb, sfk_lo + s * 64 + kb * 32, HI_SF);
+                }
+                if (has_ds) {
+                  // buffer i sits i*2048 bytes higher, so its distance to the shared zero chunk is i*2048 smaller
+                  const uint32_t i = (uint32_t)(s * 2 + t);
+                  tc_mma_bf16(tm_Sbuf, a1_lo, HI_SF, b1_lo + i * 128u - ((i * 128u) << 16), HI_SF, idesc_r1, 0);
+                }
 #pragma unroll
-              for (int kb = 0; kb < kKB; ++kb)
-                tc_mma_nvf4(tm_Sbuf, q_lo + t * (L::kQBytes >> 4) + kb * 2, HI_QK, k_lo + s * (L::kKBytes >> 4) + kb * 2, HI_QK,
-                            idesc_qk, tm_sfq + 8 * t + 4 * kb, tm_sfk + 4 * kb, (has_ds || kb > 0) ? 1u : 0u);
-              tc_commit(bars + Bars::s_full + 8 * t);
+                for (int kb = 0; kb < kKB; ++kb)
+                  tc_mma_nvf4(tm_Sbuf, q_lo + t * (L::kQBytes >> 4) + kb * 2, HI_QK, k_lo + s * (L::kKBytes >> 4) + kb * 2, HI_QK,
+                              idesc_qk, tm_sfq + 8 * t + 4 * kb, tm_sfk + 4 * kb, (has_ds || kb > 0) ? 1u : 0u);
+                tc_commit(bars + Bars::s_full + 8 * t);
+                if (it == wk.n_max - 1) tc_commit(bars + Bars::q_empty + 8 * t);   // last read of this Q tile
+              }
+              __syncwarp();
+              first = false;
               ++nqk;
-              if (it == wk.n_max - 1) tc_commit(bars + Bars::q_empty + 8 * t);   // last read of this Q tile
             }
-            if (ok) tc_commit(bars + Bars::k_empty + 8 * s);
+            if (ok && lane == 0) tc_commit(bars + Bars::k_empty + 8 * s);
           }
         }
         if (!ok) {
           // giving up: let every MMA / scale copy already issued finish before tensor memory is freed
-          tc_commit(bars + Bars::drain);
+          if (lane == 0) tc_commit(bars + Bars::drain);
           mbar_wait(bars + Bars::drain, 0, 1u << 16);
         }
-      } else if (warp == 11 && lane == 0) {
+      } else if (warp == 15) {
         // ---------------------------------------------------------------- PV issuer
         // O_t += P^_t V^ for both tiles, from its own thread so that waiting for P^ never delays the next QK.
-        // The first key tile of a work item overwrites O_t (no accumulate) - once the epilogue of the previous item
-        // in that slot has read it out.
+        // The first key tile of a work item overwrites O_t (no accumulate).
         constexpr uint32_t idesc_pv = make_idesc_nvf4(kBlockM, D);
         constexpr uint32_t HI_PV = (512u >> 4) | (1u << 14) | (4u << 29);
         constexpr uint32_t HI_SF = (128u >> 4) | (1u << 14);
@@ -599,291 +634,310 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         const uint32_t v_lo = ((sbase + L::v) >> 4) | LBO1;
         const uint32_t sfv_lo = (sbase + L::sfv) >> 4, sfp_lo = (sbase + L::sfp) >> 4;
         bool ok = true;
-        uint32_t g = 0, pv_cnt[2] = {0, 0}, n_epi[2] = {0, 0};
+        uint32_t g = 0, pv_cnt[2] = {0, 0};
+#pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked>(P, w);
+#pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             const bool act1 = j < wk.n_t[1];
             // the V stage and its scale factors do not depend on the softmax: fetch them before waiting for P
-            if (!(ok = wait_bar_dyn(bars + Bars::v_full + 8 * s, (g / kStages) & 1, issuer_hint, abort_s, P.status, 24))) break;
+            if (!(ok = wait_bar<false>(bars + Bars::v_full + 8 * s, (g / kStages) & 1, abort_s, P.status, 24))) break;
             tc_fence_after();
+            if (lane == 0)
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfv + 4 * kb, sfv_lo + s * 64 + kb * 32, HI_SF);
+              for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfv + 4 * kb, sfv_lo + s * 64 + kb * 32, HI_SF);
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
               const bool act = t == 0 ? (j < wk.n_t[0]) : act1;
               if (!(ok && act)) continue;
               const bool first_tile = it == wk.n_max - wk.n_t[t];
-              if (!(ok = wait_bar_dyn(bars + Bars::p_full + 8 * t, pv_cnt[t] & 1, issuer_hint, abort_s, P.status, 26))) break;
-              if (first_tile) {
-                if (n_epi[t] > 0 && !(ok = wait_bar_dyn(bars + Bars::o_free + 8 * t, (n_epi[t] - 1) & 1, issuer_hint, abort_s, P.status, 22))) break;
-                ++n_epi[t];
-              }
+              if (!(ok = wait_bar<false>(bars + Bars::p_full + 8 * t, pv_cnt[t] & 1, abort_s, P.status, 26))) break;
               tc_fence_after();
+              if (lane == 0) {
 #pragma unroll
-              for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfp + 8 * t + 4 * kb, sfp_lo + t * 64 + kb * 32, HI_SF);
+                for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfp + 8 * t + 4 * kb, sfp_lo + t * 64 + kb * 32, HI_SF);
 #pragma unroll
-              for (int kb = 0; kb < 2; ++kb)
-                tc_mma_nvf4_ta(tmem + t * D, tm_P + 16 * t + 8 * kb, v_lo + s * (L::kVBytes >> 4) + kb * 2, HI_PV,
-                               idesc_pv, tm_sfp + 8 * t + 4 * kb, tm_sfv + 4 * kb, (first_tile && kb == 0) ? 0u : 1u);
-              tc_commit(bars + Bars::pv_done + 8 * t);
+                for (int kb = 0; kb < 2; ++kb)
+                  tc_mma_nvf4_ta(tmem + t * D, tm_P + 16 * t + 8 * kb, v_lo + s * (L::kVBytes >> 4) + kb * 2, HI_PV,
+                                 idesc_pv, tm_sfp + 8 * t + 4 * kb, tm_sfv + 4 * kb, (first_tile && kb == 0) ? 0u : 1u);
+                tc_commit(bars + Bars::pv_done + 8 * t);
+                if (t == 1 || !act1) tc_commit(bars + Bars::v_empty + 8 * s);   // last PV of this stage
+              }
+              __syncwarp();
               ++pv_cnt[t];
-              if (t == 1 || !act1) tc_commit(bars + Bars::v_empty + 8 * s);   // last PV of this stage
             }
           }
         }
         if (!ok) {
-          tc_commit(bars + Bars::drain + 8);
+          if (lane == 0) tc_commit(bars + Bars::drain + 8);
           mbar_wait(bars + Bars::drain + 8, 0, 1u << 16);
         }
       }
     } else {
-      // ------------------------------------------------------------------ softmax
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegSplit<D>::softmax));
-      const int t = warp >> 2;                                   // query tile slot of this warpgroup
-      const int row = threadIdx.x & 127;                         // tensor-memory lane
-      const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-      const uint32_t tm_S = tm_Sbuf + lane_addr;
-      const uint32_t tm_O = tmem + t * D + lane_addr;
+      const int quarter = warp & 3;
+      const int row = quarter * 32 + lane;                       // tensor-memory lane
+      const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
       const float c = P.scale_log2;
-      const uint32_t tm_Prow = tm_P + 16 * t + lane_addr;        // this row of P^: 16 columns of 8 codes
-      uint32_t* sfp_row = reinterpret_cast<uint32_t*>(smem + L::sfp + t * 1024 + sf_atom_offset(row, 0));
-      const uint32_t bar_s = bars + Bars::s_full + 8 * t, bar_p = bars + Bars::p_full + 8 * t;
-      const uint32_t bar_pv = bars + Bars::pv_done + 8 * t;
-      uint32_t sc = 0;                                           // key tiles processed so far by this warpgroup
-      uint32_t ne = 0;                                           // epilogue rendezvous so far
-      uint32_t g0 = 0;                                           // K/V stages the CTA used before this work item
       bool ok = true;
-      for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-        const Work wk = get_work<kCausal, kPacked>(P, w);
-        const int n_mine = wk.n_t[t];
-        const uint32_t g_first = g0 + (uint32_t)(wk.n_max - n_mine);   // stage counter of this tile's first key tile
-        g0 += (uint32_t)wk.n_max;
-        const int qt = 2 * wk.pair + t;
-        const int q0 = qt * kBlockM, qpos = q0 + row;
-#if SAGE3_VARLEN_BUILD
-        __nv_bfloat16* orow = P.out + wk.hq * P.o_sh + (int64_t)(wk.q_base + qpos) * P.o_sn;   // packed output
-#else
-        __nv_bfloat16* orow = P.out + wk.b * P.o_sb + wk.hq * P.o_sh + (int64_t)qpos * P.o_sn;
-#endif
-        if (n_mine == 0) {
-          // query tile that sees no key at all (causal, more queries than keys): zeros, like the
-          // reference's store_zero (fwd_epilogue.cu:150-183); nothing if the tile does not exist
-          if (SEQ_TILE_EXISTS && qpos < SEQ_NQ) {
-            for (int i = 0; i < P.d_out / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
-            if (P.lse) P.lse[((int64_t)wk.b * P.Hq + wk.hq) * P.Nq + qpos] = -INFINITY;
-          }
-          continue;
-        }
-        // last visible key (slot): key padding, and the bottom-right aligned causal diagonal - in K-packing mode
-        // the slots of the tokens up to the diagonal one
-        auto causal_limit = [&](const int qp) {
-          const int tok = qp + SEQ_NK_LOG - SEQ_NQ;              // last visible key token
-          if (!kPacked) return tok;
-          return tok < 0 ? -1 : packed_slot_of_token(tok);
-        };
-        const int key_lim = min(SEQ_NK - 1, kCausal ? causal_limit(qpos) : 0x7fffffff);
-        const int first_row_lim = kCausal ? causal_limit(q0) : 0x7fffffff;
-        float m_ref = -INFINITY, l = 0.f;                        // reference maximum (raw score units), row sum
+      if (warp < 8) {
+        // ---------------------------------------------------------------- softmax
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegSplit::softmax));
+        const int t = warp >> 2;                                 // query tile slot of this warpgroup
+        const uint32_t tm_S = tm_Sbuf + lane_addr;
+        const uint32_t tm_Prow = tm_P + 16 * t + lane_addr;      // this row of P^: 16 columns of 8 codes
+        uint32_t* sfp_row = reinterpret_cast<uint32_t*>(smem + L::sfp + t * 1024 + sf_atom_offset(row, 0));
+        volatile float* alpha_row = reinterpret_cast<volatile float*>(smem + L::alpha) + t * 128 + row;
+        volatile float* l_row = reinterpret_cast<volatile float*>(smem + L::lx) + t * 256 + row;   // [2 items][l, m]
+        const uint32_t bar_s = bars + Bars::s_full + 8 * t, bar_p = bars + Bars::p_full + 8 * t;
+        const uint32_t bar_pv = bars + Bars::pv_done + 8 * t, bar_c = bars + Bars::corr + 8 * (2 * quarter + t);
+        uint32_t sc = 0;                                         // key tiles processed so far by this warpgroup
+        uint32_t g0 = 0;                                         // K/V stages the CTA used before this work item
+        uint32_t items = 0;
+#pragma unroll 1
+        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const int n_mine = t == 0 ? wk.n_t[0] : wk.n_t[1];
+          const uint32_t g_first = g0 + (uint32_t)(wk.n_max - n_mine);   // stage counter of this tile's first key tile
+          g0 += (uint32_t)wk.n_max;
+          if (n_mine == 0) continue;
+          const int q0 = (2 * wk.pair + t) * kBlockM, qpos = q0 + row;
+          // last visible key (slot): key padding, and the bottom-right aligned causal diagonal - in K-packing mode
+          // the slots of the tokens up to the diagonal one
+          auto causal_limit = [&](const int qp) {
+            const int tok = qp + SEQ_NK_LOG - SEQ_NQ;            // last visible key token
+            if (!kPacked) return tok;
+            return tok < 0 ? -1 : packed_slot_of_token(tok);
+          };
+          const int key_lim = min(SEQ_NK - 1, kCausal ? causal_limit(qpos) : 0x7fffffff);
+          const int first_row_lim = kCausal ? causal_limit(q0) : 0x7fffffff;
+          float m_run = kNoMax, l = 0.f;                         // row maximum so far (raw score units), row sum
 
-        for (int it = 0; it < n_mine; ++it, ++sc) {
-          const int j = n_mine - 1 - it;
-          const int n0 = j * kBlockN;
-          const bool need_mask = (n0 + kBlockN - 1 >= SEQ_NK) || (kCausal && n0 + kBlockN - 1 > first_row_lim);
-          if (!(ok = wait_bar<false>(bar_s, sc & 1, abort_s, P.status, 30))) break;
-          tc_fence_after();
-          uint32_t s[128];
-          float bm[8];
-          load_scores(tm_S, s);
-          // the scores are in registers: the Q.K^T of the other query tile may overwrite the buffer
-          tc_fence_before();
-          mbar_arrive(bars + Bars::s_free);
-          if (kPacked) {
-            // lambda of this key tile arrived with its K stage, i.e. before the Q.K^T MMA whose completion was
-            // awaited above.  Its slot is rewritten 2*kStages key tiles later, which the producer can only do
-            // after the Q.K^T of tile g+kStages is complete - issued after both warpgroups finished tile g.
-            const uint32_t g = g_first + (uint32_t)it;
-            const float* lam_s = reinterpret_cast<const float*>(smem + L::lam) + (g % (2 * kStages)) * 128;
-#pragma unroll
-            for (int blk = 0; blk < 8; ++blk) apply_lambda(&s[16 * blk], lam_s + 16 * blk);
-          }
-          if (need_mask) {
-            const int lim = key_lim - n0;                        // columns beyond it are masked
-#pragma unroll
-            for (int i = 0; i < 128; ++i) s[i] = (i > lim) ? 0xff800000u : s[i];
-          }
-          if (kPacked && P.slot_first) {
-            // the other K-packing variant (fwd_mainloop.cu:847-891): the mean slot carries the (masked) score of the
-            // group's first token - its V row holds that token's FP4 remainder - except, under the causal mask, in
-            // the group of the diagonal token and beyond
-            const int qk = qpos + SEQ_NK_LOG - SEQ_NQ;           // the diagonal key token of this row
-            const int last_group = kCausal ? (qk < 0 ? -1 : qk / 15 - 1) : 0x7ffffff;   // last group whose slot may be used
-#pragma unroll
-            for (int blk = 0; blk < 8; ++blk) {
-              const int col = n0 + 16 * blk;
-              const bool usable = !kCausal || (col < SEQ_NK && (col >> 4) <= last_group);
-              s[16 * blk] = usable ? s[16 * blk + 1] : 0xff800000u;
-            }
-          }
-#pragma unroll
-          for (int blk = 0; blk < 8; ++blk)
-            bm[blk] = max16(&s[16 * blk]);
-          const float m_loc = fmax3(fmax3(bm[0], bm[1], bm[2]), fmax3(bm[3], bm[4], bm[5]), fmaxf(bm[6], bm[7]));
-          // O_t *= alpha for the rows whose reference maximum moves, in place in tensor memory - but only after this
-          // tile's exponentials (below): by then the P.V of the previous key tile, which must land first, has long
-          // finished, so nothing waits for it.  Warps in which no row's maximum moved skip the pass.
-          float alpha = 1.0f;
-          bool rescale = false;
-          if (it == 0) {
-            m_ref = m_loc;                                       // O_t is overwritten by this tile's P.V
-          } else {
-            // (-inf) - (-inf) = NaN compares false: a row that has seen no key yet and sees none now stays put
-            const bool grow = (m_loc - m_ref) * c > kLazyLog2;
-            rescale = __any_sync(0xffffffffu, grow);
-            if (grow) {
-              alpha = ex2_approx((m_ref - m_loc) * c);
-              m_ref = m_loc;
-              l *= alpha;
-            }
-          }
-          const float m_fin = (m_ref == -INFINITY) ? 0.f : m_ref;
-          const float off = fmaf(m_fin, c, kLog2InvTop);          // P = 2^(s*c - off) in (0, 2688]
-          float neg_e[8], sb[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float e = fmaf(bm[i], c, kLog2Inv6);
-            sb[i] = ex2_approx(e - off);
-            neg_e[i] = (bm[i] == -INFINITY) ? 0.f : -e;
-          }
-          // P^ and its scales of the previous key tile must have been consumed by its P.V MMAs
-          if (sc > 0 && !(ok = wait_bar<false>(bar_pv, (sc - 1) & 1, abort_s, P.status, 31))) break;
-          sfp_row[0] = f32x2_to_e4m3x2(sb[0], sb[1]) | (f32x2_to_e4m3x2(sb[2], sb[3]) << 16);     // keys 0-63 of the tile
-          sfp_row[128] = f32x2_to_e4m3x2(sb[4], sb[5]) | (f32x2_to_e4m3x2(sb[6], sb[7]) << 16);   // keys 64-127
-          l += exp_quantise_store<kPacked>(s, c, neg_e, sb, tm_Prow, P.slot_first);
-          if (rescale) {
-            if (!(ok = wait_bar<false>(bar_pv, (sc - 1) & 1, abort_s, P.status, 32))) break;
+#pragma unroll 1
+          for (int it = 0; it < n_mine; ++it, ++sc) {
+            const int n0 = (n_mine - 1 - it) * kBlockN;
+            const bool need_mask = (n0 + kBlockN - 1 >= SEQ_NK) || (kCausal && n0 + kBlockN - 1 > first_row_lim);
+            if (!(ok = wait_bar_soon(bar_s, sc & 1, abort_s, P.status, 30))) break;
             tc_fence_after();
-            const float2 al2 = make_float2(alpha, alpha);
-            // the whole O row at once (the score registers are free by now): all loads in flight together, one
-            // wait, then scale and store - a chunk-by-chunk round trip would expose the tensor-memory latency 8 times
-            uint32_t o[D];
+            uint32_t s[128];
+            float bm[8];
+            load_scores(tm_S, s);
+            // the scores are in registers: the Q.K^T of the other query tile may overwrite the buffer
+            tc_fence_before();
+            mbar_arrive_if(lane == 0, bars + Bars::s_free);
+            if (kPacked) {
+              // lambda of this key tile arrived with its K stage, i.e. before the Q.K^T MMA whose completion was
+              // awaited above.  Its slot is rewritten 2*kStages key tiles later, which the producer can only do
+              // after the Q.K^T of tile g+kStages is complete - issued after both warpgroups finished tile g.
+              const uint32_t g = g_first + (uint32_t)it;
+              const float* lam_s = reinterpret_cast<const float*>(smem + L::lam) + (g % (2 * kStages)) * 128;
 #pragma unroll
-            for (int ch = 0; ch < D / 32; ++ch) tmem_ld32(tm_O + 32 * ch, *reinterpret_cast<uint32_t (*)[32]>(&o[32 * ch]));
-            tmem_wait_ld();
+              for (int blk = 0; blk < 8; ++blk) apply_lambda(&s[16 * blk], lam_s + 16 * blk);
+            }
+            if (need_mask) {
+              const int lim = key_lim - n0;                      // columns beyond it are masked
 #pragma unroll
-            for (int i = 0; i < D / 2; ++i) {
-              const float2 x = ffma2(make_float2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), al2,
-                                     make_float2(0.f, 0.f));
-              o[2 * i] = __float_as_uint(x.x); o[2 * i + 1] = __float_as_uint(x.y);
+              for (int i = 0; i < 128; ++i) s[i] = (i > lim) ? 0xff800000u : s[i];
+            }
+            if (kPacked && P.slot_first) {
+              // the other K-packing variant (fwd_mainloop.cu:847-891): the mean slot carries the (masked) score of the
+              // group's first token - its V row holds that token's FP4 remainder - except, under the causal mask, in
+              // the group of the diagonal token and beyond
+              const int qk = qpos + SEQ_NK_LOG - SEQ_NQ;         // the diagonal key token of this row
+              const int last_group = kCausal ? (qk < 0 ? -1 : qk / 15 - 1) : 0x7ffffff;   // last group whose slot may be used
+#pragma unroll
+              for (int blk = 0; blk < 8; ++blk) {
+                const int col = n0 + 16 * blk;
+                const bool usable = !kCausal || (col < SEQ_NK && (col >> 4) <= last_group);
+                s[16 * blk] = usable ? s[16 * blk + 1] : 0xff800000u;
+              }
             }
 #pragma unroll
-            for (int ch = 0; ch < D / 16; ++ch) tmem_st16(tm_O + 16 * ch, *reinterpret_cast<const uint32_t (*)[16]>(&o[16 * ch]));
+            for (int blk = 0; blk < 8; ++blk) bm[blk] = max16(&s[16 * blk]);
+            const float m_loc = fmax3(fmax3(bm[0], bm[1], bm[2]), fmax3(bm[3], bm[4], bm[5]), fmaxf(bm[6], bm[7]));
+            const float m_new = fmaxf(m_run, m_loc);
+            const float alpha = ex2_approx((m_run - m_new) * c);
+            l *= alpha;
+            m_run = m_new;
+            const float off = fmaf(m_new, c, kLog2Inv2688);       // P = 2^(s*c - off) in (0, 2688]
+            float neg_e[8], sb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float e = fmaf(bm[i], c, kLog2Inv6);
+              sb[i] = ex2_approx(e - off);
+              neg_e[i] = -e;
+            }
+            // the P.V MMAs of the previous key tile are complete: P^ and its scales may be rewritten, O rescaled
+            if (sc > 0 && !(ok = wait_bar_soon(bar_pv, (sc - 1) & 1, abort_s, P.status, 31))) break;
+            *alpha_row = alpha;
+            __syncwarp();
+            mbar_arrive_if(lane == 0, bar_c);
+            sfp_row[0] = f32x2_to_e4m3x2(sb[0], sb[1]) | (f32x2_to_e4m3x2(sb[2], sb[3]) << 16);     // keys 0-63 of the tile
+            sfp_row[128] = f32x2_to_e4m3x2(sb[4], sb[5]) | (f32x2_to_e4m3x2(sb[6], sb[7]) << 16);   // keys 64-127
+            l += exp_quantise_store<kPacked>(s, c, neg_e, sb, tm_Prow, P.slot_first);
+            if (it == n_mine - 1) {
+              l_row[(items & 1) * 512] = l;
+              l_row[(items & 1) * 512 + 128] = m_run;
+            }
+            // P^ written: hand the tile to the PV issuer.  The codes went to tensor memory (tcgen05.st), their block
+            // scales to shared memory for the issuer's tcgen05.cp.
             tmem_wait_st();
+            tc_fence_before();
+            fence_proxy_async_smem();
+            __syncwarp();
+            mbar_arrive_if(lane == 0, bar_p);
           }
-          // P^ written (and O_t rescaled if it had to be): hand the tile to the PV issuer.  The codes went to tensor
-          // memory (tcgen05.st), their block scales to shared memory for the issuer's tcgen05.cp.
-          tmem_wait_st();
-          tc_fence_before();
-          fence_proxy_async_smem();
-          mbar_arrive(bar_p);
+          ++items;
         }
+      } else {
+        // ---------------------------------------------------------------- O: rescaling and output
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit::corr));
+        uint32_t sc[2] = {0, 0}, items[2] = {0, 0};              // key tiles / work items so far per query tile slot
+#pragma unroll 1
+        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+          const Work wk = get_work<kCausal, kPacked>(P, w);
+          // O_t *= alpha for the rows whose maximum moved, in place in tensor memory, between the P.V of the previous
+          // key tile and that of this one; warps in which no row's maximum moved skip it.  The first key tile of an
+          // item overwrites O_t: this arrival then says that the previous item's output has been read.
+#pragma unroll 1
+          for (int it = 0; ok && it < wk.n_max; ++it) {
+#pragma unroll 1
+            for (int t = 0; t < 2; ++t) {
+              const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
+              if (wk.n_max - 1 - it >= n_t) continue;
+              uint32_t& cnt = t == 0 ? sc[0] : sc[1];
+              if (!(ok = wait_bar<false>(bars + Bars::corr + 8 * (2 * quarter + t), cnt & 1, abort_s, P.status, 32))) break;
+              ++cnt;
+              const float alpha = *(reinterpret_cast<volatile float*>(smem + L::alpha) + t * 128 + row);
+              if (it != wk.n_max - n_t && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                tc_fence_after();
+                const uint32_t tm_O = tmem + t * D + lane_addr;
+                const float2 al2 = make_float2(alpha, alpha);
+                uint32_t o[64];
+#pragma unroll 1
+                for (int hf = 0; hf < D / 64; ++hf) {
+                  tmem_ld32(tm_O + hf * 64, *reinterpret_cast<uint32_t (*)[32]>(&o[0]));
+                  tmem_ld32(tm_O + hf * 64 + 32, *reinterpret_cast<uint32_t (*)[32]>(&o[32]));
+                  tmem_wait_ld();
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) {
+                    const float2 x = ffma2(make_float2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), al2,
+                                           make_float2(0.f, 0.f));
+                    o[2 * i] = __float_as_uint(x.x); o[2 * i + 1] = __float_as_uint(x.y);
+                  }
+#pragma unroll
+                  for (int ch = 0; ch < 4; ++ch)
+                    tmem_st16(tm_O + hf * 64 + 16 * ch, *reinterpret_cast<const uint32_t (*)[16]>(&o[16 * ch]));
+                }
+                tmem_wait_st();
+                tc_fence_before();
+              }
+              __syncwarp();
+              mbar_arrive_if(lane == 0, bars + Bars::p_full + 8 * t);
+            }
+          }
+          if (!ok) break;
 
-        // ---- epilogue: O / l -> bf16 -> global.  D=128, dense batches: through a swizzled staging tile in shared
-        // memory and one TMA store per 64 columns - a thread owns a whole output row, so direct stores put 32
-        // different rows into every store instruction.  D=64 (half the bytes; measured 4 % slower with the staging)
-        // and packed variable-length outputs (a tile must not spill into the next sequence) store directly.
-        if (!ok) break;
-        if (!(ok = wait_bar<false>(bar_pv, (sc - 1) & 1, abort_s, P.status, 33))) break;   // the last P.V has landed
-        tc_fence_after();
-        const float inv = (l == 0.f || l != l) ? 0.f : 1.0f / l;
-        const float2 inv2 = make_float2(inv, inv);
-        if (kTmaStore) {
-          uint8_t* stage = smem + L::ostage + t * (D / 64) * L::kOStage;
-          const uint32_t bar_e = bars + Bars::epi + 8 * t;
-          // the stores of the previous work item must have left the staging tile
-          if (row == 0) bulk_wait_read0();
-          mbar_arrive(bar_e);
-          if (!(ok = wait_bar<false>(bar_e, ne & 1, abort_s, P.status, 35))) break;
-          ++ne;
-          uint32_t oa[16], ob[16];
-          tmem_ld16(tm_O, oa);
-#pragma unroll
-          for (int ch = 0; ch < D / 16; ++ch) {
-            uint32_t (&o)[16] = (ch & 1) ? ob : oa;
-            uint32_t (&on)[16] = (ch & 1) ? oa : ob;
-            tmem_wait_ld();
-            if (ch + 1 < D / 16) tmem_ld16(tm_O + (ch + 1) * 16, on);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint4 v;
-              float2 x;
-              x = ffma2(make_float2(__uint_as_float(o[8 * h + 0]), __uint_as_float(o[8 * h + 1])), inv2, make_float2(0.f, 0.f));
-              v.x = pack_bf16(x.x, x.y);
-              x = ffma2(make_float2(__uint_as_float(o[8 * h + 2]), __uint_as_float(o[8 * h + 3])), inv2, make_float2(0.f, 0.f));
-              v.y = pack_bf16(x.x, x.y);
-              x = ffma2(make_float2(__uint_as_float(o[8 * h + 4]), __uint_as_float(o[8 * h + 5])), inv2, make_float2(0.f, 0.f));
-              v.z = pack_bf16(x.x, x.y);
-              x = ffma2(make_float2(__uint_as_float(o[8 * h + 6]), __uint_as_float(o[8 * h + 7])), inv2, make_float2(0.f, 0.f));
-              v.w = pack_bf16(x.x, x.y);
-              const int i = 2 * ch + h;                          // 16-byte chunk of the 256-byte output row
-              *reinterpret_cast<uint4*>(stage + (i >> 3) * L::kOStage + row * 128 + (((i & 7) ^ (row & 7)) << 4)) = v;
-            }
-          }
-          // O_t is in registers / shared memory: the first P.V of the next work item may overwrite it
-          tc_fence_before();
-          mbar_arrive(bars + Bars::o_free + 8 * t);
-          fence_proxy_async_smem();
-          mbar_arrive(bar_e);
-          if (!(ok = wait_bar<false>(bar_e, ne & 1, abort_s, P.status, 36))) break;
-          ++ne;
-          if (row == 0) {
-#pragma unroll
-            for (int hcol = 0; hcol < D / 64; ++hcol)
-              tma_store_4d(&tm_o, sbase + L::ostage + (t * (D / 64) + hcol) * L::kOStage, 64 * hcol,
-                           P.o_token_first ? q0 : wk.hq, P.o_token_first ? wk.hq : q0, wk.b);
-            bulk_commit_group();
-          }
-        } else {
-          const bool live = qpos < SEQ_NQ;
-          uint32_t oa[16], ob[16];
-          tmem_ld16(tm_O, oa);
-#pragma unroll
-          for (int ch = 0; ch < D / 16; ++ch) {
-            uint32_t (&o)[16] = (ch & 1) ? ob : oa;
-            uint32_t (&on)[16] = (ch & 1) ? oa : ob;
-            tmem_wait_ld();
-            if (ch + 1 < D / 16) tmem_ld16(tm_O + (ch + 1) * 16, on);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint4 v;
-              v.x = pack_bf16(__uint_as_float(o[8 * h + 0]) * inv, __uint_as_float(o[8 * h + 1]) * inv);
-              v.y = pack_bf16(__uint_as_float(o[8 * h + 2]) * inv, __uint_as_float(o[8 * h + 3]) * inv);
-              v.z = pack_bf16(__uint_as_float(o[8 * h + 4]) * inv, __uint_as_float(o[8 * h + 5]) * inv);
-              v.w = pack_bf16(__uint_as_float(o[8 * h + 6]) * inv, __uint_as_float(o[8 * h + 7]) * inv);
-              if (live && (2 * ch + h) * 8 < P.d_out) reinterpret_cast<uint4*>(orow)[2 * ch + h] = v;
-            }
-          }
-          tc_fence_before();
-          mbar_arrive(bars + Bars::o_free + 8 * t);
-        }
-        if (qpos < SEQ_NQ) {
-          if (P.lse) {
-            // natural-log sum of exp(sm_scale * s) over the row (l carries the factor 2688 / 2^kLazyLog2)
+          // ---- output: O / l -> bf16 -> global.  D=128, dense batches: through a swizzled staging tile in shared
+          // memory and two TMA stores per warp (32 rows x 64 columns) - a thread owns an output row, so direct
+          // stores put 32 different rows into every store instruction.  D=64 (half the bytes) and packed
+          // variable-length outputs (a tile must not spill into the next sequence) store directly.
+#pragma unroll 1
+          for (int t = 0; t < 2; ++t) {
+            const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
+            const int qt = 2 * wk.pair + t, q0 = qt * kBlockM, qpos = q0 + row;
+            const bool live = SEQ_TILE_EXISTS && qpos < SEQ_NQ;
+#if SAGE3_VARLEN_BUILD
+            __nv_bfloat16* orow = P.out + wk.hq * P.o_sh + (int64_t)(wk.q_base + qpos) * P.o_sn;   // packed output
+#else
+            __nv_bfloat16* orow = P.out + wk.b * P.o_sb + wk.hq * P.o_sh + (int64_t)qpos * P.o_sn;
+#endif
             const int64_t li = ((int64_t)wk.b * P.Hq + wk.hq) * P.Nq + qpos;
-            float v = (l == 0.f) ? -INFINITY : (m_ref * c + log2f(l) + kLog2InvTop) * (1.0f / kLog2e);
-            if (P.lse_add != nullptr) v = fmaf(P.lse_add[li], c * (1.0f / kLog2e), v);
-            P.lse[li] = v;
+            if (n_t == 0) {
+              // query tile that sees no key at all (causal, more queries than keys): zeros, like the
+              // reference's store_zero (fwd_epilogue.cu:150-183); nothing if the tile does not exist
+              if (live) {
+#pragma unroll 1
+                for (int i = 0; i < P.d_out / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
+                if (P.lse) P.lse[li] = -INFINITY;
+              }
+              continue;
+            }
+            const uint32_t last = (t == 0 ? sc[0] : sc[1]) - 1;
+            uint32_t& ni = t == 0 ? items[0] : items[1];
+            // the last key tile's row sum is there, and its P.V has landed
+            if (!(ok = wait_bar<false>(bars + Bars::p_full + 8 * t, last & 1, abort_s, P.status, 33))) break;
+            const volatile float* l_row = reinterpret_cast<const volatile float*>(smem + L::lx) + t * 256 + row + (ni & 1) * 512;
+            const float l = l_row[0], m = l_row[128];
+            ++ni;
+            if (!(ok = wait_bar<false>(bars + Bars::pv_done + 8 * t, last & 1, abort_s, P.status, 34))) break;
+            tc_fence_after();
+            const uint32_t tm_O = tmem + t * D + lane_addr;
+            const bool keyless = m == kNoMax;                    // a row that has seen no key: zeros, LSE -inf
+            const float inv = (keyless || l != l) ? 0.f : 1.0f / l;
+            const float2 inv2 = make_float2(inv, inv);
+            const uint32_t stage_off = L::ostage + (t * 4 + quarter) * (D / 64) * L::kOStage;
+            uint8_t* stage = smem + stage_off + lane * 128;
+            if (kTmaStore) {
+              // the stores of this warp's previous output tiles must have left the staging tile
+              if (lane == 0) bulk_wait_read0();
+              __syncwarp();
+            }
+#pragma unroll 1
+            for (int ch = 0; ch < D / 32; ++ch) {
+              uint32_t o[32];
+              tmem_ld32(tm_O + 32 * ch, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                uint4 v;
+                float2 x;
+                x = ffma2(make_float2(__uint_as_float(o[8 * h + 0]), __uint_as_float(o[8 * h + 1])), inv2, make_float2(0.f, 0.f));
+                v.x = pack_bf16(x.x, x.y);
+                x = ffma2(make_float2(__uint_as_float(o[8 * h + 2]), __uint_as_float(o[8 * h + 3])), inv2, make_float2(0.f, 0.f));
+                v.y = pack_bf16(x.x, x.y);
+                x = ffma2(make_float2(__uint_as_float(o[8 * h + 4]), __uint_as_float(o[8 * h + 5])), inv2, make_float2(0.f, 0.f));
+                v.z = pack_bf16(x.x, x.y);
+                x = ffma2(make_float2(__uint_as_float(o[8 * h + 6]), __uint_as_float(o[8 * h + 7])), inv2, make_float2(0.f, 0.f));
+                v.w = pack_bf16(x.x, x.y);
+                const int i = 4 * ch + h;                        // 16-byte chunk of the output row
+                if (kTmaStore)
+                  *reinterpret_cast<uint4*>(stage + (i >> 3) * L::kOStage + (((i & 7) ^ (lane & 7)) << 4)) = v;
+                else if (live && 8 * i < P.d_out)
+                  *reinterpret_cast<uint4*>(orow + 8 * i) = v;
+              }
+            }
+            tc_fence_before();
+            if (kTmaStore) {
+              fence_proxy_async_smem();
+              __syncwarp();
+              const int n_row = q0 + 32 * quarter;
+              if (lane == 0 && n_row < P.Nq) {
+#pragma unroll
+                for (int hcol = 0; hcol < D / 64; ++hcol)
+                  if (64 * hcol < P.d_out)
+                    tma_store_4d(&tm_o, sbase + stage_off + hcol * L::kOStage, 64 * hcol,
+                                 P.o_token_first ? n_row : wk.hq, P.o_token_first ? wk.hq : n_row, wk.b);
+                bulk_commit_group();
+              }
+            }
+            if (live && P.lse) {
+              // natural-log sum of exp(sm_scale * s) over the row (l carries the factor 2688)
+              float v = keyless ? -INFINITY : (m * c + log2f(l) + kLog2Inv2688) * (1.0f / kLog2e);
+              if (P.lse_add != nullptr) v = fmaf(P.lse_add[li], c * (1.0f / kLog2e), v);
+              P.lse[li] = v;
+            }
           }
         }
+        if (kTmaStore && lane == 0) bulk_wait_read0();   // the last output tiles have left shared memory before the CTA ends
       }
-      if (kTmaStore && row == 0) bulk_wait_read0();   // the last output tiles have left shared memory before the CTA ends
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem, 512);
+  if (warp == 13) tmem_dealloc(tmem, 512);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -903,7 +957,7 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint32_t row_byte
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// bf16 output [B][Hq][Nq][D] with arbitrary element strides, box = 128 rows x 64 columns (128 bytes, swizzled).
+// bf16 output [B][Hq][Nq][D] with arbitrary element strides, box = 32 rows x 64 columns (128 bytes, swizzled).
 // Tensor-map strides must grow with the dimension, so tokens and heads are ordered by their stride ("HND": D, N,
 // H, B; "NHD": D, H, N, B); *n_dim tells the kernel which coordinate is the token.
 bool make_out_map(CUtensorMap* m, const void* base, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn,
@@ -918,11 +972,11 @@ bool make_out_map(CUtensorMap* m, const void* base, int B, int H, int N, int D, 
   cuuint32_t box[4] = {64, 1, 1, 1};
   const cuuint64_t s_n = (cuuint64_t)sn * 2, s_h = (cuuint64_t)sh * 2;
   if (n_first) {
-    dims[1] = N; dims[2] = H; box[1] = 128;
+    dims[1] = N; dims[2] = H; box[1] = 32;
     strides[0] = N > 1 ? s_n : (cuuint64_t)D * 2;
     strides[1] = H > 1 ? s_h : strides[0] * N;
   } else {
-    dims[1] = H; dims[2] = N; box[2] = 128;
+    dims[1] = H; dims[2] = N; box[2] = 32;
     strides[0] = s_h;
     strides[1] = N > 1 ? s_n : strides[0] * H;
   }
@@ -976,7 +1030,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   if (dev < 0 || dev >= 64 || !__atomic_load_n(&ready[dev], __ATOMIC_ACQUIRE)) {
     cudaFuncAttributes fa;
     if ((e = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess) return e;
-    if (fa.numRegs * kAttnThreads < 256 * RegSplit<D>::softmax + 128 * RegSplit<D>::role) return cudaErrorLaunchOutOfResources;
+    if (fa.numRegs * kAttnThreads < 256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role)) return cudaErrorLaunchOutOfResources;
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total + 1024)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], 1, __ATOMIC_RELEASE);
   }

@@ -149,40 +149,56 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   }
   return ok != 0;
 }
-// Bounded wait: gives up after `limit` polls and reports failure instead of hanging the SM.
+// Bounded wait: polls until the phase completes, at most `limit` times, and says whether it did.  The loop is one asm
+// block of a handful of instructions: left to the compiler it was unrolled at every one of the kernels' many waits,
+// and the instruction cache paid for it.
+template <int kHintNs = 0>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = (1u << 26)) {
-  for (uint32_t i = 0; i < limit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
+  uint32_t ok;
+  if constexpr (kHintNs > 0) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\n"
+        "POLL:\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n"
+        "@p bra DONE;\n"
+        "add.u32 n, n, -1;\n"
+        "setp.ne.u32 p, n, 0;\n"
+        "@p bra POLL;\n"
+        "DONE:\n"
+        "min.u32 %0, n, 1;\n}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit), "r"((uint32_t)kHintNs) : "memory");
+  } else {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\n"
+        "POLL:\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "@p bra DONE;\n"
+        "add.u32 n, n, -1;\n"
+        "setp.ne.u32 p, n, 0;\n"
+        "@p bra POLL;\n"
+        "DONE:\n"
+        "min.u32 %0, n, 1;\n}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+  }
+  return ok != 0;
 }
 
-// Bounded wait on an mbarrier phase used by the kernels' roles; also gives up as soon as any CTA has reported a
-// failure through *status.  A failing poll parks the thread for about 1.5 us (kHinted: about 4 us), so the default
-// limit of 2^21 polls is 3 to 8 seconds; which flavour is faster was measured per role: the shorter park costs
-// issue slots but reacts sooner.  On giving up it raises the CTA's abort flag, records `code` in *status (first
-// writer wins) and returns false - the caller then unwinds instead of hanging the SM.
+// Bounded wait of the kernels' roles.  A failing poll takes 80 ns (a lone lane, or a busy CTA) to 4 us (a parked
+// warp), so the default limit is 0.15 to 8 seconds.  On giving up it raises the CTA's abort flag, records `code` in
+// *status (first writer wins) and returns false - the caller then unwinds instead of hanging the SM.
 template <bool kHinted, uint32_t kPolls = (1u << 21)>
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  for (uint32_t i = 0; i < kPolls; ++i) {
-    if (mbar_try_wait<kHinted ? 20000 : 0>(bar, parity)) return true;
-    if ((i & 1023u) == 1023u && (*abort_s != 0 || *reinterpret_cast<volatile int*>(status) != 0)) break;
-  }
+  if (mbar_wait<kHinted ? 20000 : 0>(bar, parity, kPolls)) return true;
   *abort_s = 1;
   atomicCAS(status, 0, code);
   return false;
 }
 
-// The same with the flavour of the poll chosen at run time (uniform per kernel launch).
-template <uint32_t kPolls = (1u << 21)>
-__device__ __forceinline__ bool wait_bar_dyn(uint32_t bar, uint32_t parity, const bool hinted, volatile int* abort_s,
-                                             int* status, int code) {
-  for (uint32_t i = 0; i < kPolls; ++i) {
-    if (hinted ? mbar_try_wait<20000>(bar, parity) : mbar_try_wait<0>(bar, parity)) return true;
-    if ((i & 1023u) == 1023u && (*abort_s != 0 || *reinterpret_cast<volatile int*>(status) != 0)) break;
-  }
-  *abort_s = 1;
-  atomicCAS(status, 0, code);
-  return false;
+// The same for a phase that has usually completed by now: a plain test first (17 cycles; a try_wait on a completed
+// phase takes 160), then the parking wait.
+__device__ __forceinline__ bool wait_bar_soon(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
+  if (mbar_try_wait<-1>(bar, parity)) return true;
+  return wait_bar<false>(bar, parity, abort_s, status, code);
 }
 
 // The same for a whole warp that goes on to warp-wide instructions (tcgen05.ld / st, votes): every lane gets the

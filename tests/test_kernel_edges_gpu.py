@@ -1,0 +1,31 @@
+"""The kernels at the sizes where their tiling can go wrong, against the CPU restatement of the reference arithmetic.
+
+Tolerance as in ``test_attn_gpu.py``: cosine similarity >= 0.999 and relative L1 <= 2e-2, LSE within 2e-3.
+"""
+import pytest
+import torch
+
+import sageattention_b200 as sa
+from oracle import sage3
+from tests import _util as U
+from tests.test_attn_gpu import COS_MIN, REL_L1_MAX, oracle_on_device_operands
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one and two key tiles, a last key tile of one key, query tiles without a partner, query tiles that see no key or one
+# key tile while their partner sees more, heads whose work items land on several rounds of the persistent grid
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,causal", [
+    (1, 2, 2, 1, 129, 128, False), (1, 2, 1, 129, 1, 64, False), (1, 4, 2, 257, 383, 128, True), (1, 4, 4, 640, 130, 128, True),
+    (1, 4, 4, 511, 129, 64, True), (3, 60, 20, 129, 128, 128, True), (3, 60, 20, 385, 257, 64, False)])
+def test_attention_at_tile_edges(B, Hq, Hkv, Nq, Nk, D, causal):
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, D, seed=Nq + Nk + D, device=DEV)
+    z = sa.quantize_qkv(q, k, v)
+    out, lse = sa.fp4_attention(z, is_causal=causal, return_lse=True, check_status=True)
+    want, want_lse = oracle_on_device_operands(z, D ** -0.5, causal, return_lse=True)
+    cos, l1 = sage3.accuracy(out.float().cpu(), want.to(torch.bfloat16).float())
+    assert torch.isfinite(out).all() and cos >= COS_MIN and l1 <= REL_L1_MAX, (cos, l1)
+    fin = torch.isfinite(want_lse)
+    assert torch.allclose(lse.cpu()[fin], want_lse[fin], atol=2e-3, rtol=1e-4)
+    assert bool(torch.isneginf(lse.cpu()[~fin]).all())
