@@ -418,6 +418,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     for (int i = 0; i < 8; ++i) mbar_init(bars + Bars::corr + 8 * i, 1);
     mbar_init(bars + Bars::drain, 1);
     mbar_init(bars + Bars::drain + 8, 1);
+    // the operands are there once the kernel before is complete (one thread waits for it, the barriers below pass that on)
+    pdl_wait();
     // a failure reported by an earlier CTA (or an earlier launch that shares *status) stops new work
     const int bad = *reinterpret_cast<volatile int*>(P.status) != 0;
     *abort_s = bad;
@@ -1023,22 +1025,22 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  // once per device and instantiation: opt in to the shared memory, and make sure the register hand-over inside
-  // the kernel stays within the pool this build of it is launched with (it would block forever otherwise)
-  static unsigned char ready[64] = {};
-  if (dev < 0 || dev >= 64 || !__atomic_load_n(&ready[dev], __ATOMIC_ACQUIRE)) {
+  // once per device and instantiation: look up its SM count, opt in to the shared memory, and make sure the register
+  // hand-over inside the kernel stays within the pool this build of it is launched with (it would block forever otherwise)
+  static int ready[64] = {};                               // SM count
+  if (dev >= 0 && dev < 64) sms = __atomic_load_n(&ready[dev], __ATOMIC_ACQUIRE);
+  if (sms == 0) {
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     cudaFuncAttributes fa;
     if ((e = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess) return e;
     if (fa.numRegs * kAttnThreads < 256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role)) return cudaErrorLaunchOutOfResources;
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total + 1024)) != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], 1, __ATOMIC_RELEASE);
+    if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], sms, __ATOMIC_RELEASE);
   }
   const int64_t work = (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
   const int64_t ctas = sms - a.sm_margin > 1 ? sms - a.sm_margin : 1;
   const int64_t grid = work < ctas ? work : ctas;
-  kern<<<(unsigned)grid, kAttnThreads, L::total + 1024, stream>>>(tq, tk, tv, to, P);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)grid), kAttnThreads, L::total + 1024, stream, a.after_delta_s, tq, tk, tv, to, P);
 }
 
 }  // namespace

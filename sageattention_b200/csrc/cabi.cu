@@ -90,7 +90,8 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
   return SAGE3_OK;
 }
 
-static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int* cu_k, void* stream_) {
+static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int* cu_k, void* stream_,
+                          int* zero_status = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (int st = check_tensor(a->q)) return st;
@@ -105,13 +106,17 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   if (a->per_block_mean < -1 || a->per_block_mean > 1) return SAGE3_ERR_ARGUMENT;
   if (!head_dim_ok(a->head_dim_in, s.D)) return SAGE3_ERR_ARGUMENT;
 
-  const void* km = nullptr;
-  if (a->k.ptr && a->smooth_k) {
-    if (a->km_in) {
-      km = a->km_in;
+  // K means: the caller's; or, where only the delta_s kernel needs them, partial sums taken beside the quantisation of Q
+  // and V and added up there; or from a launch of their own
+  const void* km = a->k.ptr && a->smooth_k ? a->km_in : nullptr;
+  void* partial = nullptr;
+  if (a->k.ptr && a->smooth_k && km == nullptr) {
+    if (!a->km || !a->scratch || !aligned16(a->scratch)) return SAGE3_ERR_ARGUMENT;
+    if (a->scratch_bytes < sage3::quant_scratch_bytes(s.B, s.Hkv, s.Nk, s.D)) return SAGE3_ERR_ARGUMENT;
+    // (a whole-sequence Q mean uses the same scratch)
+    if (a->delta_s != nullptr && a->q_dot_km == nullptr && a->per_block_mean == 1) {
+      partial = a->scratch;
     } else {
-      if (!a->km || !a->scratch || !aligned16(a->scratch)) return SAGE3_ERR_ARGUMENT;
-      if (a->scratch_bytes < sage3::quant_scratch_bytes(s.B, s.Hkv, s.Nk, s.D)) return SAGE3_ERR_ARGUMENT;
       cudaError_t e = sage3::launch_channel_mean(a->k.ptr, a->k.stride_b, a->k.stride_h, a->k.stride_n, s.B, s.Hkv,
                                                  s.Nk, s.D, (float)s.Nk, a->scratch, a->km, stream, cu_k, a->head_dim_in);
       if (e != cudaSuccess) return cuda_fail(e);
@@ -135,16 +140,17 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   const bool k_in_ds = a->delta_s != nullptr && a->k.ptr != nullptr;
   if (a->delta_s != nullptr && (!a->q.ptr || !a->k.ptr || a->per_block_mean < 0)) return SAGE3_ERR_ARGUMENT;
   sage3::QuantArgs q{};
-  q.q = a->q.ptr; q.k = k_in_ds ? nullptr : a->k.ptr; q.v = a->v.ptr;
+  q.q = a->q.ptr; q.k = a->k.ptr; q.v = a->v.ptr;
   q.q_sb = a->q.stride_b; q.q_sh = a->q.stride_h; q.q_sn = a->q.stride_n;
   q.k_sb = a->k.stride_b; q.k_sh = a->k.stride_h; q.k_sn = a->k.stride_n;
   q.v_sb = a->v.stride_b; q.v_sh = a->v.stride_h; q.v_sn = a->v.stride_n;
   q.B = s.B; q.Hq = s.Hq; q.Hkv = s.Hkv; q.Nq = s.Nq; q.Nk = s.Nk; q.D = s.D;
   q.q_mean_mode = a->per_block_mean == 1 ? 1 : (a->per_block_mean == 0 ? 2 : 0);
-  q.km = km;
+  q.km = km; q.partial = partial;
+  q.zero_status = zero_status;
   q.q_mean_seq = a->per_block_mean == 0 ? a->qm : nullptr;
   q.qm_override = a->per_block_mean == 1 ? a->qm_in : nullptr;
-  q.q_codes = a->q_codes; q.q_sf = a->q_sf; q.k_codes = a->k_codes; q.k_sf = a->k_sf;
+  q.q_codes = a->q_codes; q.q_sf = a->q_sf; q.k_codes = k_in_ds ? nullptr : a->k_codes; q.k_sf = a->k_sf;
   q.vt_codes = a->vt_codes; q.vt_sf = a->vt_sf; q.qm = a->qm;
   q.cu_q = cu_q; q.cu_k = cu_k;
   q.d_in = a->head_dim_in;
@@ -158,7 +164,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   if (a->delta_s != nullptr) {
     sage3::DeltaSArgs d{};
     d.qm = a->qm; d.k = a->k.ptr; d.k_sb = a->k.stride_b; d.k_sh = a->k.stride_h; d.k_sn = a->k.stride_n;
-    d.km = km; d.ds = a->delta_s; d.cu_k = cu_k;
+    d.km = km; d.partial = partial; d.km_out = a->km; d.ds = a->delta_s; d.cu_k = cu_k; d.after_quant = true;
     d.k_codes = a->k_codes; d.k_sf = a->k_sf; d.status = a->device_status; d.d_in = a->head_dim_in;
     d.B = s.B; d.Hq = s.Hq; d.Hkv = s.Hkv; d.Tq = a->per_block_mean == 1 ? Tq : 1; d.Nk = s.Nk; d.D = s.D;
     e = sage3::launch_delta_s(d, stream);
@@ -170,7 +176,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
 int sage3_quant_qkv(const sage3_quant_args* a, void* stream) { return quant_qkv_impl(a, nullptr, nullptr, stream); }
 
 static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const int* cu_q, const int* cu_k, void* stream_,
-                         int slot_first = 0, bool zero_status = true) {
+                         int slot_first = 0, bool zero_status = true, bool after_delta_s = false) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (!a->q_codes || !a->q_sf || !a->k_codes || !a->k_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status)
@@ -203,6 +209,7 @@ static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const 
   k.d_out = a->out_head_dim;
   k.sm_margin = a->sm_margin;
   k.cu_q = cu_q; k.cu_k = cu_k;
+  k.after_delta_s = after_delta_s;
   e = (cu_q != nullptr || cu_k != nullptr) ? sage3::launch_attn_fwd_varlen(k, stream) : sage3::launch_attn_fwd(k, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   return SAGE3_OK;
@@ -281,18 +288,14 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   const float sm_scale = a->sm_scale > 0.f ? a->sm_scale : 1.0f / sqrtf((float)d_real);
   q.head_dim_in = a->head_dim;
   q.delta_s = a->per_block_mean >= 0 ? ds : nullptr;
-  // one status word for the whole call: zeroed here, the preprocessing kernels and the attention kernel report in it
+  // one status word for the whole call: zeroed by the quantisation kernel, the later ones report in it
   q.device_status = status;
-  {
-    cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)stream);
-    if (e != cudaSuccess) return cuda_fail(e);
-  }
   if (a->km_out && !a->smooth_k) {
     // no mean is removed: the caller's LSE correction term must vanish
     cudaError_t e = cudaMemsetAsync(a->km_out, 0, z.km, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e);
   }
-  if (int st = sage3_quant_qkv(&q, stream)) return st;
+  if (int st = quant_qkv_impl(&q, nullptr, nullptr, stream, status)) return st;
   sage3_attn_args t{};
   t.shape = a->shape;
   t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;
@@ -303,7 +306,7 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   t.lse_add = q.q_dot_km;
   t.out_head_dim = a->head_dim;
   t.sm_margin = a->sm_margin;
-  return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false);
+  return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false, /*after_delta_s=*/t.delta_s != nullptr);
 }
 
 int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
@@ -331,11 +334,7 @@ int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   int32_t* status = reinterpret_cast<int32_t*>(take(4));
   if (a->device_status) status = a->device_status;
   q.device_status = status;
-  {
-    cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)stream);
-    if (e != cudaSuccess) return cuda_fail(e);
-  }
-  if (int st = quant_qkv_impl(&q, a->cu_seqlens_q, a->cu_seqlens_k, stream)) return st;
+  if (int st = quant_qkv_impl(&q, a->cu_seqlens_q, a->cu_seqlens_k, stream, status)) return st;
   sage3_attn_args t{};
   t.shape = a->shape;
   t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;
@@ -345,7 +344,7 @@ int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   t.lse = nullptr;
   t.sm_scale = a->sm_scale > 0.f ? a->sm_scale : 1.0f / sqrtf((float)a->shape.D);
   t.is_causal = a->is_causal; t.device_status = status;
-  return attn_fwd_impl(&t, nullptr, a->cu_seqlens_q, a->cu_seqlens_k, stream, 0, /*zero_status=*/false);
+  return attn_fwd_impl(&t, nullptr, a->cu_seqlens_q, a->cu_seqlens_k, stream, 0, /*zero_status=*/false, /*after_delta_s=*/true);
 }
 
 int sage3_k_mean_static(const sage3_shape* shape, const sage3_tensor* k, void* km_out, void* stream) {

@@ -208,9 +208,20 @@ __device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, vol
   return __all_sync(0xffffffffu, wait_bar<kHinted, kPolls>(bar, parity, abort_s, status, code));
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start its prologue / wait until the previous one is
+// complete and its writes are visible.  Both do nothing in a kernel that was launched without the attribute.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+
+// 16 bytes global -> shared without a register in between; zeros if !valid
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // shared -> global tile store through a 4-D tensor map (rows outside the tensor are clipped by the hardware);
 // completion is tracked in bulk groups of the issuing thread

@@ -11,15 +11,23 @@
 // One CTA per (128-key tile, kv head): the K tile is read from HBM ONCE, smoothed in registers, quantised (the
 // same device function as the fused quantisation kernel, so codes and scales are bit-identical) and laid out
 // in shared memory as the B operand of tcgen05.mma kind::f16; the Q block means of every query head of the GQA
-// group (rows of A, 128 query blocks at a time) are multiplied against it with the accumulator in tensor
+// group (contiguous in memory, so the group counts as one list of rows of A, 128 at a time: the four heads of a decode
+// step are one MMA instead of four) are multiplied against it with the accumulator in tensor
 // memory; the [128 query blocks x 128 keys] result goes as bf16 through a swizzled staging tile in shared memory
 // and leaves with two TMA stores (whole 128-byte lines; rows beyond the last query block are clipped by the
-// tensor map).  HBM-bound: the output ([Tq x 128] bf16 per CTA and query head) dominates the traffic.
+// tensor map).  HBM-bound: the output ([Tq x 128] bf16 per CTA and query head) dominates the traffic, in a chain of
+// dependent steps per CTA.  Up to 128 rows of A (kMulti = false) there is one round, and what counts is how many CTAs an
+// SM holds: the staging tile lies over the A tile, which has been consumed by then, and A comes by cp.async instead of
+// through registers - three CTAs per SM instead of two (B8 Hq32 Hkv8 Nk4096, one query: 77 -> 42 us).  Several rounds
+// want the next A tile on its way during the current one: it waits in registers, two CTAs per SM (B1 H40 N32760: 330 us;
+// 390 with three CTAs and no A ahead).
 //
 // Operand layout in shared memory (K-major, no swizzle): 8-row x 16-byte core matrices; the 16 row groups of one
 // 8-channel chunk are contiguous (128 B apart), chunks are kChunk bytes apart - 16 bytes more than their size so
 // that the 16 lanes which write one row's chunks hit different banks.
 #include <cuda.h>
+
+#include <atomic>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -34,34 +42,58 @@ constexpr uint32_t kChunk = 128 * 16 + 16;            // one 8-channel chunk of 
 
 struct KDsParams {
   const __nv_bfloat16 *qm, *k, *km;
+  const float* partial;                                // K channel sums when km is null (both null: no smoothing)
+  __nv_bfloat16* km_out;
+  int chunks;
   int64_t k_sb, k_sh, k_sn;
   uint8_t *k_codes, *k_sf;                             // null: K is quantised elsewhere
   __nv_bfloat16* ds;
   int* status;                                         // optional device status word
-  int Hq, Hkv, Tq, Tk, Nk;
+  int Hkv, rows, Tk, Nk;                               // rows = query heads per kv head x query blocks per head
   const int* cu_k;
   int d_in;                                            // channels the K rows really have; the rest are zero
 };
 
 constexpr int kDsStageBytes = 2 * 128 * 128;          // output staging: [2 key halves][128 rows x 128 bytes], 128-byte swizzle
+// in front of the K tile: the staging tile and the A tile, or (one round) one place for both
+__host__ __device__ constexpr int ds_front_bytes(int D, bool multi) {
+  const int a = (D / 8) * (int)kChunk;
+  return multi ? kDsStageBytes + a : (a > kDsStageBytes ? a : kDsStageBytes);
+}
 
-template <int D>
-__global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
+template <int D, bool kMulti>
+__global__ void __launch_bounds__(kThreads, kMulti ? 2 : 3) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
                                                                       const KDsParams P) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   constexpr uint32_t kTileBytes = CH * kChunk;
   extern __shared__ uint8_t dyn_raw[];
   uint8_t* dyn_smem = dyn_raw + ((1024u - (smem_u32(dyn_raw) & 1023u)) & 1023u);   // the swizzled staging tile needs it
   uint8_t* stage = dyn_smem;                           // output staging (first: 1024-byte aligned)
-  uint8_t* sB = dyn_smem + kDsStageBytes;              // smoothed K tile  [CH][kChunk]
-  uint8_t* sA = sB + kTileBytes;                       // 128 Q block means [CH][kChunk]
-  uint8_t* sf_smem = sA + kTileBytes;                  // 2048 B
+  uint8_t* sA = dyn_smem + (kMulti ? kDsStageBytes : 0);   // 128 Q block means [CH][kChunk]
+  uint8_t* sB = dyn_smem + ds_front_bytes(D, kMulti);  // smoothed K tile  [CH][kChunk]
+  uint8_t* sf_smem = sB + kTileBytes;                  // 2048 B
   uint8_t* misc = sf_smem + 2048;                      // mbarrier (8 B), tensor-memory slot (4 B), abort flag (4 B)
   const uint32_t bar = smem_u32(misc), slot = smem_u32(misc + 8);
   int* abort_s = reinterpret_cast<int*>(misc + 12);
-  const int tile = blockIdx.x, bh = blockIdx.y, b = bh / P.Hkv, hkv = bh % P.Hkv, G = P.Hq / P.Hkv;
+  const int tile = blockIdx.x, bh = blockIdx.y, b = bh / P.Hkv, hkv = bh % P.Hkv;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, c = t % CH, rl = t / CH;
 
+  // ---- the K tile: load, smooth, quantise, lay out as the B operand
+  int Nk = P.Nk;
+  if (P.cu_k != nullptr) {
+    Nk = min(P.cu_k[b + 1] - P.cu_k[b], Nk);           // a packed batch: this sequence, cut at max_seqlen
+    if (tile * kTile >= Nk) {                          // beyond the sequence: nothing reads this tile or its delta_s
+      pdl_wait();                                      // (this grid never ends before the one it follows)
+      return;
+    }
+  }
+  const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + c * 8;
+  uint4 w[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {                       // all loads in flight before the first use
+    const int n = tile * kTile + p * RPP + rl;
+    w[p] = (n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
+  }
   if (t == 0) {
     mbar_init(bar, 1);
     *abort_s = 0;
@@ -71,21 +103,30 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
     tmem_alloc(slot, 128);
     tmem_relinquish();
   }
-
-  // ---- the K tile: load, smooth, quantise, lay out as the B operand
-  int Nk = P.Nk;
-  if (P.cu_k != nullptr) Nk = min(P.cu_k[b + 1] - P.cu_k[b], Nk);   // a packed batch: this sequence, cut at max_seqlen
-  const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + c * 8;
-  uint4 w[NP];
+  __syncthreads();
+  // only now: the attention kernel that may come in takes all of tensor memory, and waits for this grid
+  pdl_launch_dependents();
+  pdl_wait();                                          // the sums and block means of the launch before
+  // A: Q block means of rows round*128 ... +127 (zeros beyond the last one)
+  const __nv_bfloat16* qm_g = P.qm + (int64_t)bh * P.rows * D + c * 8;
+  uint4 a_next[kMulti ? NP : 1];
+  auto load_a = [&](const int round) {
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {                       // all loads in flight before the first use
-    const int n = tile * kTile + p * RPP + rl;
-    w[p] = (n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
-  }
-  if (P.km != nullptr) {
-    const uint4 m = *reinterpret_cast<const uint4*>(P.km + (int64_t)bh * D + c * 8);
-    const float mean[8] = {bf16_lo(m.x), bf16_hi(m.x), bf16_lo(m.y), bf16_hi(m.y),
-                           bf16_lo(m.z), bf16_hi(m.z), bf16_lo(m.w), bf16_hi(m.w)};
+    for (int p = 0; p < NP; ++p) {
+      const int row = p * RPP + rl, m = round * 128 + row;
+      if constexpr (kMulti)
+        a_next[p] = m < P.rows ? __ldcg(reinterpret_cast<const uint4*>(qm_g + (int64_t)m * D)) : make_uint4(0, 0, 0, 0);
+      else
+        cp_async16(smem_u32(sA) + c * kChunk + (row >> 3) * 128 + (row & 7) * 16, qm_g + (int64_t)min(m, P.rows - 1) * D, m < P.rows);
+    }
+  };
+  if (!kMulti) load_a(0);
+  if (P.km != nullptr || P.partial != nullptr) {
+    static_assert(kMaxChunks * D * 4 <= (int)kTileBytes, "partial rows of the K mean");
+    float mean[8];
+    k_mean<D>(P.km, P.partial + (int64_t)bh * P.chunks * D, P.chunks, (float)max(Nk, 1), bh, reinterpret_cast<float*>(sB),
+              tile == 0 ? P.km_out : nullptr, mean);
+    __syncthreads();                                   // every thread has its means: sB takes the K tile
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       if (tile * kTile + p * RPP + rl < Nk) {          // padding rows stay zero (the reference subtracts before padding)
@@ -110,37 +151,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(misc + 8);
 
-  // ---- delta_s: for every query head of the group, 128 query blocks at a time
+  // ---- delta_s: for the query blocks of all heads of the group, 128 at a time
   constexpr uint32_t idesc = make_idesc_bf16(128, 128);
   constexpr uint32_t HI = (128u >> 4) | (1u << 14);                     // 8-row groups 128 B apart, no swizzle
   const uint32_t a_lo = (smem_u32(sA) >> 4) | ((kChunk >> 4) << 16);    // leading (K) offset = one chunk
   const uint32_t b_lo = (smem_u32(sB) >> 4) | ((kChunk >> 4) << 16);
-  const int n_mb = (P.Tq + 127) / 128;
-  uint32_t iter = 0;
   bool ok = true;
-  // rounds = (query head of the group, block of 128 query blocks); the A tile of the next round is fetched into
-  // registers while the current round's MMA runs and its result is written out
-  const int rounds = G * n_mb;
-  auto load_a = [&](uint4 (&a)[NP], const int round) {
-    const int hq = hkv * G + round / n_mb, mb = round % n_mb;
-    const __nv_bfloat16* qm_h = P.qm + ((int64_t)b * P.Hq + hq) * P.Tq * D;
+  const int rounds = kMulti ? (P.rows + 127) / 128 : 1;
+  if (kMulti) load_a(0);
+  for (int round = 0; round < rounds && ok; ++round) {
+    if constexpr (kMulti) {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int m = mb * 128 + p * RPP + rl;
-      a[p] = m < P.Tq ? __ldg(reinterpret_cast<const uint4*>(qm_h + (int64_t)m * D + c * 8)) : make_uint4(0, 0, 0, 0);
+      for (int p = 0; p < NP; ++p) {
+        const int row = p * RPP + rl;
+        *reinterpret_cast<uint4*>(sA + c * kChunk + (row >> 3) * 128 + (row & 7) * 16) = a_next[p];
+      }
+      if (t == 0) bulk_wait_read0();                   // the previous round's stores have left the staging tile
+    } else {
+      cp_async_wait_all();
     }
-  };
-  uint4 a_next[NP];
-  load_a(a_next, 0);
-  for (int round = 0; round < rounds && ok; ++round, ++iter) {
-    const int hq = hkv * G + round / n_mb, mb = round % n_mb;
-    // A: block means of query blocks mb*128 ... +127 (zeros beyond the last one)
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int row = p * RPP + rl;
-      *reinterpret_cast<uint4*>(sA + c * kChunk + (row >> 3) * 128 + (row & 7) * 16) = a_next[p];
-    }
-    if (t == 0) bulk_wait_read0();                     // the previous round's stores have left the staging tile
     fence_proxy_async_smem();
     __syncthreads();
     if (t == 0) {
@@ -150,12 +179,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
         tc_mma_bf16(tmem, a_lo + kk * (2 * kChunk >> 4), HI, b_lo + kk * (2 * kChunk >> 4), HI, idesc, kk > 0 ? 1u : 0u);
       tc_commit(bar);
     }
-    if (round + 1 < rounds) load_a(a_next, round + 1);
+    if (kMulti && round + 1 < rounds) load_a(round + 1);
     // bounded: a few microseconds normally; gives up after about a second
     if (P.status != nullptr) {
-      ok = wait_bar_warp<false, (1u << 19)>(bar, iter & 1, abort_s, P.status, 50);
+      ok = wait_bar_warp<false, (1u << 19)>(bar, round & 1, abort_s, P.status, 50);
     } else {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, iter & 1, 1u << 19));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, round & 1, 1u << 19));
     }
     tc_fence_after();
     if (ok) {
@@ -182,9 +211,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
     tc_fence_before();
     __syncthreads();                                   // the staging tile is complete (and the accumulator read)
     if (ok && t == 0) {
-      const int z = b * P.Hq + hq;
-      tma_store_3d(&tm_ds, smem_u32(stage), tile * kTile, mb * 128, z);
-      tma_store_3d(&tm_ds, smem_u32(stage) + 128 * 128, tile * kTile + 64, mb * 128, z);
+      tma_store_3d(&tm_ds, smem_u32(stage), tile * kTile, round * 128, bh);
+      tma_store_3d(&tm_ds, smem_u32(stage) + 128 * 128, tile * kTile + 64, round * 128, bh);
       bulk_commit_group();
     }
     // the accumulator and the A tile are rewritten by the next round; every thread leaves the loop together
@@ -194,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   if (t == 0) bulk_wait_read0();                       // the last stores have read the staging tile before the CTA ends
   if (!ok && t == 0) {
     // the MMAs issued last may still be running: give them time to drain before tensor memory is freed
-    mbar_wait(bar, iter & 1, 1u << 16);
+    mbar_wait(bar, (rounds - 1) & 1, 1u << 16);
   }
   tc_fence_before();
   __syncthreads();
@@ -209,33 +237,42 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   P.k_sb = a.k_sb; P.k_sh = a.k_sh; P.k_sn = a.k_sn;
   P.k_codes = (uint8_t*)a.k_codes; P.k_sf = (uint8_t*)a.k_sf;
   P.ds = (__nv_bfloat16*)a.ds; P.status = a.status;
-  P.Hq = a.Hq; P.Hkv = a.Hkv; P.Tq = a.Tq; P.Nk = a.Nk; P.Tk = (a.Nk + 127) / 128;
+  P.partial = (const float*)a.partial; P.km_out = (__nv_bfloat16*)a.km_out;
+  int chunk_tokens;
+  quant_chunks(a.B * a.Hkv, a.Nk, &P.chunks, &chunk_tokens);
+  P.Hkv = a.Hkv; P.rows = a.Hq / a.Hkv * a.Tq; P.Nk = a.Nk; P.Tk = (a.Nk + 127) / 128;
   P.cu_k = a.cu_k;
   P.d_in = (a.d_in > 0 && a.d_in <= a.D) ? a.d_in : a.D;
   dim3 grid(P.Tk, a.B * a.Hkv);
-  // delta_s as a 3-D bf16 tensor (key, query block, batch x query head); store boxes of 64 keys x 128 query blocks
+  // delta_s as a 3-D bf16 tensor (key, query block of the GQA group, batch x kv head); store boxes of 64 keys x 128 rows
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return cudaErrorInvalidValue;
   CUtensorMap tm;
   {
     const cuuint64_t nk_pad = (cuuint64_t)P.Tk * kTile;
-    cuuint64_t dims[3] = {nk_pad, (cuuint64_t)a.Tq, (cuuint64_t)a.B * a.Hq};
-    cuuint64_t strides[2] = {nk_pad * 2, nk_pad * 2 * (cuuint64_t)a.Tq};
+    cuuint64_t dims[3] = {nk_pad, (cuuint64_t)P.rows, (cuuint64_t)a.B * a.Hkv};
+    cuuint64_t strides[2] = {nk_pad * 2, nk_pad * 2 * (cuuint64_t)P.rows};
     cuuint32_t box[3] = {64, 128, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     if (enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a.ds, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
   }
-  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
-  // per device and cheap, so set on every call rather than cached per process
-  cudaError_t e = a.D == 128
-      ? cudaFuncSetAttribute(k_quant_delta_s_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-      : cudaFuncSetAttribute(k_quant_delta_s_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const bool multi = P.rows > 128;
+  const int smem = ds_front_bytes(a.D, multi) + (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
+  static std::atomic<unsigned long long> ready[4];      // per kernel: devices on which the shared memory was asked for
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (a.D == 128) k_quant_delta_s_kernel<128><<<grid, kThreads, smem, stream>>>(tm, P);
-  else            k_quant_delta_s_kernel<64><<<grid, kThreads, smem, stream>>>(tm, P);
-  return cudaGetLastError();
+  auto kern = a.D == 128 ? (multi ? k_quant_delta_s_kernel<128, true> : k_quant_delta_s_kernel<128, false>)
+                         : (multi ? k_quant_delta_s_kernel<64, true> : k_quant_delta_s_kernel<64, false>);
+  auto& done = ready[(a.D == 128 ? 2 : 0) + (multi ? 1 : 0)];
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev >= 64 || !(done.load(std::memory_order_acquire) & bit)) {
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    if (dev < 64) done.fetch_or(bit, std::memory_order_release);
+  }
+  return launch_pdl(kern, grid, kThreads, smem, stream, a.after_quant, tm, P);
 }
 
 }  // namespace sage3

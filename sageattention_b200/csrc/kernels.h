@@ -6,12 +6,28 @@
 
 namespace sage3 {
 
+// Launch; with `pdl` as a programmatic dependent of the kernel before it on the stream (the kernel then waits with
+// griddepcontrol.wait before it touches anything that one writes).
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool pdl, const A&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at; c.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kern, args...);
+}
+
 struct QuantArgs {
   const void *q, *k, *v;                  // bf16, last dim contiguous; any of them may be null (skipped)
   int64_t q_sb, q_sh, q_sn, k_sb, k_sh, k_sn, v_sb, v_sh, v_sn;   // element strides
   int B, Hq, Hkv, Nq, Nk, D;
   int q_mean_mode;                        // 0 none, 1 per 128-token block, 2 whole sequence
-  const void* km;                         // bf16 [B,Hkv,D] or null (no K smoothing)
+  const void* km;                         // bf16 [B,Hkv,D]: the K means, where the caller has them
+  void* partial = nullptr;                // or fp32 scratch (quant_scratch_bytes): this launch only takes the partial sums
+                                          //   of K, for launch_delta_s; both null: no K smoothing
+  int* zero_status = nullptr;             // optional device word to zero
   const void* q_mean_seq;                 // bf16 [B,Hq,D]   (mode 2)
   const void* qm_override;                // fp32 [B,Hq,Tq,D] or null (mode 1)
   void *q_codes, *q_sf, *k_codes, *k_sf, *vt_codes, *vt_sf, *qm;
@@ -25,6 +41,7 @@ struct QuantArgs {
 };
 
 size_t quant_scratch_bytes(int B, int H, int N, int D);
+void quant_chunks(int BH, int N, int* chunks, int* chunk_tokens);   // how the channel sums of BH heads are cut into partial rows
 cudaError_t launch_channel_mean(const void* x, int64_t sb, int64_t sh, int64_t sn, int B, int H, int N, int D,
                                 float divisor, void* scratch, void* mean_out, cudaStream_t stream,
                                 const int* cu = nullptr, int d_in = 0);
@@ -48,7 +65,9 @@ struct DeltaSArgs {
   const void* qm;                         // bf16 [B,Hq,Tq,D]
   const void* k;                          // bf16 raw K, strides below
   int64_t k_sb, k_sh, k_sn;
-  const void* km;                         // bf16 [B,Hkv,D] or null
+  const void* km;                         // bf16 [B,Hkv,D], or null: then from
+  const void* partial = nullptr;          //   the partial sums that launch_quant_qkv took (both null: no smoothing)
+  void* km_out = nullptr;                 // bf16 [B,Hkv,D]: receives the means found from partial sums
   void* ds;                               // bf16 [B,Hq,Tq,Nk_pad]
   int B, Hq, Hkv, Tq, Nk, D;
   const int* cu_k = nullptr;              // variable-length batches, see QuantArgs
@@ -56,6 +75,7 @@ struct DeltaSArgs {
   void* k_sf = nullptr;                   //   smoothed K tile it holds (the K role of the quantisation kernel)
   int* status = nullptr;                  // optional device status word for the kernel's bounded wait
   int d_in = 0;                           // as in QuantArgs
+  bool after_quant = false;               // launched right behind launch_quant_qkv on the same stream: may overlap its end
 };
 cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream);
 
@@ -77,6 +97,7 @@ struct AttnArgs {
   int sm_margin = 0;                      // SMs left free for kernels running beside the persistent attention kernel
   const int* cu_q = nullptr;              // variable-length batches, see QuantArgs; out is then [tokens, Hq, D]
   const int* cu_k = nullptr;
+  bool after_delta_s = false;             // launched right behind launch_delta_s on the same stream: may overlap its end
 };
 cudaError_t launch_attn_fwd(const AttnArgs& a, cudaStream_t stream);
 cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream);   // cu_q / cu_k given

@@ -30,29 +30,18 @@
 namespace sage3 {
 
 // ------------------------------------------------------------------------------------------------
-// Channel sums over tokens (K channel mean; also the whole-sequence Q mean when per_block_mean=0).
-// grid = (chunks, B*H).  Each CTA writes one fp32 partial row; the last CTA of a (b,h) to finish
-// adds the partial rows in chunk order (deterministic) and writes mean = sum / divisor as bf16.
-// scratch: partial[B*H][chunks][D] fp32 followed by counters[B*H] u32 (zeroed by the host).
+// Channel sums over tokens (K channel mean; also the whole-sequence Q mean when per_block_mean=0): fp32 sums of one
+// chunk of tokens -> one partial row [D].  Rows of a head are always added in chunk order, so the mean is deterministic
+// and does not depend on who adds them (this file's mean kernel, or k_mean in quant_rows.cuh).
 // ------------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(kThreads) channel_mean_kernel(
-    const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
-    int chunk_tokens, float divisor, float* __restrict__ partial, unsigned int* __restrict__ counters,
-    __nv_bfloat16* __restrict__ mean_out, const int* __restrict__ cu, int d_in) {
+__device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict__ base, const int64_t sn, const int N,
+                                                const int chunk, const int chunk_tokens, const int d_in,
+                                                float* __restrict__ prow, float* red) {
   constexpr int CH = D / 8;              // 16-byte chunks per row
   constexpr int RPP = kThreads / CH;     // rows per pass
-  __shared__ float red[RPP][D];
-  __shared__ bool is_last;
-  const int bh = blockIdx.y, b = bh / H, h = bh % H;
-  const int chunk = blockIdx.x, nchunks = gridDim.x;
   const int t = threadIdx.x, c = t % CH, rl = t / CH;
-  // variable-length batch: sequence b starts at token cu[b] of the packed tensor and has its own length
-  if (cu != nullptr) {
-    N = min(cu[b + 1] - cu[b], N);         // never beyond the caller's max_seqlen (the grid covers no more)
-    divisor = (float)max(N, 1);
-  }
-  const __nv_bfloat16* base = x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh + c * 8;
+  base += c * 8;
   const int n0 = chunk * chunk_tokens;
   const int n1 = min(N, n0 + chunk_tokens);
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -72,15 +61,35 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) red[rl][c * 8 + i] = acc[i];
+  for (int i = 0; i < 8; ++i) red[rl * D + c * 8 + i] = acc[i];
   __syncthreads();
-  float* prow = partial + ((int64_t)bh * nchunks + chunk) * D;
   if (t < D) {
     float s = 0.f;
 #pragma unroll
-    for (int r = 0; r < RPP; ++r) s += red[r][t];
+    for (int r = 0; r < RPP; ++r) s += red[r * D + t];
     prow[t] = s;
   }
+}
+
+// The sums and the mean in one launch: grid = (chunks, B*H), the last CTA of a (b,h) to finish adds the partial rows
+// and writes mean = sum / divisor as bf16.
+// scratch: partial[B*H][chunks][D] fp32 followed by counters[B*H] u32 (zeroed by the host).
+template <int D>
+__global__ void __launch_bounds__(kThreads) channel_mean_kernel(
+    const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
+    int chunk_tokens, float divisor, float* __restrict__ partial, unsigned int* __restrict__ counters,
+    __nv_bfloat16* __restrict__ mean_out, const int* __restrict__ cu, int d_in) {
+  __shared__ float red[(kThreads / (D / 8)) * D];
+  __shared__ bool is_last;
+  const int bh = blockIdx.y, b = bh / H, h = bh % H;
+  const int chunk = blockIdx.x, nchunks = gridDim.x, t = threadIdx.x;
+  // variable-length batch: sequence b starts at token cu[b] of the packed tensor and has its own length
+  if (cu != nullptr) {
+    N = min(cu[b + 1] - cu[b], N);         // never beyond the caller's max_seqlen (the grid covers no more)
+    divisor = (float)max(N, 1);
+  }
+  channel_partial<D>(x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh, sn, N, chunk, chunk_tokens, d_in,
+                     partial + ((int64_t)bh * nchunks + chunk) * D, red);
   __threadfence();
   __syncthreads();
   if (t == 0) is_last = (atomicAdd(&counters[bh], 1u) == (unsigned)(nchunks - 1));
@@ -90,6 +99,7 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
     if (t < D) {
       const float* p = partial + (int64_t)bh * nchunks * D + t;
       float s = 0.f;
+#pragma unroll 8
       for (int i = 0; i < nchunks; ++i) s += __ldcg(p + (int64_t)i * D);
       mean_out[(int64_t)bh * D + t] = __float2bfloat16_rn(s / divisor);
     }
@@ -110,18 +120,35 @@ struct QuantLaunch {
   int q_blocks, k_blocks, v_blocks;      // CTAs per role
   const int *cu_q, *cu_k;                // variable-length batches (else null)
   int d_in;                              // channels the input rows really have (<= D, multiple of 8); the rest are zero
+  int s_blocks, chunks, chunk_tokens;    // CTAs of the K channel-sum role (0: none), chunks per head, tokens per chunk
+  float* partial;                        // [B,Hkv,chunks,D] fp32 K channel sums, written by that role
+  int* zero_status;                      // status word of the whole operator call, zeroed here (optional)
   float* q_dot_km;                       // optional fp32 [B,Hq,Nq]: raw q . K channel mean of the row's kv head
   const __nv_bfloat16* km_for_q;         //   (the term K smoothing removes from every score of the row)
 };
 
+// 64 registers: four CTAs per SM, each with a whole 32 KB tile in flight (B1 H40 N32760 D128, with the K sums: 240 us;
+// 260 at three per SM)
 template <int D>
-__global__ void __launch_bounds__(kThreads) quant_qkv_kernel(const QuantLaunch P) {
+__global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunch P) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   __shared__ __align__(16) uint8_t sf_smem[2048];
-  __shared__ float red[kThreads / 32][D];
+  __shared__ float red[RPP * D];
   __shared__ float mean_s[D];
   const int t = threadIdx.x, c = t % CH, rl = t / CH;
   int bid = blockIdx.x;
+  pdl_launch_dependents();                 // the K kernel may come in and fetch its tiles as SMs fall idle
+  if (bid == 0 && t == 0 && P.zero_status != nullptr) *P.zero_status = 0;
+
+  if (bid < P.s_blocks) {
+    // ----------------------------------------------------------------------------- K channel-sum role
+    const int chunk = bid % P.chunks, bh = bid / P.chunks, b = bh / P.Hkv, h = bh % P.Hkv;
+    const int N = P.cu_k ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
+    channel_partial<D>(P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + h * P.k_sh, P.k_sn, N, chunk, P.chunk_tokens,
+                       P.d_in, P.partial + (int64_t)bid * D, red);
+    return;
+  }
+  bid -= P.s_blocks;
 
   if (bid < P.q_blocks + P.k_blocks) {
     // ----------------------------------------------------------------------------- Q / K roles
@@ -136,6 +163,11 @@ __global__ void __launch_bounds__(kThreads) quant_qkv_kernel(const QuantLaunch P
     if (cu != nullptr) {                   // sequence b of a packed [tokens, H, D] tensor
       N = min(cu[b + 1] - cu[b], N);       // cut at max_seqlen, which sizes the output layouts
       src = (is_q ? P.q + h * P.q_sh : P.k + h * P.k_sh) + (int64_t)cu[b] * sn;
+      if (is_q && tile * kTile >= N) {     // beyond the sequence: only the block mean is read (for delta_s rows that no
+        if (P.q_mean_mode == 1 && rl == 0) //   query uses), so it must at least be a number
+          *reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 8) = make_uint4(0, 0, 0, 0);
+        return;
+      }
     }
     uint4 w[NP];
 #pragma unroll
@@ -191,13 +223,13 @@ __global__ void __launch_bounds__(kThreads) quant_qkv_kernel(const QuantLaunch P
         }
         if ((t & 31) < CH) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) red[t >> 5][c * 8 + i] = acc[i];
+          for (int i = 0; i < 8; ++i) red[(t >> 5) * D + c * 8 + i] = acc[i];
         }
         __syncthreads();
         if (t < D) {
           float s = 0.f;
 #pragma unroll
-          for (int r = 0; r < kThreads / 32; ++r) s += red[r][t];
+          for (int r = 0; r < kThreads / 32; ++r) s += red[r * D + t];
           mean_s[t] = s * (1.0f / kTile);
         }
         __syncthreads();
@@ -256,12 +288,12 @@ __global__ void __launch_bounds__(kThreads) quant_qkv_kernel(const QuantLaunch P
   const int64_t total = (int64_t)P.B * P.Hkv * P.Tk;
   for (int i = t; i < 2048 / 16; i += kThreads) reinterpret_cast<uint4*>(sf_smem)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  if (gt < total) {
-    const int tile = (int)(gt % P.Tk), bh = (int)(gt / P.Tk), b = bh / P.Hkv, h = bh % P.Hkv;
+  const int tile = (int)(gt % P.Tk), bh = (int)(gt / P.Tk), b = bh / P.Hkv, h = bh % P.Hkv;
+  const int Nv = P.cu_k && gt < total ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
+  if (gt < total && tile * kTile < Nv) {                  // (nothing reads a V tile beyond its sequence)
     const int c4 = (warp % WPT) * 4 + (lane >> 3);        // group of 4 channels
     const int blk = lane & 7;                              // 16-token block
     const __nv_bfloat16* src = P.v + (P.cu_k ? (int64_t)P.cu_k[b] * P.v_sn : b * P.v_sb) + h * P.v_sh + c4 * 4;
-    const int Nv = P.cu_k ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
     uint2 x[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -309,7 +341,7 @@ static int pick_chunk_tokens(int N, int BH) {
   // enough CTAs (8 per SM on 148 SMs) to keep the memory system full, but at most 64 partial rows per (b,h)
   int chunk = 4096;
   while (chunk > 256 && (int64_t)BH * ((N + chunk - 1) / chunk) < 1184) chunk >>= 1;
-  while ((N + chunk - 1) / chunk > 64) chunk <<= 1;
+  while ((N + chunk - 1) / chunk > kMaxChunks) chunk <<= 1;
   return chunk;
 }
 
@@ -343,6 +375,11 @@ cudaError_t launch_channel_mean(const void* x, int64_t sb, int64_t sh, int64_t s
   return cudaGetLastError();
 }
 
+void quant_chunks(int BH, int N, int* chunks, int* chunk_tokens) {
+  *chunk_tokens = pick_chunk_tokens(N, BH);
+  *chunks = (N + *chunk_tokens - 1) / *chunk_tokens;
+}
+
 cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   QuantLaunch P;
   P.q = (const __nv_bfloat16*)a.q; P.k = (const __nv_bfloat16*)a.k; P.v = (const __nv_bfloat16*)a.v;
@@ -360,13 +397,17 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   P.qm = (__nv_bfloat16*)a.qm;
   P.cu_q = a.cu_q; P.cu_k = a.cu_k;
   P.d_in = (a.d_in > 0 && a.d_in <= a.D) ? a.d_in : a.D;
+  P.partial = (float*)a.partial;
+  P.zero_status = a.zero_status;
+  quant_chunks(a.B * a.Hkv, a.Nk, &P.chunks, &P.chunk_tokens);
+  P.s_blocks = a.partial != nullptr ? a.B * a.Hkv * P.chunks : 0;
   P.q_dot_km = (a.q_dot_km != nullptr && a.km != nullptr && a.cu_q == nullptr) ? (float*)a.q_dot_km : nullptr;
   P.km_for_q = (const __nv_bfloat16*)a.km;
   P.q_blocks = a.q ? a.B * a.Hq * P.Tq : 0;
-  P.k_blocks = a.k ? a.B * a.Hkv * P.Tk : 0;
+  P.k_blocks = a.k && a.k_codes ? a.B * a.Hkv * P.Tk : 0;
   const int tpb = a.D == 128 ? 1 : 2;
   P.v_blocks = a.v ? (int)(((int64_t)a.B * a.Hkv * P.Tk + tpb - 1) / tpb) : 0;
-  const int grid = P.q_blocks + P.k_blocks + P.v_blocks;
+  const int grid = P.s_blocks + P.q_blocks + P.k_blocks + P.v_blocks;
   if (grid == 0) return cudaSuccess;
   if (a.D == 128) quant_qkv_kernel<128><<<grid, kThreads, 0, stream>>>(P);
   else            quant_qkv_kernel<64><<<grid, kThreads, 0, stream>>>(P);

@@ -9,6 +9,46 @@ namespace sage3 {
 constexpr int kTile = 128;
 constexpr int kThreads = 256;
 
+// The 8 channels of this thread (chunk threadIdx.x % (D/8)) of a head's K mean: from `km` where it is given, else from
+// the partial sums, by the whole CTA; also written to km_out if that is not null.  `stage`: shared memory for kMaxChunks
+// partial rows - they are fetched all at once, so that the CTA waits for memory once and not once per few rows (the K
+// kernel at B1 H40 N32760: 328 us, 356 with a chain of loads).
+constexpr int kMaxChunks = 64;             // at most so many partial rows per head (pick_chunk_tokens, quant.cu)
+template <int D>
+__device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, const float* __restrict__ partial, const int nchunks,
+                                       const float divisor, const int64_t bh, float* stage, __nv_bfloat16* km_out,
+                                       float (&mean)[8]) {
+  const int t = threadIdx.x, c = t % (D / 8);
+  if (km != nullptr) {
+    const uint4 m = *reinterpret_cast<const uint4*>(km + bh * D + c * 8);
+    mean[0] = bf16_lo(m.x); mean[1] = bf16_hi(m.x); mean[2] = bf16_lo(m.y); mean[3] = bf16_hi(m.y);
+    mean[4] = bf16_lo(m.z); mean[5] = bf16_hi(m.z); mean[6] = bf16_lo(m.w); mean[7] = bf16_hi(m.w);
+    return;
+  }
+  constexpr int V = kMaxChunks * D / 4 / kThreads;
+  const int nv = nchunks * D / 4;
+  float4 x[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (i * kThreads + t < nv) x[i] = __ldcg(reinterpret_cast<const float4*>(partial) + i * kThreads + t);
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (i * kThreads + t < nv) reinterpret_cast<float4*>(stage)[i * kThreads + t] = x[i];
+  __syncthreads();
+  float s = 0.f;
+  if (t < D)
+    for (int i = 0; i < nchunks; ++i) s += stage[i * D + t];
+  __syncthreads();
+  if (t < D) {
+    const __nv_bfloat16 m = __float2bfloat16_rn(s / divisor);
+    stage[t] = __bfloat162float(m);
+    if (km_out != nullptr) km_out[bh * D + t] = m;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) mean[i] = stage[c * 8 + i];
+}
+
 // Row-wise quantisation of one 128-token tile held in registers (Q and K roles).
 // Thread t owns 8 consecutive channels (chunk c) of rows rl, rl+RPP, ... ; w[p] = 4 packed bf16x2.
 // ------------------------------------------------------------------------------------------------

@@ -29,3 +29,24 @@ def test_attention_at_tile_edges(B, Hq, Hkv, Nq, Nk, D, causal):
     fin = torch.isfinite(want_lse)
     assert torch.allclose(lse.cpu()[fin], want_lse[fin], atol=2e-3, rtol=1e-4)
     assert bool(torch.isneginf(lse.cpu()[~fin]).all())
+
+
+# K means added up from partial sums in the K kernel, which takes the query blocks of a whole GQA group as one list of rows:
+# one row, 128 and 129 of them, sums of one chunk of tokens and of many, a head dim with channels to fill up
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D", [
+    (1, 8, 2, 1, 300, 128), (2, 8, 8, 16384, 129, 64), (1, 4, 1, 32 * 128 + 1, 257, 128), (1, 12, 2, 300, 20000, 64), (1, 4, 2, 260, 511, 96)])
+def test_k_means_and_delta_s_of_the_operator(B, Hq, Hkv, Nq, Nk, D):
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, 128 if D == 96 else D, seed=Nq + Nk, device=DEV)
+    if D == 96:
+        out = sa.sageattn(q[..., :96], k[..., :96], v[..., :96], sm_scale=0.1, check_status=True)
+        want = sa.sageattn(*(torch.nn.functional.pad(t[..., :96], (0, 32)) for t in (q, k, v)), sm_scale=0.1)[..., :96]
+        assert torch.equal(out, want)
+        return
+    z = sa.quantize_qkv(q, k, v)
+    ref_km = k.float().mean(dim=2).to(torch.bfloat16).float()
+    assert ((z.km.float() - ref_km).abs() <= ref_km.abs() * 2.0 ** -7 + 1e-3).all()
+    ks = (k.float() - z.km.float()[:, :, None]).to(torch.bfloat16).float().repeat_interleave(Hq // Hkv, dim=1)
+    want = torch.matmul(z.qm.float(), ks.transpose(-1, -2))
+    assert torch.allclose(z.delta_s[..., :Nk].float(), want, atol=2e-2 * float(want.abs().max()), rtol=1e-2)
+    assert (z.delta_s[..., Nk:] == 0).all()
+    assert torch.equal(sa.sageattn(q, k, v, check_status=True), sa.fp4_attention(z))
