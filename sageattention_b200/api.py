@@ -18,6 +18,7 @@ raise.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from dataclasses import dataclass
 from typing import Optional, Tuple
@@ -29,8 +30,21 @@ from . import _lib
 _LOG2E = 1.4426950408889634
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)                 # without building a Stream object
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_NOTHING = contextlib.nullcontext()
+
+
+def _on_device(device):
+    """Context in which `device` is the current one; nothing to do where it is already."""
+    return _NOTHING if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _as_bhnd_strides(x: torch.Tensor, tensor_layout: str):
@@ -144,7 +158,7 @@ def quantize_qkv(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tensor_layou
     a.km = out.km.data_ptr() if out.km is not None else None
     a.delta_s = out.delta_s.data_ptr() if out.delta_s is not None else None
     a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         _lib.check(lib.sage3_quant_qkv(C.byref(a), _stream_ptr(dev)), "sage3_quant_qkv")
     return out
 
@@ -180,7 +194,7 @@ def fp4_attention(qz: QuantizedQKV, sm_scale: Optional[float] = None, is_causal:
     a.sm_scale, a.is_causal = float(sm_scale), int(bool(is_causal))
     a.device_status = status.data_ptr()
     a.sm_margin = int(sm_margin)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         if qz.k_lambda is not None:
             a.shape = _lib.Shape(B, Hq, Hkv, Nq, int(qz.nk_slots), D)
             _lib.check(lib.sage3_attn_fwd_packed(C.byref(a), qz.k_lambda.data_ptr(), int(qz.mean_slot_first),
@@ -221,7 +235,7 @@ def pack_kv(k: torch.Tensor, v: torch.Tensor, tensor_layout: str = "HND", smooth
     a.k_packed, a.v_packed, a.k_lambda = kp.data_ptr(), vp.data_ptr(), lam.data_ptr()
     a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
     a.split_first = int(bool(split_first))
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         _lib.check(lib.sage3_pack_kv(C.byref(a), _stream_ptr(dev)), "sage3_pack_kv")
     return kp, vp, lam, km
 
@@ -277,6 +291,53 @@ def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
     """
     if attn_mask is not None:
         raise NotImplementedError("attn_mask is not supported (the reference ignores it as well)")
+    if sm_scale is not None:
+        sm_scale = float(sm_scale)
+    key = (q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.device, tensor_layout,
+           bool(is_causal), sm_scale, bool(per_block_mean), bool(smooth_k), sm_margin)
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin)
+        if len(_plans) >= _MAX_PLANS:
+            _plans.clear()
+        _plans[key] = plan
+    if plan.pad:
+        # head dims that are no multiple of 8 are padded here first, as the reference does (core.py:925-937, :990)
+        d_og = q.shape[-1]
+        q, k, v = (torch.nn.functional.pad(t, (0, plan.pad)) for t in (q, k, v))
+        res = sageattn3_blackwell(q, k, v, tensor_layout=tensor_layout, is_causal=is_causal,
+                                  sm_scale=d_og ** -0.5 if sm_scale is None else sm_scale, per_block_mean=per_block_mean,
+                                  return_lse=return_lse, smooth_k=smooth_k, check_status=check_status, sm_margin=sm_margin)
+        return (res[0][..., :d_og].contiguous(), res[1]) if return_lse else res[..., :d_og].contiguous()
+    dev = plan.device
+    out = torch.empty_like(q)
+    ws = torch.empty(plan.workspace, dtype=torch.uint8, device=dev)
+    lse = torch.empty(plan.lse_shape, dtype=torch.float32, device=dev) if return_lse else None
+    # the status word has a place in the workspace; it is only kept apart where the caller wants it read back
+    status = torch.empty(1, dtype=torch.int32, device=dev) if check_status else None
+    with _on_device(dev):
+        stream = _stream_ptr(dev)
+        st = plan.run(plan.args, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None if lse is None else lse.data_ptr(),
+                      ws.data_ptr(), None if status is None else status.data_ptr(), stream)
+        if st:
+            _lib.check(st, "sage3_attention")
+        if check_status:
+            _lib.check(_lib.load().sage3_read_device_status(status.data_ptr(), stream, None), "attention kernel")
+    return (out, lse) if return_lse else out
+
+
+# What a call with given shapes, strides and options needs, worked out once: the checks, the sizes and the argument
+# struct but for its pointers (a call on the smallest problems took 42 us of host time, 15 us of it this).  Read-only
+# after it is made, so that threads may share it; no device memory is held.
+_MAX_PLANS = 1024
+_plans = {}
+
+
+class _Plan:
+    __slots__ = ("pad", "device", "workspace", "lse_shape", "struct", "args", "run")
+
+
+def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin) -> _Plan:
     lib = _lib.load()
     _check_device(q)
     for t in (q, k, v):
@@ -292,46 +353,31 @@ def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
     # head-dim padding of sageattention/core.py:925-937: below 64 -> 64, between 64 and 128 -> 128, zeros in the
     # extra channels, default scale from the original head dim, output cut back (:990).  The kernels read rows of the
     # original width and take the rest as zero, so nothing is copied - if the width is a multiple of 8 (16-byte
-    # loads); other widths are padded here first, as the reference does.
-    d_og = D
+    # loads); other widths are padded before the call.
     if D > 128:
         raise ValueError(f"Unsupported head_dim: {D}")                            # core.py:937
-    if D not in (64, 128) and D % 8 != 0:
-        pad = (64 if D < 64 else 128) - D
-        if sm_scale is None:
-            sm_scale = D ** -0.5
-        q, k, v = (torch.nn.functional.pad(t, (0, pad)) for t in (q, k, v))
-        res = sageattn3_blackwell(q, k, v, tensor_layout=tensor_layout, is_causal=is_causal, sm_scale=sm_scale,
-                                  per_block_mean=per_block_mean, return_lse=return_lse, smooth_k=smooth_k,
-                                  check_status=check_status, sm_margin=sm_margin)
-        return (res[0][..., :d_og].contiguous(), res[1]) if return_lse else res[..., :d_og].contiguous()
-    if D not in (64, 128):
-        D = 64 if D < 64 else 128
-    dev = q.device
+    p = _Plan()
+    Dp = 64 if D <= 64 else 128
+    p.pad = 0 if D % 8 == 0 else Dp - D
+    if p.pad:
+        return p
     pbm = int(bool(per_block_mean))
-    z = buffer_sizes(B, Hq, Hkv, Nq, Nk, D, pbm)
-    out = torch.empty_like(q)
-    _, _, _, _, osb, osh, osn = _as_bhnd_strides(out, tensor_layout)
-    ws = torch.empty(int(z.workspace), dtype=torch.uint8, device=dev)
-    lse = torch.empty((B, Hq, Nq), dtype=torch.float32, device=dev) if return_lse else None
-    status = torch.empty(1, dtype=torch.int32, device=dev)
-    a = _lib.FwdArgs()
-    a.shape = _lib.Shape(B, Hq, Hkv, Nq, Nk, D)
-    a.q, a.k, a.v = _tensor_arg(q, qsb, qsh, qsn), _tensor_arg(k, ksb, ksh, ksn), _tensor_arg(v, vsb, vsh, vsn)
-    a.out, a.out_stride_b, a.out_stride_h, a.out_stride_n = out.data_ptr(), osb, osh, osn
-    a.lse = lse.data_ptr() if lse is not None else None
+    z = buffer_sizes(B, Hq, Hkv, Nq, Nk, Dp, pbm)
+    _, _, _, _, osb, osh, osn = _as_bhnd_strides(torch.empty_like(q, device="meta"), tensor_layout)
+    a = p.struct = _lib.FwdArgs()
+    a.shape = _lib.Shape(B, Hq, Hkv, Nq, Nk, Dp)
+    a.q, a.k, a.v = _lib.Tensor(None, qsb, qsh, qsn), _lib.Tensor(None, ksb, ksh, ksn), _lib.Tensor(None, vsb, vsh, vsn)
+    a.out_stride_b, a.out_stride_h, a.out_stride_n = osb, osh, osn
     a.km_out = None           # the K-mean term of the LSE is put back on the device (q . km in the quantisation kernel)
     a.sm_scale = float(sm_scale) if sm_scale is not None else 0.0
     a.is_causal, a.per_block_mean, a.smooth_k = int(bool(is_causal)), pbm, int(bool(smooth_k))
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    a.device_status = status.data_ptr()
-    a.head_dim = d_og if d_og != D else 0
+    a.workspace_bytes = int(z.workspace)
+    a.head_dim = D if D != Dp else 0
     a.sm_margin = int(sm_margin)
-    with torch.cuda.device(dev):
-        _lib.check(lib.sage3_attention(C.byref(a), _stream_ptr(dev)), "sage3_attention")
-        if check_status:
-            _lib.check(lib.sage3_read_device_status(status.data_ptr(), _stream_ptr(dev), None), "attention kernel")
-    return (out, lse) if return_lse else out
+    p.args = C.byref(a)
+    p.device, p.workspace, p.lse_shape = q.device, int(z.workspace), (B, Hq, Nq)
+    p.run = lib.sage3_attention_run
+    return p
 
 
 def sageattn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tensor_layout: str = "HND", is_causal: bool = False,
@@ -339,7 +385,6 @@ def sageattn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tensor_layout: s
     """Automatic entry point (``sageattention/core.py:79-157``).  The reference picks a kernel family
     by GPU architecture and raises ``ValueError`` for architectures it has no kernel for; this build
     has exactly one family, the FP4 kernels for compute capability 10.x."""
-    _check_device(q)
     return sageattn3_blackwell(q, k, v, tensor_layout=tensor_layout, is_causal=is_causal, sm_scale=sm_scale,
                                return_lse=return_lse, **kwargs)
 
@@ -390,7 +435,7 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
     a.is_causal, a.smooth_k = int(bool(is_causal)), int(bool(smooth_k))
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     a.device_status = status.data_ptr()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         _lib.check(lib.sage3_attention_varlen(C.byref(a), _stream_ptr(dev)), "sage3_attention_varlen")
         if check_status:
             _lib.check(lib.sage3_read_device_status(status.data_ptr(), _stream_ptr(dev), None), "attention kernel")

@@ -309,6 +309,15 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false, /*after_delta_s=*/t.delta_s != nullptr);
 }
 
+int sage3_attention_run(const sage3_fwd_args* args, const void* q, const void* k, const void* v, void* out, float* lse,
+                        void* workspace, int32_t* device_status, void* stream) {
+  if (args == nullptr) return SAGE3_ERR_ARGUMENT;
+  sage3_fwd_args a = *args;
+  a.q.ptr = q; a.k.ptr = k; a.v.ptr = v;
+  a.out = out; a.lse = lse; a.workspace = workspace; a.device_status = device_status;
+  return sage3_attention(&a, stream);
+}
+
 int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   if (a == nullptr || a->workspace == nullptr || a->out == nullptr) return SAGE3_ERR_ARGUMENT;
   if (!a->q || !a->k || !a->v || !a->cu_seqlens_q || !a->cu_seqlens_k) return SAGE3_ERR_ARGUMENT;
