@@ -445,13 +445,50 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
 _host_streams = {}
 
 
+_HOST_PIECE_BYTES = 24 << 20      # of q, k, v: 0.4 ms of copying, which hides the host work of a piece's calls
+
+
+def _host_pieces(B: int, Hkv: int, head_bytes: int, head_chunks) -> list:
+    """Pieces (first, last + 1 batch entry, first, last + 1 kv head) in which a host tensor goes through the GPU, each
+    contiguous in host memory: some heads of one batch entry, or some whole batch entries.  They carry about
+    ``_HOST_PIECE_BYTES``; where that is several heads, sizes ramp up from one head at the start and down to one at the
+    end, so that the first kernel starts after a small copy and little is left to copy out after the last."""
+    if isinstance(head_chunks, (list, tuple)):
+        sizes = [int(n) for n in head_chunks]                    # explicit group sizes (kv heads per group)
+        if sum(sizes) != Hkv or min(sizes) < 1:
+            raise ValueError(f"head_chunks {sizes} must be positive and add up to the {Hkv} kv heads")
+        plan = [sizes] * B
+    else:
+        entries = _HOST_PIECE_BYTES // max(1, Hkv * head_bytes)
+        if entries >= 1 or int(head_chunks) <= 1:
+            n = max(1, entries)
+            return [(b, min(b + n, B), 0, Hkv) for b in range(0, B, n)]
+        base = max(1, _HOST_PIECE_BYTES // head_bytes)
+        ramp = [n for n in (1, 2, 4) if n < base]
+        plan = []
+        for b in range(B):
+            up, down = (ramp if b == 0 else []), (ramp[::-1] if b == B - 1 else [])
+            while sum(up) + sum(down) > Hkv:
+                up, down = up[:-1], down[1:]
+            left = Hkv - sum(up) - sum(down)
+            plan.append(up + [base] * (left // base) + ([left % base] if left % base else []) + down)
+    pieces = []
+    for b, sizes in enumerate(plan):
+        h = 0
+        for n in sizes:
+            pieces.append((b, b + 1, h, h + n))
+            h += n
+    return pieces
+
+
 def sageattn_from_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: Optional[torch.Tensor] = None,
                        device=None, head_chunks=8, is_causal: bool = False, sm_scale: Optional[float] = None,
                        **kwargs) -> torch.Tensor:
-    """Attention on HOST tensors (HND ``[B,H,N,D]`` bf16, ideally pinned): the heads are processed in
-    ``head_chunks`` groups of kv heads (a number, or an explicit list of kv heads per group), and the host-to-device copy of group ``i+1`` and the
-    device-to-host copy of group ``i-1`` run on their own streams while group ``i`` is computed (groups
-    alternate between two compute streams so that their kernels overlap at the seams), so the
+    """Attention on HOST tensors (HND ``[B,H,N,D]`` bf16, ideally pinned): they go through the GPU in pieces of some kv
+    heads of a batch entry, or of some whole batch entries where these are small (``head_chunks`` = 1: never less than a
+    whole entry; a list: the kv heads per piece), and the host-to-device copy of piece ``i+1`` and the device-to-host
+    copy of piece ``i-1`` run on their own streams while piece ``i`` is computed (pieces alternate between two compute
+    streams so that their kernels overlap at the seams), so the
     PCIe transfers hide behind the kernels (or the other way round).  Returns the output as a host tensor
     (``out`` if given, else a new pinned tensor).  The work is ordered after the caller's current stream
     and the current stream waits for the last copy, so CUDA events recorded around the call time all of it;
@@ -466,79 +503,39 @@ def sageattn_from_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: O
     g = Hq // Hkv
     if out is None:
         out = torch.empty_like(q).pin_memory()
-    # group sizes: about Hkv / head_chunks heads, but ramping up from one head at the start and down to one at
-    # the end, so that the first kernel starts after a small copy and little is left to copy out after the last.
-    # A group should also carry enough bytes (about 96 MB of q, k, v) for its copy to be worth a pipeline stage:
-    # every group costs a few host-side calls, which small problems cannot hide.
-    if isinstance(head_chunks, (list, tuple)):
-        sizes = [int(n) for n in head_chunks]                    # explicit group sizes (kv heads per group)
-        if sum(sizes) != Hkv or min(sizes) < 1:
-            raise ValueError(f"head_chunks {sizes} must be positive and add up to the {Hkv} kv heads")
-    else:
-        in_bytes = (q.numel() + k.numel() + v.numel()) * q.element_size()
-        head_chunks = max(1, min(head_chunks, int(in_bytes // (96 << 20)) or 1))
-        base = max(1, Hkv // max(1, min(head_chunks, Hkv)))
-        ramp = [n for n in (1, 2, 4) if n < base] if head_chunks > 1 else []
-        sizes = list(ramp)
-        left = Hkv - sum(ramp)
-        tail = [n for n in reversed(ramp) if n <= left - base]      # keep at least one full group in the middle
-        left -= sum(tail)
-        while left > 0:
-            sizes.append(min(base, left))
-            left -= sizes[-1]
-        sizes += tail
-    bounds = [0]
-    for n in sizes:
-        bounds.append(bounds[-1] + n)
-    assert bounds[-1] == Hkv
-    chunks = len(sizes)
+    pieces = _host_pieces(B, Hkv, (q.numel() + k.numel() + v.numel()) * q.element_size() // (B * Hkv), head_chunks)
     if dev not in _host_streams:
         _host_streams[dev] = tuple(torch.cuda.Stream(dev) for _ in range(4))
     s_in, s_run_a, s_run_b, s_out = _host_streams[dev]
     cur = torch.cuda.current_stream(dev)
-    start = torch.cuda.Event()
-    start.record(cur)
+    # whole-problem buffers from the current stream's pool: everything below starts after that stream's present end and
+    # it waits for everything below, so they need no further bookkeeping
+    qd, kd, vd = (torch.empty(t.shape, dtype=t.dtype, device=dev) for t in (q, k, v))
+    start = cur.record_event()
     for st in (s_in, s_run_a, s_run_b, s_out):
         st.wait_event(start)
     keep = []
-    for c in range(chunks):
-        h0, h1 = bounds[c], bounds[c + 1]
-        if h0 == h1:
-            continue
+    for i, (b0, b1, h0, h1) in enumerate(pieces):
+        sq, sk = (slice(b0, b1), slice(h0 * g, h1 * g)), (slice(b0, b1), slice(h0, h1))
         with torch.cuda.stream(s_in):
-            # one copy per batch entry: q[b, h0:h1] is one contiguous block of a [B,H,N,D] tensor, q[:, h0:h1] is not
-            # (for B > 1 a strided host-to-device copy falls back to a slow path)
-            qd = torch.empty((B, (h1 - h0) * g, Nq, D), dtype=q.dtype, device=dev)
-            kd = torch.empty((B, h1 - h0) + tuple(k.shape[2:]), dtype=k.dtype, device=dev)
-            vd = torch.empty_like(kd)
-            for b in range(B):
-                qd[b].copy_(q[b, h0 * g:h1 * g], non_blocking=True)
-                kd[b].copy_(k[b, h0:h1], non_blocking=True)
-                vd[b].copy_(v[b, h0:h1], non_blocking=True)
-            ev_in = torch.cuda.Event()
-            ev_in.record(s_in)
-        # groups alternate between two compute streams: the attention kernel is persistent (one CTA per SM), so
-        # the kernels of the next group fill the SMs that the last, partly filled round of this group leaves idle
-        s_run = s_run_a if c % 2 == 0 else s_run_b
+            qd[sq].copy_(q[sq], non_blocking=True)
+            kd[sk].copy_(k[sk], non_blocking=True)
+            vd[sk].copy_(v[sk], non_blocking=True)
+            ev_in = s_in.record_event()
+        # the attention kernel is persistent (one CTA per SM): on two streams in turn, the kernels of the next piece fill
+        # the SMs that the last, partly filled round of this piece leaves idle
+        s_run = s_run_b if i % 2 else s_run_a
         with torch.cuda.stream(s_run):
             s_run.wait_event(ev_in)
-            od = sageattn3_blackwell(qd, kd, vd, tensor_layout="HND", is_causal=is_causal, sm_scale=sm_scale, **kwargs)
-            ev_run = torch.cuda.Event()
-            ev_run.record(s_run)
+            o = sageattn3_blackwell(qd[sq], kd[sk], vd[sk], tensor_layout="HND", is_causal=is_causal, sm_scale=sm_scale, **kwargs)
+            ev_run = s_run.record_event()
         with torch.cuda.stream(s_out):
             s_out.wait_event(ev_run)
-            for b in range(B):
-                out[b, h0 * g:h1 * g].copy_(od[b], non_blocking=True)
-        keep.append((qd, kd, vd, od))
-    done = torch.cuda.Event()
-    done.record(s_out)
-    cur.wait_event(done)
-    for st in (s_run_a, s_run_b):                 # nothing of this call may outlive the caller's next operation
-        ev = torch.cuda.Event()
-        ev.record(st)
-        cur.wait_event(ev)
-    # the device buffers were allocated on side streams: tell the allocator the current stream orders their reuse
-    for tensors in keep:
-        for t in tensors:
-            t.record_stream(cur)
+            out[sq].copy_(o, non_blocking=True)
+        keep.append(o)
+    for st in (s_out, s_run_a, s_run_b):          # nothing of this call may outlive the caller's next operation
+        cur.wait_event(st.record_event())
+    # the outputs came from the compute streams' pools: tell the allocator that the current stream orders their reuse
+    for o in keep:
+        o.record_stream(cur)
     return out
