@@ -19,7 +19,8 @@
 // P, its block scales and the row sum are the reference's value for value.
 //
 // One persistent CTA per SM walks a static list of work items (round r: item r*grid + i, odd rounds in
-// reverse CTA order; causal items sorted by falling cost over all heads);
+// reverse CTA order; causal items sorted by falling cost over all heads, those of variable-length batches by an order that
+// the quantisation kernel made);
 // an item is TWO adjacent 128-row query tiles of one head, which share every K / V tile.  All
 // barrier phases keep counting across items, so the loads, the first Q.K^T and the first softmax of the next item are
 // under way while the output of the current one is stored.  16 warps:
@@ -171,6 +172,7 @@ struct KParams {
 #if SAGE3_VARLEN_BUILD
   const int *cu_q, *cu_k; // token offsets of the sequences (device int32 [B+1]); Nq, Nk, Tq, Tk then describe the
                           // LONGEST sequence, i.e. the rectangular operand layouts
+  const int *order, *n_order; // pairs of query tiles that exist (sequence * pairs + pair), heaviest first, and their number
 #endif
 };
 
@@ -323,6 +325,11 @@ __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
   Work k;
   const int n_pairs = (P.Tq + 1) >> 1;
   int bh;
+#if SAGE3_VARLEN_BUILD
+  const int entry = P.order[w / P.Hq];
+  k.pair = entry % n_pairs;
+  bh = entry / n_pairs * P.Hq + w % P.Hq;
+#else
   if (kCausal) {
     // item cost grows with the pair index: heaviest pairs of all heads first, so that the rounds of
     // the static schedule hand out work of falling, nearly equal cost
@@ -334,6 +341,7 @@ __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
     k.pair = n_pairs - 1 - (w % n_pairs);
     bh = w / n_pairs;
   }
+#endif
   k.b = bh / P.Hq;
   k.hq = bh % P.Hq;
   k.hkv = k.hq / (P.Hq / P.Hkv);
@@ -397,7 +405,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   volatile int* abort_s = reinterpret_cast<volatile int*>(smem + L::bars + Bars::abort_flag);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool has_ds = P.ds != nullptr;
-  const int total_work = P.B * P.Hq * ((P.Tq + 1) >> 1);
 
   if (threadIdx.x == 0) {
     for (int t = 0; t < 2; ++t) {
@@ -450,6 +457,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   // read once after the barrier: every warp takes the same branch, so the register hand-over
   // below (setmaxnreg) is always executed by whole warpgroups
   const bool run = *reinterpret_cast<volatile int*>(smem + L::bars + Bars::run_flag) != 0;
+#if SAGE3_VARLEN_BUILD
+  const int total_work = *P.n_order * P.Hq;
+#else
+  const int total_work = P.B * P.Hq * ((P.Tq + 1) >> 1);
+#endif
   // The CTA is persistent: every role walks the same static list of work items (blockIdx.x, +gridDim.x, ...)
   // and all barrier phases simply keep counting across items, so the loads, MMAs and softmax of the
   // next item start while the tail of the current one is still being finished.
@@ -1019,6 +1031,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.Nk_log = kPacked ? (a.Nk / 16) * 15 + (a.Nk % 16 == 0 ? 0 : a.Nk % 16 - 1) : a.Nk;
 #if SAGE3_VARLEN_BUILD
   P.cu_q = a.cu_q; P.cu_k = a.cu_k;
+  P.order = a.order; P.n_order = a.n_order;
 #endif
   auto kern = attn_fwd_kernel<D, kCausal, kPacked>;
   // persistent CTAs: one per SM (registers and tensor memory allow exactly one), each walks the work list
@@ -1048,7 +1061,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
 #if SAGE3_VARLEN_BUILD
 cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream) {
   // offsets come in pairs; no K-packing and no LSE for packed batches
-  if (a.cu_q == nullptr || a.cu_k == nullptr || a.k_lambda != nullptr || a.lse != nullptr) return cudaErrorInvalidValue;
+  if (a.cu_q == nullptr || a.cu_k == nullptr || a.order == nullptr || a.n_order == nullptr || a.k_lambda != nullptr || a.lse != nullptr) return cudaErrorInvalidValue;
   if (a.D == 128) return a.causal ? launch<128, true, false>(a, stream) : launch<128, false, false>(a, stream);
   if (a.D == 64) return a.causal ? launch<64, true, false>(a, stream) : launch<64, false, false>(a, stream);
   return cudaErrorInvalidValue;

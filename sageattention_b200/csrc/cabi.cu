@@ -91,7 +91,7 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
 }
 
 static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int* cu_k, void* stream_,
-                          int* zero_status = nullptr) {
+                          int* zero_status = nullptr, int* order = nullptr, int* n_order = nullptr, int causal = 0) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (int st = check_tensor(a->q)) return st;
@@ -148,6 +148,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   q.q_mean_mode = a->per_block_mean == 1 ? 1 : (a->per_block_mean == 0 ? 2 : 0);
   q.km = km; q.partial = partial;
   q.zero_status = zero_status;
+  q.order = order; q.n_order = n_order; q.causal = causal;
   q.q_mean_seq = a->per_block_mean == 0 ? a->qm : nullptr;
   q.qm_override = a->per_block_mean == 1 ? a->qm_in : nullptr;
   q.q_codes = a->q_codes; q.q_sf = a->q_sf; q.k_codes = k_in_ds ? nullptr : a->k_codes; q.k_sf = a->k_sf;
@@ -176,7 +177,8 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
 int sage3_quant_qkv(const sage3_quant_args* a, void* stream) { return quant_qkv_impl(a, nullptr, nullptr, stream); }
 
 static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const int* cu_q, const int* cu_k, void* stream_,
-                         int slot_first = 0, bool zero_status = true, bool after_delta_s = false) {
+                         int slot_first = 0, bool zero_status = true, bool after_delta_s = false,
+                         const int* order = nullptr, const int* n_order = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (!a->q_codes || !a->q_sf || !a->k_codes || !a->k_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status)
@@ -210,6 +212,7 @@ static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const 
   k.sm_margin = a->sm_margin;
   k.cu_q = cu_q; k.cu_k = cu_k;
   k.after_delta_s = after_delta_s;
+  k.order = order; k.n_order = n_order;
   e = (cu_q != nullptr || cu_k != nullptr) ? sage3::launch_attn_fwd_varlen(k, stream) : sage3::launch_attn_fwd(k, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   return SAGE3_OK;
@@ -338,12 +341,15 @@ int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   q.qm = take(z.qm);
   q.km = take(z.km);
   q.delta_s = take(z.delta_s);
-  take(z.q_dot_km);                                   // no LSE for packed batches (the reference returns none)
+  // no LSE for packed batches (the reference returns none): the room of its term takes the work order, one entry per pair
+  // of query tiles and sequence (a word per query, head and sequence is always enough), their number goes behind the status
+  int* order = reinterpret_cast<int*>(take(z.q_dot_km));
   q.scratch = take(z.scratch); q.scratch_bytes = z.scratch;
-  int32_t* status = reinterpret_cast<int32_t*>(take(4));
+  int32_t* status = reinterpret_cast<int32_t*>(take(8));
+  int* n_order = status + 1;
   if (a->device_status) status = a->device_status;
   q.device_status = status;
-  if (int st = quant_qkv_impl(&q, a->cu_seqlens_q, a->cu_seqlens_k, stream, status)) return st;
+  if (int st = quant_qkv_impl(&q, a->cu_seqlens_q, a->cu_seqlens_k, stream, status, order, n_order, a->is_causal)) return st;
   sage3_attn_args t{};
   t.shape = a->shape;
   t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;
@@ -353,7 +359,8 @@ int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   t.lse = nullptr;
   t.sm_scale = a->sm_scale > 0.f ? a->sm_scale : 1.0f / sqrtf((float)a->shape.D);
   t.is_causal = a->is_causal; t.device_status = status;
-  return attn_fwd_impl(&t, nullptr, a->cu_seqlens_q, a->cu_seqlens_k, stream, 0, /*zero_status=*/false, /*after_delta_s=*/true);
+  return attn_fwd_impl(&t, nullptr, a->cu_seqlens_q, a->cu_seqlens_k, stream, 0, /*zero_status=*/false, /*after_delta_s=*/true,
+                       order, n_order);
 }
 
 int sage3_k_mean_static(const sage3_shape* shape, const sage3_tensor* k, void* km_out, void* stream) {

@@ -28,6 +28,9 @@ struct QuantArgs {
   void* partial = nullptr;                // or fp32 scratch (quant_scratch_bytes): this launch only takes the partial sums
                                           //   of K, for launch_delta_s; both null: no K smoothing
   int* zero_status = nullptr;             // optional device word to zero
+  int* order = nullptr;                   // variable-length batches: receives the attention kernel's work order, at most
+  int* n_order = nullptr;                 //   B * ceil(ceil(Nq / 128) / 2) entries, and their number (both or neither)
+  int causal = 0;                         //   (what the work of an entry depends on)
   const void* q_mean_seq;                 // bf16 [B,Hq,D]   (mode 2)
   const void* qm_override;                // fp32 [B,Hq,Tq,D] or null (mode 1)
   void *q_codes, *q_sf, *k_codes, *k_sf, *vt_codes, *vt_sf, *qm;
@@ -97,6 +100,8 @@ struct AttnArgs {
   int sm_margin = 0;                      // SMs left free for kernels running beside the persistent attention kernel
   const int* cu_q = nullptr;              // variable-length batches, see QuantArgs; out is then [tokens, Hq, D]
   const int* cu_k = nullptr;
+  const int* order = nullptr;             // with cu_q, cu_k: the work order that launch_quant_qkv left, and
+  const int* n_order = nullptr;           //   its length
   bool after_delta_s = false;             // launched right behind launch_delta_s on the same stream: may overlap its end
 };
 cudaError_t launch_attn_fwd(const AttnArgs& a, cudaStream_t stream);

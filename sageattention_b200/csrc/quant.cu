@@ -123,9 +123,61 @@ struct QuantLaunch {
   int s_blocks, chunks, chunk_tokens;    // CTAs of the K channel-sum role (0: none), chunks per head, tokens per chunk
   float* partial;                        // [B,Hkv,chunks,D] fp32 K channel sums, written by that role
   int* zero_status;                      // status word of the whole operator call, zeroed here (optional)
+  int o_blocks, causal;                  // 1: the work-order role of a variable-length batch runs
+  int *order, *n_order;                  // its result: (sequence, pair of query tiles) entries and their number
   float* q_dot_km;                       // optional fp32 [B,Hq,Nq]: raw q . K channel mean of the row's kv head
   const __nv_bfloat16* km_for_q;         //   (the term K smoothing removes from every score of the row)
 };
+
+// Work order of a variable-length batch for the attention kernel's static schedule: the pairs of query tiles that exist,
+// by falling number of key tiles they visit, as sequence * pairs + pair.  One CTA, counting sort (costs above the table
+// are scaled into it); the order within a bin is whatever the atomics make it, the results do not depend on it.
+// Without it the schedule dealt out items as if every sequence were the longest: 16 causal sequences of 187 to 3000
+// tokens, 32 heads, took 452 us.
+constexpr int kOrderBins = 2048;
+__device__ __forceinline__ void varlen_order(const QuantLaunch& P, int* hist) {
+  const int t = threadIdx.x, n_pairs = (P.Tq + 1) >> 1, n = P.B * n_pairs;
+  const int scale = (2 * P.Tk + kOrderBins) / kOrderBins;       // costs 0 ... 2 Tk
+  auto bin_of = [&](const int e) {                              // heaviest in bin 0; -1: no such query tiles
+    const int b = e / n_pairs, q0 = (e % n_pairs) * 2 * kTile;
+    const int nq = min(P.cu_q[b + 1] - P.cu_q[b], P.Nq), nk = min(P.cu_k[b + 1] - P.cu_k[b], P.Nk);
+    if (q0 >= nq) return -1;
+    int cost = 0;
+    for (int s = 0; s < 2; ++s) {
+      const int end = min(q0 + (s + 1) * kTile, nq);
+      if (q0 + s * kTile >= nq) break;
+      const int keys = P.causal ? min(nk, end + nk - nq) : nk;
+      cost += keys <= 0 ? 0 : (keys + kTile - 1) / kTile;
+    }
+    return kOrderBins - 1 - cost / scale;
+  };
+  for (int i = t; i < kOrderBins; i += kThreads) hist[i] = 0;
+  __syncthreads();
+  for (int e = t; e < n; e += kThreads) {
+    const int bin = bin_of(e);
+    if (bin >= 0) atomicAdd(&hist[bin], 1);
+  }
+  __syncthreads();
+  if (t < 32) {                                                 // exclusive prefix sum by one warp
+    int base = 0;
+    for (int i = t; i < kOrderBins; i += 32) {
+      const int v = hist[i];
+      int x = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (t >= o) x += y;
+      }
+      hist[i] = base + x - v;
+      base += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (t == 0) *P.n_order = base;
+  }
+  __syncthreads();
+  for (int e = t; e < n; e += kThreads) {
+    const int bin = bin_of(e);
+    if (bin >= 0) P.order[atomicAdd(&hist[bin], 1)] = e;
+  }
+}
 
 // 64 registers: four CTAs per SM, each with a whole 32 KB tile in flight (B1 H40 N32760 D128, with the K sums: 240 us;
 // 260 at three per SM)
@@ -140,6 +192,12 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   pdl_launch_dependents();                 // the K kernel may come in and fetch its tiles as SMs fall idle
   if (bid == 0 && t == 0 && P.zero_status != nullptr) *P.zero_status = 0;
 
+  if (bid < P.o_blocks) {
+    static_assert(sizeof(red) >= kOrderBins * sizeof(int), "histogram");
+    varlen_order(P, reinterpret_cast<int*>(red));
+    return;
+  }
+  bid -= P.o_blocks;
   if (bid < P.s_blocks) {
     // ----------------------------------------------------------------------------- K channel-sum role
     const int chunk = bid % P.chunks, bh = bid / P.chunks, b = bh / P.Hkv, h = bh % P.Hkv;
@@ -407,7 +465,9 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   P.k_blocks = a.k && a.k_codes ? a.B * a.Hkv * P.Tk : 0;
   const int tpb = a.D == 128 ? 1 : 2;
   P.v_blocks = a.v ? (int)(((int64_t)a.B * a.Hkv * P.Tk + tpb - 1) / tpb) : 0;
-  const int grid = P.s_blocks + P.q_blocks + P.k_blocks + P.v_blocks;
+  P.order = a.order; P.n_order = a.n_order; P.causal = a.causal;
+  P.o_blocks = a.order != nullptr ? 1 : 0;
+  const int grid = P.o_blocks + P.s_blocks + P.q_blocks + P.k_blocks + P.v_blocks;
   if (grid == 0) return cudaSuccess;
   if (a.D == 128) quant_qkv_kernel<128><<<grid, kThreads, 0, stream>>>(P);
   else            quant_qkv_kernel<64><<<grid, kThreads, 0, stream>>>(P);

@@ -50,3 +50,21 @@ def test_k_means_and_delta_s_of_the_operator(B, Hq, Hkv, Nq, Nk, D):
     assert torch.allclose(z.delta_s[..., :Nk].float(), want, atol=2e-2 * float(want.abs().max()), rtol=1e-2)
     assert (z.delta_s[..., Nk:] == 0).all()
     assert torch.equal(sa.sageattn(q, k, v, check_status=True), sa.fp4_attention(z))
+
+
+# the work order of variable-length batches: more entries than threads and than SMs, sequences of no and one query, one
+# tile, two and three; and one sequence alone
+@pytest.mark.parametrize("n,causal,D", [(300, True, 128), (300, False, 64), (1, True, 64)])
+def test_varlen_work_order_reaches_every_query_tile(n, causal, D):
+    lens = [(0, 1, 128, 129, 256, 257, 385)[(5 * i + 3) % 7] for i in range(n)]
+    g = torch.Generator().manual_seed(n)
+    q, k, v = (torch.randn(sum(lens), h, D, generator=g).to(torch.bfloat16).to(DEV) for h in (4, 2, 2))
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    out = sa.sageattn_varlen(q, k, v, cu, cu, max(lens), max(lens), is_causal=causal, check_status=True)
+    for i in range(n):
+        s = slice(int(cu[i]), int(cu[i + 1]))
+        if lens[i] > 0 and (i < 14 or i > n - 8):
+            one = sa.sageattn(q[s][None], k[s][None], v[s][None], tensor_layout="NHD", is_causal=causal)[0]
+            cos, l1 = sage3.accuracy(out[s].float().cpu(), one.float().cpu())
+            assert cos >= 0.9995 and l1 <= 2e-2, (i, lens[i], cos, l1)
+    assert torch.isfinite(out).all() and (out.float().abs().amax(dim=(1, 2)) > 0).all()
