@@ -163,6 +163,7 @@ struct KParams {
   int* status;
   int64_t o_sb, o_sh, o_sn;
   int B, Hq, Hkv, Nq, Nk, Tq, Tk, ds_rows;
+  int list_tiles;        // kList: query tiles of the heads of a kv head
   float scale_log2;      // sm_scale * log2(e)
   const float* lam;      // K-packing mode: lambda per key slot, fp32 [B,Hkv,Tk*128]; Nk is the packed length
   int Nk_log;            // number of key tokens (= Nk unless packed)
@@ -301,9 +302,11 @@ __device__ __forceinline__ int packed_len_of(const int len) {
   return len <= 0 ? 0 : (len / 15) * 16 + (len % 15 == 0 ? 0 : len % 15 + 1);
 }
 
-// One unit of work of a CTA: two adjacent query tiles of one head.
+// One unit of work of a CTA: two adjacent query tiles of one head - or, in the kList kernels, of the list of all query
+// tiles of the heads that share a kv head: with an odd number of tiles every head would have an item of a single tile,
+// which costs three quarters of a full one.
 struct Work {
-  int b, hq, hkv, pair;
+  int b, hq, hkv, pair;  // (kList: hq = first head of the list, pair = place in it)
 #if SAGE3_VARLEN_BUILD
   int Nq, Nk;            // lengths of this item's sequence
   int q_base;            // first token of the sequence in the packed output
@@ -320,17 +323,33 @@ __device__ __forceinline__ int work_at(const int r, const int total) {
   return w < total ? w : -1;
 }
 
-template <bool kCausal, bool kPacked>
+// head and query tile (>= Tq: there is none) of tile t of a work item
+template <bool kList>
+__device__ __forceinline__ int head_of(const KParams& P, const Work& k, const int t) {
+  return kList ? k.hq + (2 * k.pair + t) / P.Tq : k.hq;
+}
+template <bool kList>
+__device__ __forceinline__ int tile_of(const KParams& P, const Work& k, const int t) {
+  const int u = 2 * k.pair + t;
+  if (!kList) return u;
+  return u < P.list_tiles ? u % P.Tq : P.Tq;
+}
+
+template <bool kCausal, bool kPacked, bool kList>
 __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
   Work k;
-  const int n_pairs = (P.Tq + 1) >> 1;
+  const int n_pairs = ((kList ? P.list_tiles : P.Tq) + 1) >> 1;
   int bh;
 #if SAGE3_VARLEN_BUILD
   const int entry = P.order[w / P.Hq];
   k.pair = entry % n_pairs;
   bh = entry / n_pairs * P.Hq + w % P.Hq;
 #else
-  if (kCausal) {
+  if (kList) {
+    // equal cost, as below
+    k.pair = n_pairs - 1 - (w % n_pairs);
+    bh = w / n_pairs * (P.Hq / P.Hkv);
+  } else if (kCausal) {
     // item cost grows with the pair index: heaviest pairs of all heads first, so that the rounds of
     // the static schedule hand out work of falling, nearly equal cost
     const int n_bh = P.B * P.Hq;
@@ -369,7 +388,7 @@ __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
 #else
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int qt = 2 * k.pair + t;
+    const int qt = tile_of<kList>(P, k, t);
     int n = 0;
     if (qt < P.Tq) {
       n = P.Tk;
@@ -387,7 +406,7 @@ __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
   return k;
 }
 
-template <int D, bool kCausal, bool kPacked>
+template <int D, bool kCausal, bool kPacked, bool kList>
 __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                                    const __grid_constant__ CUtensorMap tm_k,
                                                                    const __grid_constant__ CUtensorMap tm_v,
@@ -405,6 +424,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   volatile int* abort_s = reinterpret_cast<volatile int*>(smem + L::bars + Bars::abort_flag);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool has_ds = P.ds != nullptr;
+#if !SAGE3_VARLEN_BUILD
+  const int total_work = kList ? P.B * P.Hkv * ((P.list_tiles + 1) >> 1) : P.B * P.Hq * ((P.Tq + 1) >> 1);
+#endif
 
   if (threadIdx.x == 0) {
     for (int t = 0; t < 2; ++t) {
@@ -459,8 +481,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   const bool run = *reinterpret_cast<volatile int*>(smem + L::bars + Bars::run_flag) != 0;
 #if SAGE3_VARLEN_BUILD
   const int total_work = *P.n_order * P.Hq;
-#else
-  const int total_work = P.B * P.Hq * ((P.Tq + 1) >> 1);
 #endif
   // The CTA is persistent: every role walks the same static list of work items (blockIdx.x, +gridDim.x, ...)
   // and all barrier phases simply keep counting across items, so the loads, MMAs and softmax of the
@@ -477,12 +497,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         bool ok = true;
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
           int64_t ds_row[2];
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             const int qt = 2 * wk.pair + t;
-            ds_row[t] = ((int64_t)wk.b * P.Hq + wk.hq) * P.ds_rows + (P.ds_rows == 1 ? 0 : qt);
+            if (kList) ds_row[t] = ((int64_t)wk.b * P.Hq + head_of<kList>(P, wk, t)) * P.ds_rows + (P.ds_rows == 1 ? 0 : tile_of<kList>(P, wk, t));
+            else ds_row[t] = ((int64_t)wk.b * P.Hq + wk.hq) * P.ds_rows + (P.ds_rows == 1 ? 0 : qt);
             if (ok && wk.n_t[t] > 0) {
               // the slot's previous Q tile must have been read by its last QK MMA
               if (qn[t] > 0 && !(ok = wait_bar<false>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1, abort_s, P.status, 12))) break;
@@ -546,7 +567,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         bool ok = true;
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
@@ -585,7 +606,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t qn[2] = {0, 0};              // Q tiles taken so far per slot
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
@@ -651,7 +672,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t g = 0, pv_cnt[2] = {0, 0};
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
@@ -711,12 +732,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t items = 0;
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
           const int n_mine = t == 0 ? wk.n_t[0] : wk.n_t[1];
           const uint32_t g_first = g0 + (uint32_t)(wk.n_max - n_mine);   // stage counter of this tile's first key tile
           g0 += (uint32_t)wk.n_max;
           if (n_mine == 0) continue;
-          const int q0 = (2 * wk.pair + t) * kBlockM, qpos = q0 + row;
+          const int q0 = tile_of<kList>(P, wk, t) * kBlockM, qpos = q0 + row;
           // last visible key (slot): key padding, and the bottom-right aligned causal diagonal - in K-packing mode
           // the slots of the tokens up to the diagonal one
           auto causal_limit = [&](const int qp) {
@@ -810,7 +831,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t sc[2] = {0, 0}, items[2] = {0, 0};              // key tiles / work items so far per query tile slot
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
-          const Work wk = get_work<kCausal, kPacked>(P, w);
+          const Work wk = get_work<kCausal, kPacked, kList>(P, w);
           // O_t *= alpha for the rows whose maximum moved, in place in tensor memory, between the P.V of the previous
           // key tile and that of this one; warps in which no row's maximum moved skip it.  The first key tile of an
           // item overwrites O_t: this arrival then says that the previous item's output has been read.
@@ -860,14 +881,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll 1
           for (int t = 0; t < 2; ++t) {
             const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
-            const int qt = 2 * wk.pair + t, q0 = qt * kBlockM, qpos = q0 + row;
+            const int hq = head_of<kList>(P, wk, t), qt = tile_of<kList>(P, wk, t), q0 = qt * kBlockM, qpos = q0 + row;
             const bool live = SEQ_TILE_EXISTS && qpos < SEQ_NQ;
 #if SAGE3_VARLEN_BUILD
-            __nv_bfloat16* orow = P.out + wk.hq * P.o_sh + (int64_t)(wk.q_base + qpos) * P.o_sn;   // packed output
+            __nv_bfloat16* orow = P.out + hq * P.o_sh + (int64_t)(wk.q_base + qpos) * P.o_sn;   // packed output
 #else
-            __nv_bfloat16* orow = P.out + wk.b * P.o_sb + wk.hq * P.o_sh + (int64_t)qpos * P.o_sn;
+            __nv_bfloat16* orow = P.out + wk.b * P.o_sb + hq * P.o_sh + (int64_t)qpos * P.o_sn;
 #endif
-            const int64_t li = ((int64_t)wk.b * P.Hq + wk.hq) * P.Nq + qpos;
+            const int64_t li = ((int64_t)wk.b * P.Hq + hq) * P.Nq + qpos;
             if (n_t == 0) {
               // query tile that sees no key at all (causal, more queries than keys): zeros, like the
               // reference's store_zero (fwd_epilogue.cu:150-183); nothing if the tile does not exist
@@ -932,7 +953,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
                 for (int hcol = 0; hcol < D / 64; ++hcol)
                   if (64 * hcol < P.d_out)
                     tma_store_4d(&tm_o, sbase + stage_off + hcol * L::kOStage, 64 * hcol,
-                                 P.o_token_first ? n_row : wk.hq, P.o_token_first ? wk.hq : n_row, wk.b);
+                                 P.o_token_first ? n_row : hq, P.o_token_first ? hq : n_row, wk.b);
                 bulk_commit_group();
               }
             }
@@ -1001,7 +1022,7 @@ bool make_out_map(CUtensorMap* m, const void* base, int B, int H, int N, int D, 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int D, bool kCausal, bool kPacked>
+template <int D, bool kCausal, bool kPacked, bool kList>
 cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   using L = Smem<D>;
   const int Tq = (a.Nq + 127) / 128, Tk = (a.Nk + 127) / 128;
@@ -1023,6 +1044,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.o_sb = a.o_sb; P.o_sh = a.o_sh; P.o_sn = a.o_sn;
   P.B = a.B; P.Hq = a.Hq; P.Hkv = a.Hkv; P.Nq = a.Nq; P.Nk = a.Nk; P.Tq = Tq; P.Tk = Tk; P.ds_rows = a.ds_rows;
   P.scale_log2 = a.sm_scale * kLog2e;
+  P.list_tiles = a.Hq / a.Hkv * Tq;
   P.o_token_first = o_ndim == 1;
   P.lam = a.k_lambda;
   P.slot_first = kPacked && a.slot_first != 0;
@@ -1033,7 +1055,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.cu_q = a.cu_q; P.cu_k = a.cu_k;
   P.order = a.order; P.n_order = a.n_order;
 #endif
-  auto kern = attn_fwd_kernel<D, kCausal, kPacked>;
+  auto kern = attn_fwd_kernel<D, kCausal, kPacked, kList>;
   // persistent CTAs: one per SM (registers and tensor memory allow exactly one), each walks the work list
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1050,7 +1072,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total + 1024)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], sms, __ATOMIC_RELEASE);
   }
-  const int64_t work = (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
+  const int64_t work = kList ? (int64_t)a.B * a.Hkv * ((P.list_tiles + 1) / 2) : (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
   const int64_t ctas = sms - a.sm_margin > 1 ? sms - a.sm_margin : 1;
   const int64_t grid = work < ctas ? work : ctas;
   return launch_pdl(kern, dim3((unsigned)grid), kAttnThreads, L::total + 1024, stream, a.after_delta_s, tq, tk, tv, to, P);
@@ -1062,19 +1084,27 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
 cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream) {
   // offsets come in pairs; no K-packing and no LSE for packed batches
   if (a.cu_q == nullptr || a.cu_k == nullptr || a.order == nullptr || a.n_order == nullptr || a.k_lambda != nullptr || a.lse != nullptr) return cudaErrorInvalidValue;
-  if (a.D == 128) return a.causal ? launch<128, true, false>(a, stream) : launch<128, false, false>(a, stream);
-  if (a.D == 64) return a.causal ? launch<64, true, false>(a, stream) : launch<64, false, false>(a, stream);
+  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, stream) : launch<128, false, false, false>(a, stream);
+  if (a.D == 64) return a.causal ? launch<64, true, false, false>(a, stream) : launch<64, false, false, false>(a, stream);
   return cudaErrorInvalidValue;
 }
 #else
 cudaError_t launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
   if (a.D != 128 && a.D != 64) return cudaErrorInvalidValue;
   if (a.k_lambda) {
-    if (a.D == 128) return a.causal ? launch<128, true, true>(a, stream) : launch<128, false, true>(a, stream);
-    return a.causal ? launch<64, true, true>(a, stream) : launch<64, false, true>(a, stream);
+    if (a.D == 128) return a.causal ? launch<128, true, true, false>(a, stream) : launch<128, false, true, false>(a, stream);
+    return a.causal ? launch<64, true, true, false>(a, stream) : launch<64, false, true, false>(a, stream);
   }
-  if (a.D == 128) return a.causal ? launch<128, true, false>(a, stream) : launch<128, false, false>(a, stream);
-  return a.causal ? launch<64, true, false>(a, stream) : launch<64, false, false>(a, stream);
+  // Query tiles paired across the heads of a GQA group: where every head has an odd number of them, and the two of a pair
+  // visit the same keys - one tile per head (decoding: B8 Hq32 Hkv8 Nk4096, 84 -> 62 us), or no causal mask.  (Kernels of
+  // their own: the index arithmetic in the common ones cost those up to 5 %.)
+  const int Tq = (a.Nq + 127) / 128;
+  if (a.Hq > a.Hkv && (Tq & 1) && (Tq == 1 || !a.causal)) {
+    if (a.D == 128) return a.causal ? launch<128, true, false, true>(a, stream) : launch<128, false, false, true>(a, stream);
+    return a.causal ? launch<64, true, false, true>(a, stream) : launch<64, false, false, true>(a, stream);
+  }
+  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, stream) : launch<128, false, false, false>(a, stream);
+  return a.causal ? launch<64, true, false, false>(a, stream) : launch<64, false, false, false>(a, stream);
 }
 
 #endif
