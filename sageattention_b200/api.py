@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import math
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
@@ -445,25 +446,30 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
 _host_streams = {}
 
 
-_HOST_PIECE_BYTES = 24 << 20      # of q, k, v: 0.4 ms of copying, which hides the host work of a piece's calls
+def _host_piece_bytes(total: int) -> int:
+    """How much of q, k, v a piece carries: filling and draining the pipeline costs in proportion to it, the gaps between
+    copies and kernels in inverse proportion, so the best size grows with the root of the whole.  Measured best for 25 /
+    100 / 201 / 403 MB: 12 / 24 - 36 / 36 / 48 MB; less than 12 MB never paid."""
+    return max(12 << 20, int(math.sqrt(total * 6e6)))
 
 
 def _host_pieces(B: int, Hkv: int, head_bytes: int, head_chunks) -> list:
     """Pieces (first, last + 1 batch entry, first, last + 1 kv head) in which a host tensor goes through the GPU, each
-    contiguous in host memory: some heads of one batch entry, or some whole batch entries.  They carry about
-    ``_HOST_PIECE_BYTES``; where that is several heads, sizes ramp up from one head at the start and down to one at the
+    contiguous in host memory: some heads of one batch entry, or some whole batch entries.  Several heads at a time
+    ramp up from one head at the start and down to one at the
     end, so that the first kernel starts after a small copy and little is left to copy out after the last."""
+    want = _host_piece_bytes(B * Hkv * head_bytes)
     if isinstance(head_chunks, (list, tuple)):
         sizes = [int(n) for n in head_chunks]                    # explicit group sizes (kv heads per group)
         if sum(sizes) != Hkv or min(sizes) < 1:
             raise ValueError(f"head_chunks {sizes} must be positive and add up to the {Hkv} kv heads")
         plan = [sizes] * B
     else:
-        entries = _HOST_PIECE_BYTES // max(1, Hkv * head_bytes)
+        entries = want // max(1, Hkv * head_bytes)
         if entries >= 1 or int(head_chunks) <= 1:
             n = max(1, entries)
             return [(b, min(b + n, B), 0, Hkv) for b in range(0, B, n)]
-        base = max(1, _HOST_PIECE_BYTES // head_bytes)
+        base = max(1, round(want / head_bytes))
         ramp = [n for n in (1, 2, 4) if n < base]
         plan = []
         for b in range(B):
