@@ -224,6 +224,13 @@ SAGE3_API int sage3_attention_varlen(const sage3_varlen_args* args, void* stream
 SAGE3_API int sage3_packed_rows(int nk);   /* 16 * ceil(nk / 15): rows of the packed tensors                */
 SAGE3_API int sage3_packed_len(int nk);    /* occupied slots: 16 per full group, tokens + 1 for a partial one */
 SAGE3_API int sage3_pack_kv(const sage3_pack_args* args, void* stream);
+/* The whole K-packing operator in one call, from raw tokens: K is packed inside the K kernel and V on its way through the
+ * quantiser, so no packed tensors are written.  args: shape (Nk = key tokens), strides of q, k, v and out, sm_scale,
+ * is_causal, per_block_mean (0 or 1) and workspace_bytes are used; split_first and mean_slot_first as above. */
+SAGE3_API int sage3_attention_packed_workspace(const sage3_shape* shape, int per_block_mean, size_t* bytes);
+SAGE3_API int sage3_attention_packed_run(const sage3_fwd_args* args, int split_first, int mean_slot_first, const void* q,
+                                         const void* k, const void* v, void* out, void* workspace, int32_t* device_status,
+                                         void* stream);
 SAGE3_API int sage3_attn_fwd_packed(const sage3_attn_args* args, const float* k_lambda, int32_t mean_slot_first,
                                     void* stream);
 

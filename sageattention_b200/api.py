@@ -251,7 +251,6 @@ def sageattn4_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
     (``fwd_mainloop.cu:878-888``): True = per-128-token Q mean, the mean slot is masked out; False =
     whole-sequence Q mean, the mean slot takes the first token's score.  ``v_trick`` (default
     ``not per_block_mean``, ``api.py:180-181``) selects the split-first V layout.  ``quant_block`` must be 16."""
-    lib = _lib.load()
     if attn_mask is not None:
         raise NotImplementedError("attn_mask is not supported (the reference ignores it, api.py:250)")
     if quant_block != 16:
@@ -260,16 +259,26 @@ def sageattn4_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
         raise ValueError(f"Unsupported Headdim {q.shape[-1]}")
     if v_trick is None:
         v_trick = not per_block_mean
-    kp, vp, lam, _ = pack_kv(k, v, tensor_layout, smooth_k=True, split_first=bool(v_trick))
-    if tensor_layout == "NHD":
-        kp, vp = kp.transpose(1, 2), vp.transpose(1, 2)          # views; the quantiser takes strides
-    qz = quantize_qkv(q, kp, vp, tensor_layout, per_block_mean=bool(per_block_mean), smooth_k=False)
-    qz.k_lambda = lam
-    qz.mean_slot_first = not per_block_mean
-    Nk = k.shape[2] if tensor_layout == "HND" else k.shape[1]
-    qz.nk_slots = lib.sage3_packed_len(Nk)
-    return fp4_attention(qz, sm_scale=sm_scale, is_causal=is_causal, tensor_layout=tensor_layout,
-                         check_status=check_status)
+    if sm_scale is not None:
+        sm_scale = float(sm_scale)
+    key = ("packed", q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.device,
+           tensor_layout, bool(is_causal), sm_scale, bool(per_block_mean))
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _keep_plan(key, _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, True, 0, packed=True))
+    dev = plan.device
+    out = torch.empty_like(q)
+    ws = torch.empty(plan.workspace, dtype=torch.uint8, device=dev)
+    status = torch.empty(1, dtype=torch.int32, device=dev) if check_status else None
+    with _on_device(dev):
+        stream = _stream_ptr(dev)
+        st = plan.run(plan.args, int(bool(v_trick)), int(not per_block_mean), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                      ws.data_ptr(), None if status is None else status.data_ptr(), stream)
+        if st:
+            _lib.check(st, "sage3_attention_packed_run")
+        if check_status:
+            _lib.check(_lib.load().sage3_read_device_status(status.data_ptr(), stream, None), "attention kernel")
+    return out
 
 
 def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tensor_layout: str = "HND",
@@ -298,10 +307,7 @@ def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
            bool(is_causal), sm_scale, bool(per_block_mean), bool(smooth_k), sm_margin)
     plan = _plans.get(key)
     if plan is None:
-        plan = _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin)
-        if len(_plans) >= _MAX_PLANS:
-            _plans.clear()
-        _plans[key] = plan
+        plan = _keep_plan(key, _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin))
     if plan.pad:
         # head dims that are no multiple of 8 are padded here first, as the reference does (core.py:925-937, :990)
         d_og = q.shape[-1]
@@ -334,11 +340,18 @@ _MAX_PLANS = 1024
 _plans = {}
 
 
+def _keep_plan(key, plan):
+    if len(_plans) >= _MAX_PLANS:
+        _plans.clear()
+    _plans[key] = plan
+    return plan
+
+
 class _Plan:
     __slots__ = ("pad", "device", "workspace", "lse_shape", "struct", "args", "run")
 
 
-def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin) -> _Plan:
+def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin, packed=False) -> _Plan:
     lib = _lib.load()
     _check_device(q)
     for t in (q, k, v):
@@ -372,12 +385,17 @@ def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smoo
     a.km_out = None           # the K-mean term of the LSE is put back on the device (q . km in the quantisation kernel)
     a.sm_scale = float(sm_scale) if sm_scale is not None else 0.0
     a.is_causal, a.per_block_mean, a.smooth_k = int(bool(is_causal)), pbm, int(bool(smooth_k))
-    a.workspace_bytes = int(z.workspace)
+    workspace = int(z.workspace)
+    p.run = lib.sage3_attention_run
+    if packed:
+        n = C.c_size_t()
+        _lib.check(lib.sage3_attention_packed_workspace(C.byref(a.shape), pbm, C.byref(n)), "sage3_attention_packed_workspace")
+        workspace, p.run = n.value, lib.sage3_attention_packed_run
+    a.workspace_bytes = workspace
     a.head_dim = D if D != Dp else 0
     a.sm_margin = int(sm_margin)
     p.args = C.byref(a)
-    p.device, p.workspace, p.lse_shape = q.device, int(z.workspace), (B, Hq, Nq)
-    p.run = lib.sage3_attention_run
+    p.device, p.workspace, p.lse_shape = q.device, workspace, (B, Hq, Nq)
     return p
 
 

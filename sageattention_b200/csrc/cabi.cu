@@ -91,7 +91,8 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
 }
 
 static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int* cu_k, void* stream_,
-                          int* zero_status = nullptr, int* order = nullptr, int* n_order = nullptr, int causal = 0) {
+                          int* zero_status = nullptr, int* order = nullptr, int* n_order = nullptr, int causal = 0,
+                          float* k_lambda = nullptr, int split_first = 0) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (int st = check_tensor(a->q)) return st;
@@ -149,6 +150,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   q.km = km; q.partial = partial;
   q.zero_status = zero_status;
   q.order = order; q.n_order = n_order; q.causal = causal;
+  q.pack = k_lambda != nullptr; q.split_first = split_first != 0;
   q.q_mean_seq = a->per_block_mean == 0 ? a->qm : nullptr;
   q.qm_override = a->per_block_mean == 1 ? a->qm_in : nullptr;
   q.q_codes = a->q_codes; q.q_sf = a->q_sf; q.k_codes = k_in_ds ? nullptr : a->k_codes; q.k_sf = a->k_sf;
@@ -165,7 +167,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   if (a->delta_s != nullptr) {
     sage3::DeltaSArgs d{};
     d.qm = a->qm; d.k = a->k.ptr; d.k_sb = a->k.stride_b; d.k_sh = a->k.stride_h; d.k_sn = a->k.stride_n;
-    d.km = km; d.partial = partial; d.km_out = a->km; d.ds = a->delta_s; d.cu_k = cu_k; d.after_quant = true;
+    d.km = km; d.partial = partial; d.km_out = a->km; d.ds = a->delta_s; d.cu_k = cu_k; d.k_lambda = k_lambda; d.after_quant = true;
     d.k_codes = a->k_codes; d.k_sf = a->k_sf; d.status = a->device_status; d.d_in = a->head_dim_in;
     d.B = s.B; d.Hq = s.Hq; d.Hkv = s.Hkv; d.Tq = a->per_block_mean == 1 ? Tq : 1; d.Nk = s.Nk; d.D = s.D;
     e = sage3::launch_delta_s(d, stream);
@@ -319,6 +321,63 @@ int sage3_attention_run(const sage3_fwd_args* args, const void* q, const void* k
   a.q.ptr = q; a.k.ptr = k; a.v.ptr = v;
   a.out = out; a.lse = lse; a.workspace = workspace; a.device_status = device_status;
   return sage3_attention(&a, stream);
+}
+
+// Parts of the workspace of the K-packing operator: those of a problem with as many keys as there are slots, the scratch of
+// the token means and the lambdas
+static int packed_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes* z, size_t* lam, size_t* total) {
+  if (shape == nullptr || (per_block_mean != 0 && per_block_mean != 1)) return SAGE3_ERR_ARGUMENT;
+  sage3_shape s = *shape;
+  s.Nk = sage3_packed_rows(s.Nk);
+  if (int st = sage3_buffer_sizes(&s, per_block_mean, z)) return st;
+  const size_t sk = sage3::quant_scratch_bytes(s.B, s.Hkv, shape->Nk, s.D);
+  if (sk > z->scratch) { z->workspace += align256(sk) - align256(z->scratch); z->scratch = sk; }
+  *lam = (size_t)s.B * s.Hkv * ((s.Nk + 127) / 128) * 128 * sizeof(float);
+  *total = z->workspace + align256(*lam);
+  return SAGE3_OK;
+}
+
+int sage3_attention_packed_workspace(const sage3_shape* shape, int per_block_mean, size_t* bytes) {
+  sage3_sizes z;
+  size_t lam;
+  if (bytes == nullptr) return SAGE3_ERR_ARGUMENT;
+  return packed_sizes(shape, per_block_mean, &z, &lam, bytes);
+}
+
+int sage3_attention_packed_run(const sage3_fwd_args* a, int split_first, int mean_slot_first, const void* qp, const void* kp,
+                               const void* vp, void* out, void* workspace, int32_t* device_status, void* stream) {
+  if (a == nullptr || workspace == nullptr || out == nullptr || !qp || !kp || !vp) return SAGE3_ERR_ARGUMENT;
+  sage3_sizes z;
+  size_t lam_bytes, total;
+  if (int st = packed_sizes(&a->shape, a->per_block_mean, &z, &lam_bytes, &total)) return st;
+  if (a->workspace_bytes < total || (reinterpret_cast<uintptr_t>(workspace) & 255)) return SAGE3_ERR_ARGUMENT;
+  char* w = reinterpret_cast<char*>(workspace);
+  auto take = [&](size_t n) { char* p = w; w += align256(n); return (void*)p; };
+  sage3_quant_args q{};
+  q.shape = a->shape; q.q = a->q; q.k = a->k; q.v = a->v;
+  q.q.ptr = qp; q.k.ptr = kp; q.v.ptr = vp;
+  q.per_block_mean = a->per_block_mean; q.smooth_k = 1;
+  q.q_codes = take(z.q_codes); q.q_sf = take(z.q_sf); q.k_codes = take(z.k_codes); q.k_sf = take(z.k_sf);
+  q.vt_codes = take(z.vt_codes); q.vt_sf = take(z.vt_sf);
+  q.qm = take(z.qm);
+  q.km = take(z.km);
+  q.delta_s = take(z.delta_s);
+  q.scratch = take(z.scratch); q.scratch_bytes = z.scratch;
+  float* lam = reinterpret_cast<float*>(take(lam_bytes));
+  int32_t* status = reinterpret_cast<int32_t*>(take(4));
+  if (device_status) status = device_status;
+  q.device_status = status;
+  if (int st = quant_qkv_impl(&q, nullptr, nullptr, stream, status, nullptr, nullptr, 0, lam, split_first)) return st;
+  sage3_attn_args t{};
+  t.shape = a->shape;
+  t.shape.Nk = sage3_packed_len(a->shape.Nk);
+  t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;
+  t.delta_s = q.delta_s;
+  t.delta_s_rows = a->per_block_mean == 1 ? (a->shape.Nq + 127) / 128 : 1;
+  t.out = out; t.out_stride_b = a->out_stride_b; t.out_stride_h = a->out_stride_h; t.out_stride_n = a->out_stride_n;
+  t.sm_scale = a->sm_scale > 0.f ? a->sm_scale : 1.0f / sqrtf((float)a->shape.D);
+  t.is_causal = a->is_causal; t.device_status = status;
+  return attn_fwd_impl(&t, lam, nullptr, nullptr, stream, mean_slot_first != 0, /*zero_status=*/false, /*after_delta_s=*/true);
 }
 
 int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {

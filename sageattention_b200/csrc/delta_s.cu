@@ -22,6 +22,10 @@
 // want the next A tile on its way during the current one: it waits in registers, two CTAs per SM (B1 H40 N32760: 330 us;
 // 390 with three CTAs and no A ahead).
 //
+// kPack: K-packing mode (pack.cu) on the way in - a tile is 8 groups of 16 slots, its 120 tokens are smoothed, laid out
+// and turned into mean and residuals by one warp per group, in place in the operand tile; the lambdas leave from here.
+// (B4 H32 N2048 D128: a packing kernel in front, whose output this one and the V quantiser read back, took 111 us.)
+//
 // Operand layout in shared memory (K-major, no swizzle): 8-row x 16-byte core matrices; the 16 row groups of one
 // 8-channel chunk are contiguous (128 B apart), chunks are kChunk bytes apart - 16 bytes more than their size so
 // that the 16 lanes which write one row's chunks hit different banks.
@@ -31,6 +35,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "pack_group.cuh"
 #include "quant_rows.cuh"
 #include "tensor_map.h"
 
@@ -49,6 +54,7 @@ struct KDsParams {
   uint8_t *k_codes, *k_sf;                             // null: K is quantised elsewhere
   __nv_bfloat16* ds;
   int* status;                                         // optional device status word
+  float* lam;                                          // kPack: fp32 [B,Hkv,Tk*128]
   int Hkv, rows, Tk, Nk;                               // rows = query heads per kv head x query blocks per head
   const int* cu_k;
   int d_in;                                            // channels the K rows really have; the rest are zero
@@ -61,8 +67,8 @@ __host__ __device__ constexpr int ds_front_bytes(int D, bool multi) {
   return multi ? kDsStageBytes + a : (a > kDsStageBytes ? a : kDsStageBytes);
 }
 
-template <int D, bool kMulti>
-__global__ void __launch_bounds__(kThreads, kMulti ? 2 : 3) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
+template <int D, bool kMulti, bool kPack>
+__global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
                                                                       const KDsParams P) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   constexpr uint32_t kTileBytes = CH * kChunk;
@@ -88,11 +94,16 @@ __global__ void __launch_bounds__(kThreads, kMulti ? 2 : 3) k_quant_delta_s_kern
     }
   }
   const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + c * 8;
+  // token in slot `row` of the tile (kPack: 16 slots hold 15 tokens, none the first)
+  auto token_of = [&](const int row) {
+    if (!kPack) return tile * kTile + row;
+    return (row & 15) == 0 ? -1 : (tile * (kTile / 16) + (row >> 4)) * kGroup + (row & 15) - 1;
+  };
   uint4 w[NP];
 #pragma unroll
   for (int p = 0; p < NP; ++p) {                       // all loads in flight before the first use
-    const int n = tile * kTile + p * RPP + rl;
-    w[p] = (n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
+    const int n = token_of(p * RPP + rl);
+    w[p] = (n >= 0 && n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
   }
   if (t == 0) {
     mbar_init(bar, 1);
@@ -129,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, kMulti ? 2 : 3) k_quant_delta_s_kern
     __syncthreads();                                   // every thread has its means: sB takes the K tile
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      if (tile * kTile + p * RPP + rl < Nk) {          // padding rows stay zero (the reference subtracts before padding)
+      if (const int n = token_of(p * RPP + rl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
         w[p].x = pack_bf16(bf16_lo(w[p].x) - mean[0], bf16_hi(w[p].x) - mean[1]);
         w[p].y = pack_bf16(bf16_lo(w[p].y) - mean[2], bf16_hi(w[p].y) - mean[3]);
         w[p].z = pack_bf16(bf16_lo(w[p].z) - mean[4], bf16_hi(w[p].z) - mean[5]);
@@ -141,6 +152,37 @@ __global__ void __launch_bounds__(kThreads, kMulti ? 2 : 3) k_quant_delta_s_kern
   for (int p = 0; p < NP; ++p) {
     const int row = p * RPP + rl;
     *reinterpret_cast<uint4*>(sB + c * kChunk + (row >> 3) * 128 + (row & 7) * 16) = w[p];
+  }
+  if constexpr (kPack) {
+    // one warp per group: rows 16 warp ... +15 of the tile, lane l channels l*C ... (8-channel chunks of sB)
+    constexpr int C = D / 32;
+    __syncthreads();
+    uint8_t* grp = sB + (lane * C / 8) * kChunk + (lane * C % 8) * 2 + warp * 256;
+    auto at = [&](const int slot) { return grp + (slot >> 3) * 128 + (slot & 7) * 16; };
+    auto put = [&](const int slot, const float (&r)[C]) {
+      if constexpr (C == 4) *reinterpret_cast<uint2*>(at(slot)) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
+      else                  *reinterpret_cast<uint32_t*>(at(slot)) = pack_bf16(r[0], r[1]);
+    };
+    float x[kGroup][C], m[C];
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+      if constexpr (C == 4) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(at(j + 1));
+        x[j][0] = bf16_lo(raw.x); x[j][1] = bf16_hi(raw.x); x[j][2] = bf16_lo(raw.y); x[j][3] = bf16_hi(raw.y);
+      } else {
+        const uint32_t raw = *reinterpret_cast<const uint32_t*>(at(j + 1));
+        x[j][0] = bf16_lo(raw); x[j][1] = bf16_hi(raw);
+      }
+    }
+    const float my_lam = pack_group<C>(x, lane, m, [&](const int j, const float (&r)[C]) { put(j + 1, r); });
+    put(0, m);
+    if (lane < 16) P.lam[((int64_t)bh * P.Tk + tile) * kTile + warp * 16 + lane] = my_lam;
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int row = p * RPP + rl;
+      w[p] = *reinterpret_cast<const uint4*>(sB + c * kChunk + (row >> 3) * 128 + (row & 7) * 16);
+    }
   }
   if (P.k_codes != nullptr) {
     const int64_t kt = (int64_t)bh * P.Tk + tile;
@@ -240,7 +282,8 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   P.partial = (const float*)a.partial; P.km_out = (__nv_bfloat16*)a.km_out;
   int chunk_tokens;
   quant_chunks(a.B * a.Hkv, a.Nk, &P.chunks, &chunk_tokens);
-  P.Hkv = a.Hkv; P.rows = a.Hq / a.Hkv * a.Tq; P.Nk = a.Nk; P.Tk = (a.Nk + 127) / 128;
+  P.Hkv = a.Hkv; P.rows = a.Hq / a.Hkv * a.Tq; P.Nk = a.Nk; P.lam = a.k_lambda;
+  P.Tk = ((a.k_lambda ? (a.Nk + kGroup - 1) / kGroup * 16 : a.Nk) + 127) / 128;
   P.cu_k = a.cu_k;
   P.d_in = (a.d_in > 0 && a.d_in <= a.D) ? a.d_in : a.D;
   dim3 grid(P.Tk, a.B * a.Hkv);
@@ -260,13 +303,18 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   }
   const bool multi = P.rows > 128;
   const int smem = ds_front_bytes(a.D, multi) + (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
-  static std::atomic<unsigned long long> ready[4];      // per kernel: devices on which the shared memory was asked for
+  static std::atomic<unsigned long long> ready[8];      // per kernel: devices on which the shared memory was asked for
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  auto kern = a.D == 128 ? (multi ? k_quant_delta_s_kernel<128, true> : k_quant_delta_s_kernel<128, false>)
-                         : (multi ? k_quant_delta_s_kernel<64, true> : k_quant_delta_s_kernel<64, false>);
-  auto& done = ready[(a.D == 128 ? 2 : 0) + (multi ? 1 : 0)];
+  using Kern = void (*)(CUtensorMap, KDsParams);
+  static const Kern kerns[8] = {k_quant_delta_s_kernel<64, false, false>,  k_quant_delta_s_kernel<64, true, false>,
+                                k_quant_delta_s_kernel<128, false, false>, k_quant_delta_s_kernel<128, true, false>,
+                                k_quant_delta_s_kernel<64, false, true>,   k_quant_delta_s_kernel<64, true, true>,
+                                k_quant_delta_s_kernel<128, false, true>,  k_quant_delta_s_kernel<128, true, true>};
+  const int which = (a.k_lambda ? 4 : 0) + (a.D == 128 ? 2 : 0) + (multi ? 1 : 0);
+  const Kern kern = kerns[which];
+  auto& done = ready[which];
   const unsigned long long bit = 1ull << (dev & 63);
   if (dev >= 64 || !(done.load(std::memory_order_acquire) & bit)) {
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;

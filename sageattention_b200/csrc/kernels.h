@@ -28,6 +28,7 @@ struct QuantArgs {
   void* partial = nullptr;                // or fp32 scratch (quant_scratch_bytes): this launch only takes the partial sums
                                           //   of K, for launch_delta_s; both null: no K smoothing
   int* zero_status = nullptr;             // optional device word to zero
+  bool pack = false, split_first = false; // K-packing mode: V goes to slots (see pack.cu) as it is quantised; K elsewhere
   int* order = nullptr;                   // variable-length batches: receives the attention kernel's work order, at most
   int* n_order = nullptr;                 //   B * ceil(ceil(Nq / 128) / 2) entries, and their number (both or neither)
   int causal = 0;                         //   (what the work of an entry depends on)
@@ -78,6 +79,7 @@ struct DeltaSArgs {
   void* k_sf = nullptr;                   //   smoothed K tile it holds (the K role of the quantisation kernel)
   int* status = nullptr;                  // optional device status word for the kernel's bounded wait
   int d_in = 0;                           // as in QuantArgs
+  float* k_lambda = nullptr;              // K-packing mode: K (Nk tokens) is packed on the way in, lambdas go here
   bool after_quant = false;               // launched right behind launch_quant_qkv on the same stream: may overlap its end
 };
 cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream);

@@ -19,20 +19,13 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "pack_group.cuh"
 
 namespace sage3 {
 
 namespace {
 
 constexpr int kPackThreads = 256;
-constexpr int kGroup = 15;
-
-// magnitude of an E2M1 code: 0, 0.5, 1, 1.5, 2, 3, 4, 6 (sign in bit 3)
-__device__ __forceinline__ float e2m1_value(const uint32_t code) {
-  const uint32_t mag = code & 7u;
-  const float lvl = mag < 2 ? 0.5f * mag : (mag < 4 ? 1.0f + 0.5f * (mag - 2) : (mag < 6 ? 2.0f + (mag - 4) : (mag == 6 ? 4.0f : 6.0f)));
-  return (code & 8u) ? -lvl : lvl;
-}
 
 template <int D>
 __global__ void __launch_bounds__(kPackThreads) pack_kv_kernel(
@@ -41,7 +34,6 @@ __global__ void __launch_bounds__(kPackThreads) pack_kv_kernel(
     const __nv_bfloat16* __restrict__ km, __nv_bfloat16* __restrict__ kp, __nv_bfloat16* __restrict__ vp,
     float* __restrict__ lam, int H, int N, int G, int lam_len, int split_first) {
   constexpr int C = D / 32;                         // channels per lane (4 or 2)
-  constexpr int kLanesPerBlock = 16 / C;            // lanes that share one 16-channel scale block
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
@@ -60,9 +52,6 @@ __global__ void __launch_bounds__(kPackThreads) pack_kv_kernel(
     const int t0 = g * kGroup;
     // ---- load the 15 rows, centre them (bf16 arithmetic of `k - k.mean()`: fp32 subtract, round to bf16)
     float x[kGroup][C];
-    float sum[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) sum[c] = 0.f;
 #pragma unroll
     for (int j = 0; j < kGroup; ++j) {
       const int t = t0 + j;
@@ -80,68 +69,22 @@ __global__ void __launch_bounds__(kPackThreads) pack_kv_kernel(
 #pragma unroll
         for (int c = 0; c < C; ++c) x[j][c] = 0.f;
       }
-#pragma unroll
-      for (int c = 0; c < C; ++c) sum[c] += x[j][c];
     }
-    // ---- group mean -> bf16 -> block-scaled FP4 round trip along the head dimension (16-channel blocks)
-    float m[C];
-    float amax = 0.f;
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      m[c] = __bfloat162float(__float2bfloat16(__fdiv_rn(sum[c], (float)kGroup)));
-      amax = fmaxf(amax, fabsf(m[c]));
-    }
-#pragma unroll
-    for (int o = 1; o < kLanesPerBlock; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = e4m3_to_f32(f32_to_e4m3(__fdiv_rn(amax, 6.0f)));
-    const float inv = scale == 0.f ? 0.f : __frcp_rn(scale);
-    {
-      float sc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c = 0; c < C; ++c) sc[c] = __fmul_rn(m[c], inv);
-      // E2M1 round-to-nearest-even with saturation, then back to fp32 through the 8 magnitudes
-      uint32_t codes = f32x8_to_e2m1x8(sc[0], sc[1], sc[2], sc[3], 0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        m[c] = __bfloat162float(__float2bfloat16(__fmul_rn(e2m1_value((codes >> (4 * c)) & 0xFu), scale)));
-      }
-    }
-    // ---- direction = m / |m|^2
-    float nsq = 0.f;
-#pragma unroll
-    for (int c = 0; c < C; ++c) nsq = fmaf(m[c], m[c], nsq);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nsq += __shfl_xor_sync(0xffffffffu, nsq, o);
-    float dir[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) dir[c] = nsq > 0.f ? __fdiv_rn(m[c], nsq) : 0.f;
-
-    // ---- slot 0: the rounded mean
+    // ---- slots 1..15: residuals; slot 0: the rounded mean
     const int64_t row0 = (int64_t)g * 16;
-    if constexpr (C == 4) {
-      *reinterpret_cast<uint2*>(kpb + row0 * D) = make_uint2(pack_bf16(m[0], m[1]), pack_bf16(m[2], m[3]));
-    } else {
-      *reinterpret_cast<uint32_t*>(kpb + row0 * D) = pack_bf16(m[0], m[1]);
-    }
-    // ---- slots 1..15: lambda and residual
-    float my_lam = 0.f;                               // lane s keeps lambda of slot s
-#pragma unroll
-    for (int j = 0; j < kGroup; ++j) {
-      float dot = 0.f;
-#pragma unroll
-      for (int c = 0; c < C; ++c) dot = fmaf(x[j][c], dir[c], dot);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      if (lane == j + 1) my_lam = dot;
-      float r[C];
-#pragma unroll
-      for (int c = 0; c < C; ++c) r[c] = __fsub_rn(x[j][c], __fmul_rn(dot, m[c]));
+    float m[C];
+    const float my_lam = pack_group<C>(x, lane, m, [&](const int j, const float (&r)[C]) {
       const int64_t row = row0 + 1 + j;
       if constexpr (C == 4) {
         *reinterpret_cast<uint2*>(kpb + row * D) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
       } else {
         *reinterpret_cast<uint32_t*>(kpb + row * D) = pack_bf16(r[0], r[1]);
       }
+    });
+    if constexpr (C == 4) {
+      *reinterpret_cast<uint2*>(kpb + row0 * D) = make_uint2(pack_bf16(m[0], m[1]), pack_bf16(m[2], m[3]));
+    } else {
+      *reinterpret_cast<uint32_t*>(kpb + row0 * D) = pack_bf16(m[0], m[1]);
     }
     // ---- V: the 15 rows behind their slots; slot 0 zero, or (split first) the first row in two FP4 terms
     if (vpb) {
@@ -163,19 +106,12 @@ __global__ void __launch_bounds__(kPackThreads) pack_kv_kernel(
 #pragma unroll
       for (int c = 0; c < C; ++c) slot[c] = 0.f;
       if (split_first) {
-        // what scaled_fp4_quant_trans will make of the first row: one scale per channel over the group's 16 slots
-        // (slot 0 still zero), emulation arithmetic of api.py:77-110 (true division, round to nearest even)
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           float amax = 0.f;
 #pragma unroll
           for (int j = 0; j < kGroup; ++j) amax = fmaxf(amax, fabsf(vf[j][c]));
-          const float scale = e4m3_to_f32(f32_to_e4m3(__fdiv_rn(amax, 6.0f)));
-          const float inv = scale == 0.f ? 0.f : __frcp_rn(scale);
-          const uint32_t code = f32x8_to_e2m1x8(__fmul_rn(vf[0][c], inv), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f) & 0xFu;
-          const float hi = __bfloat162float(__float2bfloat16(__fmul_rn(e2m1_value(code), scale)));
-          slot[c] = __fsub_rn(vf[0][c], hi);
-          vf[0][c] = hi;
+          slot[c] = split_first_value(vf[0][c], amax);
         }
       }
       if constexpr (C == 4) {

@@ -25,6 +25,7 @@
 //   qm         : [T][D] bf16 block means of Q;  km : [D] bf16 channel means of K
 #include "common.cuh"
 #include "kernels.h"
+#include "pack_group.cuh"
 #include "quant_rows.cuh"
 
 namespace sage3 {
@@ -123,6 +124,7 @@ struct QuantLaunch {
   int s_blocks, chunks, chunk_tokens;    // CTAs of the K channel-sum role (0: none), chunks per head, tokens per chunk
   float* partial;                        // [B,Hkv,chunks,D] fp32 K channel sums, written by that role
   int* zero_status;                      // status word of the whole operator call, zeroed here (optional)
+  bool pack, split_first;                // K-packing mode: Nk tokens in Tk tiles of slots; V layout of its two variants
   int o_blocks, causal;                  // 1: the work-order role of a variable-length batch runs
   int *order, *n_order;                  // its result: (sequence, pair of query tiles) entries and their number
   float* q_dot_km;                       // optional fp32 [B,Hq,Nq]: raw q . K channel mean of the row's kv head
@@ -348,15 +350,17 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   __syncthreads();
   const int tile = (int)(gt % P.Tk), bh = (int)(gt / P.Tk), b = bh / P.Hkv, h = bh % P.Hkv;
   const int Nv = P.cu_k && gt < total ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
-  if (gt < total && tile * kTile < Nv) {                  // (nothing reads a V tile beyond its sequence)
+  if (gt < total && (P.pack || tile * kTile < Nv)) {      // (nothing reads a V tile beyond its sequence)
     const int c4 = (warp % WPT) * 4 + (lane >> 3);        // group of 4 channels
     const int blk = lane & 7;                              // 16-token block
     const __nv_bfloat16* src = P.v + (P.cu_k ? (int64_t)P.cu_k[b] * P.v_sn : b * P.v_sb) + h * P.v_sh + c4 * 4;
+    // K-packing mode: a block is a group, 15 tokens behind an empty slot
+    const int n0 = P.pack ? (tile * 8 + blk) * kGroup - 1 : tile * kTile + blk * 16;
     uint2 x[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const int n = tile * kTile + blk * 16 + i;
-      x[i] = (n < Nv && c4 * 4 < P.d_in) ? *reinterpret_cast<const uint2*>(src + (int64_t)n * P.v_sn) : make_uint2(0, 0);
+      const int n = n0 + i;
+      x[i] = (n < Nv && c4 * 4 < P.d_in && !(P.pack && i == 0)) ? *reinterpret_cast<const uint2*>(src + (int64_t)n * P.v_sn) : make_uint2(0, 0);
     }
     uint8_t* codes = P.vt_codes + gt * (D * 64);
 #pragma unroll
@@ -370,6 +374,12 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       float amax = 0.f;
 #pragma unroll
       for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
+      if (P.split_first) {
+        f[0] = __bfloat162float(__float2bfloat16_rn(split_first_value(f[1], amax)));
+        amax = fmaxf(fabsf(f[0]), fabsf(f[1]));
+#pragma unroll
+        for (int i = 2; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
+      }
       uint32_t sfb; float inv;
       block_scale(amax, sfb, inv);
       uint2 o;
@@ -445,7 +455,8 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   P.k_sb = a.k_sb; P.k_sh = a.k_sh; P.k_sn = a.k_sn;
   P.v_sb = a.v_sb; P.v_sh = a.v_sh; P.v_sn = a.v_sn;
   P.B = a.B; P.Hq = a.Hq; P.Hkv = a.Hkv; P.Nq = a.Nq; P.Nk = a.Nk;
-  P.Tq = (a.Nq + kTile - 1) / kTile; P.Tk = (a.Nk + kTile - 1) / kTile;
+  P.Tq = (a.Nq + kTile - 1) / kTile; P.pack = a.pack; P.split_first = a.pack && a.split_first;
+  P.Tk = ((a.pack ? (a.Nk + kGroup - 1) / kGroup * 16 : a.Nk) + kTile - 1) / kTile;
   P.q_mean_mode = a.q_mean_mode;
   P.km = (const __nv_bfloat16*)a.km; P.q_mean_seq = (const __nv_bfloat16*)a.q_mean_seq;
   P.qm_override = (const float*)a.qm_override;

@@ -68,3 +68,19 @@ def test_varlen_work_order_reaches_every_query_tile(n, causal, D):
             cos, l1 = sage3.accuracy(out[s].float().cpu(), one.float().cpu())
             assert cos >= 0.9995 and l1 <= 2e-2, (i, lens[i], cos, l1)
     assert torch.isfinite(out).all() and (out.float().abs().amax(dim=(1, 2)) > 0).all()
+
+
+# the K-packing operator packs on the way into the quantisers: bit for bit what pack_kv + quantize_qkv + fp4_attention give;
+# part of a group, one group, a whole tile of groups and one token more, several rounds of query blocks in the K kernel
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,causal,pbm,layout", [
+    (1, 2, 2, 40, 1, 128, False, True, "HND"), (2, 4, 2, 130, 15, 64, False, False, "NHD"), (1, 4, 2, 300, 120, 128, True, True, "HND"),
+    (2, 2, 2, 257, 121, 64, True, False, "HND"), (1, 8, 1, 2200, 2200, 128, True, True, "NHD"), (1, 8, 1, 2200, 1000, 64, False, False, "NHD")])
+def test_packing_operator_equals_its_parts(B, Hq, Hkv, Nq, Nk, D, causal, pbm, layout):
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, D, seed=Nq + Nk, layout=layout, device=DEV)
+    got = sa.sageattn4_blackwell(q, k, v, tensor_layout=layout, is_causal=causal, per_block_mean=pbm, check_status=True)
+    kp, vp, lam, _ = sa.pack_kv(k, v, layout, split_first=not pbm)
+    if layout == "NHD":
+        kp, vp = kp.transpose(1, 2), vp.transpose(1, 2)
+    z = sa.quantize_qkv(q, kp, vp, layout, per_block_mean=pbm, smooth_k=False)
+    z.k_lambda, z.mean_slot_first, z.nk_slots = lam, not pbm, sa._lib.load().sage3_packed_len(Nk)
+    assert torch.equal(got, sa.fp4_attention(z, is_causal=causal, tensor_layout=layout))
