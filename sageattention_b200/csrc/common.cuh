@@ -25,10 +25,27 @@ __device__ __forceinline__ float rcp_approx_ftz(float a) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
-__device__ __forceinline__ float mul_ftz(float a, float b) {
-  float r;
-  asm("mul.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
+// packed fp32x2 arithmetic: one issue slot for two elements, each rounded as by the scalar instruction
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2_ftz(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
 }
 __device__ __forceinline__ float ex2_approx(float a) {
   float r;
@@ -75,9 +92,20 @@ __device__ __forceinline__ uint32_t f32x8_to_e2m1x8(float a0, float a1, float a2
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+__device__ __forceinline__ float2 bf16x2_to_f32(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)); }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&p);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float2 v) { return pack_bf16(v.x, v.y); }
+// x - mean in fp32, rounded to bf16 (what a bf16 tensor subtraction does), for 8 channels; neg = -mean
+__device__ __forceinline__ uint4 subtract_mean(const uint4& w, const float2 (&neg)[4]) {
+  return make_uint4(pack_bf16(fadd2(bf16x2_to_f32(w.x), neg[0])), pack_bf16(fadd2(bf16x2_to_f32(w.y), neg[1])),
+                    pack_bf16(fadd2(bf16x2_to_f32(w.z), neg[2])), pack_bf16(fadd2(bf16x2_to_f32(w.w), neg[3])));
+}
+__device__ __forceinline__ void add_channels(float2 (&acc)[4], const uint4& w) {
+  acc[0] = fadd2(acc[0], bf16x2_to_f32(w.x)); acc[1] = fadd2(acc[1], bf16x2_to_f32(w.y));
+  acc[2] = fadd2(acc[2], bf16x2_to_f32(w.z)); acc[3] = fadd2(acc[3], bf16x2_to_f32(w.w));
 }
 __device__ __forceinline__ uint32_t habsmax2(uint32_t a, uint32_t b) {   // per-half max(|a|,|b|)
   __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&a);

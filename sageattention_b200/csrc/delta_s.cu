@@ -138,13 +138,11 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     k_mean<D>(P.km, P.partial + (int64_t)bh * P.chunks * D, P.chunks, (float)max(Nk, 1), bh, reinterpret_cast<float*>(sB),
               tile == 0 ? P.km_out : nullptr, mean);
     __syncthreads();                                   // every thread has its means: sB takes the K tile
+    const float2 neg[4] = {{-mean[0], -mean[1]}, {-mean[2], -mean[3]}, {-mean[4], -mean[5]}, {-mean[6], -mean[7]}};
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       if (const int n = token_of(p * RPP + rl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
-        w[p].x = pack_bf16(bf16_lo(w[p].x) - mean[0], bf16_hi(w[p].x) - mean[1]);
-        w[p].y = pack_bf16(bf16_lo(w[p].y) - mean[2], bf16_hi(w[p].y) - mean[3]);
-        w[p].z = pack_bf16(bf16_lo(w[p].z) - mean[4], bf16_hi(w[p].z) - mean[5]);
-        w[p].w = pack_bf16(bf16_lo(w[p].w) - mean[6], bf16_hi(w[p].w) - mean[7]);
+        w[p] = subtract_mean(w[p], neg);
       }
     }
   }

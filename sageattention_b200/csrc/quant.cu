@@ -45,7 +45,7 @@ __device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict_
   base += c * 8;
   const int n0 = chunk * chunk_tokens;
   const int n1 = min(N, n0 + chunk_tokens);
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  float2 acc[4] = {};
   for (int n = n0 + rl; n < n1; n += RPP * 4) {
     uint4 v[4];
 #pragma unroll
@@ -54,15 +54,10 @@ __device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict_
       v[u] = (nn < n1 && c * 8 < d_in) ? *reinterpret_cast<const uint4*>(base + (int64_t)nn * sn) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      acc[0] += bf16_lo(v[u].x); acc[1] += bf16_hi(v[u].x);
-      acc[2] += bf16_lo(v[u].y); acc[3] += bf16_hi(v[u].y);
-      acc[4] += bf16_lo(v[u].z); acc[5] += bf16_hi(v[u].z);
-      acc[6] += bf16_lo(v[u].w); acc[7] += bf16_hi(v[u].w);
-    }
+    for (int u = 0; u < 4; ++u) add_channels(acc, v[u]);
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) red[rl * D + c * 8 + i] = acc[i];
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(red + rl * D + c * 8 + 2 * i) = acc[i];
   __syncthreads();
   if (t < D) {
     float s = 0.f;
@@ -80,7 +75,7 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
     int chunk_tokens, float divisor, float* __restrict__ partial, unsigned int* __restrict__ counters,
     __nv_bfloat16* __restrict__ mean_out, const int* __restrict__ cu, int d_in) {
-  __shared__ float red[(kThreads / (D / 8)) * D];
+  __shared__ __align__(16) float red[(kThreads / (D / 8)) * D];
   __shared__ bool is_last;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const int chunk = blockIdx.x, nchunks = gridDim.x, t = threadIdx.x;
@@ -187,7 +182,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunch P) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   __shared__ __align__(16) uint8_t sf_smem[2048];
-  __shared__ float red[RPP * D];
+  __shared__ __align__(16) float red[RPP * D];
   __shared__ float mean_s[D];
   const int t = threadIdx.x, c = t % CH, rl = t / CH;
   int bid = blockIdx.x;
@@ -263,14 +258,12 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
         for (int i = 0; i < 8; ++i) mean[i] = mp[i];
       } else {
         // fp32 column sums over the tile's 128 rows (zero rows of the padding included), / 128
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        float2 acc2[4] = {};
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          acc[0] += bf16_lo(w[p].x); acc[1] += bf16_hi(w[p].x);
-          acc[2] += bf16_lo(w[p].y); acc[3] += bf16_hi(w[p].y);
-          acc[4] += bf16_lo(w[p].z); acc[5] += bf16_hi(w[p].z);
-          acc[6] += bf16_lo(w[p].w); acc[7] += bf16_hi(w[p].w);
-        }
+        for (int p = 0; p < NP; ++p) add_channels(acc2, w[p]);
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { acc[2 * i] = acc2[i].x; acc[2 * i + 1] = acc2[i].y; }
         if (CH == 16) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
@@ -317,15 +310,11 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       // x - mean in fp32, rounded to bf16 (what a bf16 tensor subtraction does).  Q: padding rows
       // become -mean like the reference (it pads before subtracting); K: padding rows stay zero
       // (the reference subtracts before padding).
+      const float2 neg[4] = {{-mean[0], -mean[1]}, {-mean[2], -mean[3]}, {-mean[4], -mean[5]}, {-mean[6], -mean[7]}};
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const int n = tile * kTile + p * RPP + rl;
-        if (is_q || n < N) {
-          w[p].x = pack_bf16(bf16_lo(w[p].x) - mean[0], bf16_hi(w[p].x) - mean[1]);
-          w[p].y = pack_bf16(bf16_lo(w[p].y) - mean[2], bf16_hi(w[p].y) - mean[3]);
-          w[p].z = pack_bf16(bf16_lo(w[p].z) - mean[4], bf16_hi(w[p].z) - mean[5]);
-          w[p].w = pack_bf16(bf16_lo(w[p].w) - mean[6], bf16_hi(w[p].w) - mean[7]);
-        }
+        if (is_q || n < N) w[p] = subtract_mean(w[p], neg);
       }
     }
     uint8_t* codes = (is_q ? P.q_codes : P.k_codes) + ((int64_t)bh * T + tile) * (kTile * D / 2);
@@ -363,6 +352,10 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       x[i] = (n < Nv && c4 * 4 < P.d_in && !(P.pack && i == 0)) ? *reinterpret_cast<const uint2*>(src + (int64_t)n * P.v_sn) : make_uint2(0, 0);
     }
     uint8_t* codes = P.vt_codes + gt * (D * 64);
+    // largest magnitudes of the 4 channels, two at a time (bf16 comparisons are exact)
+    uint32_t m01 = habsmax2(x[0].x, x[1].x), m23 = habsmax2(x[0].y, x[1].y);
+#pragma unroll
+    for (int i = 2; i < 16; ++i) { m01 = habsmax2(m01, x[i].x); m23 = habsmax2(m23, x[i].y); }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float f[16];
@@ -371,9 +364,8 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
         uint32_t wv = (j < 2) ? x[i].x : x[i].y;
         f[i] = (j & 1) ? bf16_hi(wv) : bf16_lo(wv);
       }
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
+      const uint32_t mv = j < 2 ? m01 : m23;
+      float amax = (j & 1) ? bf16_hi(mv) : bf16_lo(mv);
       if (P.split_first) {
         f[0] = __bfloat162float(__float2bfloat16_rn(split_first_value(f[1], amax)));
         amax = fmaxf(fabsf(f[0]), fabsf(f[1]));
@@ -382,11 +374,15 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       }
       uint32_t sfb; float inv;
       block_scale(amax, sfb, inv);
+      const float2 inv2 = make_float2(inv, inv);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 y = mul2_ftz(make_float2(f[2 * i], f[2 * i + 1]), inv2);
+        f[2 * i] = y.x; f[2 * i + 1] = y.y;
+      }
       uint2 o;
-      o.x = f32x8_to_e2m1x8(mul_ftz(f[0], inv), mul_ftz(f[1], inv), mul_ftz(f[2], inv), mul_ftz(f[3], inv),
-                            mul_ftz(f[4], inv), mul_ftz(f[5], inv), mul_ftz(f[6], inv), mul_ftz(f[7], inv));
-      o.y = f32x8_to_e2m1x8(mul_ftz(f[8], inv), mul_ftz(f[9], inv), mul_ftz(f[10], inv), mul_ftz(f[11], inv),
-                            mul_ftz(f[12], inv), mul_ftz(f[13], inv), mul_ftz(f[14], inv), mul_ftz(f[15], inv));
+      o.x = f32x8_to_e2m1x8(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
+      o.y = f32x8_to_e2m1x8(f[8], f[9], f[10], f[11], f[12], f[13], f[14], f[15]);
       const int d = c4 * 4 + j;
       *reinterpret_cast<uint2*>(codes + d * 64 + blk * 8) = o;
       sf_smem[tl * 1024 + (blk >> 2) * 512 + sf_atom_offset(d, blk & 3)] = (uint8_t)sfb;

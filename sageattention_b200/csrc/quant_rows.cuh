@@ -66,10 +66,10 @@ __device__ __forceinline__ void quant_rows_store(const uint4 (&w)[kTile / (kThre
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));       // 16-element block = 2 threads
     uint32_t sfb; float inv;
     block_scale(amax, sfb, inv);
-    uint32_t code = f32x8_to_e2m1x8(
-        mul_ftz(bf16_lo(w[p].x), inv), mul_ftz(bf16_hi(w[p].x), inv), mul_ftz(bf16_lo(w[p].y), inv),
-        mul_ftz(bf16_hi(w[p].y), inv), mul_ftz(bf16_lo(w[p].z), inv), mul_ftz(bf16_hi(w[p].z), inv),
-        mul_ftz(bf16_lo(w[p].w), inv), mul_ftz(bf16_hi(w[p].w), inv));
+    const float2 inv2 = make_float2(inv, inv);
+    const float2 f0 = mul2_ftz(bf16x2_to_f32(w[p].x), inv2), f1 = mul2_ftz(bf16x2_to_f32(w[p].y), inv2);
+    const float2 f2 = mul2_ftz(bf16x2_to_f32(w[p].z), inv2), f3 = mul2_ftz(bf16x2_to_f32(w[p].w), inv2);
+    const uint32_t code = f32x8_to_e2m1x8(f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y);
     *reinterpret_cast<uint32_t*>(codes_tile + row * (D / 2) + c * 4) = code;
     if ((c & 1) == 0) {
       const int blk = c >> 1;                                        // 16-channel block index
