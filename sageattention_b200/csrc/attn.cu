@@ -98,10 +98,6 @@ constexpr int kLaunchRegs = 128;
 struct RegSplit { static constexpr int softmax = 192, corr = 80, role = 48; };
 static_assert(256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role) <= kAttnThreads * kLaunchRegs,
               "setmaxnreg split exceeds the CTA's register pool");
-constexpr float kNoMax = -1.0e30f;                     // row maximum where no key has been visible
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLog2Inv2688 = -11.392317422778762f;   // log2(1 / (448 * 6))  softmax_fused.h:33
-constexpr float kLog2Inv6 = -2.584962500721156f;       // log2(1 / 6)          softmax_fused.h:34
 
 template <int D>
 struct Smem {

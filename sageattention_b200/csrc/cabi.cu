@@ -86,7 +86,8 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
   out->status = 4;
   out->workspace = align256(out->q_codes) + align256(out->q_sf) + align256(out->k_codes) + align256(out->k_sf) +
                    align256(out->vt_codes) + align256(out->vt_sf) + align256(out->qm) + align256(out->km) +
-                   align256(out->delta_s) + align256(out->q_dot_km) + align256(out->scratch) + 256;
+                   align256(out->delta_s) + align256(out->q_dot_km) + align256(out->scratch) + 256 +
+                   sage3::decode_scratch_bytes(s.B, s.Hq, s.Hkv, s.Nq, s.Nk, s.D);
   return SAGE3_OK;
 }
 
@@ -180,7 +181,7 @@ int sage3_quant_qkv(const sage3_quant_args* a, void* stream) { return quant_qkv_
 
 static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const int* cu_q, const int* cu_k, void* stream_,
                          int slot_first = 0, bool zero_status = true, bool after_delta_s = false,
-                         const int* order = nullptr, const int* n_order = nullptr) {
+                         const int* order = nullptr, const int* n_order = nullptr, void* decode_scratch = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (!a->q_codes || !a->q_sf || !a->k_codes || !a->k_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status)
@@ -215,7 +216,8 @@ static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const 
   k.cu_q = cu_q; k.cu_k = cu_k;
   k.after_delta_s = after_delta_s;
   k.order = order; k.n_order = n_order;
-  e = (cu_q != nullptr || cu_k != nullptr) ? sage3::launch_attn_fwd_varlen(k, stream) : sage3::launch_attn_fwd(k, stream);
+  if (decode_scratch != nullptr) e = sage3::launch_attn_decode(k, decode_scratch, stream);
+  else e = (cu_q != nullptr || cu_k != nullptr) ? sage3::launch_attn_fwd_varlen(k, stream) : sage3::launch_attn_fwd(k, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   return SAGE3_OK;
 }
@@ -286,6 +288,7 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   float* qk = reinterpret_cast<float*>(take(z.q_dot_km));
   q.scratch = take(z.scratch); q.scratch_bytes = z.scratch;
   int32_t* status = reinterpret_cast<int32_t*>(take(4));
+  void* decode_scratch = sage3::decode_fits(a->shape.Hq, a->shape.Hkv, a->shape.Nq, a->shape.Nk) ? w : nullptr;
   if (a->device_status) status = a->device_status;
   if (a->lse && a->smooth_k) q.q_dot_km = qk;
   if (!head_dim_ok(a->head_dim, a->shape.D)) return SAGE3_ERR_ARGUMENT;
@@ -311,7 +314,8 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   t.lse_add = q.q_dot_km;
   t.out_head_dim = a->head_dim;
   t.sm_margin = a->sm_margin;
-  return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false, /*after_delta_s=*/t.delta_s != nullptr);
+  return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false, /*after_delta_s=*/t.delta_s != nullptr,
+                       nullptr, nullptr, decode_scratch);
 }
 
 int sage3_attention_run(const sage3_fwd_args* args, const void* q, const void* k, const void* v, void* out, float* lse,

@@ -53,6 +53,11 @@ __device__ __forceinline__ float ex2_approx(float a) {
   return r;
 }
 
+constexpr float kNoMax = -1.0e30f;                     // row maximum where no key has been visible
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLog2Inv2688 = -11.392317422778762f;   // log2(1 / (448 * 6))  softmax_fused.h:33
+constexpr float kLog2Inv6 = -2.584962500721156f;       // log2(1 / 6)          softmax_fused.h:34
+
 // fp32 -> E4M3 (round to nearest even, saturate to 448); returns the byte.
 __device__ __forceinline__ uint32_t f32_to_e4m3(float x) {
   uint16_t r;

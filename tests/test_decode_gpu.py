@@ -1,0 +1,51 @@
+"""Few query rows per head: the operator splits the keys over the chip there.  Against the CPU restatement of the reference
+arithmetic, tolerance as in ``test_attn_gpu.py``: cosine similarity >= 0.999 and relative L1 <= 2e-2, LSE within 2e-3.
+"""
+import pytest
+import torch
+
+import sageattention_b200 as sa
+from oracle import sage3
+from tests import _util as U
+from tests.test_attn_gpu import COS_MIN, REL_L1_MAX, oracle_on_device_operands
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# the fewest key tiles (and one fewer: the other kernel), a last tile of one key, key tiles that do not fill the runs, runs of
+# several tiles; 1, 8, 9, 16 and 17 rows per kv head and the most there can be; causal rows that see the last keys or not
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,causal", [
+    (1, 2, 2, 1, 896, 128, False), (1, 2, 2, 1, 897, 128, False), (2, 4, 2, 4, 1023, 64, True), (1, 9, 1, 1, 1025, 64, False),
+    (1, 2, 2, 8, 1153, 128, True), (1, 4, 1, 4, 2000, 128, True), (1, 17, 1, 1, 1000, 128, False), (1, 64, 2, 4, 1100, 64, True),
+    (1, 2, 1, 2, 33000, 128, True), (1, 2, 1, 1, 65537, 64, False), (40, 32, 8, 1, 1500, 128, False)])
+def test_few_query_rows(B, Hq, Hkv, Nq, Nk, D, causal):
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, D, seed=Nq + Nk + D, device=DEV)
+    out = sa.sageattn(q, k, v, is_causal=causal, check_status=True)
+    out2, lse = sa.sageattn(q, k, v, is_causal=causal, return_lse=True, check_status=True)
+    assert torch.allclose(out.float(), out2.float(), atol=2e-3, rtol=2e-2)
+    z = sa.quantize_qkv(q, k, v)
+    other, other_lse = sa.fp4_attention(z, is_causal=causal, return_lse=True)
+    assert torch.isfinite(out).all()
+    assert sage3.accuracy(out.float().cpu(), other.float().cpu())[1] <= 1e-3
+    if B * Hq <= 64:
+        want, want_lse = oracle_on_device_operands(z, D ** -0.5, causal, return_lse=True)
+        cos, l1 = sage3.accuracy(out.float().cpu(), want.to(torch.bfloat16).float())
+        assert cos >= COS_MIN and l1 <= REL_L1_MAX, (cos, l1)
+    # (the kernel's own LSE lacks the K-mean term, which the operator adds)
+    term = D ** -0.5 * torch.einsum("bhnd,bhd->bhn", q.float(), z.km.float().repeat_interleave(Hq // Hkv, dim=1))
+    assert torch.allclose(lse, other_lse + term, atol=4e-3, rtol=1e-4)
+
+
+def test_few_query_rows_in_other_layouts():
+    q, k, v = U.make_qkv(2, 8, 2, 3, 1300, 128, seed=5, device=DEV)
+    want = sa.sageattn(q, k, v, is_causal=True)
+    nhd = [t.transpose(1, 2).contiguous() for t in (q, k, v)]
+    assert torch.equal(sa.sageattn(*nhd, tensor_layout="NHD", is_causal=True).transpose(1, 2), want)
+    narrow = sa.sageattn(q[..., :72], k[..., :72], v[..., :72], sm_scale=0.1)
+    full = sa.sageattn(*(torch.nn.functional.pad(t[..., :72], (0, 56)) for t in (q, k, v)), sm_scale=0.1)
+    assert torch.equal(narrow, full[..., :72])
+    # more queries than keys cannot be few; no key smoothing and one mean per sequence can
+    for kw in ({"smooth_k": False}, {"per_block_mean": False}):
+        a = sa.sageattn3_blackwell(q, k, v, **kw)
+        assert torch.isfinite(a).all() and sage3.accuracy(a.float().cpu(), sa.sageattn(q, k, v).float().cpu())[0] > 0.9
