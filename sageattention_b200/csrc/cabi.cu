@@ -93,7 +93,7 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
 
 static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int* cu_k, void* stream_,
                           int* zero_status = nullptr, int* order = nullptr, int* n_order = nullptr, int causal = 0,
-                          float* k_lambda = nullptr, int split_first = 0) {
+                          float* k_lambda = nullptr, int split_first = 0, sage3::DeltaSArgs* k_later = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (int st = check_tensor(a->q)) return st;
@@ -171,6 +171,10 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
     d.km = km; d.partial = partial; d.km_out = a->km; d.ds = a->delta_s; d.cu_k = cu_k; d.k_lambda = k_lambda; d.after_quant = true;
     d.k_codes = a->k_codes; d.k_sf = a->k_sf; d.status = a->device_status; d.d_in = a->head_dim_in;
     d.B = s.B; d.Hq = s.Hq; d.Hkv = s.Hkv; d.Tq = a->per_block_mean == 1 ? Tq : 1; d.Nk = s.Nk; d.D = s.D;
+    if (k_later != nullptr) {                            // the caller's kernel does what this launch would
+      *k_later = d;
+      return SAGE3_OK;
+    }
     e = sage3::launch_delta_s(d, stream);
     if (e != cudaSuccess) return cuda_fail(e);
   }
@@ -181,7 +185,7 @@ int sage3_quant_qkv(const sage3_quant_args* a, void* stream) { return quant_qkv_
 
 static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const int* cu_q, const int* cu_k, void* stream_,
                          int slot_first = 0, bool zero_status = true, bool after_delta_s = false,
-                         const int* order = nullptr, const int* n_order = nullptr, void* decode_scratch = nullptr) {
+                         const int* order = nullptr, const int* n_order = nullptr, const sage3::DeltaSArgs* decode_k = nullptr, void* decode_scratch = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
   if (!a->q_codes || !a->q_sf || !a->k_codes || !a->k_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status)
@@ -216,7 +220,7 @@ static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const 
   k.cu_q = cu_q; k.cu_k = cu_k;
   k.after_delta_s = after_delta_s;
   k.order = order; k.n_order = n_order;
-  if (decode_scratch != nullptr) e = sage3::launch_attn_decode(k, decode_scratch, stream);
+  if (decode_k != nullptr) e = sage3::launch_attn_decode(k, *decode_k, decode_scratch, stream);
   else e = (cu_q != nullptr || cu_k != nullptr) ? sage3::launch_attn_fwd_varlen(k, stream) : sage3::launch_attn_fwd(k, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   return SAGE3_OK;
@@ -288,7 +292,9 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   float* qk = reinterpret_cast<float*>(take(z.q_dot_km));
   q.scratch = take(z.scratch); q.scratch_bytes = z.scratch;
   int32_t* status = reinterpret_cast<int32_t*>(take(4));
-  void* decode_scratch = sage3::decode_fits(a->shape.Hq, a->shape.Hkv, a->shape.Nq, a->shape.Nk) ? w : nullptr;
+  const bool decode = a->per_block_mean >= 0 && sage3::decode_fits(a->shape.Hq, a->shape.Hkv, a->shape.Nq, a->shape.Nk);
+  sage3::DeltaSArgs decode_k{};
+  void* decode_scratch = w;
   if (a->device_status) status = a->device_status;
   if (a->lse && a->smooth_k) q.q_dot_km = qk;
   if (!head_dim_ok(a->head_dim, a->shape.D)) return SAGE3_ERR_ARGUMENT;
@@ -303,7 +309,7 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
     cudaError_t e = cudaMemsetAsync(a->km_out, 0, z.km, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e);
   }
-  if (int st = quant_qkv_impl(&q, nullptr, nullptr, stream, status)) return st;
+  if (int st = quant_qkv_impl(&q, nullptr, nullptr, stream, status, nullptr, nullptr, 0, nullptr, 0, decode ? &decode_k : nullptr)) return st;
   sage3_attn_args t{};
   t.shape = a->shape;
   t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;
@@ -315,7 +321,7 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   t.out_head_dim = a->head_dim;
   t.sm_margin = a->sm_margin;
   return attn_fwd_impl(&t, nullptr, nullptr, nullptr, stream, 0, /*zero_status=*/false, /*after_delta_s=*/t.delta_s != nullptr,
-                       nullptr, nullptr, decode_scratch);
+                       nullptr, nullptr, decode ? &decode_k : nullptr, decode_scratch);
 }
 
 int sage3_attention_run(const sage3_fwd_args* args, const void* q, const void* k, const void* v, void* out, float* lse,

@@ -2,7 +2,8 @@
 // those of attn.cu, the work is split over the keys instead of the query rows.  There a tile of 128 query rows is worked on
 // whole, and its key tiles one after another: P is rounded relative to the running row maximum, so a tile has to know the
 // maximum of all tiles before it.  Here that maximum comes from a pass of its own:
-//   decode_scores_kernel   one warp per key tile: scores of all rows that share the kv head -> memory, and their tile maxima
+//   decode_scores_kernel   one CTA per key tile: K is smoothed and quantised on the way, scores of all rows that share the kv
+//                          head (with delta_s) -> memory, and their tile maxima
 //   decode_output_kernel   one warp per run of key tiles: running maximum before the run from the tile maxima, P^, P^.V^;
 //                          partial outputs; the last CTA of a kv head to finish adds them up
 // The FP4 rows that are long - keys, channels of V^T - are the 16-row operand of mma.m16n8k16, the query rows the 8 columns:
@@ -26,10 +27,16 @@ namespace {
 constexpr int kTile = 128;
 constexpr int kWarps = 4, kThreads = 32 * kWarps;
 constexpr int kMaxChunks = 64;                           // CTAs of the output kernel per kv head
+constexpr int kMaxRows = 64;                             // query rows per kv head
 
 struct DecodeParams {
-  const uint8_t *q_codes, *q_sf, *k_codes, *k_sf, *vt_codes, *vt_sf;
-  const __nv_bfloat16* ds;
+  const uint8_t *q_codes, *q_sf, *vt_codes, *vt_sf;
+  const __nv_bfloat16 *k, *qm, *km;                      // km: the K mean, or
+  const float* partial;                                  // its partial sums, [kv][mean_chunks][D], or neither
+  __nv_bfloat16* km_out;
+  int64_t k_sb, k_sh, k_sn;
+  int Hkv, mean_chunks, d_in;
+  bool smooth;
   __nv_bfloat16* out;
   float* lse;
   const float* lse_add;
@@ -39,7 +46,7 @@ struct DecodeParams {
   int run, chunks;                                       // output kernel: key tiles per warp, CTAs per kv head
   float scale_log2, sm_scale;
   float *scores, *tile_max, *o_part, *l_part, *m_part;   // [kv][rows][Tk*128], [kv][rows][Tk], [kv][rows][chunks] ([D])
-  int* counter;                                          // [kv][groups of rows]
+  int* counter;                                          // [kv][rows]: CTAs of the output kernel that are done with a group of rows
 };
 
 __device__ __forceinline__ uint32_t e2m1x2_to_half2(const float lo, const float hi) {   // rounded to E2M1, as halves
@@ -111,78 +118,146 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t a0, const
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT = groups of 8 query rows
-template <int D, int NT>
+__device__ __forceinline__ void mma16816_bf16(float (&d)[4], const uint32_t a0, const uint32_t a1, const uint32_t a2, const uint32_t a3,
+                                              const uint32_t b0, const uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// One CTA per key tile, each warp two times 16 keys: K is smoothed, quantised and multiplied where it was loaded - a lane has
+// whole 16-channel blocks of a row - so neither its codes nor delta_s exist in memory.
+template <int D>
 __global__ __launch_bounds__(kThreads) void decode_scores_kernel(const DecodeParams P) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
-  const int unit = blockIdx.x * kWarps + (threadIdx.x >> 5), r0 = blockIdx.y * 8 * NT;
+  constexpr int W = D / 8;                               // words of a lane's quarter of a row, as halves or bf16
+  extern __shared__ __align__(16) uint32_t frag[];       // [groups of 8 query rows][W / 4][32 lanes][4]: Q^, then their Q means
+  __shared__ __align__(16) float neg_mean[D];
+  __shared__ float tmax[8][kMaxRows];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
+  const int tile = blockIdx.x, kv = blockIdx.y, groups = (P.rows + 7) / 8;
   pdl_launch_dependents();
-  if (unit >= P.kvs * P.Tk) return;
-  const int kv = unit / P.Tk, tile = unit % P.Tk;
-  // columns of the result fragment: queries 2 tg and 2 tg + 1 of each group.  Head of query row r, counted over the batch: kv
-  // heads are numbered b * Hkv + h, so it is kv * G + r / Nq
-  int64_t ds_row[NT][2];
-  int lim[NT][2];
+  const __nv_bfloat16* src = P.k + kv / P.Hkv * P.k_sb + kv % P.Hkv * P.k_sh + tg * (D / 4);
+  uint4 w[4][W / 4];                                     // rows 32 warp + g + 0, 8, 16, 24 of the tile
 #pragma unroll
-  for (int n = 0; n < NT; ++n)
+  for (int i = 0; i < 4; ++i) {
+    const int key = tile * kTile + 32 * warp + g + 8 * i;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int r = r0 + 8 * n + 2 * tg + j, head = r < P.rows ? r / P.Nq : 0;
-      ds_row[n][j] = ((int64_t)kv * P.G + head) * P.Tk * kTile;
-      lim[n][j] = P.causal ? min(P.Nk - 1, r - head * P.Nq + P.Nk - P.Nq) : P.Nk - 1;      // last visible key
-    }
+    for (int j = 0; j < W / 4; ++j)
+      w[i][j] = key < P.Nk && tg * (D / 4) + 8 * j < P.d_in ? *reinterpret_cast<const uint4*>(src + (int64_t)key * P.k_sn + 8 * j)
+                                                            : make_uint4(0, 0, 0, 0);
+  }
   pdl_wait();
-  if (tile == 0 && lane == 0) P.counter[kv * gridDim.y + blockIdx.y] = 0;
-  const uint8_t* kc = P.k_codes + (int64_t)unit * kTile * (D / 2);
-  const uint8_t* ks = P.k_sf + (int64_t)unit * (D / 64) * 512;
-  uint32_t q[NT][D / 8];
+  if (tile == 0 && t < P.rows) P.counter[kv * P.rows + t] = 0;
+  for (int i = t; i < groups * 64; i += kThreads) {
+    const int n = i >> 6, r = 8 * n + ((i & 31) >> 2), quarter = i & 3;      // (threads of a warp: all Q^ or all means)
+    const int64_t head = (int64_t)kv * P.G + min(r, P.rows - 1) / P.Nq;
+    uint32_t x[W];
+    if ((i & 32) == 0) {
+      RawRow<D> raw = {};
+      if (r < P.rows) raw = raw_row<D>(P.q_codes + head * kTile * (D / 2), P.q_sf + head * (D / 64) * 512, r % P.Nq, quarter);
+      expand_row<D>(raw, x);
+    } else {
 #pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    const int r = r0 + 8 * n + g;
-    RawRow<D> x = {};
-    if (r < P.rows) {
-      const int64_t head = (int64_t)kv * P.G + r / P.Nq;
-      x = raw_row<D>(P.q_codes + head * kTile * (D / 2), P.q_sf + head * (D / 64) * 512, r % P.Nq, tg);
+      for (int j = 0; j < W / 4; ++j)
+        reinterpret_cast<uint4*>(x)[j] = __ldcg(reinterpret_cast<const uint4*>(P.qm + head * D + quarter * (D / 4) + 8 * j));
     }
-    expand_row<D>(x, q[n]);
-  }
-  float m[NT][2];
 #pragma unroll
-  for (int n = 0; n < NT; ++n) m[n][0] = m[n][1] = kNoMax;
+    for (int j = 0; j < W / 4; ++j)
+      reinterpret_cast<uint4*>(frag)[((i >> 5) * (W / 4) + j) * 32 + (i & 31)] = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+  }
+  if (t < D) {
+    // the mean: given, or from the partial sums (same order and rounding as in the other K kernel), or none
+    float m = 0.f;
+    if (P.km != nullptr) {
+      m = __bfloat162float(P.km[(int64_t)kv * D + t]);
+    } else if (P.partial != nullptr) {
+      const float* p = P.partial + (int64_t)kv * P.mean_chunks * D + t;
+      float s = 0.f;
+#pragma unroll 16
+      for (int i = 0; i < P.mean_chunks; ++i) s += __ldcg(p + i * D);
+      const __nv_bfloat16 b = __float2bfloat16_rn(s / (float)P.Nk);
+      if (tile == 0 && P.km_out != nullptr) P.km_out[(int64_t)kv * D + t] = b;
+      m = __bfloat162float(b);
+    }
+    neg_mean[t] = -m;
+  }
+  __syncthreads();
   const int64_t ld = (int64_t)P.Tk * kTile;
-#pragma unroll 4
-  for (int mt = 0; mt < 8; ++mt) {
-    const int row = 16 * mt + g, key = tile * kTile + row;
-    uint32_t k0[D / 8], k1[D / 8];
-    expand_row<D>(raw_row<D>(kc, ks, row, tg), k0);
-    expand_row<D>(raw_row<D>(kc, ks, row + 8, tg), k1);
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-      if (P.ds != nullptr) {
+  for (int mt = 0; mt < 2; ++mt) {
+    uint32_t kb[2][W], kq[2][W];                         // smoothed rows, the same quantised
 #pragma unroll
-        for (int i = 0; i < 4; ++i) s[i] = __bfloat162float(P.ds[ds_row[n][i & 1] + key + (i >> 1) * 8]);
+    for (int i = 0; i < 2; ++i) {
+      const int key = tile * kTile + 32 * warp + 16 * mt + 8 * i + g;
+      uint32_t amax[W / 4];
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j) {
+        uint4 x = w[2 * mt + i][j];
+        const float4 a = *reinterpret_cast<const float4*>(&neg_mean[tg * (D / 4) + 8 * j]);
+        const float4 b = *reinterpret_cast<const float4*>(&neg_mean[tg * (D / 4) + 8 * j + 4]);
+        const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
+        if (P.smooth && key < P.Nk) x = subtract_mean(x, neg);             // padding rows stay zero
+        kb[i][4 * j] = x.x; kb[i][4 * j + 1] = x.y; kb[i][4 * j + 2] = x.z; kb[i][4 * j + 3] = x.w;
+        amax[j] = habsmax2(habsmax2(x.x, x.y), habsmax2(x.z, x.w));
       }
 #pragma unroll
-      for (int j = 0; j < D / 16; ++j) mma16816(s, k0[2 * j], k1[2 * j], k0[2 * j + 1], k1[2 * j + 1], q[n][2 * j], q[n][2 * j + 1]);
+      for (int blk = 0; blk < W / 8; ++blk) {
+        const uint32_t m2 = habsmax2(amax[2 * blk], amax[2 * blk + 1]);
+        uint32_t sfb, sf2, unused;
+        float inv;
+        block_scale(fmaxf(bf16_lo(m2), bf16_hi(m2)), sfb, inv);
+        scales2(sfb, sf2, unused);
+        const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + 8 * n + 2 * tg + (i & 1), kk = key + (i >> 1) * 8;
-        if (kk > lim[n][i & 1]) s[i] = __uint_as_float(0xff800000u);
-        if (r < P.rows) P.scores[((int64_t)kv * P.rows + r) * ld + kk] = s[i];
-        m[n][i & 1] = fmaxf(m[n][i & 1], s[i]);
+        for (int j = 8 * blk; j < 8 * blk + 8; ++j) {
+          const float2 x = mul2_ftz(bf16x2_to_f32(kb[i][j]), inv2);
+          kq[i][j] = hmul2(e2m1x2_to_half2(x.x, x.y), sf2);
+        }
+      }
+    }
+    const int key = tile * kTile + 32 * warp + 16 * mt + g;
+#pragma unroll 1
+    for (int n = 0; n < groups; ++n) {
+      const uint4* f = reinterpret_cast<const uint4*>(frag) + n * 2 * (W / 4) * 32 + lane;
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j) {                  // delta_s
+        const uint4 b = f[(W / 4 + j) * 32];
+        mma16816_bf16(s, kb[0][4 * j], kb[1][4 * j], kb[0][4 * j + 1], kb[1][4 * j + 1], b.x, b.y);
+        mma16816_bf16(s, kb[0][4 * j + 2], kb[1][4 * j + 2], kb[0][4 * j + 3], kb[1][4 * j + 3], b.z, b.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = __bfloat162float(__float2bfloat16_rn(s[i]));
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j) {
+        const uint4 b = f[j * 32];
+        mma16816(s, kq[0][4 * j], kq[1][4 * j], kq[0][4 * j + 1], kq[1][4 * j + 1], b.x, b.y);
+        mma16816(s, kq[0][4 * j + 2], kq[1][4 * j + 2], kq[0][4 * j + 3], kq[1][4 * j + 3], b.z, b.w);
+      }
+      // columns: query rows 8 n + 2 tg and + 1, rows: keys `key` and + 8
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = 8 * n + 2 * tg + j;
+        const int lim = P.causal ? min(P.Nk - 1, r % P.Nq + P.Nk - P.Nq) : P.Nk - 1;       // last visible key
+        const float lo = key <= lim ? s[j] : __uint_as_float(0xff800000u), hi = key + 8 <= lim ? s[2 + j] : __uint_as_float(0xff800000u);
+        if (r < P.rows) {
+          float* row = P.scores + ((int64_t)kv * P.rows + r) * ld + key;
+          row[0] = lo;
+          row[8] = hi;
+        }
+        float m = fmaxf(fmaxf(lo, hi), kNoMax);
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+        if (g == 0) tmax[2 * warp + mt][r] = m;
       }
     }
   }
+  __syncthreads();
+  if (t < P.rows) {
+    float m = tmax[0][t];
 #pragma unroll
-  for (int n = 0; n < NT; ++n)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-      for (int x = 4; x < 32; x <<= 1) m[n][j] = fmaxf(m[n][j], __shfl_xor_sync(0xffffffffu, m[n][j], x));
-      const int r = r0 + 8 * n + 2 * tg + j;
-      if (g == 0 && r < P.rows) P.tile_max[((int64_t)kv * P.rows + r) * P.Tk + tile] = m[n][j];
-    }
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, tmax[i][t]);
+    P.tile_max[((int64_t)kv * P.rows + t) * P.Tk + tile] = m;
+  }
 }
 
 // Key tiles from the last to the first, as in attn.cu; a warp takes `run` of them, a CTA 4 * run.
@@ -314,7 +389,7 @@ __global__ __launch_bounds__(kThreads) void decode_output_kernel(const DecodePar
   if (P.chunks > 1) {
     __threadfence();
     __syncthreads();
-    if (t == 0) last_s = atomicAdd(P.counter + kv * gridDim.y + blockIdx.y, 1) == P.chunks - 1;
+    if (t == 0) last_s = atomicAdd(P.counter + kv * P.rows + blockIdx.y, 1) == P.chunks - 1;
     __syncthreads();
     if (!last_s) return;
     __threadfence();
@@ -384,8 +459,8 @@ cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
   const int even = (int)(((int64_t)units * groups + 148 * 16 - 1) / (148 * 16)), most = (P.Tk + kWarps * kMaxChunks - 1) / (kWarps * kMaxChunks);
   P.run = even > most ? even : most;
   P.chunks = (P.Tk + kWarps * P.run - 1) / (kWarps * P.run);
-  cudaError_t e = launch_pdl(decode_scores_kernel<D, NT>, dim3((unsigned)((units + kWarps - 1) / kWarps), groups), kThreads, 0, stream,
-                             overlap, P);
+  const size_t frag = (size_t)(P.rows + 7) / 8 * 2 * 32 * (D / 8) * 4;         // 32 KB at most
+  cudaError_t e = launch_pdl(decode_scores_kernel<D>, dim3(P.Tk, P.kvs), kThreads, frag, stream, overlap, P);
   if (e != cudaSuccess) return e;
   return launch_pdl(decode_output_kernel<D, NT>, dim3((unsigned)(P.kvs * P.chunks), groups), kThreads, 0, stream, true, P);
 }
@@ -394,7 +469,7 @@ cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
 
 bool decode_fits(int Hq, int Hkv, int Nq, int Nk) {
   const int rows = Hq / Hkv * Nq;
-  return Nk > 7 * kTile && rows <= 128 && (Nq <= 4 || rows <= 8);
+  return Nk > 7 * kTile && rows <= kMaxRows && (Nq <= 4 || rows <= 8);
 }
 
 size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D) {
@@ -404,12 +479,20 @@ size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D) {
          2 * align256(rows * chunks * 4) + align256(rows * 4);
 }
 
-cudaError_t launch_attn_decode(const AttnArgs& a, void* scratch, cudaStream_t stream) {
+cudaError_t launch_attn_decode(const AttnArgs& a, const DeltaSArgs& k, void* scratch, cudaStream_t stream) {
   if ((a.D != 128 && a.D != 64) || !decode_fits(a.Hq, a.Hkv, a.Nq, a.Nk)) return cudaErrorInvalidValue;
   DecodeParams P;
-  P.q_codes = (const uint8_t*)a.q_codes; P.q_sf = (const uint8_t*)a.q_sf; P.k_codes = (const uint8_t*)a.k_codes;
-  P.k_sf = (const uint8_t*)a.k_sf; P.vt_codes = (const uint8_t*)a.vt_codes; P.vt_sf = (const uint8_t*)a.vt_sf;
-  P.ds = (const __nv_bfloat16*)a.ds; P.out = (__nv_bfloat16*)a.out; P.lse = a.lse; P.lse_add = a.lse_add;
+  P.q_codes = (const uint8_t*)a.q_codes; P.q_sf = (const uint8_t*)a.q_sf;
+  P.vt_codes = (const uint8_t*)a.vt_codes; P.vt_sf = (const uint8_t*)a.vt_sf;
+  P.k = (const __nv_bfloat16*)k.k; P.k_sb = k.k_sb; P.k_sh = k.k_sh; P.k_sn = k.k_sn;
+  P.qm = (const __nv_bfloat16*)k.qm; P.km = (const __nv_bfloat16*)k.km; P.partial = (const float*)k.partial;
+  P.km_out = (__nv_bfloat16*)k.km_out;
+  P.smooth = P.km != nullptr || P.partial != nullptr;
+  int chunk_tokens;
+  quant_chunks(a.B * a.Hkv, a.Nk, &P.mean_chunks, &chunk_tokens);
+  P.d_in = (k.d_in > 0 && k.d_in <= a.D) ? k.d_in : a.D;
+  P.Hkv = a.Hkv;
+  P.out = (__nv_bfloat16*)a.out; P.lse = a.lse; P.lse_add = a.lse_add;
   P.o_sb = a.o_sb; P.o_sh = a.o_sh; P.o_sn = a.o_sn;
   P.kvs = a.B * a.Hkv; P.Hq = a.Hq; P.G = a.Hq / a.Hkv; P.Nq = a.Nq; P.Nk = a.Nk; P.Tk = (a.Nk + kTile - 1) / kTile;
   P.rows = P.G * a.Nq;
@@ -425,8 +508,8 @@ cudaError_t launch_attn_decode(const AttnArgs& a, void* scratch, cudaStream_t st
   P.l_part = (float*)take(rows * chunks * 4);
   P.m_part = (float*)take(rows * chunks * 4);
   P.counter = (int*)take(rows * 4);
-  if (a.D == 128) return P.rows <= 8 ? launch<128, 1>(P, a.after_delta_s, stream) : launch<128, 2>(P, a.after_delta_s, stream);
-  return P.rows <= 8 ? launch<64, 1>(P, a.after_delta_s, stream) : launch<64, 2>(P, a.after_delta_s, stream);
+  if (a.D == 128) return P.rows <= 8 ? launch<128, 1>(P, k.after_quant, stream) : launch<128, 2>(P, k.after_quant, stream);
+  return P.rows <= 8 ? launch<64, 1>(P, k.after_quant, stream) : launch<64, 2>(P, k.after_quant, stream);
 }
 
 }  // namespace sage3

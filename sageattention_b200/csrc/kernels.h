@@ -112,7 +112,8 @@ cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream);   //
 // Attention of a few query rows per head (decode.cu); scratch of decode_scratch_bytes, 0 where decode_fits says no.
 bool decode_fits(int Hq, int Hkv, int Nq, int Nk);
 size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D);
-cudaError_t launch_attn_decode(const AttnArgs& a, void* scratch, cudaStream_t stream);
+// K is taken as it is, with the means and Q block means that launch_delta_s would get; no codes of K, no delta_s.
+cudaError_t launch_attn_decode(const AttnArgs& a, const DeltaSArgs& k, void* scratch, cudaStream_t stream);
 
 // Back-to-back block-scaled FP4 MMAs on resident operands, one CTA per SM (peak.cu); *ctas = CTAs launched.
 cudaError_t launch_fp4_mma_peak(int n_cols, int bursts, int* status, cudaStream_t stream, int* ctas);
