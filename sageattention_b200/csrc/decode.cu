@@ -10,8 +10,8 @@
 // tcgen05's smallest tile has 128 rows of the other kind, and its operands would have to go through shared and tensor
 // memory.  Values are expanded to halves together with their block scale, which is exact (2 + 4 significant bits, 2^-10 ...
 // 2688), products are exact and sums fp32.  The order of elements along the contraction is free as long as both operands have
-// the same: a lane takes a quarter of a row, contiguous, so it loads it with one instruction - and of P a lane then holds 32
-// keys of one query, i.e. whole quantisation blocks: their maxima, scales and codes need no exchange between lanes.
+// the same: a lane takes whole quantisation blocks of a
+// row, so that maxima, scales and codes need no exchange between lanes.
 // What bounds it: on a full chip the expansion of the codes (32 instructions per row and lane, the MMA are 8), on few heads
 // the latency of a few dependent loads.
 #include <cuda_fp16.h>
@@ -25,7 +25,8 @@ namespace sage3 {
 namespace {
 
 constexpr int kTile = 128;
-constexpr int kWarps = 4, kThreads = 32 * kWarps;
+constexpr int kWarps = 4, kThreads = 32 * kWarps;        // output kernel
+constexpr int kScoreThreads = 256;
 constexpr int kMaxChunks = 64;                           // CTAs of the output kernel per kv head
 constexpr int kMaxRows = 64;                             // query rows per kv head
 
@@ -43,6 +44,7 @@ struct DecodeParams {
   int64_t o_sb, o_sh, o_sn;
   int kvs, Hq, G, Nq, Nk, Tk, rows;                      // kv heads of the batch; rows = G * Nq query rows share one
   int causal, d_out;
+  int score_run;                                         // scores kernel: key tiles per CTA
   int run, chunks;                                       // output kernel: key tiles per warp, CTAs per kv head
   float scale_log2, sm_scale;
   float *scores, *tile_max, *o_part, *l_part, *m_part;   // [kv][rows][Tk*128], [kv][rows][Tk], [kv][rows][chunks] ([D])
@@ -87,152 +89,171 @@ __device__ __forceinline__ void scales2(const uint32_t bytes, uint32_t& lo2, uin
   lo2 = __byte_perm(h, h, 0x1010);
   hi2 = __byte_perm(h, h, 0x3232);
 }
-// Row of E values (E = 128 or 64) of the tile whose codes and scale atoms start at `codes`, `sf`: the quarter of lane `tg` of
-// the four that share it, as E / 8 half pairs.  `raw` and `expand` apart: all loads of a tile go out first.
-template <int E> struct RawRow { uint32_t w[E / 32], sf; };
-template <int E>
-__device__ __forceinline__ RawRow<E> raw_row(const uint8_t* codes, const uint8_t* sf, const int row, const int tg) {
-  RawRow<E> x;
-  const uint8_t* s = sf + (row & 31) * 16 + (row >> 5) * 4;
-  if (E == 128) {
-    const uint4 v = *reinterpret_cast<const uint4*>(codes + row * 64 + tg * 16);
-    x.w[0] = v.x; x.w[1] = v.y; x.w[E / 32 - 2] = v.z; x.w[E / 32 - 1] = v.w;
-    x.sf = *reinterpret_cast<const uint16_t*>(s + (tg >> 1) * 512 + (tg & 1) * 2);
-  } else {
-    const uint2 v = *reinterpret_cast<const uint2*>(codes + row * 32 + tg * 8);
-    x.w[0] = v.x; x.w[1] = v.y;
-    x.sf = s[tg];
+// What lane `tg` of the four that share a row holds of it, as words of two codes or values:
+//   V^T, P (128 keys)   keys 32 tg ... + 31: one 16-byte load of codes
+//   Q, K (D channels)   16-channel blocks tg and (D=128) tg + 4: the four lanes' loads of bf16 K fall into one line, which
+//                       is what the L1 is short of (a quarter of a row per lane: two lines, 88 -> 85 us for the whole operator at B8 H32/8 Nk4096)
+struct RawRow { uint32_t w[4], sf; };
+__device__ __forceinline__ RawRow raw_keys(const uint8_t* codes, const uint8_t* sf, const int row, const int tg) {
+  const uint4 v = *reinterpret_cast<const uint4*>(codes + row * 64 + tg * 16);
+  return {{v.x, v.y, v.z, v.w}, *reinterpret_cast<const uint16_t*>(sf + (tg >> 1) * 512 + sf_atom_offset(row, (tg & 1) * 2))};
+}
+template <int D>
+__device__ __forceinline__ RawRow raw_channels(const uint8_t* codes, const uint8_t* sf, const int row, const int tg) {
+  RawRow x = {};
+#pragma unroll
+  for (int i = 0; i < D / 64; ++i) {
+    const uint2 v = *reinterpret_cast<const uint2*>(codes + row * (D / 2) + (tg + 4 * i) * 8);
+    x.w[2 * i] = v.x; x.w[2 * i + 1] = v.y;
+    x.sf |= (uint32_t)sf[i * 512 + sf_atom_offset(row, tg)] << (8 * i);
   }
   return x;
 }
-template <int E>
-__device__ __forceinline__ void expand_row(const RawRow<E>& x, uint32_t (&h)[E / 8]) {
+template <int W>
+__device__ __forceinline__ void expand_row(const RawRow& x, uint32_t (&h)[W]) {
   uint32_t s0, s1;
   scales2(x.sf, s0, s1);
 #pragma unroll
-  for (int i = 0; i < E / 32; ++i) expand8(x.w[i], i < 2 ? s0 : s1, &h[4 * i]);
+  for (int i = 0; i < W / 4; ++i) expand8(x.w[i], i < 2 ? s0 : s1, &h[4 * i]);
 }
+template <bool kBf16>
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t a0, const uint32_t a1, const uint32_t a2, const uint32_t a3,
                                          const uint32_t b0, const uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  if (kBf16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-
-__device__ __forceinline__ void mma16816_bf16(float (&d)[4], const uint32_t a0, const uint32_t a1, const uint32_t a2, const uint32_t a3,
-                                              const uint32_t b0, const uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// One CTA per key tile, each warp two times 16 keys: K is smoothed, quantised and multiplied where it was loaded - a lane has
-// whole 16-channel blocks of a row - so neither its codes nor delta_s exist in memory.
-template <int D>
-__global__ __launch_bounds__(kThreads) void decode_scores_kernel(const DecodeParams P) {
-  constexpr int W = D / 8;                               // words of a lane's quarter of a row, as halves or bf16
-  extern __shared__ __align__(16) uint32_t frag[];       // [groups of 8 query rows][W / 4][32 lanes][4]: Q^, then their Q means
-  __shared__ __align__(16) float neg_mean[D];
-  __shared__ float tmax[8][kMaxRows];
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
-  const int tile = blockIdx.x, kv = blockIdx.y, groups = (P.rows + 7) / 8;
-  pdl_launch_dependents();
-  const __nv_bfloat16* src = P.k + kv / P.Hkv * P.k_sb + kv % P.Hkv * P.k_sh + tg * (D / 4);
-  uint4 w[4][W / 4];                                     // rows 32 warp + g + 0, 8, 16, 24 of the tile
+// 16 keys (parts of rows in registers) times 8 query rows (parts as vectors, 32 lanes apart, in shared memory)
+template <bool kBf16, int W>
+__device__ __forceinline__ void product(float (&s)[4], const uint32_t (&k)[2][W], const uint4* f) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int key = tile * kTile + 32 * warp + g + 8 * i;
-#pragma unroll
-    for (int j = 0; j < W / 4; ++j)
-      w[i][j] = key < P.Nk && tg * (D / 4) + 8 * j < P.d_in ? *reinterpret_cast<const uint4*>(src + (int64_t)key * P.k_sn + 8 * j)
-                                                            : make_uint4(0, 0, 0, 0);
+  for (int j = 0; j < W / 4; ++j) {
+    const uint4 b = f[j * 32];
+    mma16816<kBf16>(s, k[0][4 * j], k[1][4 * j], k[0][4 * j + 1], k[1][4 * j + 1], b.x, b.y);
+    mma16816<kBf16>(s, k[0][4 * j + 2], k[1][4 * j + 2], k[0][4 * j + 3], k[1][4 * j + 3], b.z, b.w);
   }
+}
+
+// Where the score of key `k` of a tile lies: key 32 a + 4 b + c at 16 b + 4 a + c, so that the output kernel's four lanes
+// read 64 contiguous bytes.
+__device__ __forceinline__ constexpr int score_place(const int k) { return (k & 28) * 4 + (k >> 5) * 4 + (k & 3); }
+
+// A CTA takes `score_run` key tiles one after another, each warp 16 keys of a tile, and fetches the rows of the next while it
+// works on the present one.  K is smoothed, quantised and multiplied where it was loaded, so neither its codes nor delta_s
+// exist in memory.  kOne: at most 8 query rows; the quantised rows then take the registers of the smoothed ones.
+// (One tile per CTA of four warps, 32 keys each: 47 us at B8 H32/8 Nk4096, now 26.)
+template <int D, bool kOne>
+__global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores_kernel(const DecodeParams P) {
+  constexpr int W = D / 8;                               // words of a lane's part of a row, as halves or bf16
+  extern __shared__ __align__(16) uint32_t frag[];       // [groups of 8 query rows][W / 4][32 lanes][4]: Q^, then their Q means
+  __shared__ __align__(16) float neg_mean[D + D / 8];    // four words further every 32 channels, for the banks
+  __shared__ float tmax[2][8][kOne ? 8 : kMaxRows];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
+  const int kv = blockIdx.y, groups = kOne ? 1 : (P.rows + 7) / 8;
+  const int first = blockIdx.x * P.score_run, end = min(first + P.score_run, P.Tk);
+  pdl_launch_dependents();
+  const __nv_bfloat16* src = P.k + kv / P.Hkv * P.k_sb + kv % P.Hkv * P.k_sh;
+  auto channel = [](const int quarter, const int j) { return 16 * (quarter + 4 * (j >> 1)) + 8 * (j & 1); };   // first of 8
+  uint4 w[2][W / 4];                                     // rows 16 warp + g and + 8 of the tile
+  auto load = [&](const int tile) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int key = tile * kTile + 16 * warp + g + 8 * i;
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j)
+        w[i][j] = key < P.Nk && channel(tg, j) < P.d_in ? *reinterpret_cast<const uint4*>(src + (int64_t)key * P.k_sn + channel(tg, j))
+                                                        : make_uint4(0, 0, 0, 0);
+    }
+  };
+  load(first);
   pdl_wait();
-  if (tile == 0 && t < P.rows) P.counter[kv * P.rows + t] = 0;
-  for (int i = t; i < groups * 64; i += kThreads) {
+  if (blockIdx.x == 0 && t < P.rows) P.counter[kv * P.rows + t] = 0;
+  for (int i = t; i < groups * 64; i += kScoreThreads) {
     const int n = i >> 6, r = 8 * n + ((i & 31) >> 2), quarter = i & 3;      // (threads of a warp: all Q^ or all means)
     const int64_t head = (int64_t)kv * P.G + min(r, P.rows - 1) / P.Nq;
     uint32_t x[W];
     if ((i & 32) == 0) {
-      RawRow<D> raw = {};
-      if (r < P.rows) raw = raw_row<D>(P.q_codes + head * kTile * (D / 2), P.q_sf + head * (D / 64) * 512, r % P.Nq, quarter);
-      expand_row<D>(raw, x);
+      RawRow raw = {};
+      if (r < P.rows) raw = raw_channels<D>(P.q_codes + head * kTile * (D / 2), P.q_sf + head * (D / 64) * 512, r % P.Nq, quarter);
+      expand_row(raw, x);
     } else {
 #pragma unroll
       for (int j = 0; j < W / 4; ++j)
-        reinterpret_cast<uint4*>(x)[j] = __ldcg(reinterpret_cast<const uint4*>(P.qm + head * D + quarter * (D / 4) + 8 * j));
+        reinterpret_cast<uint4*>(x)[j] = __ldcg(reinterpret_cast<const uint4*>(P.qm + head * D + channel(quarter, j)));
     }
 #pragma unroll
     for (int j = 0; j < W / 4; ++j)
       reinterpret_cast<uint4*>(frag)[((i >> 5) * (W / 4) + j) * 32 + (i & 31)] = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
   }
-  if (t < D) {
+  if (t >= kScoreThreads - D) {
     // the mean: given, or from the partial sums (same order and rounding as in the other K kernel), or none
+    const int d = t - (kScoreThreads - D);
     float m = 0.f;
     if (P.km != nullptr) {
-      m = __bfloat162float(P.km[(int64_t)kv * D + t]);
+      m = __bfloat162float(P.km[(int64_t)kv * D + d]);
     } else if (P.partial != nullptr) {
-      const float* p = P.partial + (int64_t)kv * P.mean_chunks * D + t;
+      const float* p = P.partial + (int64_t)kv * P.mean_chunks * D + d;
       float s = 0.f;
 #pragma unroll 16
       for (int i = 0; i < P.mean_chunks; ++i) s += __ldcg(p + i * D);
       const __nv_bfloat16 b = __float2bfloat16_rn(s / (float)P.Nk);
-      if (tile == 0 && P.km_out != nullptr) P.km_out[(int64_t)kv * D + t] = b;
+      if (blockIdx.x == 0 && P.km_out != nullptr) P.km_out[(int64_t)kv * D + d] = b;
       m = __bfloat162float(b);
     }
-    neg_mean[t] = -m;
+    neg_mean[d + d / 32 * 4] = -m;
   }
   __syncthreads();
   const int64_t ld = (int64_t)P.Tk * kTile;
+#pragma unroll 1
+  for (int tile = first; tile < end; ++tile) {
+    uint32_t kb[2][W];                                   // smoothed rows
+    uint32_t amax[2][W / 4];
+    const int key = tile * kTile + 16 * warp + g;
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
-    uint32_t kb[2][W], kq[2][W];                         // smoothed rows, the same quantised
+    for (int j = 0; j < W / 4; ++j) {
+      const float* nm = &neg_mean[channel(tg, j) + channel(tg, j) / 32 * 4];
+      const float4 a = *reinterpret_cast<const float4*>(nm), b = *reinterpret_cast<const float4*>(nm + 4);
+      const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int key = tile * kTile + 32 * warp + 16 * mt + 8 * i + g;
-      uint32_t amax[W / 4];
-#pragma unroll
-      for (int j = 0; j < W / 4; ++j) {
-        uint4 x = w[2 * mt + i][j];
-        const float4 a = *reinterpret_cast<const float4*>(&neg_mean[tg * (D / 4) + 8 * j]);
-        const float4 b = *reinterpret_cast<const float4*>(&neg_mean[tg * (D / 4) + 8 * j + 4]);
-        const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
-        if (P.smooth && key < P.Nk) x = subtract_mean(x, neg);             // padding rows stay zero
+      for (int i = 0; i < 2; ++i) {
+        uint4 x = w[i][j];
+        if (P.smooth && key + 8 * i < P.Nk) x = subtract_mean(x, neg);     // padding rows stay zero
         kb[i][4 * j] = x.x; kb[i][4 * j + 1] = x.y; kb[i][4 * j + 2] = x.z; kb[i][4 * j + 3] = x.w;
-        amax[j] = habsmax2(habsmax2(x.x, x.y), habsmax2(x.z, x.w));
-      }
-#pragma unroll
-      for (int blk = 0; blk < W / 8; ++blk) {
-        const uint32_t m2 = habsmax2(amax[2 * blk], amax[2 * blk + 1]);
-        uint32_t sfb, sf2, unused;
-        float inv;
-        block_scale(fmaxf(bf16_lo(m2), bf16_hi(m2)), sfb, inv);
-        scales2(sfb, sf2, unused);
-        const float2 inv2 = make_float2(inv, inv);
-#pragma unroll
-        for (int j = 8 * blk; j < 8 * blk + 8; ++j) {
-          const float2 x = mul2_ftz(bf16x2_to_f32(kb[i][j]), inv2);
-          kq[i][j] = hmul2(e2m1x2_to_half2(x.x, x.y), sf2);
-        }
+        amax[i][j] = habsmax2(habsmax2(x.x, x.y), habsmax2(x.z, x.w));
       }
     }
-    const int key = tile * kTile + 32 * warp + 16 * mt + g;
-#pragma unroll 1
-    for (int n = 0; n < groups; ++n) {
-      const uint4* f = reinterpret_cast<const uint4*>(frag) + n * 2 * (W / 4) * 32 + lane;
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < W / 4; ++j) {                  // delta_s
-        const uint4 b = f[(W / 4 + j) * 32];
-        mma16816_bf16(s, kb[0][4 * j], kb[1][4 * j], kb[0][4 * j + 1], kb[1][4 * j + 1], b.x, b.y);
-        mma16816_bf16(s, kb[0][4 * j + 2], kb[1][4 * j + 2], kb[0][4 * j + 3], kb[1][4 * j + 3], b.z, b.w);
-      }
+    if (tile + 1 < end) load(tile + 1);
+    // scores start from delta_s
+    auto delta_s = [&](float (&s)[4], const int n) {
+      s[0] = s[1] = s[2] = s[3] = 0.f;
+      product<true, W>(s, kb, reinterpret_cast<const uint4*>(frag) + (2 * n + 1) * (W / 4) * 32 + lane);
 #pragma unroll
       for (int i = 0; i < 4; ++i) s[i] = __bfloat162float(__float2bfloat16_rn(s[i]));
+    };
+    auto quantise = [&](uint32_t (&kq)[2][W]) {
 #pragma unroll
-      for (int j = 0; j < W / 4; ++j) {
-        const uint4 b = f[j * 32];
-        mma16816(s, kq[0][4 * j], kq[1][4 * j], kq[0][4 * j + 1], kq[1][4 * j + 1], b.x, b.y);
-        mma16816(s, kq[0][4 * j + 2], kq[1][4 * j + 2], kq[0][4 * j + 3], kq[1][4 * j + 3], b.z, b.w);
+      for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int blk = 0; blk < W / 8; ++blk) {
+          const uint32_t m2 = habsmax2(amax[i][2 * blk], amax[i][2 * blk + 1]);
+          uint32_t sfb, sf2, unused;
+          float inv;
+          block_scale(fmaxf(bf16_lo(m2), bf16_hi(m2)), sfb, inv);
+          scales2(sfb, sf2, unused);
+          const float2 inv2 = make_float2(inv, inv);
+#pragma unroll
+          for (int j = 8 * blk; j < 8 * blk + 8; ++j) {
+            const float2 x = mul2_ftz(bf16x2_to_f32(kb[i][j]), inv2);
+            kq[i][j] = hmul2(e2m1x2_to_half2(x.x, x.y), sf2);
+          }
+        }
       }
+    };
+    auto scores = [&](float (&s)[4], const uint32_t (&kq)[2][W], const int n) {
+      product<false, W>(s, kq, reinterpret_cast<const uint4*>(frag) + 2 * n * (W / 4) * 32 + lane);
       // columns: query rows 8 n + 2 tg and + 1, rows: keys `key` and + 8
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -240,29 +261,43 @@ __global__ __launch_bounds__(kThreads) void decode_scores_kernel(const DecodePar
         const int lim = P.causal ? min(P.Nk - 1, r % P.Nq + P.Nk - P.Nq) : P.Nk - 1;       // last visible key
         const float lo = key <= lim ? s[j] : __uint_as_float(0xff800000u), hi = key + 8 <= lim ? s[2 + j] : __uint_as_float(0xff800000u);
         if (r < P.rows) {
-          float* row = P.scores + ((int64_t)kv * P.rows + r) * ld + key;
+          float* row = P.scores + ((int64_t)kv * P.rows + r) * ld + tile * kTile + score_place(16 * warp + g);
           row[0] = lo;
-          row[8] = hi;
+          row[score_place(8)] = hi;
         }
         float m = fmaxf(fmaxf(lo, hi), kNoMax);
 #pragma unroll
         for (int x = 4; x < 32; x <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
-        if (g == 0) tmax[2 * warp + mt][r] = m;
+        if (g == 0) tmax[tile & 1][warp][r] = m;
+      }
+    };
+    float s[4];
+    if constexpr (kOne) {
+      delta_s(s, 0);
+      quantise(kb);
+      scores(s, kb, 0);
+    } else {
+      uint32_t kq[2][W];
+      quantise(kq);
+#pragma unroll 1
+      for (int n = 0; n < groups; ++n) {
+        delta_s(s, n);
+        scores(s, kq, n);
       }
     }
-  }
-  __syncthreads();
-  if (t < P.rows) {
-    float m = tmax[0][t];
+    __syncthreads();                                     // (the other half of tmax is written next)
+    if (t < P.rows) {
+      float m = tmax[tile & 1][0][t];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) m = fmaxf(m, tmax[i][t]);
-    P.tile_max[((int64_t)kv * P.rows + t) * P.Tk + tile] = m;
+      for (int i = 1; i < 8; ++i) m = fmaxf(m, tmax[tile & 1][i][t]);
+      P.tile_max[((int64_t)kv * P.rows + t) * P.Tk + tile] = m;
+    }
   }
 }
 
 // Key tiles from the last to the first, as in attn.cu; a warp takes `run` of them, a CTA 4 * run.
 template <int D, int NT>
-__global__ __launch_bounds__(kThreads) void decode_output_kernel(const DecodeParams P) {
+__global__ __launch_bounds__(kThreads, NT == 1 ? 4 : 3) void decode_output_kernel(const DecodeParams P) {
   constexpr int MT = D / 16, RO = 8 * NT;
   __shared__ __align__(16) float o_s[kWarps][RO][D + 4];
   __shared__ float m_s[kWarps][RO], l_s[kWarps][RO];
@@ -302,7 +337,7 @@ __global__ __launch_bounds__(kThreads) void decode_output_kernel(const DecodePar
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float off = __uint_as_float(0xff800000u);
-        s[i] = live ? *reinterpret_cast<const float4*>(P.scores + row * ld + tile * kTile + 32 * tg + 4 * i)
+        s[i] = live ? *reinterpret_cast<const float4*>(P.scores + row * ld + tile * kTile + 16 * i + 4 * tg)
                     : make_float4(off, off, off, off);
       }
       const float m_new = fmaxf(m_run[n], live ? P.tile_max[row * P.Tk + tile] : kNoMax);
@@ -340,12 +375,12 @@ __global__ __launch_bounds__(kThreads) void decode_output_kernel(const DecodePar
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
       uint32_t v0[16], v1[16];
-      expand_row<128>(raw_row<128>(vc, vs, 16 * mt + g, tg), v0);
-      expand_row<128>(raw_row<128>(vc, vs, 16 * mt + g + 8, tg), v1);
+      expand_row(raw_keys(vc, vs, 16 * mt + g, tg), v0);
+      expand_row(raw_keys(vc, vs, 16 * mt + g + 8, tg), v1);
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) mma16816(o[n][mt], v0[2 * j], v1[2 * j], v0[2 * j + 1], v1[2 * j + 1], p[n][2 * j], p[n][2 * j + 1]);
+        for (int j = 0; j < 8; ++j) mma16816<false>(o[n][mt], v0[2 * j], v1[2 * j], v0[2 * j + 1], v1[2 * j + 1], p[n][2 * j], p[n][2 * j + 1]);
     }
   }
 
@@ -460,7 +495,16 @@ cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
   P.run = even > most ? even : most;
   P.chunks = (P.Tk + kWarps * P.run - 1) / (kWarps * P.run);
   const size_t frag = (size_t)(P.rows + 7) / 8 * 2 * 32 * (D / 8) * 4;         // 32 KB at most
-  cudaError_t e = launch_pdl(decode_scores_kernel<D>, dim3(P.Tk, P.kvs), kThreads, frag, stream, overlap, P);
+  // key tiles per CTA of the scores kernel: the fewest tile times on 148 SMs, a CTA's start counted as one
+  const int slots = 148 * (D == 128 ? 2 : 3);
+  int64_t best = INT64_MAX;
+  for (int run = 1; run <= 16; ++run) {
+    const int64_t ctas = (int64_t)((P.Tk + run - 1) / run) * P.kvs, cost = (ctas + slots - 1) / slots * (run + 1);
+    if (cost < best) { best = cost; P.score_run = run; }
+  }
+  const dim3 grid((P.Tk + P.score_run - 1) / P.score_run, P.kvs);
+  cudaError_t e = launch_pdl(P.rows <= 8 ? decode_scores_kernel<D, true> : decode_scores_kernel<D, false>, grid, kScoreThreads, frag, stream,
+                             overlap, P);
   if (e != cudaSuccess) return e;
   return launch_pdl(decode_output_kernel<D, NT>, dim3((unsigned)(P.kvs * P.chunks), groups), kThreads, 0, stream, true, P);
 }
