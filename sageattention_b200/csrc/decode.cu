@@ -511,9 +511,12 @@ cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
 
 }  // namespace
 
+// Against the tile kernels, whole operator (us): Nq=1 H32/8 Nk700 25 -> 14, Nk4096 70 -> 19; B16 H32/8 Nk4096, Nq=4 258 -> 166,
+// Nq=8 260 -> 212, but Nq=16 (64 rows) 262 -> 315; B4 H32 Nq=16 (16 rows) Nk4000 181 -> 163, Nk700 26 -> 27.  With two or three
+// key tiles there is nothing to split.
 bool decode_fits(int Hq, int Hkv, int Nq, int Nk) {
   const int rows = Hq / Hkv * Nq;
-  return Nk > 7 * kTile && rows <= kMaxRows && (Nq <= 4 || rows <= 8);
+  return Nk > 3 * kTile && rows <= kMaxRows && (Nq <= 8 || (Nq <= 16 && rows <= 32 && Nk > 1024));
 }
 
 size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D) {

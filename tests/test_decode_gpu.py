@@ -16,8 +16,8 @@ DEV = "cuda"
 # the fewest key tiles (and one fewer: the other kernel), a last tile of one key, key tiles that do not fill the runs, runs of
 # several tiles; 1, 8, 9, 16 and 17 rows per kv head and the most there can be; causal rows that see the last keys or not
 @pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,causal", [
-    (1, 2, 2, 1, 896, 128, False), (1, 2, 2, 1, 897, 128, False), (2, 4, 2, 4, 1023, 64, True), (1, 9, 1, 1, 1025, 64, False),
-    (1, 2, 2, 8, 1153, 128, True), (1, 4, 1, 4, 2000, 128, True), (1, 17, 1, 1, 1000, 128, False), (1, 64, 2, 4, 1100, 64, True),
+    (1, 2, 2, 1, 384, 128, False), (1, 2, 2, 1, 385, 128, False), (2, 4, 2, 4, 1023, 64, True), (1, 9, 1, 1, 1025, 64, False),
+    (1, 2, 2, 8, 1153, 128, True), (1, 4, 1, 4, 2000, 128, True), (1, 17, 1, 1, 1000, 128, False), (1, 16, 2, 8, 1100, 64, True), (1, 4, 2, 16, 1025, 128, True),
     (1, 2, 1, 2, 33000, 128, True), (1, 2, 1, 1, 65537, 64, False), (40, 32, 8, 1, 1500, 128, False)])
 def test_few_query_rows(B, Hq, Hkv, Nq, Nk, D, causal):
     q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, D, seed=Nq + Nk + D, device=DEV)
