@@ -16,11 +16,11 @@
 // memory; the [128 query blocks x 128 keys] result goes as bf16 through a swizzled staging tile in shared memory
 // and leaves with two TMA stores (whole 128-byte lines; rows beyond the last query block are clipped by the
 // tensor map).  HBM-bound: the output ([Tq x 128] bf16 per CTA and query head) dominates the traffic, in a chain of
-// dependent steps per CTA.  Up to 128 rows of A (kMulti = false) there is one round, and what counts is how many CTAs an
-// SM holds: the staging tile lies over the A tile, which has been consumed by then, and A comes by cp.async instead of
-// through registers - three CTAs per SM instead of two (B8 Hq32 Hkv8 Nk4096, one query: 77 -> 42 us).  Several rounds
-// want the next A tile on its way during the current one: it waits in registers, two CTAs per SM (B1 H40 N32760: 330 us;
-// 390 with three CTAs and no A ahead).
+// dependent steps per CTA.  So a CTA walks several key tiles of a head: tensor memory, barrier and K means are set up once, and
+// the next tile's rows are on their way (in the registers that the quantised tile leaves) during the MMAs and stores of the
+// present one (B4 H32 N4096 D64 52 -> 45 us, B1 H40 N9450 66 -> 57 us, B1 H40 N32760 327 -> 314 us; one tile per CTA with three
+// CTAs per SM was the best without that).  Up to 128 rows of A (kMulti = false) A is loaded once per CTA; with more, the next
+// 128 wait in registers during a round (390 us without).
 //
 // kPack: K-packing mode (pack.cu) on the way in - a tile is 8 groups of 16 slots, its 120 tokens are smoothed, laid out
 // and turned into mean and residuals by one warp per group, in place in the operand tile; the lambdas leave from here.
@@ -32,6 +32,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <cstdint>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -58,53 +59,52 @@ struct KDsParams {
   int Hkv, rows, Tk, Nk;                               // rows = query heads per kv head x query blocks per head
   const int* cu_k;
   int d_in;                                            // channels the K rows really have; the rest are zero
+  int run;                                             // key tiles per CTA
 };
 
 constexpr int kDsStageBytes = 2 * 128 * 128;          // output staging: [2 key halves][128 rows x 128 bytes], 128-byte swizzle
-// in front of the K tile: the staging tile and the A tile, or (one round) one place for both
-__host__ __device__ constexpr int ds_front_bytes(int D, bool multi) {
-  const int a = (D / 8) * (int)kChunk;
-  return multi ? kDsStageBytes + a : (a > kDsStageBytes ? a : kDsStageBytes);
-}
-
 template <int D, bool kMulti, bool kPack>
-__global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
+__global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __grid_constant__ CUtensorMap tm_ds,
                                                                       const KDsParams P) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   constexpr uint32_t kTileBytes = CH * kChunk;
   extern __shared__ uint8_t dyn_raw[];
   uint8_t* dyn_smem = dyn_raw + ((1024u - (smem_u32(dyn_raw) & 1023u)) & 1023u);   // the swizzled staging tile needs it
   uint8_t* stage = dyn_smem;                           // output staging (first: 1024-byte aligned)
-  uint8_t* sA = dyn_smem + (kMulti ? kDsStageBytes : 0);   // 128 Q block means [CH][kChunk]
-  uint8_t* sB = dyn_smem + ds_front_bytes(D, kMulti);  // smoothed K tile  [CH][kChunk]
+  uint8_t* sA = dyn_smem + kDsStageBytes;              // 128 Q block means [CH][kChunk]
+  uint8_t* sB = sA + kTileBytes;                       // smoothed K tile  [CH][kChunk]
   uint8_t* sf_smem = sB + kTileBytes;                  // 2048 B
   uint8_t* misc = sf_smem + 2048;                      // mbarrier (8 B), tensor-memory slot (4 B), abort flag (4 B)
   const uint32_t bar = smem_u32(misc), slot = smem_u32(misc + 8);
   int* abort_s = reinterpret_cast<int*>(misc + 12);
-  const int tile = blockIdx.x, bh = blockIdx.y, b = bh / P.Hkv, hkv = bh % P.Hkv;
+  const int first = blockIdx.x * P.run, bh = blockIdx.y, b = bh / P.Hkv, hkv = bh % P.Hkv;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, c = t % CH, rl = t / CH;
 
   // ---- the K tile: load, smooth, quantise, lay out as the B operand
   int Nk = P.Nk;
   if (P.cu_k != nullptr) {
     Nk = min(P.cu_k[b + 1] - P.cu_k[b], Nk);           // a packed batch: this sequence, cut at max_seqlen
-    if (tile * kTile >= Nk) {                          // beyond the sequence: nothing reads this tile or its delta_s
+    if (first * kTile >= Nk) {                          // beyond the sequence: nothing reads this tile or its delta_s
       pdl_wait();                                      // (this grid never ends before the one it follows)
       return;
     }
   }
   const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + c * 8;
-  // token in slot `row` of the tile (kPack: 16 slots hold 15 tokens, none the first)
-  auto token_of = [&](const int row) {
+  const int end = min(first + P.run, P.cu_k != nullptr ? (Nk + kTile - 1) / kTile : P.Tk);
+  // token in slot `row` of a tile (kPack: 16 slots hold 15 tokens, none the first)
+  auto token_of = [&](const int tile, const int row) {
     if (!kPack) return tile * kTile + row;
     return (row & 15) == 0 ? -1 : (tile * (kTile / 16) + (row >> 4)) * kGroup + (row & 15) - 1;
   };
   uint4 w[NP];
+  auto load = [&](const int tile) {
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {                       // all loads in flight before the first use
-    const int n = token_of(p * RPP + rl);
-    w[p] = (n >= 0 && n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
-  }
+    for (int p = 0; p < NP; ++p) {                     // all loads in flight before the first use
+      const int n = token_of(tile, p * RPP + rl);
+      w[p] = (n >= 0 && n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  load(first);
   if (t == 0) {
     mbar_init(bar, 1);
     *abort_s = 0;
@@ -114,7 +114,10 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     tmem_alloc(slot, 128);
     tmem_relinquish();
   }
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(misc + 8);
   // only now: the attention kernel that may come in takes all of tensor memory, and waits for this grid
   pdl_launch_dependents();
   pdl_wait();                                          // the sums and block means of the launch before
@@ -132,16 +135,25 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     }
   };
   if (!kMulti) load_a(0);
-  if (P.km != nullptr || P.partial != nullptr) {
+  const bool smooth = P.km != nullptr || P.partial != nullptr;
+  float2 neg[4];
+  if (smooth) {
     static_assert(kMaxChunks * D * 4 <= (int)kTileBytes, "partial rows of the K mean");
     float mean[8];
     k_mean<D>(P.km, P.partial + (int64_t)bh * P.chunks * D, P.chunks, (float)max(Nk, 1), bh, reinterpret_cast<float*>(sB),
-              tile == 0 ? P.km_out : nullptr, mean);
+              first == 0 ? P.km_out : nullptr, mean);
     __syncthreads();                                   // every thread has its means: sB takes the K tile
-    const float2 neg[4] = {{-mean[0], -mean[1]}, {-mean[2], -mean[3]}, {-mean[4], -mean[5]}, {-mean[6], -mean[7]}};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) neg[i] = make_float2(-mean[2 * i], -mean[2 * i + 1]);
+  }
+  bool ok = true;
+  uint32_t done = 0;                                   // rounds so far, of all tiles
+#pragma unroll 1
+  for (int tile = first; tile < end && ok; ++tile) {
+  if (smooth) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      if (const int n = token_of(p * RPP + rl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
+      if (const int n = token_of(tile, p * RPP + rl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
         w[p] = subtract_mean(w[p], neg);
       }
     }
@@ -186,30 +198,25 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     const int64_t kt = (int64_t)bh * P.Tk + tile;
     quant_rows_store<D>(w, P.k_codes + kt * (kTile * D / 2), P.k_sf + kt * ((D / 64) * 512), sf_smem);
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(misc + 8);
-
+  if (tile + 1 < end) load(tile + 1);
   // ---- delta_s: for the query blocks of all heads of the group, 128 at a time
   constexpr uint32_t idesc = make_idesc_bf16(128, 128);
   constexpr uint32_t HI = (128u >> 4) | (1u << 14);                     // 8-row groups 128 B apart, no swizzle
   const uint32_t a_lo = (smem_u32(sA) >> 4) | ((kChunk >> 4) << 16);    // leading (K) offset = one chunk
   const uint32_t b_lo = (smem_u32(sB) >> 4) | ((kChunk >> 4) << 16);
-  bool ok = true;
   const int rounds = kMulti ? (P.rows + 127) / 128 : 1;
   if (kMulti) load_a(0);
-  for (int round = 0; round < rounds && ok; ++round) {
+  for (int round = 0; round < rounds && ok; ++round, ++done) {
     if constexpr (kMulti) {
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const int row = p * RPP + rl;
         *reinterpret_cast<uint4*>(sA + c * kChunk + (row >> 3) * 128 + (row & 7) * 16) = a_next[p];
       }
-      if (t == 0) bulk_wait_read0();                   // the previous round's stores have left the staging tile
     } else {
       cp_async_wait_all();
     }
+    if (t == 0) bulk_wait_read0();                     // the previous round's stores have left the staging tile
     fence_proxy_async_smem();
     __syncthreads();
     if (t == 0) {
@@ -222,9 +229,9 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     if (kMulti && round + 1 < rounds) load_a(round + 1);
     // bounded: a few microseconds normally; gives up after about a second
     if (P.status != nullptr) {
-      ok = wait_bar_warp<false, (1u << 19)>(bar, round & 1, abort_s, P.status, 50);
+      ok = wait_bar_warp<false, (1u << 19)>(bar, done & 1, abort_s, P.status, 50);
     } else {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, round & 1, 1u << 19));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, done & 1, 1u << 19));
     }
     tc_fence_after();
     if (ok) {
@@ -259,10 +266,11 @@ __global__ void __launch_bounds__(kThreads, kMulti || kPack ? 2 : 3) k_quant_del
     tc_fence_before();
     ok = __syncthreads_and(ok);
   }
+  }
   if (t == 0) bulk_wait_read0();                       // the last stores have read the staging tile before the CTA ends
   if (!ok && t == 0) {
     // the MMAs issued last may still be running: give them time to drain before tensor memory is freed
-    mbar_wait(bar, (rounds - 1) & 1, 1u << 16);
+    mbar_wait(bar, (done - 1) & 1, 1u << 16);
   }
   tc_fence_before();
   __syncthreads();
@@ -284,7 +292,14 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   P.Tk = ((a.k_lambda ? (a.Nk + kGroup - 1) / kGroup * 16 : a.Nk) + 127) / 128;
   P.cu_k = a.cu_k;
   P.d_in = (a.d_in > 0 && a.d_in <= a.D) ? a.d_in : a.D;
-  dim3 grid(P.Tk, a.B * a.Hkv);
+  // key tiles per CTA: the fewest tile times on 148 SMs with two CTAs each, a CTA's start counted as one; at most two where
+  // lengths vary, since a CTA that has begun is not given to another sequence (16 prompts: 486 us, 500 with up to 16)
+  int64_t best = INT64_MAX;
+  for (int run = 1; run <= (a.cu_k != nullptr ? 2 : 16); ++run) {
+    const int64_t ctas = (int64_t)((P.Tk + run - 1) / run) * a.B * a.Hkv, cost = (ctas + 295) / 296 * (run + 1);
+    if (cost < best) { best = cost; P.run = run; }
+  }
+  const dim3 grid((P.Tk + P.run - 1) / P.run, a.B * a.Hkv);
   // delta_s as a 3-D bf16 tensor (key, query block of the GQA group, batch x kv head); store boxes of 64 keys x 128 rows
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return cudaErrorInvalidValue;
@@ -300,7 +315,7 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const bool multi = P.rows > 128;
-  const int smem = ds_front_bytes(a.D, multi) + (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
+  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
   static std::atomic<unsigned long long> ready[8];      // per kernel: devices on which the shared memory was asked for
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
