@@ -160,6 +160,8 @@ struct KParams {
   int64_t o_sb, o_sh, o_sn;
   int B, Hq, Hkv, Nq, Nk, Tq, Tk, ds_rows;
   int list_tiles;        // kList: query tiles of the heads of a kv head
+  int per_item;          // kList: how many of them make an item, 1 or 2, and
+  int list_items;        //   how many items that are
   float scale_log2;      // sm_scale * log2(e)
   const float* lam;      // K-packing mode: lambda per key slot, fp32 [B,Hkv,Tk*128]; Nk is the packed length
   int Nk_log;            // number of key tokens (= Nk unless packed)
@@ -308,19 +310,19 @@ __device__ __forceinline__ int work_at(const int r, const int total) {
 // head and query tile (>= Tq: there is none) of tile t of a work item
 template <bool kList>
 __device__ __forceinline__ int head_of(const KParams& P, const Work& k, const int t) {
-  return kList ? k.hq + (2 * k.pair + t) / P.Tq : k.hq;
+  return kList ? k.hq + (P.per_item * k.pair + t) / P.Tq : k.hq;
 }
 template <bool kList>
 __device__ __forceinline__ int tile_of(const KParams& P, const Work& k, const int t) {
-  const int u = 2 * k.pair + t;
-  if (!kList) return u;
-  return u < P.list_tiles ? u % P.Tq : P.Tq;
+  if (!kList) return 2 * k.pair + t;
+  const int u = P.per_item * k.pair + t;
+  return t < P.per_item && u < P.list_tiles ? u % P.Tq : P.Tq;
 }
 
 template <bool kCausal, bool kPacked, bool kList>
 __device__ __forceinline__ Work get_work(const KParams& P, const int w) {
   Work k;
-  const int n_pairs = ((kList ? P.list_tiles : P.Tq) + 1) >> 1;
+  const int n_pairs = kList ? P.list_items : (P.Tq + 1) >> 1;
   int bh;
 #if SAGE3_VARLEN_BUILD
   const int entry = P.order[w / P.Hq];
@@ -407,7 +409,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool has_ds = P.ds != nullptr;
 #if !SAGE3_VARLEN_BUILD
-  const int total_work = kList ? P.B * P.Hkv * ((P.list_tiles + 1) >> 1) : P.B * P.Hq * ((P.Tq + 1) >> 1);
+  const int total_work = kList ? P.B * P.Hkv * P.list_items : P.B * P.Hq * ((P.Tq + 1) >> 1);
 #endif
 
   if (threadIdx.x == 0) {
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           int64_t ds_row[2];
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
-            const int qt = 2 * wk.pair + t;
+            const int qt = (kList ? P.per_item : 2) * wk.pair + t;
             if (kList) ds_row[t] = ((int64_t)wk.b * P.Hq + head_of<kList>(P, wk, t)) * P.ds_rows + (P.ds_rows == 1 ? 0 : tile_of<kList>(P, wk, t));
             else ds_row[t] = ((int64_t)wk.b * P.Hq + wk.hq) * P.ds_rows + (P.ds_rows == 1 ? 0 : qt);
             if (ok && wk.n_t[t] > 0) {
@@ -1004,6 +1006,10 @@ bool make_out_map(CUtensorMap* m, const void* base, int B, int H, int N, int D, 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// At most one query tile per SM of a B200: one per item then (kList kernels), since an item of one takes three quarters of the
+// time of two (B1 H8 N1024 20.8 -> 16.4 us, B1 H32/8 N128 causal 10.2 -> 7.9 us).
+bool few_query_tiles(const AttnArgs& a) { return (int64_t)a.B * a.Hq * ((a.Nq + 127) / 128) <= 148; }
+
 template <int D, bool kCausal, bool kPacked, bool kList>
 cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   using L = Smem<D>;
@@ -1027,6 +1033,8 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.B = a.B; P.Hq = a.Hq; P.Hkv = a.Hkv; P.Nq = a.Nq; P.Nk = a.Nk; P.Tq = Tq; P.Tk = Tk; P.ds_rows = a.ds_rows;
   P.scale_log2 = a.sm_scale * kLog2e;
   P.list_tiles = a.Hq / a.Hkv * Tq;
+  P.per_item = few_query_tiles(a) ? 1 : 2;
+  P.list_items = (P.list_tiles + P.per_item - 1) / P.per_item;
   P.o_token_first = o_ndim == 1;
   P.lam = a.k_lambda;
   P.slot_first = kPacked && a.slot_first != 0;
@@ -1054,8 +1062,8 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total + 1024)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], sms, __ATOMIC_RELEASE);
   }
-  const int64_t work = kList ? (int64_t)a.B * a.Hkv * ((P.list_tiles + 1) / 2) : (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
   const int64_t ctas = sms - a.sm_margin > 1 ? sms - a.sm_margin : 1;
+  const int64_t work = kList ? (int64_t)a.B * a.Hkv * P.list_items : (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
   const int64_t grid = work < ctas ? work : ctas;
   return launch_pdl(kern, dim3((unsigned)grid), kAttnThreads, L::total + 1024, stream, a.after_delta_s, tq, tk, tv, to, P);
 }
@@ -1081,7 +1089,7 @@ cudaError_t launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
   // visit the same keys - one tile per head (decoding: B8 Hq32 Hkv8 Nk4096, 84 -> 62 us), or no causal mask.  (Kernels of
   // their own: the index arithmetic in the common ones cost those up to 5 %.)
   const int Tq = (a.Nq + 127) / 128;
-  if (a.Hq > a.Hkv && (Tq & 1) && (Tq == 1 || !a.causal)) {
+  if ((a.Hq > a.Hkv && (Tq & 1) && (Tq == 1 || !a.causal)) || few_query_tiles(a)) {
     if (a.D == 128) return a.causal ? launch<128, true, false, true>(a, stream) : launch<128, false, false, true>(a, stream);
     return a.causal ? launch<64, true, false, true>(a, stream) : launch<64, false, false, true>(a, stream);
   }

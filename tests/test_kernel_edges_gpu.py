@@ -84,3 +84,18 @@ def test_packing_operator_equals_its_parts(B, Hq, Hkv, Nq, Nk, D, causal, pbm, l
     z = sa.quantize_qkv(q, kp, vp, layout, per_block_mean=pbm, smooth_k=False)
     z.k_lambda, z.mean_slot_first, z.nk_slots = lam, not pbm, sa._lib.load().sage3_packed_len(Nk)
     assert torch.equal(got, sa.fp4_attention(z, is_causal=causal, tensor_layout=layout))
+
+
+# up to one query tile per SM: items of one tile, of a list that runs over the heads of a GQA group; and the sizes around that
+# many, causal or not
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,D,causal", [
+    (1, 148, 37, 100, 64, True), (1, 149, 149, 128, 64, False), (2, 37, 37, 200, 128, True), (1, 6, 2, 385, 128, False)])
+def test_one_query_tile_per_item(B, Hq, Hkv, Nq, D, causal):
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, 300, D, seed=Nq + Hq, device=DEV)
+    z = sa.quantize_qkv(q, k, v)
+    out, lse = sa.fp4_attention(z, is_causal=causal, return_lse=True, check_status=True)
+    want, want_lse = oracle_on_device_operands(z, D ** -0.5, causal, return_lse=True)
+    cos, l1 = sage3.accuracy(out.float().cpu(), want.to(torch.bfloat16).float())
+    assert torch.isfinite(out).all() and cos >= COS_MIN and l1 <= REL_L1_MAX, (cos, l1)
+    fin = torch.isfinite(want_lse)
+    assert torch.allclose(lse.cpu()[fin], want_lse[fin], atol=2e-3, rtol=1e-4)
