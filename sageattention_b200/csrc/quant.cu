@@ -35,7 +35,7 @@ namespace sage3 {
 // chunk of tokens -> one partial row [D].  Rows of a head are always added in chunk order, so the mean is deterministic
 // and does not depend on who adds them (this file's mean kernel, or k_mean in quant_rows.cuh).
 // ------------------------------------------------------------------------------------------------
-template <int D>
+template <int D, int U>                // U = passes in flight
 __device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict__ base, const int64_t sn, const int N,
                                                 const int chunk, const int chunk_tokens, const int d_in,
                                                 float* __restrict__ prow, float* red) {
@@ -46,15 +46,15 @@ __device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict_
   const int n0 = chunk * chunk_tokens;
   const int n1 = min(N, n0 + chunk_tokens);
   float2 acc[4] = {};
-  for (int n = n0 + rl; n < n1; n += RPP * 4) {
-    uint4 v[4];
+  for (int n = n0 + rl; n < n1; n += RPP * U) {
+    uint4 v[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       int nn = n + u * RPP;
       v[u] = (nn < n1 && c * 8 < d_in) ? *reinterpret_cast<const uint4*>(base + (int64_t)nn * sn) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) add_channels(acc, v[u]);
+    for (int u = 0; u < U; ++u) add_channels(acc, v[u]);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(red + rl * D + c * 8 + 2 * i) = acc[i];
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
     N = min(cu[b + 1] - cu[b], N);         // never beyond the caller's max_seqlen (the grid covers no more)
     divisor = (float)max(N, 1);
   }
-  channel_partial<D>(x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh, sn, N, chunk, chunk_tokens, d_in,
+  channel_partial<D, 4>(x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh, sn, N, chunk, chunk_tokens, d_in,
                      partial + ((int64_t)bh * nchunks + chunk) * D, red);
   __threadfence();
   __syncthreads();
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     bid -= P.s_first;
     const int chunk = bid % P.chunks, bh = bid / P.chunks, b = bh / P.Hkv, h = bh % P.Hkv;
     const int N = P.cu_k ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
-    channel_partial<D>(P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + h * P.k_sh, P.k_sn, N, chunk, P.chunk_tokens,
+    channel_partial<D, 8>(P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + h * P.k_sh, P.k_sn, N, chunk, P.chunk_tokens,
                        P.d_in, P.partial + (int64_t)bid * D, red);
     return;
   }
