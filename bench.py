@@ -633,7 +633,7 @@ def main():
                         "shorter than the slower direction (copy_bound_ms), than the operator (ms_per_step of the line) "
                         "or - when it overlaps them completely - than the two directions running at the same time "
                         "(copies_both_directions_ms)"},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": 3 * args.steps,
         "clocks": clocks,
     }
     if uly is not None:

@@ -278,5 +278,5 @@ def bench_ulysses(args, w, dist_mod, dev, ring: bool = False):
                        {"workload": "ulysses", "B": B, "H": H, "N": N, "D": D, "causal": w["causal"],
                         "sharding": f"sequence-sharded input, all-to-all to {H // world} heads per GPU, {chunks} head chunk(s)",
                         "step": "3 all-to-all + K mean + fused quant + delta_s + attention + 1 all-to-all"}),
-            "gpu_launches": 4 * (world if ring else chunks) * args.steps}), flush=True)
+            "gpu_launches": (4 * world if ring else 3 * chunks) * args.steps}), flush=True)
     dist_mod.destroy_process_group()
