@@ -424,12 +424,6 @@ cudaError_t launch_channel_mean(const void* x, int64_t sb, int64_t sh, int64_t s
                                 int d_in) {
   if (d_in <= 0 || d_in > D) d_in = D;
   int chunk = pick_chunk_tokens(N, B * H);
-  // here no other work fills the SMs' last turn, so no more CTAs than fit at once: larger chunks, if those are not more than
-  // the scratch has room for (B1 H40 N9450: 34.6 -> 28.4 us)
-  if (const int most = 1184 / (B * H); most > 0) {
-    const int larger = ((N + most - 1) / most + 63) / 64 * 64;
-    if (larger > chunk) chunk = larger;
-  }
   int nchunks = (N + chunk - 1) / chunk;
   size_t part = (size_t)B * H * nchunks * D * sizeof(float);
   part = (part + 255) & ~(size_t)255;
