@@ -11,7 +11,7 @@
 // memory.  Values are expanded to halves together with their block scale, which is exact (2 + 4 significant bits, 2^-10 ...
 // 2688), products are exact and sums fp32.  The order of elements along the contraction is free as long as both operands have
 // the same: a lane takes whole quantisation blocks of a row, so that maxima, scales and codes need no exchange between lanes.
-// What bounds it: on a full chip the conversions between the formats and their latencies (a third of the issue slots in use,
+// What bounds it: on a full chip the conversions between the formats and their latencies (half of the issue slots in use,
 // the tensor pipe 5 % busy, K at 2.7 TB/s), on few heads a chain of a few dependent loads.  Whole operator on the device,
 // against tiles of 128 query rows: B8 H32/8 Nk4096 131 -> 63 us, B1 70 -> 19, B3 H32/4 Nk16384 258 -> 56.
 #include <cuda_fp16.h>
