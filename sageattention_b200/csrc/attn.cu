@@ -185,12 +185,19 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-__device__ __forceinline__ float max16(const uint32_t* r) {
+__device__ __forceinline__ float fmax3_nan(float a, float b, float c) {      // NaN if any of them is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Largest of a 16-key block, NaNs left out.  `c` and `e` receive maxima over columns 6 to 8 and 12 to 14 that are NaN where
+// one of those is: the columns that ex2_poly takes are among them (see nan_of_poly_columns).
+__device__ __forceinline__ float max16(const uint32_t* r, float& c, float& e) {
   const float a = fmax3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
   const float b = fmax3(__uint_as_float(r[3]), __uint_as_float(r[4]), __uint_as_float(r[5]));
-  const float c = fmax3(__uint_as_float(r[6]), __uint_as_float(r[7]), __uint_as_float(r[8]));
+  c = fmax3_nan(__uint_as_float(r[6]), __uint_as_float(r[7]), __uint_as_float(r[8]));
   const float d = fmax3(__uint_as_float(r[9]), __uint_as_float(r[10]), __uint_as_float(r[11]));
-  const float e = fmax3(__uint_as_float(r[12]), __uint_as_float(r[13]), __uint_as_float(r[14]));
+  e = fmax3_nan(__uint_as_float(r[12]), __uint_as_float(r[13]), __uint_as_float(r[14]));
   return fmax3(fmax3(a, b, c), fmax3(d, e, __uint_as_float(r[15])), kNoMax);
 }
 
@@ -226,6 +233,7 @@ __device__ __forceinline__ void load_scores(const uint32_t tm_S, uint32_t (&s)[1
 // relative error (Remez exchange, computed for this file: 7.5e-8 in exact arithmetic, 2.1e-7 = 2^-22.2 evaluated in
 // fp32, the error bound of ex2.approx being 2^-22); n goes into the exponent bits.  x <= log2(6) here; below -125 (a
 // masked score) the result is 2^-125: code 0, and nothing beside the 6 that the block's largest value adds to its sum.
+// So is that of a NaN, which has to reach the row sum by another way: nan_of_poly_columns.
 __device__ __forceinline__ float2 ex2_poly(float2 x) {
   const auto both = [](const float v) { return make_float2(v, v); };
   x.x = fmaxf(x.x, -125.f); x.y = fmaxf(x.y, -125.f);
@@ -244,6 +252,17 @@ __device__ __forceinline__ float2 ex2_poly(float2 x) {
 // (B1 H10 N32760): D=128 3.98 / 3.75 / 3.65 / 3.72 ms, D=64 3.86 / 3.73 / 3.62 / 3.65 ms - more, and the 12
 // instructions per pair cost more issue slots than the unit's cycles they save.
 __device__ constexpr bool on_fma_pipe(const int blk, const int pair) { return pair == 3 || (pair == 6 && (blk & 1)); }
+// A NaN if one of the columns that take it has a NaN score, else a finite number or +inf, from the maxima that max16 leaves:
+// times 0 it goes into the row sum, so that such a row ends as one with a NaN in any other column does (its output zero, its
+// LSE NaN) whatever the place of the key.  (A row with a score of +inf has that sum anyhow: inf - inf.)  7 instructions per key
+// tile, 0.2 to 0.6 % of the kernel (B1 H40 N32760 D128 14.48 -> 14.57 ms); a select behind every polynomial would be 48.
+__device__ __forceinline__ float nan_of_poly_columns(const float (&c)[8], const float (&e)[8]) {
+  float x = kNoMax;
+#pragma unroll
+  for (int blk = 0; blk < 8; blk += 2) x = fmax3_nan(x, c[blk], c[blk + 1]);
+  x = fmax3_nan(x, e[1], e[3]);
+  return fmax3_nan(x, e[5], e[7]);
+}
 
 // P / blockscale = 2^(s*c - (bm*c + log2(1/6))) in [0, 6] -> E2M1 codes into this row's 16 tensor-memory columns of
 // P^ (8 codes per column, in key order - the A operand of the P.V MMA is read from there); returns the row sum of the unquantised P = sum over blocks of (sum of P/blockscale) * blockscale
@@ -740,7 +759,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             if (!(ok = wait_bar_soon(bar_s, sc & 1, abort_s, P.status, 30))) break;
             tc_fence_after();
             uint32_t s[128];
-            float bm[8];
+            float bm[8], c6[8], c12[8];
             load_scores(tm_S, s);
             // the scores are in registers: the Q.K^T of the other query tile may overwrite the buffer
             tc_fence_before();
@@ -773,11 +792,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               }
             }
 #pragma unroll
-            for (int blk = 0; blk < 8; ++blk) bm[blk] = max16(&s[16 * blk]);
+            for (int blk = 0; blk < 8; ++blk) bm[blk] = max16(&s[16 * blk], c6[blk], c12[blk]);
             const float m_loc = fmax3(fmax3(bm[0], bm[1], bm[2]), fmax3(bm[3], bm[4], bm[5]), fmaxf(bm[6], bm[7]));
             const float m_new = fmaxf(m_run, m_loc);
             const float alpha = ex2_approx((m_run - m_new) * c);
-            l *= alpha;
+            l = fmaf(nan_of_poly_columns(c6, c12), 0.f, l) * alpha;
             m_run = m_new;
             const float off = fmaf(m_new, c, kLog2Inv2688);       // P = 2^(s*c - off) in (0, 2688]
             float neg_e[8], sb[8];

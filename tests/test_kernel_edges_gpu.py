@@ -99,3 +99,33 @@ def test_one_query_tile_per_item(B, Hq, Hkv, Nq, D, causal):
     assert torch.isfinite(out).all() and cos >= COS_MIN and l1 <= REL_L1_MAX, (cos, l1)
     fin = torch.isfinite(want_lse)
     assert torch.allclose(lse.cpu()[fin], want_lse[fin], atol=2e-3, rtol=1e-4)
+
+
+# a key whose scores are NaN (K not smoothed, else every key is) at each place of a pair of 16-key blocks, of which some columns
+# take another exponential than the others: rows that see it are zero with a NaN LSE, rows that do not are as without it.  Two
+# tiles of query rows per item, one, packed sequences, and few query rows
+@pytest.mark.parametrize("Nq,D,causal,op", [(300, 128, False, "dense"), (300, 64, True, "dense"), (100, 128, True, "dense"),
+                                            (300, 64, False, "varlen"), (1, 128, False, "dense"), (4, 64, True, "dense")])
+def test_nan_score_counts_alike_at_every_key(Nq, D, causal, op):
+    H, Nk = 64, 600
+    q, k, v = U.make_qkv(1, H, H, Nq, Nk, D, seed=Nq + D, k_offset_std=0.0, device=DEV)
+
+    def run(k):
+        if op == "dense":
+            return sa.sageattn3_blackwell(q, k, v, is_causal=causal, smooth_k=False, return_lse=True, check_status=True)
+        cu = [torch.tensor([0, n], dtype=torch.int32, device=DEV) for n in (Nq, Nk)]
+        rows = [t[0].transpose(0, 1).contiguous() for t in (q, k, v)]
+        return sa.sageattn_varlen(*rows, *cu, Nq, Nk, is_causal=causal, smooth_k=False, check_status=True).transpose(0, 1)[None], None
+
+    want, want_lse = run(k)
+    key = Nk - 330 + torch.arange(H, device=DEV) + 128 * (torch.arange(H, device=DEV) % 2)
+    bad = k.clone()
+    bad[0, torch.arange(H, device=DEV), key, 5] = float("nan")
+    out, lse = run(bad)
+    last = torch.arange(Nq, device=DEV) + Nk - Nq if causal else torch.full((Nq,), Nk, device=DEV)   # last visible key
+    sees = last[None] >= key[:, None]
+    assert bool(sees.any()) and (Nq < 300 or not causal or not bool(sees.all()))
+    assert bool((out[0][sees] == 0).all()), sorted({int(h) % 32 for h in (out[0] != 0).any(-1).logical_and(sees).any(-1).nonzero()})
+    assert torch.equal(out[0][~sees], want[0][~sees])
+    if lse is not None:
+        assert bool(torch.isnan(lse[0][sees]).all()) and torch.equal(lse[0][~sees], want_lse[0][~sees])
