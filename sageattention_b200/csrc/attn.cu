@@ -48,7 +48,7 @@
 // (B4 Hq32 Hkv8 N8192 D128 causal: 1.79 -> 1.61 ms; B4 H32 N4096 D64: 0.815 -> 0.79 ms); all 32 lanes of a role warp
 // wait and one issues, because a wait executed by a single lane polls instead of parking and answers 40 cycles later;
 // waits for what has usually happened test once before they park (45 cycles instead of 120); the poll loop is a handful
-// of instructions in one asm block (left to the compiler it was unrolled at every wait); and 3 of 16 exponentials run on
+// of instructions in one asm block (left to the compiler it was unrolled at every wait) and uniform by a vote; and 3 of 16 exponentials run on
 // the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile.  At B1 H10 N32760 D128 the
 // kernel went from 3.86 to 3.63 ms (1560 cycles per key tile and 128 query rows; 61 % of the issue slots used).
 //
@@ -553,14 +553,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             __syncwarp();
           }
         }
-        if (*abort_s) {
+        if (__any_sync(0xffffffffu, *abort_s != 0)) {
           // giving up: the copies this thread started must land before the CTA may exit
           for (int t = 0; t < 2; ++t)
-            if (qn[t] > 0) mbar_wait(bars + Bars::q_full + 8 * t, (qn[t] - 1) & 1, 1u << 16);
+            if (qn[t] > 0) mbar_wait<true>(bars + Bars::q_full + 8 * t, (qn[t] - 1) & 1, 1u << 16);
           for (uint32_t i = (gk > (uint32_t)kStages ? gk - kStages : 0); i < gk; ++i)
-            mbar_wait(bars + Bars::k_full + 8 * (i % kStages), (i / kStages) & 1, 1u << 16);
+            mbar_wait<true>(bars + Bars::k_full + 8 * (i % kStages), (i / kStages) & 1, 1u << 16);
           for (uint32_t i = (g > (uint32_t)kStages ? g - kStages : 0); i < g; ++i)
-            mbar_wait(bars + Bars::v_full + 8 * (i % kStages), (i / kStages) & 1, 1u << 16);
+            mbar_wait<true>(bars + Bars::v_full + 8 * (i % kStages), (i / kStages) & 1, 1u << 16);
         }
       } else if (warp == 14 && has_ds) {
         // ---------------------------------------------------------------- delta_s -> rank-1 B operand
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         if (!ok) {
           // giving up: let every MMA / scale copy already issued finish before tensor memory is freed
           if (lane == 0) tc_commit(bars + Bars::drain);
-          mbar_wait(bars + Bars::drain, 0, 1u << 16);
+          mbar_wait<true>(bars + Bars::drain, 0, 1u << 16);
         }
       } else if (warp == 15) {
         // ---------------------------------------------------------------- PV issuer
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         }
         if (!ok) {
           if (lane == 0) tc_commit(bars + Bars::drain + 8);
-          mbar_wait(bars + Bars::drain + 8, 0, 1u << 16);
+          mbar_wait<true>(bars + Bars::drain + 8, 0, 1u << 16);
         }
       }
     } else {

@@ -155,73 +155,57 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// One poll of an mbarrier phase.  kHintNs > 0: try_wait with a suspend-time hint (measured on B200: a failing
-// poll returns after about 4 us whatever the hint); 0: try_wait without hint (about 1.5 us); < 0: a plain test
-// that never parks (7 ns).  A parked thread resumes as soon as the phase completes.
-template <int kHintNs = 0>
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+// One look at an mbarrier phase, without parking.  (Measured on B200: 7 ns; a failing try_wait of a whole warp returns after 4 us,
+// with and without a suspend-time hint.  A parked thread resumes as soon as the phase completes.)
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  if constexpr (kHintNs > 0) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"((uint32_t)kHintNs) : "memory");
-  } else if constexpr (kHintNs == 0) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  } else {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  }
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
 // Bounded wait: polls until the phase completes, at most `limit` times, and says whether it did.  The loop is one asm
 // block of a handful of instructions: left to the compiler it was unrolled at every one of the kernels' many waits,
-// and the instruction cache paid for it.
-template <int kHintNs = 0>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = (1u << 26)) {
+// and the instruction cache paid for it.  kWarp: by all 32 lanes of a warp, which leave it together and with the same answer,
+// each poll being a vote.
+template <bool kWarp = false, bool kHinted = false>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
   uint32_t ok;
-  if constexpr (kHintNs > 0) {
-    asm volatile(
-        "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\n"
-        "POLL:\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n"
-        "@p bra DONE;\n"
-        "add.u32 n, n, -1;\n"
-        "setp.ne.u32 p, n, 0;\n"
-        "@p bra POLL;\n"
-        "DONE:\n"
-        "min.u32 %0, n, 1;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit), "r"((uint32_t)kHintNs) : "memory");
-  } else {
-    asm volatile(
-        "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\n"
-        "POLL:\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "@p bra DONE;\n"
-        "add.u32 n, n, -1;\n"
-        "setp.ne.u32 p, n, 0;\n"
-        "@p bra POLL;\n"
-        "DONE:\n"
-        "min.u32 %0, n, 1;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
-  }
+#define SAGE3_WAIT(TRY, VOTE)                                                                   \
+  "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\nPOLL:\n"                                    \
+  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2" TRY ";\n" VOTE                         \
+  "@p bra DONE;\nadd.u32 n, n, -1;\nsetp.ne.u32 p, n, 0;\n@p bra POLL;\nDONE:\nmin.u32 %0, n, 1;\n}"
+#define SAGE3_VOTE "vote.sync.all.pred p, p, 0xffffffff;\n"
+  if constexpr (kWarp && kHinted)
+    asm volatile(SAGE3_WAIT(", %4", SAGE3_VOTE) : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit), "r"(20000u) : "memory");
+  else if constexpr (kWarp)
+    asm volatile(SAGE3_WAIT("", SAGE3_VOTE) : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+  else
+    asm volatile(SAGE3_WAIT("", "") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+#undef SAGE3_VOTE
+#undef SAGE3_WAIT
   return ok != 0;
 }
 
-// Bounded wait of the kernels' roles.  A failing poll takes 80 ns (a lone lane, or a busy CTA) to 4 us (a parked
-// warp), so the default limit is 0.15 to 8 seconds.  On giving up it raises the CTA's abort flag, records `code` in
+// Bounded wait of a whole warp of one of the kernels' roles.  On giving up it raises the CTA's abort flag, records `code` in
 // *status (first writer wins) and returns false - the caller then unwinds instead of hanging the SM.
-template <bool kHinted, uint32_t kPolls = (1u << 21)>
+//
+// The warp goes on to warp-wide instructions (tcgen05.ld / st, __syncwarp), so it must never split on a wait that ran out for
+// some of its lanes only: each poll is a vote.  That also lets the compiler treat the loops as uniform, without the code that
+// brings diverged lanes together again (16 prompts 484 -> 476 us; one vote behind a loop that is not uniform cost 6 %).
+//
+// The limit.  A failing poll takes 80 ns (a busy CTA) to 4 us (a parked warp): the default gives up after 0.02 to 1.05
+// seconds, where the longest wait of a working kernel is some 10 us.  A warp that waits does not look whether another
+// has given up: all of them wait for one another, so each runs out its own limit at about the same time, and that is why it
+// is not longer.  Looking at the flags every 1024 polls - never reached unless something is wrong - costs 2 to 25 % of the
+// attention kernel, by the room its instructions take at every wait (B1 H40 N32760 D128, 16 prompts: in the loop's slow part
+// 14.5 -> 16.4 ms, 484 -> 551 us; behind the loop 15.8, 598; one load per failing poll 14.8, 504; a function of its own does
+// not compile beside setmaxnreg).
+template <bool kHinted, uint32_t kPolls = (1u << 18)>
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  if (mbar_wait<kHinted ? 20000 : 0>(bar, parity, kPolls)) return true;
+  if (mbar_wait<true, kHinted>(bar, parity, kPolls)) return true;
   *abort_s = 1;
   atomicCAS(status, 0, code);
   return false;
@@ -230,15 +214,8 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
 // The same for a phase that has usually completed by now: a plain test first (17 cycles; a try_wait on a completed
 // phase takes 160), then the parking wait.
 __device__ __forceinline__ bool wait_bar_soon(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  if (mbar_try_wait<-1>(bar, parity)) return true;
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   return wait_bar<false>(bar, parity, abort_s, status, code);
-}
-
-// The same for a whole warp that goes on to warp-wide instructions (tcgen05.ld / st, votes): every lane gets the
-// same answer, so the warp never splits on a wait that ran out for some of its lanes only.
-template <bool kHinted, uint32_t kPolls = (1u << 21)>
-__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  return __all_sync(0xffffffffu, wait_bar<kHinted, kPolls>(bar, parity, abort_s, status, code));
 }
 
 // Programmatic dependent launch: let the next kernel of the stream start its prologue / wait until the previous one is

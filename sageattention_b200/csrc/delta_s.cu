@@ -229,9 +229,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
     if (kMulti && round + 1 < rounds) load_a(round + 1);
     // bounded: a few microseconds normally; gives up after about a second
     if (P.status != nullptr) {
-      ok = wait_bar_warp<false, (1u << 19)>(bar, done & 1, abort_s, P.status, 50);
+      ok = wait_bar<false>(bar, done & 1, abort_s, P.status, 50);
     } else {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, done & 1, 1u << 19));
+      ok = mbar_wait<true>(bar, done & 1, 1u << 18);
     }
     tc_fence_after();
     if (ok) {
