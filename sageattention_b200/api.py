@@ -351,25 +351,31 @@ class _Plan:
     __slots__ = ("pad", "device", "workspace", "lse_shape", "struct", "args", "run")
 
 
-def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin, packed=False) -> _Plan:
-    lib = _lib.load()
-    _check_device(q)
+def _check_qkv(q, k, v, tensor_layout):
+    """The operator's conditions on the tensors but for where they are; their sizes and strides."""
     for t in (q, k, v):
         if t.dtype != torch.bfloat16:
             raise AssertionError("TODO: support inputs other than bfloat16")     # api.py:257
-    B, Hq, Nq, D, qsb, qsh, qsn = _as_bhnd_strides(q, tensor_layout)
-    Bk, Hkv, Nk, Dk, ksb, ksh, ksn = _as_bhnd_strides(k, tensor_layout)
-    Bv, Hv, Nv, Dv, vsb, vsh, vsn = _as_bhnd_strides(v, tensor_layout)
-    if not (B == Bk == Bv and D == Dk == Dv and Hkv == Hv and Nk == Nv):
+    dq, dk, dv = (_as_bhnd_strides(t, tensor_layout) for t in (q, k, v))
+    B, Hq, _, D = dq[:4]
+    if dk[:4] != dv[:4] or dk[0] != B or dk[3] != D:
         raise ValueError("q, k, v shapes do not match")
-    if Hq % Hkv != 0:
+    if Hq % dk[1] != 0:
         raise ValueError("num_qo_heads must be a multiple of num_kv_heads")
+    if D > 128:
+        raise ValueError(f"Unsupported head_dim: {D}")                            # core.py:937
+    return dq, dk, dv
+
+
+def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin, packed=False) -> _Plan:
+    lib = _lib.load()
+    _check_device(q)
+    ((B, Hq, Nq, D, qsb, qsh, qsn), (_, Hkv, Nk, _, ksb, ksh, ksn),
+     (_, _, _, _, vsb, vsh, vsn)) = _check_qkv(q, k, v, tensor_layout)
     # head-dim padding of sageattention/core.py:925-937: below 64 -> 64, between 64 and 128 -> 128, zeros in the
     # extra channels, default scale from the original head dim, output cut back (:990).  The kernels read rows of the
     # original width and take the rest as zero, so nothing is copied - if the width is a multiple of 8 (16-byte
     # loads); other widths are padded before the call.
-    if D > 128:
-        raise ValueError(f"Unsupported head_dim: {D}")                            # core.py:937
     p = _Plan()
     Dp = 64 if D <= 64 else 128
     p.pad = 0 if D % 8 == 0 else Dp - D
@@ -473,9 +479,9 @@ def _host_piece_bytes(total: int) -> int:
 
 def _host_pieces(B: int, Hkv: int, head_bytes: int, head_chunks) -> list:
     """Pieces (first, last + 1 batch entry, first, last + 1 kv head) in which a host tensor goes through the GPU, each
-    contiguous in host memory: some heads of one batch entry, or some whole batch entries.  Several heads at a time
-    ramp up from one head at the start and down to one at the
-    end, so that the first kernel starts after a small copy and little is left to copy out after the last."""
+    contiguous in host memory: some heads of one batch entry (a share of one in ``head_chunks`` at least), or some whole
+    batch entries.  Several heads at a time ramp up from one head at the start and down to one at the end, so that the first
+    kernel starts after a small copy and little is left to copy out after the last."""
     want = _host_piece_bytes(B * Hkv * head_bytes)
     if isinstance(head_chunks, (list, tuple)):
         sizes = [int(n) for n in head_chunks]                    # explicit group sizes (kv heads per group)
@@ -487,7 +493,7 @@ def _host_pieces(B: int, Hkv: int, head_bytes: int, head_chunks) -> list:
         if entries >= 1 or int(head_chunks) <= 1:
             n = max(1, entries)
             return [(b, min(b + n, B), 0, Hkv) for b in range(0, B, n)]
-        base = max(1, round(want / head_bytes))
+        base = max(1, round(want / head_bytes), -(-Hkv // int(head_chunks)))
         ramp = [n for n in (1, 2, 4) if n < base]
         plan = []
         for b in range(B):
@@ -509,8 +515,8 @@ def sageattn_from_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: O
                        device=None, head_chunks=8, is_causal: bool = False, sm_scale: Optional[float] = None,
                        **kwargs) -> torch.Tensor:
     """Attention on HOST tensors (HND ``[B,H,N,D]`` bf16, ideally pinned): they go through the GPU in pieces of some kv
-    heads of a batch entry, or of some whole batch entries where these are small (``head_chunks`` = 1: never less than a
-    whole entry; a list: the kv heads per piece), and the host-to-device copy of piece ``i+1`` and the device-to-host
+    heads of a batch entry, or of some whole batch entries where these are small (``head_chunks``: into how many pieces an
+    entry is cut at most, not counting smaller ones at the very start and end; or a list: the kv heads per piece), and the host-to-device copy of piece ``i+1`` and the device-to-host
     copy of piece ``i-1`` run on their own streams while piece ``i`` is computed (pieces alternate between two compute
     streams so that their kernels overlap at the seams), so the
     PCIe transfers hide behind the kernels (or the other way round).  Returns the output as a host tensor
@@ -519,47 +525,53 @@ def sageattn_from_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: O
     the host must still synchronise before reading ``out``."""
     if q.is_cuda or k.is_cuda or v.is_cuda:
         raise ValueError("sageattn_from_host takes host tensors; use sageattn for device tensors")
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    B, Hq, Nq, D = q.shape
-    Hkv = k.shape[1]
-    if Hq % Hkv != 0:
-        raise ValueError("num_qo_heads must be a multiple of num_kv_heads")
+    # what the operator would refuse is refused before any copy is queued
+    if kwargs.get("attn_mask") is not None:
+        raise NotImplementedError("attn_mask is not supported (the reference ignores it as well)")
+    if kwargs.get("return_lse"):
+        raise TypeError("sageattn_from_host returns no log-sum-exp")
+    (B, Hq, *_), (_, Hkv, *_), _ = _check_qkv(*(torch.empty(t.shape, dtype=t.dtype, device="meta") for t in (q, k, v)), "HND")
     g = Hq // Hkv
+    pieces = _host_pieces(B, Hkv, (q.numel() + k.numel() + v.numel()) * q.element_size() // (B * Hkv), head_chunks)
+    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     if out is None:
         out = torch.empty_like(q).pin_memory()
-    pieces = _host_pieces(B, Hkv, (q.numel() + k.numel() + v.numel()) * q.element_size() // (B * Hkv), head_chunks)
     if dev not in _host_streams:
         _host_streams[dev] = tuple(torch.cuda.Stream(dev) for _ in range(4))
-    s_in, s_run_a, s_run_b, s_out = _host_streams[dev]
+    s_in, s_run_a, s_run_b, s_out = streams = _host_streams[dev]
     cur = torch.cuda.current_stream(dev)
     # whole-problem buffers from the current stream's pool: everything below starts after that stream's present end and
     # it waits for everything below, so they need no further bookkeeping
     qd, kd, vd = (torch.empty(t.shape, dtype=t.dtype, device=dev) for t in (q, k, v))
     start = cur.record_event()
-    for st in (s_in, s_run_a, s_run_b, s_out):
+    for st in streams:
         st.wait_event(start)
     keep = []
-    for i, (b0, b1, h0, h1) in enumerate(pieces):
-        sq, sk = (slice(b0, b1), slice(h0 * g, h1 * g)), (slice(b0, b1), slice(h0, h1))
-        with torch.cuda.stream(s_in):
-            qd[sq].copy_(q[sq], non_blocking=True)
-            kd[sk].copy_(k[sk], non_blocking=True)
-            vd[sk].copy_(v[sk], non_blocking=True)
-            ev_in = s_in.record_event()
-        # the attention kernel is persistent (one CTA per SM): on two streams in turn, the kernels of the next piece fill
-        # the SMs that the last, partly filled round of this piece leaves idle
-        s_run = s_run_b if i % 2 else s_run_a
-        with torch.cuda.stream(s_run):
-            s_run.wait_event(ev_in)
-            o = sageattn3_blackwell(qd[sq], kd[sk], vd[sk], tensor_layout="HND", is_causal=is_causal, sm_scale=sm_scale, **kwargs)
-            ev_run = s_run.record_event()
-        with torch.cuda.stream(s_out):
-            s_out.wait_event(ev_run)
-            out[sq].copy_(o, non_blocking=True)
-        keep.append(o)
-    for st in (s_out, s_run_a, s_run_b):          # nothing of this call may outlive the caller's next operation
-        cur.wait_event(st.record_event())
-    # the outputs came from the compute streams' pools: tell the allocator that the current stream orders their reuse
-    for o in keep:
-        o.record_stream(cur)
+    try:
+        for i, (b0, b1, h0, h1) in enumerate(pieces):
+            sq, sk = (slice(b0, b1), slice(h0 * g, h1 * g)), (slice(b0, b1), slice(h0, h1))
+            with torch.cuda.stream(s_in):
+                qd[sq].copy_(q[sq], non_blocking=True)
+                kd[sk].copy_(k[sk], non_blocking=True)
+                vd[sk].copy_(v[sk], non_blocking=True)
+                ev_in = s_in.record_event()
+            # the attention kernel is persistent (one CTA per SM): on two streams in turn, the kernels of the next piece
+            # fill the SMs that the last, partly filled round of this piece leaves idle
+            s_run = s_run_b if i % 2 else s_run_a
+            with torch.cuda.stream(s_run):
+                s_run.wait_event(ev_in)
+                o = sageattn3_blackwell(qd[sq], kd[sk], vd[sk], tensor_layout="HND", is_causal=is_causal, sm_scale=sm_scale, **kwargs)
+                keep.append(o)
+                ev_run = s_run.record_event()
+            with torch.cuda.stream(s_out):
+                s_out.wait_event(ev_run)
+                out[sq].copy_(o, non_blocking=True)
+    finally:
+        # nothing of this call may outlive the caller's next operation - also where a piece failed: copies into the buffers,
+        # which the current stream's pool is about to get back, are under way then
+        for st in streams:
+            cur.wait_event(st.record_event())
+        # the outputs came from the compute streams' pools: tell the allocator that the current stream orders their reuse
+        for o in keep:
+            o.record_stream(cur)
     return out
