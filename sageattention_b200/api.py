@@ -21,6 +21,7 @@ from __future__ import annotations
 import contextlib
 import ctypes as C
 import math
+import threading
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
@@ -335,15 +336,18 @@ def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
 
 # What a call with given shapes, strides and options needs, worked out once: the checks, the sizes and the argument
 # struct but for its pointers (a call on the smallest problems took 42 us of host time, 15 us of it this).  Read-only
-# after it is made, so that threads may share it; no device memory is held.
+# after it is made, so that threads may share it; no device memory is held.  The oldest plan makes room for a new one: in
+# generation every token has another Nk, whose plan serves the layers of one step and must not take the others with it.
 _MAX_PLANS = 1024
 _plans = {}
+_plans_lock = threading.Lock()
 
 
 def _keep_plan(key, plan):
-    if len(_plans) >= _MAX_PLANS:
-        _plans.clear()
-    _plans[key] = plan
+    with _plans_lock:
+        while len(_plans) >= _MAX_PLANS:
+            del _plans[next(iter(_plans))]
+        _plans[key] = plan
     return plan
 
 
@@ -356,15 +360,16 @@ def _check_qkv(q, k, v, tensor_layout):
     for t in (q, k, v):
         if t.dtype != torch.bfloat16:
             raise AssertionError("TODO: support inputs other than bfloat16")     # api.py:257
-    dq, dk, dv = (_as_bhnd_strides(t, tensor_layout) for t in (q, k, v))
-    B, Hq, _, D = dq[:4]
-    if dk[:4] != dv[:4] or dk[0] != B or dk[3] != D:
+    dims = B, Hq, _, D, _, _, _ = _as_bhnd_strides(q, tensor_layout)
+    dims_k = Bk, Hkv, Nk, Dk, _, _, _ = _as_bhnd_strides(k, tensor_layout)
+    dims_v = Bv, Hv, Nv, Dv, _, _, _ = _as_bhnd_strides(v, tensor_layout)
+    if not (B == Bk == Bv and D == Dk == Dv and Hkv == Hv and Nk == Nv):
         raise ValueError("q, k, v shapes do not match")
-    if Hq % dk[1] != 0:
+    if Hq % Hkv != 0:
         raise ValueError("num_qo_heads must be a multiple of num_kv_heads")
     if D > 128:
         raise ValueError(f"Unsupported head_dim: {D}")                            # core.py:937
-    return dq, dk, dv
+    return dims, dims_k, dims_v
 
 
 def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smooth_k, sm_margin, packed=False) -> _Plan:

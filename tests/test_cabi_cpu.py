@@ -137,3 +137,21 @@ def test_varlen_entry_refuses_bad_arguments_without_a_gpu():
     a = _lib.VarlenArgs()
     assert lib.sage3_attention_varlen(C.byref(a), None) == _lib.ERR_ARGUMENT      # no workspace / tensors
     assert lib.sage3_attention_varlen(None, None) == _lib.ERR_ARGUMENT
+
+
+def test_plans_of_lengths_that_do_not_come_back_push_out_the_oldest_only(monkeypatch):
+    """A generation loop has a new key length, and so a new plan, on every token; threads may add plans at once."""
+    import threading
+    from sageattention_b200 import api
+    monkeypatch.setattr(api, "_plans", {})
+    monkeypatch.setattr(api, "_MAX_PLANS", 64)
+    for i in range(100):
+        assert api._keep_plan(("len", i), i) == i
+        assert len(api._plans) == min(i + 1, 64)
+    assert list(api._plans.values()) == list(range(36, 100))
+    threads = [threading.Thread(target=lambda t=t: [api._keep_plan((t, i), i) for i in range(2000)]) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(api._plans) == 64
