@@ -129,7 +129,9 @@ typedef struct {
                                 The attention kernel is persistent, one CTA per SM, with a static work
                                 list: a CTA that finds its SM taken starts late and finishes late.  It
                                 launches min(work items, SMs - sm_margin) CTAs; results do not depend
-                                on it.  The reference has no counterpart.                            */
+                                on it.  Of no effect where sage3_attention takes the kernels for few
+                                query rows per head: short CTAs, dealt out to whatever SM is free.
+                                The reference has no counterpart.                                    */
 } sage3_attn_args;
 
 typedef struct {

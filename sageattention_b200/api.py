@@ -298,7 +298,8 @@ def sageattn3_blackwell(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tenso
     ``sm_margin`` (no counterpart in the reference): the attention kernel is persistent with one CTA per SM and a
     static work list, so a CTA whose SM is held by another kernel - a collective running beside it on another
     stream - starts late and the whole launch ends late.  With ``sm_margin = m`` it launches on ``SMs - m`` SMs
-    only; the result is the same bit for bit.
+    only; the result is the same bit for bit.  It is that kernel's: the quantisation kernels, and those that take its
+    place for few query rows per head, are many short CTAs which the hardware deals out to whatever SM is free.
     """
     if attn_mask is not None:
         raise NotImplementedError("attn_mask is not supported (the reference ignores it as well)")

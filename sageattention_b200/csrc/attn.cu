@@ -1025,12 +1025,22 @@ bool make_out_map(CUtensorMap* m, const void* base, int B, int H, int N, int D, 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// At most one query tile per SM of a B200: one per item then (kList kernels), since an item of one takes three quarters of the
-// time of two (B1 H8 N1024 20.8 -> 16.4 us, B1 H32/8 N128 causal 10.2 -> 7.9 us).
-bool few_query_tiles(const AttnArgs& a) { return (int64_t)a.B * a.Hq * ((a.Nq + 127) / 128) <= 148; }
+// At most one query tile per CTA that may run: one per item then (kList kernels), since an item of one takes three quarters of
+// the time of two (B1 H8 N1024 20.8 -> 16.4 us, B1 H32/8 N128 causal 10.2 -> 7.9 us).  CTAs, not SMs: with a margin and a tile
+// count between the two, single tiles would take two rounds where pairs take one (B1 H32/8 N512, margin 25: 20.5 -> 16.4 us; B1
+// H6/2 N3000, margin 8: 68 -> 49.6 us, but causal, where the second round is of lighter tiles, 39 -> 49).
+bool few_query_tiles(const AttnArgs& a, const int ctas) { return (int64_t)a.B * a.Hq * ((a.Nq + 127) / 128) <= ctas; }
+
+// CTAs of the persistent kernel: one per SM (registers and tensor memory allow exactly one) but for those left free
+cudaError_t cta_count(const AttnArgs& a, int* ctas) {
+  int sms = 0;
+  const cudaError_t e = sm_count(&sms);
+  *ctas = sms - a.sm_margin > 1 ? sms - a.sm_margin : 1;
+  return e;
+}
 
 template <int D, bool kCausal, bool kPacked, bool kList>
-cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
+cudaError_t launch(const AttnArgs& a, const int ctas, cudaStream_t stream) {
   using L = Smem<D>;
   const int Tq = (a.Nq + 127) / 128, Tk = (a.Nk + 127) / 128;
   CUtensorMap tq, tk, tv;
@@ -1052,7 +1062,7 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.B = a.B; P.Hq = a.Hq; P.Hkv = a.Hkv; P.Nq = a.Nq; P.Nk = a.Nk; P.Tq = Tq; P.Tk = Tk; P.ds_rows = a.ds_rows;
   P.scale_log2 = a.sm_scale * kLog2e;
   P.list_tiles = a.Hq / a.Hkv * Tq;
-  P.per_item = few_query_tiles(a) ? 1 : 2;
+  P.per_item = few_query_tiles(a, ctas) ? 1 : 2;
   P.list_items = (P.list_tiles + P.per_item - 1) / P.per_item;
   P.o_token_first = o_ndim == 1;
   P.lam = a.k_lambda;
@@ -1065,23 +1075,19 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
   P.order = a.order; P.n_order = a.n_order;
 #endif
   auto kern = attn_fwd_kernel<D, kCausal, kPacked, kList>;
-  // persistent CTAs: one per SM (registers and tensor memory allow exactly one), each walks the work list
-  int dev = 0, sms = 0;
+  int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  // once per device and instantiation: look up its SM count, opt in to the shared memory, and make sure the register
-  // hand-over inside the kernel stays within the pool this build of it is launched with (it would block forever otherwise)
-  static int ready[64] = {};                               // SM count
-  if (dev >= 0 && dev < 64) sms = __atomic_load_n(&ready[dev], __ATOMIC_ACQUIRE);
-  if (sms == 0) {
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  // once per device and instantiation: opt in to the shared memory, and make sure the register hand-over inside the kernel
+  // stays within the pool this build of it is launched with (it would block forever otherwise)
+  static bool ready[64] = {};
+  if (dev >= 64 || !__atomic_load_n(&ready[dev], __ATOMIC_ACQUIRE)) {
     cudaFuncAttributes fa;
     if ((e = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess) return e;
     if (fa.numRegs * kAttnThreads < 256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role)) return cudaErrorLaunchOutOfResources;
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total + 1024)) != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) __atomic_store_n(&ready[dev], sms, __ATOMIC_RELEASE);
+    if (dev < 64) __atomic_store_n(&ready[dev], true, __ATOMIC_RELEASE);
   }
-  const int64_t ctas = sms - a.sm_margin > 1 ? sms - a.sm_margin : 1;
   const int64_t work = kList ? (int64_t)a.B * a.Hkv * P.list_items : (int64_t)a.B * a.Hq * ((Tq + 1) / 2);
   const int64_t grid = work < ctas ? work : ctas;
   return launch_pdl(kern, dim3((unsigned)grid), kAttnThreads, L::total + 1024, stream, a.after_delta_s, tq, tk, tv, to, P);
@@ -1093,27 +1099,31 @@ cudaError_t launch(const AttnArgs& a, cudaStream_t stream) {
 cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream) {
   // offsets come in pairs; no K-packing and no LSE for packed batches
   if (a.cu_q == nullptr || a.cu_k == nullptr || a.order == nullptr || a.n_order == nullptr || a.k_lambda != nullptr || a.lse != nullptr) return cudaErrorInvalidValue;
-  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, stream) : launch<128, false, false, false>(a, stream);
-  if (a.D == 64) return a.causal ? launch<64, true, false, false>(a, stream) : launch<64, false, false, false>(a, stream);
+  int ctas;
+  if (cudaError_t e = cta_count(a, &ctas); e != cudaSuccess) return e;
+  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, ctas, stream) : launch<128, false, false, false>(a, ctas, stream);
+  if (a.D == 64) return a.causal ? launch<64, true, false, false>(a, ctas, stream) : launch<64, false, false, false>(a, ctas, stream);
   return cudaErrorInvalidValue;
 }
 #else
 cudaError_t launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
   if (a.D != 128 && a.D != 64) return cudaErrorInvalidValue;
+  int ctas;
+  if (cudaError_t e = cta_count(a, &ctas); e != cudaSuccess) return e;
   if (a.k_lambda) {
-    if (a.D == 128) return a.causal ? launch<128, true, true, false>(a, stream) : launch<128, false, true, false>(a, stream);
-    return a.causal ? launch<64, true, true, false>(a, stream) : launch<64, false, true, false>(a, stream);
+    if (a.D == 128) return a.causal ? launch<128, true, true, false>(a, ctas, stream) : launch<128, false, true, false>(a, ctas, stream);
+    return a.causal ? launch<64, true, true, false>(a, ctas, stream) : launch<64, false, true, false>(a, ctas, stream);
   }
   // Query tiles paired across the heads of a GQA group: where every head has an odd number of them, and the two of a pair
   // visit the same keys - one tile per head (decoding: B8 Hq32 Hkv8 Nk4096, 84 -> 62 us), or no causal mask.  (Kernels of
   // their own: the index arithmetic in the common ones cost those up to 5 %.)
   const int Tq = (a.Nq + 127) / 128;
-  if ((a.Hq > a.Hkv && (Tq & 1) && (Tq == 1 || !a.causal)) || few_query_tiles(a)) {
-    if (a.D == 128) return a.causal ? launch<128, true, false, true>(a, stream) : launch<128, false, false, true>(a, stream);
-    return a.causal ? launch<64, true, false, true>(a, stream) : launch<64, false, false, true>(a, stream);
+  if ((a.Hq > a.Hkv && (Tq & 1) && (Tq == 1 || !a.causal)) || few_query_tiles(a, ctas)) {
+    if (a.D == 128) return a.causal ? launch<128, true, false, true>(a, ctas, stream) : launch<128, false, false, true>(a, ctas, stream);
+    return a.causal ? launch<64, true, false, true>(a, ctas, stream) : launch<64, false, false, true>(a, ctas, stream);
   }
-  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, stream) : launch<128, false, false, false>(a, stream);
-  return a.causal ? launch<64, true, false, false>(a, stream) : launch<64, false, false, false>(a, stream);
+  if (a.D == 128) return a.causal ? launch<128, true, false, false>(a, ctas, stream) : launch<128, false, false, false>(a, ctas, stream);
+  return a.causal ? launch<64, true, false, false>(a, ctas, stream) : launch<64, false, false, false>(a, ctas, stream);
 }
 
 #endif

@@ -494,21 +494,24 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 template <int D, int NT>
 cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
+  int sms;
+  cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
   const int groups = (P.rows + 8 * NT - 1) / (8 * NT), units = P.kvs * P.Tk;
-  // runs: 16 warps per SM of a B200, at most kMaxChunks CTAs per kv head
-  const int even = (int)(((int64_t)units * groups + 148 * 16 - 1) / (148 * 16)), most = (P.Tk + kWarps * kMaxChunks - 1) / (kWarps * kMaxChunks);
+  // runs: 16 warps per SM, at most kMaxChunks CTAs per kv head
+  const int even = (int)(((int64_t)units * groups + sms * 16 - 1) / (sms * 16)), most = (P.Tk + kWarps * kMaxChunks - 1) / (kWarps * kMaxChunks);
   P.run = even > most ? even : most;
   P.chunks = (P.Tk + kWarps * P.run - 1) / (kWarps * P.run);
   const size_t frag = (size_t)(P.rows + 7) / 8 * 2 * 32 * (D / 8) * 4;         // 32 KB at most
-  // key tiles per CTA of the scores kernel: the fewest tile times on 148 SMs, a CTA's start counted as one
-  const int slots = 148 * (D == 128 ? 2 : 3);
+  // key tiles per CTA of the scores kernel: the fewest tile times, a CTA's start counted as one
+  const int slots = sms * (D == 128 ? 2 : 3);
   int64_t best = INT64_MAX;
   for (int run = 1; run <= 16; ++run) {
     const int64_t ctas = (int64_t)((P.Tk + run - 1) / run) * P.kvs, cost = (ctas + slots - 1) / slots * (run + 1);
     if (cost < best) { best = cost; P.score_run = run; }
   }
   const dim3 grid((P.Tk + P.score_run - 1) / P.score_run, P.kvs);
-  cudaError_t e = launch_pdl(P.rows <= 8 ? decode_scores_kernel<D, true> : decode_scores_kernel<D, false>, grid, kScoreThreads, frag, stream,
+  e = launch_pdl(P.rows <= 8 ? decode_scores_kernel<D, true> : decode_scores_kernel<D, false>, grid, kScoreThreads, frag, stream,
                              overlap, P);
   if (e != cudaSuccess) return e;
   return launch_pdl(decode_output_kernel<D, NT>, dim3((unsigned)(P.kvs * P.chunks), groups), kThreads, 0, stream, true, P);

@@ -292,11 +292,14 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   P.Tk = ((a.k_lambda ? (a.Nk + kGroup - 1) / kGroup * 16 : a.Nk) + 127) / 128;
   P.cu_k = a.cu_k;
   P.d_in = (a.d_in > 0 && a.d_in <= a.D) ? a.d_in : a.D;
-  // key tiles per CTA: the fewest tile times on 148 SMs with two CTAs each, a CTA's start counted as one; at most two where
+  // key tiles per CTA: the fewest tile times on SMs with two CTAs each, a CTA's start counted as one; at most two where
   // lengths vary, since a CTA that has begun is not given to another sequence (16 prompts: 486 us, 500 with up to 16)
+  int sms;
+  cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
   int64_t best = INT64_MAX;
   for (int run = 1; run <= (a.cu_k != nullptr ? 2 : 16); ++run) {
-    const int64_t ctas = (int64_t)((P.Tk + run - 1) / run) * a.B * a.Hkv, cost = (ctas + 295) / 296 * (run + 1);
+    const int64_t ctas = (int64_t)((P.Tk + run - 1) / run) * a.B * a.Hkv, cost = (ctas + 2 * sms - 1) / (2 * sms) * (run + 1);
     if (cost < best) { best = cost; P.run = run; }
   }
   const dim3 grid((P.Tk + P.run - 1) / P.run, a.B * a.Hkv);
@@ -318,8 +321,7 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
   const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
   static std::atomic<unsigned long long> ready[8];      // per kernel: devices on which the shared memory was asked for
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   using Kern = void (*)(CUtensorMap, KDsParams);
   static const Kern kerns[8] = {k_quant_delta_s_kernel<64, false, false>,  k_quant_delta_s_kernel<64, true, false>,
                                 k_quant_delta_s_kernel<128, false, false>, k_quant_delta_s_kernel<128, true, false>,

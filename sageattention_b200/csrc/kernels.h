@@ -4,7 +4,20 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace sage3 {
+
+// SMs of the current device, asked for once per device
+inline cudaError_t sm_count(int* sms) {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  if (dev < 64 && (*sms = known[dev].load(std::memory_order_relaxed)) != 0) return cudaSuccess;
+  if (cudaError_t e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev); e != cudaSuccess) return e;
+  if (dev < 64) known[dev].store(*sms, std::memory_order_relaxed);
+  return cudaSuccess;
+}
 
 // Launch; with `pdl` as a programmatic dependent of the kernel before it on the stream (the kernel then waits with
 // griddepcontrol.wait before it touches anything that one writes).

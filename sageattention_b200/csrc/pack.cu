@@ -141,7 +141,9 @@ cudaError_t launch_pack_kv(const PackArgs& a, cudaStream_t stream) {
   const int per_block = kPackThreads / 32;
   int gx = (G + per_block - 1) / per_block;
   // enough blocks to fill the GPU a few times over; warps loop over the remaining groups
-  const int cap = max(1, (148 * 16) / max(1, a.B * a.Hkv));
+  int sms;
+  if (cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
+  const int cap = max(1, (sms * 16) / max(1, a.B * a.Hkv));
   if (gx > cap) gx = cap;
   dim3 grid(gx, a.B * a.Hkv);
   auto K = (const __nv_bfloat16*)a.k;

@@ -129,3 +129,12 @@ def test_nan_score_counts_alike_at_every_key(Nq, D, causal, op):
     assert torch.equal(out[0][~sees], want[0][~sees])
     if lse is not None:
         assert bool(torch.isnan(lse[0][sees]).all()) and torch.equal(lse[0][~sees], want_lse[0][~sees])
+
+
+# as many query tiles as CTAs with a margin, one more and one fewer (items of one or of two tiles), and few query rows per head,
+# whose kernels have no margin: the same bits
+@pytest.mark.parametrize("Hq,Hkv,Nq,margin", [(100, 100, 128, 47), (100, 100, 128, 48), (100, 100, 128, 49), (35, 7, 300, 43), (35, 7, 300, 44), (8, 2, 1, 100)])
+def test_sm_margin_around_one_query_tile_per_cta(Hq, Hkv, Nq, margin):
+    q, k, v = U.make_qkv(1, Hq, Hkv, Nq, 500, 128, seed=Hq + Nq, device=DEV)
+    want = sa.sageattn(q, k, v, is_causal=True)
+    assert torch.equal(sa.sageattn(q, k, v, is_causal=True, sm_margin=margin, check_status=True), want)
