@@ -80,7 +80,8 @@ typedef struct {
   size_t q_dot_km;  /* fp32 [B,Hq,Nq]: raw q . K channel mean (the LSE term K smoothing removes)  */
   size_t scratch;   /* reduction scratch of the channel-mean kernel                               */
   size_t status;    /* one int32 on the device                                                    */
-  size_t workspace; /* all of the above packed (256-byte aligned parts), for sage3_attention      */
+  size_t workspace; /* all of the above packed (256-byte aligned parts): enough for sage3_attention
+                       (sage3_attention_workspace says what it takes) and sage3_attention_varlen  */
 } sage3_sizes;        /* Tq = ceil(Nq/128), Tk = ceil(Nk/128)                                        */
 
 typedef struct {
@@ -146,7 +147,7 @@ typedef struct {
   int32_t is_causal;
   int32_t per_block_mean;    /* as in sage3_quant_args                                               */
   int32_t smooth_k;
-  void* workspace;           /* >= sage3_sizes.workspace bytes, 256-byte aligned                     */
+  void* workspace;           /* >= sage3_attention_workspace bytes, 256-byte aligned                 */
   size_t workspace_bytes;
   int32_t* device_status;    /* optional device int32 (see sage3_attn_args); NULL: one inside the
                                 workspace is used and cannot be read back by the caller              */
@@ -201,6 +202,8 @@ SAGE3_API const char* sage3_status_string(int status);
 SAGE3_API int sage3_last_cuda_error(void);
 
 SAGE3_API int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes* out);
+/* What sage3_attention takes of sage3_sizes.workspace: with few query rows per head K leaves neither codes nor delta_s. */
+SAGE3_API int sage3_attention_workspace(const sage3_shape* shape, int per_block_mean, size_t* bytes);
 
 SAGE3_API int sage3_quant_qkv(const sage3_quant_args* args, void* stream);
 SAGE3_API int sage3_attn_fwd(const sage3_attn_args* args, void* stream);

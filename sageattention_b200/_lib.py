@@ -82,7 +82,7 @@ class VarlenArgs(C.Structure):
 
 
 EXPORTS = ("sage3_version", "sage3_status_string", "sage3_last_cuda_error", "sage3_buffer_sizes",
-           "sage3_quant_qkv", "sage3_attn_fwd", "sage3_attention", "sage3_attention_run", "sage3_attention_packed_workspace", "sage3_attention_packed_run", "sage3_read_device_status",
+           "sage3_quant_qkv", "sage3_attn_fwd", "sage3_attention", "sage3_attention_run", "sage3_attention_workspace", "sage3_attention_packed_workspace", "sage3_attention_packed_run", "sage3_read_device_status",
            "sage3_k_mean_static", "sage3_packed_rows", "sage3_packed_len", "sage3_pack_kv",
            "sage3_attn_fwd_packed", "sage3_attention_varlen", "sage3_fp4_mma_peak", "sage3_selftest_bounded_wait")
 
@@ -107,6 +107,7 @@ def load() -> C.CDLL:
     lib.sage3_attn_fwd.argtypes = [C.POINTER(AttnArgs), C.c_void_p]
     lib.sage3_attention.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
     lib.sage3_attention_run.argtypes = [C.POINTER(FwdArgs)] + [C.c_void_p] * 8
+    lib.sage3_attention_workspace.argtypes = [C.POINTER(Shape), C.c_int, C.POINTER(C.c_size_t)]
     lib.sage3_attention_packed_workspace.argtypes = [C.POINTER(Shape), C.c_int, C.POINTER(C.c_size_t)]
     lib.sage3_attention_packed_run.argtypes = [C.POINTER(FwdArgs), C.c_int, C.c_int] + [C.c_void_p] * 7
     lib.sage3_read_device_status.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_int32)]

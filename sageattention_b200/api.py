@@ -388,7 +388,6 @@ def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smoo
     if p.pad:
         return p
     pbm = int(bool(per_block_mean))
-    z = buffer_sizes(B, Hq, Hkv, Nq, Nk, Dp, pbm)
     _, _, _, _, osb, osh, osn = _as_bhnd_strides(torch.empty_like(q, device="meta"), tensor_layout)
     a = p.struct = _lib.FwdArgs()
     a.shape = _lib.Shape(B, Hq, Hkv, Nq, Nk, Dp)
@@ -397,12 +396,11 @@ def _make_plan(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean, smoo
     a.km_out = None           # the K-mean term of the LSE is put back on the device (q . km in the quantisation kernel)
     a.sm_scale = float(sm_scale) if sm_scale is not None else 0.0
     a.is_causal, a.per_block_mean, a.smooth_k = int(bool(is_causal)), pbm, int(bool(smooth_k))
-    workspace = int(z.workspace)
-    p.run = lib.sage3_attention_run
-    if packed:
-        n = C.c_size_t()
-        _lib.check(lib.sage3_attention_packed_workspace(C.byref(a.shape), pbm, C.byref(n)), "sage3_attention_packed_workspace")
-        workspace, p.run = n.value, lib.sage3_attention_packed_run
+    size, p.run = ((lib.sage3_attention_packed_workspace, lib.sage3_attention_packed_run) if packed else
+                   (lib.sage3_attention_workspace, lib.sage3_attention_run))
+    n = C.c_size_t()
+    _lib.check(size(C.byref(a.shape), pbm, C.byref(n)), "workspace size")
+    workspace = n.value
     a.workspace_bytes = workspace
     a.head_dim = D if D != Dp else 0
     a.sm_margin = int(sm_margin)

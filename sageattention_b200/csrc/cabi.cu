@@ -43,6 +43,19 @@ inline int check_tensor(const sage3_tensor& t) {
   return SAGE3_OK;
 }
 
+// Workspace of the tile kernels, and of those for few query rows per head, which leave no codes of K and no delta_s
+inline size_t tiles_bytes(const sage3_sizes& z) {
+  return align256(z.q_codes) + align256(z.q_sf) + align256(z.k_codes) + align256(z.k_sf) + align256(z.vt_codes) + align256(z.vt_sf) +
+         align256(z.qm) + align256(z.km) + align256(z.delta_s) + align256(z.q_dot_km) + align256(z.scratch) + 256;
+}
+inline bool takes_decode(const sage3_shape& s, int per_block_mean) {
+  return per_block_mean >= 0 && sage3::decode_fits(s.Hq, s.Hkv, s.Nq, s.Nk);
+}
+inline size_t decode_bytes(const sage3_sizes& z, const sage3_shape& s) {
+  return tiles_bytes(z) - align256(z.k_codes) - align256(z.k_sf) - align256(z.delta_s) +
+         sage3::decode_scratch_bytes(s.B, s.Hq, s.Hkv, s.Nq, s.Nk, s.D);
+}
+
 }  // namespace
 
 extern "C" {
@@ -84,10 +97,17 @@ int sage3_buffer_sizes(const sage3_shape* shape, int per_block_mean, sage3_sizes
   size_t sq = sage3::quant_scratch_bytes(s.B, s.Hq, s.Nq, s.D);
   out->scratch = sk > sq ? sk : sq;
   out->status = 4;
-  out->workspace = align256(out->q_codes) + align256(out->q_sf) + align256(out->k_codes) + align256(out->k_sf) +
-                   align256(out->vt_codes) + align256(out->vt_sf) + align256(out->qm) + align256(out->km) +
-                   align256(out->delta_s) + align256(out->q_dot_km) + align256(out->scratch) + 256 +
-                   sage3::decode_scratch_bytes(s.B, s.Hq, s.Hkv, s.Nq, s.Nk, s.D);
+  // enough for every entry point that takes this shape; what sage3_attention needs is sage3_attention_workspace
+  out->workspace = tiles_bytes(*out);
+  if (takes_decode(s, per_block_mean) && decode_bytes(*out, s) > out->workspace) out->workspace = decode_bytes(*out, s);
+  return SAGE3_OK;
+}
+
+int sage3_attention_workspace(const sage3_shape* shape, int per_block_mean, size_t* bytes) {
+  sage3_sizes z;
+  if (bytes == nullptr) return SAGE3_ERR_ARGUMENT;
+  if (int st = sage3_buffer_sizes(shape, per_block_mean, &z)) return st;
+  *bytes = takes_decode(*shape, per_block_mean) ? decode_bytes(z, *shape) : tiles_bytes(z);
   return SAGE3_OK;
 }
 
@@ -102,7 +122,8 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   cudaStream_t stream = (cudaStream_t)stream_;
   const sage3_shape& s = a->shape;
   if (a->q.ptr && (!a->q_codes || !a->q_sf)) return SAGE3_ERR_ARGUMENT;
-  if (a->k.ptr && (!a->k_codes || !a->k_sf)) return SAGE3_ERR_ARGUMENT;
+  const bool ds = a->delta_s != nullptr || k_later != nullptr;         // K goes on to the K kernel, or to what stands in for it
+  if (a->k.ptr && (!a->k_codes || !a->k_sf) && k_later == nullptr) return SAGE3_ERR_ARGUMENT;
   if (a->v.ptr && (!a->vt_codes || !a->vt_sf)) return SAGE3_ERR_ARGUMENT;
   if (a->q.ptr && a->per_block_mean >= 0 && !a->qm) return SAGE3_ERR_ARGUMENT;
   if (a->per_block_mean < -1 || a->per_block_mean > 1) return SAGE3_ERR_ARGUMENT;
@@ -116,7 +137,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
     if (!a->km || !a->scratch || !aligned16(a->scratch)) return SAGE3_ERR_ARGUMENT;
     if (a->scratch_bytes < sage3::quant_scratch_bytes(s.B, s.Hkv, s.Nk, s.D)) return SAGE3_ERR_ARGUMENT;
     // (a whole-sequence Q mean uses the same scratch)
-    if (a->delta_s != nullptr && a->q_dot_km == nullptr && a->per_block_mean == 1) {
+    if (ds && a->q_dot_km == nullptr && a->per_block_mean == 1) {
       partial = a->scratch;
     } else {
       cudaError_t e = sage3::launch_channel_mean(a->k.ptr, a->k.stride_b, a->k.stride_h, a->k.stride_n, s.B, s.Hkv,
@@ -139,8 +160,8 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
 
   // with delta_s requested, K is quantised by the delta_s kernel, which has the smoothed tile in hand anyway
   if (a->delta_s != nullptr && !aligned16(a->delta_s)) return SAGE3_ERR_ARGUMENT;     // written through a tensor map
-  const bool k_in_ds = a->delta_s != nullptr && a->k.ptr != nullptr;
-  if (a->delta_s != nullptr && (!a->q.ptr || !a->k.ptr || a->per_block_mean < 0)) return SAGE3_ERR_ARGUMENT;
+  const bool k_in_ds = ds && a->k.ptr != nullptr;
+  if (ds && (!a->q.ptr || !a->k.ptr || a->per_block_mean < 0)) return SAGE3_ERR_ARGUMENT;
   sage3::QuantArgs q{};
   q.q = a->q.ptr; q.k = a->k.ptr; q.v = a->v.ptr;
   q.q_sb = a->q.stride_b; q.q_sh = a->q.stride_h; q.q_sn = a->q.stride_n;
@@ -165,7 +186,7 @@ static int quant_qkv_impl(const sage3_quant_args* a, const int* cu_q, const int*
   cudaError_t e = sage3::launch_quant_qkv(q, stream);
   if (e != cudaSuccess) return cuda_fail(e);
 
-  if (a->delta_s != nullptr) {
+  if (ds) {
     sage3::DeltaSArgs d{};
     d.qm = a->qm; d.k = a->k.ptr; d.k_sb = a->k.stride_b; d.k_sh = a->k.stride_h; d.k_sn = a->k.stride_n;
     d.km = km; d.partial = partial; d.km_out = a->km; d.ds = a->delta_s; d.cu_k = cu_k; d.k_lambda = k_lambda; d.after_quant = true;
@@ -188,8 +209,8 @@ static int attn_fwd_impl(const sage3_attn_args* a, const float* k_lambda, const 
                          const int* order = nullptr, const int* n_order = nullptr, const sage3::DeltaSArgs* decode_k = nullptr, void* decode_scratch = nullptr) {
   if (a == nullptr) return SAGE3_ERR_ARGUMENT;
   if (int st = check_shape(a->shape)) return st;
-  if (!a->q_codes || !a->q_sf || !a->k_codes || !a->k_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status)
-    return SAGE3_ERR_ARGUMENT;
+  if (!a->q_codes || !a->q_sf || !a->vt_codes || !a->vt_sf || !a->out || !a->device_status) return SAGE3_ERR_ARGUMENT;
+  if (decode_k == nullptr && (!a->k_codes || !a->k_sf)) return SAGE3_ERR_ARGUMENT;
   if (!aligned16(a->q_codes) || !aligned16(a->k_codes) || !aligned16(a->vt_codes) || !aligned16(a->q_sf) ||
       !aligned16(a->k_sf) || !aligned16(a->vt_sf) || !aligned16(a->out) || (a->delta_s && !aligned16(a->delta_s)))
     return SAGE3_ERR_ARGUMENT;
@@ -277,24 +298,29 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
   if (!a->q.ptr || !a->k.ptr || !a->v.ptr) return SAGE3_ERR_ARGUMENT;
   sage3_sizes z;
   if (int st = sage3_buffer_sizes(&a->shape, a->per_block_mean, &z)) return st;
-  if (a->workspace_bytes < z.workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255)) return SAGE3_ERR_ARGUMENT;
+  const bool decode = takes_decode(a->shape, a->per_block_mean);
+  const size_t need = decode ? decode_bytes(z, a->shape) : tiles_bytes(z);
+  if (a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 255)) return SAGE3_ERR_ARGUMENT;
   char* w = reinterpret_cast<char*>(a->workspace);
   auto take = [&](size_t n) { char* p = w; w += align256(n); return (void*)p; };
   sage3_quant_args q{};
   q.shape = a->shape; q.q = a->q; q.k = a->k; q.v = a->v;
   q.per_block_mean = a->per_block_mean; q.smooth_k = a->smooth_k;
-  q.q_codes = take(z.q_codes); q.q_sf = take(z.q_sf); q.k_codes = take(z.k_codes); q.k_sf = take(z.k_sf);
-  q.vt_codes = take(z.vt_codes); q.vt_sf = take(z.vt_sf);
+  q.q_codes = take(z.q_codes); q.q_sf = take(z.q_sf); q.vt_codes = take(z.vt_codes); q.vt_sf = take(z.vt_sf);
   q.qm = take(z.qm);
   void* km_ws = take(z.km);
   q.km = a->km_out ? a->km_out : km_ws;
-  void* ds = take(z.delta_s);
   float* qk = reinterpret_cast<float*>(take(z.q_dot_km));
   q.scratch = take(z.scratch); q.scratch_bytes = z.scratch;
   int32_t* status = reinterpret_cast<int32_t*>(take(4));
-  const bool decode = a->per_block_mean >= 0 && sage3::decode_fits(a->shape.Hq, a->shape.Hkv, a->shape.Nq, a->shape.Nk);
   sage3::DeltaSArgs decode_k{};
-  void* decode_scratch = w;
+  void *ds = nullptr, *decode_scratch = nullptr;
+  if (decode) {
+    decode_scratch = w;
+  } else {
+    q.k_codes = take(z.k_codes); q.k_sf = take(z.k_sf);
+    ds = take(z.delta_s);
+  }
   if (a->device_status) status = a->device_status;
   if (a->lse && a->smooth_k) q.q_dot_km = qk;
   if (!head_dim_ok(a->head_dim, a->shape.D)) return SAGE3_ERR_ARGUMENT;
@@ -341,9 +367,9 @@ static int packed_sizes(const sage3_shape* shape, int per_block_mean, sage3_size
   s.Nk = sage3_packed_rows(s.Nk);
   if (int st = sage3_buffer_sizes(&s, per_block_mean, z)) return st;
   const size_t sk = sage3::quant_scratch_bytes(s.B, s.Hkv, shape->Nk, s.D);
-  if (sk > z->scratch) { z->workspace += align256(sk) - align256(z->scratch); z->scratch = sk; }
+  if (sk > z->scratch) z->scratch = sk;
   *lam = (size_t)s.B * s.Hkv * ((s.Nk + 127) / 128) * 128 * sizeof(float);
-  *total = z->workspace + align256(*lam);
+  *total = tiles_bytes(*z) + align256(*lam);
   return SAGE3_OK;
 }
 
@@ -396,7 +422,7 @@ int sage3_attention_varlen(const sage3_varlen_args* a, void* stream) {
   if ((a->out_stride_h % 8) || (a->out_stride_n % 8)) return SAGE3_ERR_ARGUMENT;
   sage3_sizes z;
   if (int st = sage3_buffer_sizes(&a->shape, 1, &z)) return st;
-  if (a->workspace_bytes < z.workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255)) return SAGE3_ERR_ARGUMENT;
+  if (a->workspace_bytes < tiles_bytes(z) || (reinterpret_cast<uintptr_t>(a->workspace) & 255)) return SAGE3_ERR_ARGUMENT;
   char* w = reinterpret_cast<char*>(a->workspace);
   auto take = [&](size_t n) { char* p = w; w += align256(n); return (void*)p; };
   sage3_quant_args q{};

@@ -155,3 +155,38 @@ def test_plans_of_lengths_that_do_not_come_back_push_out_the_oldest_only(monkeyp
     for t in threads:
         t.join()
     assert len(api._plans) == 64
+
+
+def test_workspace_of_few_query_rows_holds_only_what_their_kernels_use():
+    """With few query rows per head K leaves neither codes nor delta_s, but scores and partial outputs; batches of packed
+    sequences and the K-packing operator never take those kernels, whatever their lengths."""
+    lib = _lib.load()
+    up = lambda n: (n + 255) // 256 * 256
+    z, n = _lib.Sizes(), C.c_size_t()
+
+    def tiles():
+        parts = ("q_codes", "q_sf", "k_codes", "k_sf", "vt_codes", "vt_sf", "qm", "km", "delta_s", "q_dot_km", "scratch")
+        return sum(up(getattr(z, p)) for p in parts) + 256
+
+    def sizes(s, pbm=1):
+        assert lib.sage3_buffer_sizes(C.byref(s), pbm, C.byref(z)) == _lib.OK
+        assert lib.sage3_attention_workspace(C.byref(s), pbm, C.byref(n)) == _lib.OK
+        return n.value
+
+    for pbm in (0, 1):
+        few = sizes(_lib.Shape(8, 32, 8, 1, 4096, 128), pbm)
+        rows, tk, chunks = 8 * 32, 32, 32
+        scratch = up(rows * tk * 512) + up(rows * tk * 4) + up(rows * chunks * 512) + 2 * up(rows * chunks * 4) + up(rows * 4)
+        assert few == tiles() - up(z.k_codes) - up(z.k_sf) - up(z.delta_s) + scratch
+        assert few < z.workspace == tiles()
+    # 64 rows: the scores outweigh the codes, and sage3_sizes.workspace is enough for either kind of kernel
+    assert sizes(_lib.Shape(1, 8, 1, 8, 8192, 64)) == z.workspace > tiles()
+    for s, pbm in ((_lib.Shape(2, 4, 2, 300, 700, 128), 1), (_lib.Shape(8, 32, 8, 1, 4096, 128), -1)):
+        assert sizes(s, pbm) == z.workspace == tiles()
+    # K-packing: the parts of a problem with as many keys as there are slots, and the lambdas
+    assert lib.sage3_attention_packed_workspace(C.byref(_lib.Shape(8, 32, 8, 1, 1500, 128)), 1, C.byref(n)) == _lib.OK
+    packed = n.value
+    sizes(_lib.Shape(8, 32, 8, 1, 1600, 128))
+    assert packed == tiles() + up(8 * 8 * 13 * 128 * 4)
+    assert lib.sage3_attention_workspace(None, 1, C.byref(n)) == _lib.ERR_ARGUMENT
+    assert lib.sage3_attention_workspace(C.byref(_lib.Shape(1, 1, 1, 1, 1, 128)), 1, None) == _lib.ERR_ARGUMENT

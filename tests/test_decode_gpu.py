@@ -49,3 +49,34 @@ def test_few_query_rows_in_other_layouts():
     for kw in ({"smooth_k": False}, {"per_block_mean": False}):
         a = sa.sageattn3_blackwell(q, k, v, **kw)
         assert torch.isfinite(a).all() and sage3.accuracy(a.float().cpu(), sa.sageattn(q, k, v).float().cpu())[0] > 0.9
+
+
+# the workspace that sage3_attention_workspace asks for is enough, and all that is written; one byte less is refused
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,lse", [(2, 8, 2, 1, 1300, 128, True), (1, 8, 1, 8, 3000, 64, False), (1, 4, 2, 300, 500, 128, True)])
+def test_workspace_is_not_overrun(B, Hq, Hkv, Nq, Nk, D, lse):
+    import ctypes as C
+    from sageattention_b200 import _lib
+    lib = _lib.load()
+    q, k, v = U.make_qkv(B, Hq, Hkv, Nq, Nk, D, seed=Nk, device=DEV)
+    want = sa.sageattn(q, k, v, return_lse=True)
+    n = C.c_size_t()
+    a = _lib.FwdArgs()
+    a.shape = _lib.Shape(B, Hq, Hkv, Nq, Nk, D)
+    a.per_block_mean = a.smooth_k = 1
+    assert lib.sage3_attention_workspace(C.byref(a.shape), 1, C.byref(n)) == _lib.OK
+    ws = torch.full((n.value + 65536,), 0xA5, dtype=torch.uint8, device=DEV)
+    out, lse_out = torch.empty_like(q), torch.empty(B, Hq, Nq, dtype=torch.float32, device=DEV)
+    for t, x in (("q", q), ("k", k), ("v", v)):
+        setattr(a, t, _lib.Tensor(None, x.stride(0), x.stride(1), x.stride(2)))
+    a.out_stride_b, a.out_stride_h, a.out_stride_n = out.stride(0), out.stride(1), out.stride(2)
+    stream = torch.cuda.current_stream().cuda_stream
+    for nbytes, status in ((n.value - 1, _lib.ERR_ARGUMENT), (n.value, _lib.OK)):
+        a.workspace_bytes = nbytes
+        assert lib.sage3_attention_run(C.byref(a), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                                       lse_out.data_ptr() if lse else None, ws.data_ptr(), None, stream) == status
+    torch.cuda.synchronize()
+    assert bool((ws[n.value:] == 0xA5).all())
+    if lse:
+        assert torch.equal(out, want[0]) and torch.equal(lse_out, want[1])
+    else:
+        assert torch.equal(out, sa.sageattn(q, k, v))
