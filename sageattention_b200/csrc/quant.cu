@@ -476,7 +476,9 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   P.v_blocks = a.v ? (int)(((int64_t)a.B * a.Hkv * P.Tk + tpb - 1) / tpb) : 0;
   // K sums come last where K fits in L2, so that the K kernel finds it there (with V read past the L2's favour: K-packing
   // B4 H32 N2048 325 -> 320 us, 16 prompts 490 -> 486); else first, being the longest units (B1 H40 N32760 loses 10 us else),
-  // as where K is so small that it is in L2 anyhow
+  // as where K is so small that it is in L2 anyhow.  Of a variable-length batch the padded size counts: last, the sums also wait
+  // for the CTAs of tiles beyond the sequences (by the keys there really are, 73 MB of 688: 2162 -> 2186 us, 53 MB of 999: 1110 ->
+  // 1140)
   const int64_t k_bytes = (int64_t)a.B * a.Hkv * a.Nk * a.D * 2;
   const bool fits = k_bytes <= 96 << 20 && k_bytes >= 8 << 20;
   P.s_first = fits ? P.q_blocks + P.k_blocks + P.v_blocks : 0;

@@ -138,3 +138,21 @@ def test_sm_margin_around_one_query_tile_per_cta(Hq, Hkv, Nq, margin):
     q, k, v = U.make_qkv(1, Hq, Hkv, Nq, 500, 128, seed=Hq + Nq, device=DEV)
     want = sa.sageattn(q, k, v, is_causal=True)
     assert torch.equal(sa.sageattn(q, k, v, is_causal=True, sm_margin=margin, check_status=True), want)
+
+
+# K channel sums first or last (8 to 96 MB of K, counted with the longest sequence's length) in the first launch; sequences
+# without keys among them
+@pytest.mark.parametrize("lens", [[8000] + [120, 0, 121] * 36, [2000] * 8 + [500], [100, 0, 3000]])
+def test_varlen_k_sums_first_and_last(lens):
+    g = torch.Generator().manual_seed(len(lens))
+    q, k, v = (torch.randn(sum(lens), h, 128, generator=g).to(torch.bfloat16).to(DEV) for h in (2, 2, 2))
+    k += 2.0 * torch.randn(1, 2, 128, generator=g).to(torch.bfloat16).to(DEV)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    out = sa.sageattn_varlen(q, k, v, cu, cu, max(lens), max(lens), is_causal=True, check_status=True)
+    for i in range(len(lens)):
+        s = slice(int(cu[i]), int(cu[i + 1]))
+        if lens[i] > 0 and (i < 8 or i > len(lens) - 4):
+            one = sa.sageattn(q[s][None], k[s][None], v[s][None], tensor_layout="NHD", is_causal=True)[0]
+            cos, l1 = sage3.accuracy(out[s].float().cpu(), one.float().cpu())
+            assert cos >= 0.9995 and l1 <= 2e-2, (i, lens[i], cos, l1)
+    assert torch.isfinite(out).all()
