@@ -3,8 +3,8 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--workload NAME]
 
-One "step" = one pass of the whole operator (K channel means, fused smoothing + NVFP4 quantisation,
-delta_s, FP4 attention) over one batch of seeded synthetic input.  The metric is the reference's
+One "step" = one pass of the whole operator (K channel sums + fused smoothing and NVFP4 quantisation of Q and V,
+the K pass with means, quantisation and delta_s, FP4 attention) over one batch of seeded synthetic input.  The metric is the reference's
 attention throughput ``4*B*Hq*Nq*Nk*D / t`` (halved for causal), sageattention3_blackwell/scripts/
 bench.py:151-153.  Prints ONE JSON line (rank 0).
 
@@ -607,7 +607,7 @@ def main():
         "config": {"workload": args.workload, "B": B, "Hq": Hq, "Hkv": Hkv, "N": N, "D": D, "causal": causal,
                    "sharding": f"batch x heads over {world} GPU(s), no collective",
                    "l2": "inputs (3 x %.0f MB bf16) exceed the 126 MB L2" % (B * Hq * N * D * 2 / 1e6),
-                   "step": "K mean + fused quant + delta_s + attention, inputs resident in HBM"},
+                   "step": "K sums + fused quant, K pass (means, quant, delta_s), attention; inputs resident in HBM"},
         "kernel_only": {"attention_ms": attn_ms, "attention_tops": achieved, "preprocess_ms": quant_ms,
                         "preprocess_gbs": quant_bytes / (quant_ms * 1e-3) / 1e9,
                         "preprocess_frac_of_hbm": quant_bytes / (quant_ms * 1e-3) / 1e9 / hbm,

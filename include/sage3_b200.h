@@ -212,7 +212,7 @@ SAGE3_API int sage3_attention(const sage3_fwd_args* args, void* stream);
  * threads: q, k, v, out, lse, workspace and device_status replace those of *args, which is only read. */
 SAGE3_API int sage3_attention_run(const sage3_fwd_args* args, const void* q, const void* k, const void* v, void* out,
                                   float* lse, void* workspace, int32_t* device_status, void* stream);
-/* sage3_attention for a variable-length batch in ONE pass over the same four kernels: every kernel takes
+/* sage3_attention for a variable-length batch in ONE pass over the same three kernels: every kernel takes
  * the sequence offsets and lengths from cu_seqlens_*, the operands are laid out as for a [B, longest] batch
  * and tiles beyond a sequence's end cost nothing.  Replaces the per-sequence loop a caller of the dense
  * entry points would write; the reference's own varlen operator (sageattention/core.py:334-448) belongs to

@@ -424,7 +424,7 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
                     **kwargs) -> torch.Tensor:
     """Variable-length batch (``sageattention/core.py:334-448``): q ``[sum(len_q), Hq, D]``, k/v
     ``[sum(len_k), Hkv, D]``, ``cu_seqlens_*`` the int32 prefix sums (length batch + 1, on the device).
-    One pass over the four kernels for the whole batch (``sage3_attention_varlen``); every sequence is
+    One pass over the three kernels for the whole batch (``sage3_attention_varlen``); every sequence is
     smoothed, quantised and attended on its own (K means never mix sequences); sequences without keys give
     zeros.  ``max_seqlen_*`` must bound the longest sequence - they size the workspace."""
     lib = _lib.load()

@@ -230,7 +230,7 @@ __device__ __forceinline__ void load_scores(const uint32_t tm_S, uint32_t (&s)[1
 
 // 2^x for two values on the FMA pipe (the special-function unit paces the softmax): x = n + r with n the nearest
 // integer, found by adding and subtracting 1.5 * 2^23, |r| <= 1/2; 2^r by a polynomial of degree 5, minimax in the
-// relative error (Remez exchange, computed for this file: 7.5e-8 in exact arithmetic, 2.1e-7 = 2^-22.2 evaluated in
+// relative error (Remez exchange, computed for this file: 1.5e-7 with its coefficients rounded to fp32, 2.1e-7 = 2^-22.2 evaluated in
 // fp32, the error bound of ex2.approx being 2^-22); n goes into the exponent bits.  x <= log2(6) here; below -125 (a
 // masked score) the result is 2^-125: code 0, and nothing beside the 6 that the block's largest value adds to its sum.
 // So is that of a NaN, which has to reach the row sum by another way: nan_of_poly_columns.

@@ -294,38 +294,15 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t r0, uint32_t r
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Operations on operands in shared memory take each 64-bit descriptor as (low word, high word): the issuing thread then only
+// does 32-bit adds on the low word.
 // 32 rows x 16 bytes of scale factors: shared -> tensor memory, replicated into all four
 // 32-lane quarters (what block-scaled MMAs expect).
-__device__ __forceinline__ void tc_cp_sf(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-
-// D[tmem] (+)= A[smem] * B[smem], E2M1 operands with one UE4M3 scale per 16 elements, K = 64.
-__device__ __forceinline__ void tc_mma_nvf4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
-      : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem], bf16 operands, K = 16.
-__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// The same three operations taking each 64-bit shared-memory descriptor as (low word, high word):
-// the issuing thread then only does 32-bit adds on the low word.
 __device__ __forceinline__ void tc_cp_sf(uint32_t taddr, uint32_t lo, uint32_t hi) {
   asm volatile("{\n.reg .b64 d;\nmov.b64 d, {%1, %2};\ntcgen05.cp.cta_group::1.32x128b.warpx4 [%0], d;\n}"
                ::"r"(taddr), "r"(lo), "r"(hi) : "memory");
 }
+// D[tmem] (+)= A[smem] * B[smem], E2M1 operands with one UE4M3 scale per 16 elements, K = 64.
 __device__ __forceinline__ void tc_mma_nvf4(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                             uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
   asm volatile(
@@ -346,6 +323,7 @@ __device__ __forceinline__ void tc_mma_nvf4_ta(uint32_t d_tmem, uint32_t a_tmem,
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
+// D[tmem] (+)= A[smem] * B[smem], bf16 operands, K = 16.
 __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -355,20 +333,9 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint
       ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// Shared-memory matrix descriptor for a K-major operand.
-//   swizzle_code: 0 none (8x16B core matrices), 6 = 32B, 4 = 64B, 2 = 128B swizzle
-//   sbo_bytes   : distance between consecutive groups of 8 rows
-//   lbo_bytes   : distance between the two 16-byte K chunks (unswizzled layouts only)
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t sbo_bytes, uint32_t lbo_bytes,
-                                                   uint32_t swizzle_code) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;                          // descriptor version (Blackwell)
-  d |= (uint64_t)(swizzle_code & 7) << 61;
-  return d;
-}
+// A shared-memory descriptor's low word: address >> 4, leading offset >> 4 in bits 16 on (the distance between the two 16-byte
+// K chunks where there is no swizzle, 1 else); its high word: distance between groups of 8 rows >> 4, version 1 in bit 14,
+// swizzle from bit 29 (0 none, 6 = 32 bytes, 4 = 64, 2 = 128).
 
 // Instruction descriptor for kind::mxf4nvf4, scale_vec::4X: E2M1 x E2M1 -> fp32, UE4M3 scales,
 // both operands K-major, M x N tile, K = 64.
@@ -390,23 +357,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr) : "memory");
-}
-
-// 8 consecutive fp32 columns of this thread's TMEM lane -> registers.
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr) : "memory");
-}
-// 16 consecutive fp32 columns of this thread's TMEM lane -> registers.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
 

@@ -1,6 +1,7 @@
 // Fused smoothing + NVFP4 quantisation of Q, K and V for the FP4 attention kernel (sm_100a).
 //
-// Replaces, in one launch (plus one small reduction launch for the K channel means):
+// Replaces, in one launch (the K channel means are added up from its partial sums by the next one, or, where the means
+// themselves are asked for, come from a reduction launch before it):
 //   * K minus its per-channel mean over tokens        sageattn4/api.py:184
 //   * Q zero-padded to 128 rows, minus per-128-row mean sageattn4/api.py:26-72,186-191
 //   * NVFP4 quantisation of Q                          quantization/fp4_quantization_4d.cu:164-284,414-490

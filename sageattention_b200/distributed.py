@@ -273,10 +273,10 @@ def bench_ulysses(args, w, dist_mod, dev, ring: bool = False):
             "data": "synthetic",
             "config": ({"workload": "ring", "B": B, "H": H, "N": N, "D": D, "causal": w["causal"],
                         "sharding": f"sequence-sharded input, {world} ring steps of {n} keys, K/V shards by point-to-point copies",
-                        "step": f"{world} x (K mean + fused quant + delta_s + attention) + {world - 1} K/V exchanges + LSE merges"}
+                        "step": f"{world} x (K sums + fused quant, K pass, attention) + {world - 1} K/V exchanges + LSE merges"}
                        if ring else
                        {"workload": "ulysses", "B": B, "H": H, "N": N, "D": D, "causal": w["causal"],
                         "sharding": f"sequence-sharded input, all-to-all to {H // world} heads per GPU, {chunks} head chunk(s)",
-                        "step": "3 all-to-all + K mean + fused quant + delta_s + attention + 1 all-to-all"}),
+                        "step": "3 all-to-all + K sums + fused quant, K pass, attention + 1 all-to-all"}),
             "gpu_launches": (4 * world if ring else 3 * chunks) * args.steps}), flush=True)
     dist_mod.destroy_process_group()

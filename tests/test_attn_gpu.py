@@ -213,7 +213,7 @@ def test_custom_op_runs_and_matches_direct_call():
 
 
 def test_operator_can_be_captured_in_a_cuda_graph():
-    """The whole operator (memsets + four kernels, no allocation or synchronisation inside the library) is
+    """The whole operator (three kernels, no allocation or synchronisation inside the library) is
     captured once and replayed on new input values."""
     q, k, v = U.make_qkv(2, 4, 2, 700, 700, 128, seed=21, device=DEV)
     for _ in range(2):
