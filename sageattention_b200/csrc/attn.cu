@@ -47,10 +47,11 @@
 // exponentials.  Hence: everything that is not softmax - the rescaling, the output - is other warps' work
 // (B4 Hq32 Hkv8 N8192 D128 causal: 1.79 -> 1.61 ms; B4 H32 N4096 D64: 0.815 -> 0.79 ms); all 32 lanes of a role warp
 // wait and one issues, because a wait executed by a single lane polls instead of parking and answers 40 cycles later;
-// waits for what has usually happened test once before they park (45 cycles instead of 120); the poll loop is a handful
-// of instructions in one asm block (left to the compiler it was unrolled at every wait) and uniform by a vote; and 3 of 16 exponentials run on
-// the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile.  At B1 H10 N32760 D128 the
-// kernel went from 3.86 to 3.63 ms (1560 cycles per key tile and 128 query rows; 61 % of the issue slots used).
+// waits for what has usually happened test once before they park (45 cycles instead of 120); the poll loop is a handful of
+// instructions in one asm block (left to the compiler it was unrolled at every wait) and uniform by a vote; and 3 of 16
+// exponentials run on the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile (by count, at
+// 16 a clock).  At B1 H10 N32760 D128 the kernel went from 3.86 to 3.60 ms: 1530 cycles per key tile and 128 query rows, 61 % of
+// the issue slots used, the special-function pipe 64 % busy.
 //
 // Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128), 48 columns of scale factors, P^0 and P^1 (16
 // columns each: 128 FP4 codes per row).

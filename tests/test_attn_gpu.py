@@ -276,8 +276,8 @@ def test_varlen_sequences_longer_than_max_seqlen_are_cut_not_overrun():
 
 
 def test_host_tensor_entry_point_batched_is_copy_bound_not_stride_bound():
-    """B > 1: the head groups of a [B,H,N,D] host tensor are not contiguous across the batch; the entry point copies
-    them batch entry by batch entry.  Same values as the device operator."""
+    """B > 1, entries so small that all go in one piece (cuts inside an entry, and between entries: test_host_pieces.py).
+    Same values as the device operator."""
     q, k, v = U.make_qkv(3, 8, 4, 500, 500, 128, seed=13)
     want = sa.sageattn(q.cuda(), k.cuda(), v.cuda(), is_causal=False).cpu()
     got = sa.sageattn_from_host(q.pin_memory(), k.pin_memory(), v.pin_memory(), head_chunks=4)
