@@ -628,12 +628,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
                 if (!(ok = wait_bar<true>(bars + Bars::q_full + 8 * t, qn[t] & 1, abort_s, P.status, 20))) break;
                 ++qn[t];
                 tc_fence_after();
-                if (lane == 0)
+                if (elect_one())
 #pragma unroll
                   for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfq + 8 * t + 4 * kb, sfq_lo + t * 64 + kb * 32, HI_SF);
               }
               tc_fence_after();
-              if (lane == 0) {
+              if (elect_one()) {
                 if (first) {
 #pragma unroll
                   for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfk + 4 * kb, sfk_lo + s * 64 + kb * 32, HI_SF);
@@ -654,12 +654,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               first = false;
               ++nqk;
             }
-            if (ok && lane == 0) tc_commit(bars + Bars::k_empty + 8 * s);
+            if (ok && elect_one()) tc_commit(bars + Bars::k_empty + 8 * s);
           }
         }
         if (!ok) {
           // giving up: let every MMA / scale copy already issued finish before tensor memory is freed
-          if (lane == 0) tc_commit(bars + Bars::drain);
+          if (elect_one()) tc_commit(bars + Bars::drain);
           mbar_wait<true>(bars + Bars::drain, 0, 1u << 16);
         }
       } else if (warp == 15) {
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             // the V stage and its scale factors do not depend on the softmax: fetch them before waiting for P
             if (!(ok = wait_bar<false>(bars + Bars::v_full + 8 * s, (g / kStages) & 1, abort_s, P.status, 24))) break;
             tc_fence_after();
-            if (lane == 0)
+            if (elect_one())
 #pragma unroll
               for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfv + 4 * kb, sfv_lo + s * 64 + kb * 32, HI_SF);
 #pragma unroll
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               const bool first_tile = it == wk.n_max - wk.n_t[t];
               if (!(ok = wait_bar<false>(bars + Bars::p_full + 8 * t, pv_cnt[t] & 1, abort_s, P.status, 26))) break;
               tc_fence_after();
-              if (lane == 0) {
+              if (elect_one()) {
 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfp + 8 * t + 4 * kb, sfp_lo + t * 64 + kb * 32, HI_SF);
 #pragma unroll
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           }
         }
         if (!ok) {
-          if (lane == 0) tc_commit(bars + Bars::drain + 8);
+          if (elect_one()) tc_commit(bars + Bars::drain + 8);
           mbar_wait<true>(bars + Bars::drain + 8, 0, 1u << 16);
         }
       }
