@@ -426,7 +426,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bars = sbase + L::bars;
   volatile int* abort_s = reinterpret_cast<volatile int*>(smem + L::bars + Bars::abort_flag);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // by a shuffle, so that the compiler knows it to be the same in all lanes: the roles' loops, branches and descriptors are then
+  // uniform code (16 prompts 457 -> 435 us, K-packing B4 H32 N2048 306 -> 287, B4 H32/8 N8192 causal 1708 -> 1661)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const bool has_ds = P.ds != nullptr;
 #if !SAGE3_VARLEN_BUILD
   const int total_work = kList ? P.B * P.Hkv * P.list_items : P.B * P.Hq * ((P.Tq + 1) >> 1);
