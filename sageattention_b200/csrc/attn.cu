@@ -36,7 +36,7 @@
 //   warp  12    TMA producer (Q tiles per item, then a ring of K and V stages; scale factors and the
 //               delta_s rows by plain bulk copies)
 //   warp  13    QK issuer: scale-factor copies, rank-1 delta_s MMA and Q.K^T MMAs, both tiles in turn
-//               into the ONE score buffer
+//               into the ONE score buffer (D=64: one for each)
 //   warp  14    turns each delta_s row (128 bf16) into the B operand of a rank-1 bf16 MMA
 //               (ones x delta_s) that initialises the score accumulator, so the softmax warps never
 //               touch delta_s
@@ -47,14 +47,19 @@
 // exponentials.  Hence: everything that is not softmax - the rescaling, the output - is other warps' work
 // (B4 Hq32 Hkv8 N8192 D128 causal: 1.79 -> 1.61 ms; B4 H32 N4096 D64: 0.815 -> 0.79 ms); all 32 lanes of a role warp
 // wait and one issues, because a wait executed by a single lane polls instead of parking and answers 40 cycles later;
-// waits for what has usually happened test once before they park (45 cycles instead of 120); the poll loop is a handful of
-// instructions in one asm block (left to the compiler it was unrolled at every wait) and uniform by a vote; and 3 of 16
-// exponentials run on the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile (by count, at
-// 16 a clock).  At B1 H10 N32760 D128 the kernel went from 3.86 to 3.60 ms: 1530 cycles per key tile and 128 query rows, 61 % of
-// the issue slots used, the special-function pipe 64 % busy.
+// the poll loop is a handful of instructions in one asm block (left to the compiler it was unrolled at every wait) and uniform by
+// a vote; 3 of 16 exponentials run on the FMA pipe, which takes the special-function unit from 1100 to 900 cycles per key tile (by
+// count, at 16 a clock).
+// A look at a barrier takes 150 to 200 cycles even where the phase is long complete, since it queues behind the other warp's
+// exponentials, and so do the other hand-overs of a key tile (clock stamps).  So those of the softmax lie behind one another no
+// more than they must: the next scores' barrier is looked at in the last exponentials, that of the last P.V before the first
+// exponentials, whose codes wait in registers, and P^ is handed over while the next scores are on their way.  With it and with
+// loops that are not unrolled in the issuers: B1 H10 N32760 D128 3.67 -> 3.47 ms (whole operator), D64 3.59 -> 3.33, B4 H32/8 N8192
+// causal 1.66 -> 1.59, 16 prompts 435 -> 408 us.  The arithmetic of the softmax alone, two warps per sub-partition with every barrier
+// satisfied, takes 1200 to 1250 cycles per key tile and 128 query rows; here it is 1330, and was 1530.
 //
-// Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128), 48 columns of scale factors, P^0 and P^1 (16
-// columns each: 128 FP4 codes per row).
+// Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128) (D=64: one for each query tile, [2D,2D+256)), 48 columns of scale
+// factors, P^0 and P^1 (16 columns each: 128 FP4 codes per row).
 //
 // Every wait on an mbarrier is bounded; if one gives up the CTA records a code in *status, waits
 // (bounded) for its own copies and MMAs in flight, frees its tensor memory and returns.
@@ -96,7 +101,7 @@ constexpr int kAttnThreads = 512;
 // it would block forever, so the split is checked here.  kLaunchRegs is what the compiler allocates under
 // __launch_bounds__(512, 1).
 constexpr int kLaunchRegs = 128;
-struct RegSplit { static constexpr int softmax = 192, corr = 80, role = 48; };
+struct RegSplit { static constexpr int softmax = 192, corr = 72, role = 56; };
 static_assert(256 * RegSplit::softmax + 128 * (RegSplit::corr + RegSplit::role) <= kAttnThreads * kLaunchRegs,
               "setmaxnreg split exceeds the CTA's register pool");
 
@@ -140,8 +145,8 @@ struct Bars {            // byte offsets inside the barrier block
   static constexpr int v_empty = v_full + 8 * kStages;
   static constexpr int ds_ready = v_empty + 8 * kStages;
   static constexpr int s_full = ds_ready + 8 * kStages;   // [2] Q.K^T of tile t is in the score buffer
-  static constexpr int s_free = s_full + 16;              // the score buffer has been copied into registers
-  static constexpr int p_full = s_free + 8;               // [2] P^ and its scales written (O rescaled if it had to be)
+  static constexpr int s_free = s_full + 16;              // [score buffers] the score buffer has been copied into registers
+  static constexpr int p_full = s_free + 16;              // [2] P^ and its scales written (O rescaled if it had to be)
   static constexpr int pv_done = p_full + 16;             // [2] P.V MMAs of tile t complete: P^ may be rewritten, O_t is current
   static constexpr int drain = pv_done + 16;              // [2] the issuers' last commit when giving up
   static constexpr int corr = drain + 16;                 // [4 row quarters][2] alpha of a key tile is in shared memory, O_t may be rescaled
@@ -252,7 +257,7 @@ __device__ __forceinline__ float2 ex2_poly(float2 x) {
 // Which of the 8 pairs of a 16-key block take it: 3 in 16.  Measured for 0 / 2 / 3 / 4 of 16 on rows of 256 key tiles
 // (B1 H10 N32760): D=128 3.98 / 3.75 / 3.65 / 3.72 ms, D=64 3.86 / 3.73 / 3.62 / 3.65 ms - more, and the 12
 // instructions per pair cost more issue slots than the unit's cycles they save.
-__device__ constexpr bool on_fma_pipe(const int blk, const int pair) { return pair == 3 || (pair == 6 && (blk & 1)); }
+__device__ constexpr bool on_fma_pipe(const int blk, const int pair) {  return pair == 3 || (pair == 6 && (blk & 1)); }
 // A NaN if one of the columns that take it has a NaN score, else a finite number or +inf, from the maxima that max16 leaves:
 // times 0 it goes into the row sum, so that such a row ends as one with a NaN in any other column does (its output zero, its
 // LSE NaN) whatever the place of the key.  (A row with a score of +inf has that sum anyhow: inf - inf.)  7 instructions per key
@@ -265,21 +270,19 @@ __device__ __forceinline__ float nan_of_poly_columns(const float (&c)[8], const 
   return fmax3_nan(x, e[5], e[7]);
 }
 
-// P / blockscale = 2^(s*c - (bm*c + log2(1/6))) in [0, 6] -> E2M1 codes into this row's 16 tensor-memory columns of
-// P^ (8 codes per column, in key order - the A operand of the P.V MMA is read from there); returns the row sum of the unquantised P = sum over blocks of (sum of P/blockscale) * blockscale
-// (softmax_fused.h:135-153).  neg_e[b] = -(bm_b*c + log2(1/6)), sb[b] = the block's unrounded scale.
+// Two 16-key blocks, 2 kPair and the next: P / blockscale = 2^(s*c - (bm*c + log2(1/6))) in [0, 6] -> E2M1 codes, 8 to a word in key
+// order; they go into this row's 16 tensor-memory columns of P^, from where the P.V MMA reads its A operand.  To lsum, the row sum
+// of the unquantised P, (sum of P/blockscale) * blockscale of each block is added (softmax_fused.h:135-153).
+// neg_e[b] = -(bm_b*c + log2(1/6)), sb[b] = the block's unrounded scale.
 // K-packing mode with slot_first: the first column of every block is the group's mean slot carrying a copy of the
 // first token's score; its P^ goes to the MMA like any other, but it is no token and stays out of the row sum
 // (softmax_fused.h:48-64).
-template <bool kPacked>
-__device__ __forceinline__ float exp_quantise_store(const uint32_t (&s)[128], const float c, const float (&neg_e)[8],
-                                                    const float (&sb)[8], const uint32_t tm_P,
-                                                    const bool slot_first) {
+template <bool kPacked, int kPair>
+__device__ __forceinline__ void exp_quantise(const uint32_t (&s)[128], const float c, const float (&neg_e)[8], const float (&sb)[8],
+                                             const bool slot_first, float& lsum, uint32_t (&code)[4]) {
   const float2 c2 = make_float2(c, c);
-  float lsum = 0.f;
-  uint32_t code[4];
 #pragma unroll
-  for (int blk = 0; blk < 8; ++blk) {
+  for (int blk = 2 * kPair; blk < 2 * kPair + 2; ++blk) {
     const float2 nb2 = make_float2(neg_e[blk], neg_e[blk]);
     float2 e[8];
 #pragma unroll
@@ -294,9 +297,7 @@ __device__ __forceinline__ float exp_quantise_store(const uint32_t (&s)[128], co
     lsum = fmaf(bsum, sb[blk], lsum);
     code[(blk & 1) * 2 + 0] = f32x8_to_e2m1x8(e[0].x, e[0].y, e[1].x, e[1].y, e[2].x, e[2].y, e[3].x, e[3].y);
     code[(blk & 1) * 2 + 1] = f32x8_to_e2m1x8(e[4].x, e[4].y, e[5].x, e[5].y, e[6].x, e[6].y, e[7].x, e[7].y);
-    if (blk & 1) tmem_st4(tm_P + 4 * (blk >> 1), code[0], code[1], code[2], code[3]);     // 32 keys = 4 columns
   }
-  return lsum;
 }
 
 // K-packing mode: 15 tokens occupy 16 key slots (fwd_mainloop.cu:273-303).  Last slot that token `tok` or an
@@ -417,6 +418,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
                                                                    const __grid_constant__ CUtensorMap tm_o,
                                                                    const KParams P) {
   using L = Smem<D>;
+  // Score buffers in tensor memory: one for each query tile where there is room (D=64: B4 H32 N8192 causal 1553 -> 1543 us, longer rows
+  // gain nothing)
+  constexpr int kSBufs = D == 64 ? 2 : 1;
   constexpr int kKB = D / 64;                              // K=64 blocks of the QK contraction
   constexpr uint32_t kSwzQK = (D == 128) ? 4u : 6u;        // 64-byte / 32-byte swizzle
   constexpr uint32_t kSboQK = (D == 128) ? 512u : 256u;
@@ -449,7 +453,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       mbar_init(bars + Bars::v_empty + 8 * s, 1);          // tcgen05.commit
       mbar_init(bars + Bars::ds_ready + 8 * s, 1);
     }
-    mbar_init(bars + Bars::s_free, 4);
+    for (int i = 0; i < 2; ++i) mbar_init(bars + Bars::s_free + 8 * i, 4);
     for (int i = 0; i < 8; ++i) mbar_init(bars + Bars::corr + 8 * i, 1);
     mbar_init(bars + Bars::drain, 1);
     mbar_init(bars + Bars::drain + 8, 1);
@@ -477,9 +481,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + L::bars + Bars::tmem_slot);
-  // columns: O0 [0, D)  O1 [D, 2D)  S [2D, 2D + 128)  scale factors behind
+  // columns: O0 [0, D)  O1 [D, 2D)  S [2D, 2D + 128 kSBufs)  scale factors behind
   const uint32_t tm_Sbuf = tmem + 2 * D;
-  const uint32_t tm_sfq = tm_Sbuf + 128, tm_sfk = tm_sfq + 16, tm_sfp = tm_sfk + 8, tm_sfv = tm_sfp + 16;
+  const uint32_t tm_sfq = tm_Sbuf + 128 * kSBufs, tm_sfk = tm_sfq + 16, tm_sfp = tm_sfk + 8, tm_sfv = tm_sfp + 16;
   const uint32_t tm_P = tm_sfv + 8;                       // [2] P^ codes: the A operand of the P.V MMAs, 16 columns each
 
   // read once after the barrier: every warp takes the same branch, so the register hand-over
@@ -497,10 +501,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       if (warp == 12) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_o); }
+        bool ok = true;
         uint32_t g = 0;                       // K/V stages completely issued so far
         uint32_t gk = 0;                      // K stages issued so far (g or g + 1)
         uint32_t qn[2] = {0, 0};              // Q tiles loaded so far per slot
-        bool ok = true;
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             else ds_row[t] = ((int64_t)wk.b * P.Hq + wk.hq) * P.ds_rows + (P.ds_rows == 1 ? 0 : qt);
             if (ok && wk.n_t[t] > 0) {
               // the slot's previous Q tile must have been read by its last QK MMA
-              if (qn[t] > 0 && !(ok = wait_bar<false>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1, abort_s, P.status, 12))) break;
+              if (qn[t] > 0 && !(ok = wait_bar<>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1))) break;
               const int64_t qtile = ((int64_t)wk.b * P.Hq + wk.hq) * P.Tq + qt;
               const uint32_t qb = bars + Bars::q_full + 8 * t;
               if (lane == 0) {
@@ -529,7 +533,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             const uint32_t ph = ((g / kStages) & 1) ^ 1;
-            if (!(ok = wait_bar<false>(bars + Bars::k_empty + 8 * s, ph, abort_s, P.status, 10))) break;
+            if (!(ok = wait_bar<>(bars + Bars::k_empty + 8 * s, ph))) break;
             const uint32_t kb = bars + Bars::k_full + 8 * s;
             const int nds = has_ds ? (int)(j < wk.n_t[0]) + (int)(j < wk.n_t[1]) : 0;
             if (lane == 0) {
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             }
             __syncwarp();
             ++gk;
-            if (!(ok = wait_bar<false>(bars + Bars::v_empty + 8 * s, ph, abort_s, P.status, 11))) break;
+            if (!(ok = wait_bar<>(bars + Bars::v_empty + 8 * s, ph))) break;
             const uint32_t vb = bars + Bars::v_full + 8 * s;
             if (lane == 0) {
               mbar_arrive_expect_tx(vb, L::kVBytes + L::kSfV);
@@ -556,6 +560,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             __syncwarp();
           }
         }
+        if (!ok) give_up(abort_s, P.status, 10);
         if (__any_sync(0xffffffffu, *abort_s != 0)) {
           // giving up: the copies this thread started must land before the CTA may exit
           for (int t = 0; t < 2; ++t)
@@ -569,18 +574,17 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         // ---------------------------------------------------------------- delta_s -> rank-1 B operand
         // B1 is a K-major [128 keys x 16] bf16 operand in 8x16-byte core matrices: key n's first
         // element sits at (n/8)*128 + (n%8)*16; everything else stays zero.
-        uint32_t g = 0;
         bool ok = true;
+        uint32_t s = 0, ph = 0;
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
-          for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
-            const int j = wk.n_max - 1 - it, s = g % kStages;
-            if (!(ok = wait_bar<false>(bars + Bars::k_full + 8 * s, (g / kStages) & 1, abort_s, P.status, 40))) break;
-#pragma unroll
+          for (int j = wk.n_max - 1; j >= 0; --j) {
+            if (!(ok = wait_bar<>(bars + Bars::k_full + 8 * s, ph))) break;
+#pragma unroll 1
             for (int t = 0; t < 2; ++t) {
-              if (j < wk.n_t[t]) {
+              if (j < (t == 0 ? wk.n_t[0] : wk.n_t[1])) {
                 const uint16_t* raw = reinterpret_cast<const uint16_t*>(smem + L::dsraw + (s * 2 + t) * 256);
                 uint8_t* dst = smem + L::b1 + (s * 2 + t) * 2048 + (lane >> 3) * 128 + (lane & 7) * 16;   // keys lane + 32 i
 #pragma unroll
@@ -590,8 +594,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + Bars::ds_ready + 8 * s);
+            if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
+        if (!ok) give_up(abort_s, P.status, 40);
       } else if (warp == 13) {
         // ---------------------------------------------------------------- QK issuer
         // Its instruction stream is kept minimal: every shared-memory descriptor is a constant high word (stride /
@@ -607,28 +613,34 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         const uint32_t a1_lo = ((sbase + L::a1) >> 4) | (((uint32_t)(L::zero - L::a1) >> 4) << 16);
         const uint32_t b1_lo = ((sbase + L::b1) >> 4) | (((uint32_t)(L::zero - L::b1) >> 4) << 16);
         bool ok = true;
-        uint32_t g = 0;                       // K stages consumed so far
+        uint32_t s = 0, ph = 0;               // K stage and its parity
         uint32_t nqk = 0;                     // QK groups issued so far (= uses of the score buffer)
-        uint32_t qn[2] = {0, 0};              // Q tiles taken so far per slot
+        uint32_t s_par = 0;                   // bit t: the same, odd or even, for tile t's own buffer
+        uint32_t q_par = 0;                   // bit t: parity of the Q tile to come in slot t
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
-          for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
-            const int j = wk.n_max - 1 - it, s = g % kStages;
-            const uint32_t ph = (g / kStages) & 1;
-            if (!(ok = wait_bar<true>(bars + Bars::k_full + 8 * s, ph, abort_s, P.status, 21))) break;
-            if (has_ds && !(ok = wait_bar<true>(bars + Bars::ds_ready + 8 * s, ph, abort_s, P.status, 25))) break;
-            bool first = true;
-#pragma unroll
+          for (int j = wk.n_max - 1; ok && j >= 0; --j) {
+            if (!(ok = wait_bar_uniform(bars + Bars::k_full + 8 * s, ph))) break;
+            if (has_ds && !(ok = wait_bar_uniform(bars + Bars::ds_ready + 8 * s, ph))) break;
+            uint32_t copy_k = 1;
+#pragma unroll 1
             for (int t = 0; t < 2; ++t) {
-              if (!ok || j >= wk.n_t[t]) continue;
+              const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
+              if (j >= n_t) continue;
               // the one score buffer must be free: the softmax warpgroup that got the previous Q.K^T (the other
               // query tile, or this one in the previous key tile) has copied it into registers
-              if (nqk > 0 && !(ok = wait_bar<true>(bars + Bars::s_free, (nqk - 1) & 1, abort_s, P.status, 23))) break;
-              if (it == wk.n_max - wk.n_t[t]) {                    // first key tile of this query tile
-                if (!(ok = wait_bar<true>(bars + Bars::q_full + 8 * t, qn[t] & 1, abort_s, P.status, 20))) break;
-                ++qn[t];
+              if (kSBufs == 1) {
+                if (!(ok = wait_bar_uniform(bars + Bars::s_free, (nqk - 1) & 1))) break;      // (nothing to wait for: parity 1)
+              } else {
+                if (!(ok = wait_bar_uniform(bars + Bars::s_free + 8 * t, ((s_par >> t) & 1) ^ 1))) break;
+                s_par ^= 1u << t;
+              }
+              const uint32_t tm_S = tm_Sbuf + 128 * (kSBufs - 1) * t;
+              if (j == n_t - 1) {                                  // first key tile of this query tile
+                if (!(ok = wait_bar_uniform(bars + Bars::q_full + 8 * t, (q_par >> t) & 1))) break;
+                q_par ^= 1u << t;
                 tc_fence_after();
                 if (elect_one())
 #pragma unroll
@@ -636,30 +648,32 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               }
               tc_fence_after();
               if (elect_one()) {
-                if (first) {
+                if (copy_k) {
 #pragma unroll
                   for (int kb = 0; kb < kKB; ++kb) tc_cp_sf(tm_sfk + 4 * kb, sfk_lo + s * 64 + kb * 32, HI_SF);
                 }
                 if (has_ds) {
                   // buffer i sits i*2048 bytes higher, so its distance to the shared zero chunk is i*2048 smaller
-                  const uint32_t i = (uint32_t)(s * 2 + t);
-                  tc_mma_bf16(tm_Sbuf, a1_lo, HI_SF, b1_lo + i * 128u - ((i * 128u) << 16), HI_SF, idesc_r1, 0);
+                  const uint32_t i = s * 2 + t;
+                  tc_mma_bf16(tm_S, a1_lo, HI_SF, b1_lo + i * 128u - ((i * 128u) << 16), HI_SF, idesc_r1, 0);
                 }
 #pragma unroll
                 for (int kb = 0; kb < kKB; ++kb)
-                  tc_mma_nvf4(tm_Sbuf, q_lo + t * (L::kQBytes >> 4) + kb * 2, HI_QK, k_lo + s * (L::kKBytes >> 4) + kb * 2, HI_QK,
+                  tc_mma_nvf4(tm_S, q_lo + t * (L::kQBytes >> 4) + kb * 2, HI_QK, k_lo + s * (L::kKBytes >> 4) + kb * 2, HI_QK,
                               idesc_qk, tm_sfq + 8 * t + 4 * kb, tm_sfk + 4 * kb, (has_ds || kb > 0) ? 1u : 0u);
                 tc_commit(bars + Bars::s_full + 8 * t);
-                if (it == wk.n_max - 1) tc_commit(bars + Bars::q_empty + 8 * t);   // last read of this Q tile
+                if (j == 0) tc_commit(bars + Bars::q_empty + 8 * t);   // last read of this Q tile
               }
               __syncwarp();
-              first = false;
+              copy_k = 0;
               ++nqk;
             }
             if (ok && elect_one()) tc_commit(bars + Bars::k_empty + 8 * s);
+            if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
         if (!ok) {
+          give_up(abort_s, P.status, 20);
           // giving up: let every MMA / scale copy already issued finish before tensor memory is freed
           if (elect_one()) tc_commit(bars + Bars::drain);
           mbar_wait<true>(bars + Bars::drain, 0, 1u << 16);
@@ -675,26 +689,25 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         const uint32_t v_lo = ((sbase + L::v) >> 4) | LBO1;
         const uint32_t sfv_lo = (sbase + L::sfv) >> 4, sfp_lo = (sbase + L::sfp) >> 4;
         bool ok = true;
-        uint32_t g = 0, pv_cnt[2] = {0, 0};
+        uint32_t s = 0, ph = 0;               // V stage and its parity
+        uint32_t p_par = 0;                   // bit t: parity of the P^ to come of tile t
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
-          for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
-            const int j = wk.n_max - 1 - it, s = g % kStages;
-            const bool act1 = j < wk.n_t[1];
+          for (int j = wk.n_max - 1; ok && j >= 0; --j) {
             // the V stage and its scale factors do not depend on the softmax: fetch them before waiting for P
-            if (!(ok = wait_bar<false>(bars + Bars::v_full + 8 * s, (g / kStages) & 1, abort_s, P.status, 24))) break;
+            if (!(ok = wait_bar<>(bars + Bars::v_full + 8 * s, ph))) break;
             tc_fence_after();
             if (elect_one())
 #pragma unroll
               for (int kb = 0; kb < 2; ++kb) tc_cp_sf(tm_sfv + 4 * kb, sfv_lo + s * 64 + kb * 32, HI_SF);
-#pragma unroll
+#pragma unroll 1
             for (int t = 0; t < 2; ++t) {
-              const bool act = t == 0 ? (j < wk.n_t[0]) : act1;
-              if (!(ok && act)) continue;
-              const bool first_tile = it == wk.n_max - wk.n_t[t];
-              if (!(ok = wait_bar<false>(bars + Bars::p_full + 8 * t, pv_cnt[t] & 1, abort_s, P.status, 26))) break;
+              const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
+              if (j >= n_t) continue;
+              if (!(ok = wait_bar<>(bars + Bars::p_full + 8 * t, (p_par >> t) & 1))) break;
+              p_par ^= 1u << t;
               tc_fence_after();
               if (elect_one()) {
 #pragma unroll
@@ -702,16 +715,17 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb)
                   tc_mma_nvf4_ta(tmem + t * D, tm_P + 16 * t + 8 * kb, v_lo + s * (L::kVBytes >> 4) + kb * 2, HI_PV,
-                                 idesc_pv, tm_sfp + 8 * t + 4 * kb, tm_sfv + 4 * kb, (first_tile && kb == 0) ? 0u : 1u);
+                                 idesc_pv, tm_sfp + 8 * t + 4 * kb, tm_sfv + 4 * kb, (j == n_t - 1 && kb == 0) ? 0u : 1u);
                 tc_commit(bars + Bars::pv_done + 8 * t);
-                if (t == 1 || !act1) tc_commit(bars + Bars::v_empty + 8 * s);   // last PV of this stage
               }
               __syncwarp();
-              ++pv_cnt[t];
             }
+            if (ok && elect_one()) tc_commit(bars + Bars::v_empty + 8 * s);
+            if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
         if (!ok) {
+          give_up(abort_s, P.status, 24);
           if (elect_one()) tc_commit(bars + Bars::drain + 8);
           mbar_wait<true>(bars + Bars::drain + 8, 0, 1u << 16);
         }
@@ -721,12 +735,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       const int row = quarter * 32 + lane;                       // tensor-memory lane
       const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
       const float c = P.scale_log2;
-      bool ok = true;
       if (warp < 8) {
         // ---------------------------------------------------------------- softmax
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegSplit::softmax));
+        bool ok = true;
         const int t = warp >> 2;                                 // query tile slot of this warpgroup
-        const uint32_t tm_S = tm_Sbuf + lane_addr;
+        const uint32_t tm_S = tm_Sbuf + 128 * (kSBufs - 1) * t + lane_addr;
+        const uint32_t bar_f = bars + Bars::s_free + 8 * (kSBufs - 1) * t;
         const uint32_t tm_Prow = tm_P + 16 * t + lane_addr;      // this row of P^: 16 columns of 8 codes
         uint32_t* sfp_row = reinterpret_cast<uint32_t*>(smem + L::sfp + t * 1024 + sf_atom_offset(row, 0));
         volatile float* alpha_row = reinterpret_cast<volatile float*>(smem + L::alpha) + t * 128 + row;
@@ -736,6 +751,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         uint32_t sc = 0;                                         // key tiles processed so far by this warpgroup
         uint32_t g0 = 0;                                         // K/V stages the CTA used before this work item
         uint32_t items = 0;
+        bool s_ready = false;                                    // the next tile's scores were there when last looked at
+        // P^ written: hand the tile to the PV issuer.  The codes went to tensor memory (tcgen05.st), their block
+        // scales to shared memory for the issuer's tcgen05.cp.
+        auto hand_over = [&](const bool there_is) {
+          tmem_wait_st();
+          tc_fence_before();
+          fence_proxy_async_smem();
+          __syncwarp();
+          mbar_arrive_if(lane == 0 && there_is, bar_p);
+        };
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
@@ -759,14 +784,22 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           for (int it = 0; it < n_mine; ++it, ++sc) {
             const int n0 = (n_mine - 1 - it) * kBlockN;
             const bool need_mask = (n0 + kBlockN - 1 >= SEQ_NK) || (kCausal && n0 + kBlockN - 1 > first_row_lim);
-            if (!(ok = wait_bar_soon(bar_s, sc & 1, abort_s, P.status, 30))) break;
+            // the scores are usually there by now: then P^ of the tile before is handed over while they are on their way
+            const bool ready = __all_sync(0xffffffffu, s_ready);
+            if (!ready) {
+              hand_over(it > 0);
+              if (!(ok = wait_bar<>(bar_s, sc & 1))) break;
+            }
             tc_fence_after();
             uint32_t s[128];
             float bm[8], c6[8], c12[8];
-            load_scores(tm_S, s);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tmem_ld32(tm_S + 32 * q, *reinterpret_cast<uint32_t (*)[32]>(&s[32 * q]));
+            if (ready) hand_over(it > 0);
+            tmem_wait_ld();
             // the scores are in registers: the Q.K^T of the other query tile may overwrite the buffer
             tc_fence_before();
-            mbar_arrive_if(lane == 0, bars + Bars::s_free);
+            mbar_arrive_if(lane == 0, bar_f);
             if (kPacked) {
               // lambda of this key tile arrived with its K stage, i.e. before the Q.K^T MMA whose completion was
               // awaited above.  Its slot is rewritten 2*kStages key tiles later, which the producer can only do
@@ -776,7 +809,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
               for (int blk = 0; blk < 8; ++blk) apply_lambda(&s[16 * blk], lam_s + 16 * blk);
             }
-            if (need_mask) {
+            if (__builtin_expect(need_mask, 0)) {
               const int lim = key_lim - n0;                      // columns beyond it are masked
 #pragma unroll
               for (int i = 0; i < 128; ++i) s[i] = (i > lim) ? 0xff800000u : s[i];
@@ -809,31 +842,39 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               sb[i] = ex2_approx(e - off);
               neg_e[i] = -e;
             }
+            const bool pv_ready = mbar_test(bar_pv, (sc - 1) & 1);
+            float lsum = 0.f;
+            uint32_t code[4];
+            exp_quantise<kPacked, 0>(s, c, neg_e, sb, P.slot_first, lsum, code);
             // the P.V MMAs of the previous key tile are complete: P^ and its scales may be rewritten, O rescaled
-            if (sc > 0 && !(ok = wait_bar_soon(bar_pv, (sc - 1) & 1, abort_s, P.status, 31))) break;
+            if (!__all_sync(0xffffffffu, pv_ready) && !(ok = wait_bar<>(bar_pv, (sc - 1) & 1))) break;
+            tc_fence_after();
             *alpha_row = alpha;
             __syncwarp();
             mbar_arrive_if(lane == 0, bar_c);
             sfp_row[0] = f32x2_to_e4m3x2(sb[0], sb[1]) | (f32x2_to_e4m3x2(sb[2], sb[3]) << 16);     // keys 0-63 of the tile
             sfp_row[128] = f32x2_to_e4m3x2(sb[4], sb[5]) | (f32x2_to_e4m3x2(sb[6], sb[7]) << 16);   // keys 64-127
-            l += exp_quantise_store<kPacked>(s, c, neg_e, sb, tm_Prow, P.slot_first);
-            if (it == n_mine - 1) {
-              l_row[(items & 1) * 512] = l;
-              l_row[(items & 1) * 512 + 128] = m_run;
-            }
-            // P^ written: hand the tile to the PV issuer.  The codes went to tensor memory (tcgen05.st), their block
-            // scales to shared memory for the issuer's tcgen05.cp.
-            tmem_wait_st();
-            tc_fence_before();
-            fence_proxy_async_smem();
-            __syncwarp();
-            mbar_arrive_if(lane == 0, bar_p);
+            tmem_st4(tm_Prow, code[0], code[1], code[2], code[3]);                                  // 32 keys = 4 columns
+            exp_quantise<kPacked, 1>(s, c, neg_e, sb, P.slot_first, lsum, code);
+            tmem_st4(tm_Prow + 4, code[0], code[1], code[2], code[3]);
+            exp_quantise<kPacked, 2>(s, c, neg_e, sb, P.slot_first, lsum, code);
+            tmem_st4(tm_Prow + 8, code[0], code[1], code[2], code[3]);
+            exp_quantise<kPacked, 3>(s, c, neg_e, sb, P.slot_first, lsum, code);
+            s_ready = mbar_test(bar_s, (sc + 1) & 1);
+            tmem_st4(tm_Prow + 12, code[0], code[1], code[2], code[3]);
+            l += lsum;
           }
+          if (!ok) break;
+          l_row[(items & 1) * 512] = l;
+          l_row[(items & 1) * 512 + 128] = m_run;
+          hand_over(true);
           ++items;
         }
+        if (!ok) give_up(abort_s, P.status, 30);
       } else {
         // ---------------------------------------------------------------- O: rescaling and output
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit::corr));
+        bool ok = true;
         uint32_t sc[2] = {0, 0}, items[2] = {0, 0};              // key tiles / work items so far per query tile slot
 #pragma unroll 1
         for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
@@ -848,28 +889,27 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
               if (wk.n_max - 1 - it >= n_t) continue;
               uint32_t& cnt = t == 0 ? sc[0] : sc[1];
-              if (!(ok = wait_bar<false>(bars + Bars::corr + 8 * (2 * quarter + t), cnt & 1, abort_s, P.status, 32))) break;
+              if (!(ok = wait_bar<>(bars + Bars::corr + 8 * (2 * quarter + t), cnt & 1))) break;
               ++cnt;
               const float alpha = *(reinterpret_cast<volatile float*>(smem + L::alpha) + t * 128 + row);
               if (it != wk.n_max - n_t && __any_sync(0xffffffffu, alpha != 1.0f)) {
                 tc_fence_after();
                 const uint32_t tm_O = tmem + t * D + lane_addr;
                 const float2 al2 = make_float2(alpha, alpha);
-                uint32_t o[64];
+                uint32_t o[32];
 #pragma unroll 1
-                for (int hf = 0; hf < D / 64; ++hf) {
-                  tmem_ld32(tm_O + hf * 64, *reinterpret_cast<uint32_t (*)[32]>(&o[0]));
-                  tmem_ld32(tm_O + hf * 64 + 32, *reinterpret_cast<uint32_t (*)[32]>(&o[32]));
+                for (int ch = 0; ch < D / 32; ++ch) {
+                  tmem_ld32(tm_O + ch * 32, o);
                   tmem_wait_ld();
 #pragma unroll
-                  for (int i = 0; i < 32; ++i) {
+                  for (int i = 0; i < 16; ++i) {
                     const float2 x = ffma2(make_float2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), al2,
                                            make_float2(0.f, 0.f));
                     o[2 * i] = __float_as_uint(x.x); o[2 * i + 1] = __float_as_uint(x.y);
                   }
 #pragma unroll
-                  for (int ch = 0; ch < 4; ++ch)
-                    tmem_st16(tm_O + hf * 64 + 16 * ch, *reinterpret_cast<const uint32_t (*)[16]>(&o[16 * ch]));
+                  for (int h = 0; h < 2; ++h)
+                    tmem_st16(tm_O + ch * 32 + 16 * h, *reinterpret_cast<const uint32_t (*)[16]>(&o[16 * h]));
                 }
                 tmem_wait_st();
                 tc_fence_before();
@@ -908,11 +948,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             const uint32_t last = (t == 0 ? sc[0] : sc[1]) - 1;
             uint32_t& ni = t == 0 ? items[0] : items[1];
             // the last key tile's row sum is there, and its P.V has landed
-            if (!(ok = wait_bar<false>(bars + Bars::p_full + 8 * t, last & 1, abort_s, P.status, 33))) break;
+            if (!(ok = wait_bar<>(bars + Bars::p_full + 8 * t, last & 1))) break;
             const volatile float* l_row = reinterpret_cast<const volatile float*>(smem + L::lx) + t * 256 + row + (ni & 1) * 512;
             const float l = l_row[0], m = l_row[128];
             ++ni;
-            if (!(ok = wait_bar<false>(bars + Bars::pv_done + 8 * t, last & 1, abort_s, P.status, 34))) break;
+            if (!(ok = wait_bar<>(bars + Bars::pv_done + 8 * t, last & 1))) break;
             tc_fence_after();
             const uint32_t tm_O = tmem + t * D + lane_addr;
             const bool keyless = m == kNoMax;                    // a row that has seen no key: zeros, LSE -inf
@@ -971,6 +1011,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             }
           }
         }
+        if (!ok) give_up(abort_s, P.status, 32);
         if (kTmaStore && lane == 0) bulk_wait_read0();   // the last output tiles have left shared memory before the CTA ends
       }
     }

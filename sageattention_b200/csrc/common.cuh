@@ -155,7 +155,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// One look at an mbarrier phase, without parking.  (Measured on B200: 7 ns; a failing try_wait of a whole warp returns after 4 us,
+// One look at an mbarrier phase, without parking.  (Measured on B200: 7 ns on an idle SM, 150 to 200 cycles beside a warp that
+// keeps the special-function unit busy, so it is issued well before its result is needed; a failing try_wait of a whole warp returns after 4 us,
 // with and without a suspend-time hint.  A parked thread resumes as soon as the phase completes.)
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -170,27 +171,23 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // block of a handful of instructions: left to the compiler it was unrolled at every one of the kernels' many waits,
 // and the instruction cache paid for it.  kWarp: by all 32 lanes of a warp, which leave it together and with the same answer,
 // each poll being a vote.
-template <bool kWarp = false, bool kHinted = false>
+template <bool kWarp = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
   uint32_t ok;
-#define SAGE3_WAIT(TRY, VOTE)                                                                   \
+#define SAGE3_WAIT(VOTE)                                                                        \
   "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\nPOLL:\n"                                    \
-  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2" TRY ";\n" VOTE                         \
+  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n" VOTE                                \
   "@p bra DONE;\nadd.u32 n, n, -1;\nsetp.ne.u32 p, n, 0;\n@p bra POLL;\nDONE:\nmin.u32 %0, n, 1;\n}"
-#define SAGE3_VOTE "vote.sync.all.pred p, p, 0xffffffff;\n"
-  if constexpr (kWarp && kHinted)
-    asm volatile(SAGE3_WAIT(", %4", SAGE3_VOTE) : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit), "r"(20000u) : "memory");
-  else if constexpr (kWarp)
-    asm volatile(SAGE3_WAIT("", SAGE3_VOTE) : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+  if constexpr (kWarp)
+    asm volatile(SAGE3_WAIT("vote.sync.all.pred p, p, 0xffffffff;\n") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
   else
-    asm volatile(SAGE3_WAIT("", "") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
-#undef SAGE3_VOTE
+    asm volatile(SAGE3_WAIT("") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
 #undef SAGE3_WAIT
   return ok != 0;
 }
 
-// Bounded wait of a whole warp of one of the kernels' roles.  On giving up it raises the CTA's abort flag, records `code` in
-// *status (first writer wins) and returns false - the caller then unwinds instead of hanging the SM.
+// Bounded wait of a whole warp of one of the kernels' roles.  Where it returns false the caller leaves its loops, calls give_up
+// and unwinds instead of hanging the SM.
 //
 // The warp goes on to warp-wide instructions (tcgen05.ld / st, __syncwarp), so it must never split on a wait that ran out for
 // some of its lanes only: each poll is a vote.  That also lets the compiler treat the loops as uniform, without the code that
@@ -199,23 +196,32 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 // The limit.  A failing poll takes 80 ns (a busy CTA) to 4 us (a parked warp): the default gives up after 0.02 to 1.05
 // seconds, where the longest wait of a working kernel is some 10 us.  A warp that waits does not look whether another
 // has given up: all of them wait for one another, so each runs out its own limit at about the same time, and that is why it
-// is not longer.  Looking at the flags every 1024 polls - never reached unless something is wrong - costs 2 to 25 % of the
-// attention kernel, by the room its instructions take at every wait (B1 H40 N32760 D128, 16 prompts: in the loop's slow part
-// 14.5 -> 16.4 ms, 484 -> 551 us; behind the loop 15.8, 598; one load per failing poll 14.8, 504; a function of its own does
-// not compile beside setmaxnreg).
-template <bool kHinted, uint32_t kPolls = (1u << 18)>
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  if (mbar_wait<true, kHinted>(bar, parity, kPolls)) return true;
-  *abort_s = 1;
-  atomicCAS(status, 0, code);
+// is not longer.
+template <uint32_t kPolls = (1u << 18)>
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity) {
+  return mbar_wait<true>(bar, parity, kPolls);
+}
+
+// The same as a loop that the compiler sees, so that it knows the answer to be the warp's, and with a suspend-time hint: for
+// the QK issuer (all four forms measured for each role, within 1 % of one another; this one was the best over all shapes).
+__device__ __forceinline__ bool wait_bar_uniform(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t n = 1u << 18; n != 0; --n) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
+    if (__all_sync(0xffffffffu, ok)) return true;
+  }
   return false;
 }
 
-// The same for a phase that has usually completed by now: a plain test first (17 cycles; a try_wait on a completed
-// phase takes 160), then the parking wait.
-__device__ __forceinline__ bool wait_bar_soon(uint32_t bar, uint32_t parity, volatile int* abort_s, int* status, int code) {
-  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-  return wait_bar<false>(bar, parity, abort_s, status, code);
+// A wait of this warp ran out: raises the CTA's abort flag and records `code` in *status (first writer wins).
+__device__ __forceinline__ void give_up(volatile int* abort_s, int* status, int code) {
+  *abort_s = 1;
+  atomicCAS(status, 0, code);
 }
 
 // Programmatic dependent launch: let the next kernel of the stream start its prologue / wait until the previous one is

@@ -1,4 +1,4 @@
-// Self-test of the bounded wait every role of the attention kernel uses (wait_bar, common.cuh): three warps wait, one with
+// Self-test of the bounded wait every role of the attention kernel uses (wait_bar and give_up, common.cuh): three warps wait, one with
 // a SHORT poll limit, the others with the limits that the roles have, on an mbarrier phase that nothing will ever complete.
 // The waits must run out, record their code in the status word and let the kernel return normally - no trap, no fault, no
 // hang - which is how a protocol error inside the attention kernel surfaces as SAGE3_ERR_DEVICE_WAIT on the host.  No
@@ -22,9 +22,8 @@ __global__ void __launch_bounds__(96) bounded_wait_selftest_kernel(int* status, 
   __syncthreads();
   // 2048 polls of 4 us at most: gives up after a few milliseconds
   const int warp = threadIdx.x / 32;
-  const bool done = warp == 0 ? wait_bar<false, 2048>(bar, 0, &abort_flag, status, code)
-                              : (warp == 1 ? wait_bar<false>(bar, 0, &abort_flag, status, code + 1)
-                                           : wait_bar<true>(bar, 0, &abort_flag, status, code + 2));
+  const bool done = warp == 0 ? wait_bar<2048>(bar, 0) : (warp == 1 ? wait_bar<>(bar, 0) : wait_bar_uniform(bar, 0));
+  if (!done) give_up(&abort_flag, status, code + warp);
   if (done) atomicCAS(status, 0, -1);    // cannot happen; would mean the wait saw a phase nobody completed
 }
 
