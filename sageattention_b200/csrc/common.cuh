@@ -112,12 +112,13 @@ __device__ __forceinline__ void add_channels(float2 (&acc)[4], const uint4& w) {
   acc[0] = fadd2(acc[0], bf16x2_to_f32(w.x)); acc[1] = fadd2(acc[1], bf16x2_to_f32(w.y));
   acc[2] = fadd2(acc[2], bf16x2_to_f32(w.z)); acc[3] = fadd2(acc[3], bf16x2_to_f32(w.w));
 }
-__device__ __forceinline__ uint32_t habsmax2(uint32_t a, uint32_t b) {   // per-half max(|a|,|b|)
-  __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&a);
-  __nv_bfloat162 y = *reinterpret_cast<__nv_bfloat162*>(&b);
-  __nv_bfloat162 m = __hmax2(__habs2(x), __habs2(y));
-  return *reinterpret_cast<uint32_t*>(&m);
+// Per half max(|a|, |b|), a NaN only where both are; the sign is of no meaning (xor of the two) until abs2 has cleared it.
+__device__ __forceinline__ uint32_t habsmax2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
 }
+__device__ __forceinline__ uint32_t abs2(uint32_t a) { return a & 0x7fff7fffu; }
 
 // Scale byte + reciprocal for one 16-element block whose absmax (a bf16 value) is `amax`
 // (fp4_quantization_4d.cu:224-230).

@@ -238,7 +238,7 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
       for (int i = 0; i < 2; ++i) {
 #pragma unroll
         for (int blk = 0; blk < W / 8; ++blk) {
-          const uint32_t m2 = habsmax2(amax[i][2 * blk], amax[i][2 * blk + 1]);
+          const uint32_t m2 = abs2(habsmax2(amax[i][2 * blk], amax[i][2 * blk + 1]));
           uint32_t sfb, sf2, unused;
           float inv;
           block_scale(fmaxf(bf16_lo(m2), bf16_hi(m2)), sfb, inv);

@@ -104,6 +104,19 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
   }
 }
 
+// Division by a number that the host knows, for 0 <= n < 2^31 (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994): the six of a CTA's index arithmetic were 10 % of the Q role's instructions.
+struct Div {
+  uint32_t d, mul, shift;
+  void set(uint32_t by) {
+    d = by;
+    for (shift = 0; (1ull << shift) < by; ++shift) {}
+    mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - by)) / by + 1);
+  }
+  __device__ __forceinline__ int quot(int n) const { return (int)((__umulhi(mul, (uint32_t)n) + (uint32_t)n) >> shift); }
+  __device__ __forceinline__ void split(int n, int& q, int& r) const { q = quot(n); r = n - q * (int)d; }
+};
+
 struct QuantLaunch {
   const __nv_bfloat16 *q, *k, *v;
   int64_t q_sb, q_sh, q_sn, k_sb, k_sh, k_sn, v_sb, v_sh, v_sn;
@@ -115,6 +128,7 @@ struct QuantLaunch {
   uint8_t *q_codes, *q_sf, *k_codes, *k_sf, *vt_codes, *vt_sf;
   __nv_bfloat16* qm;                     // [B,Hq,Tq,D] (mode 1)
   int q_blocks, k_blocks, v_blocks;      // CTAs per role
+  Div by_Tq, by_Tk, by_Hq, by_Hkv, by_chunks;
   const int *cu_q, *cu_k;                // variable-length batches (else null)
   int d_in;                              // channels the input rows really have (<= D, multiple of 8); the rest are zero
   int s_blocks, chunks, chunk_tokens;    // CTAs of the K channel-sum role (0: none), chunks per head, tokens per chunk
@@ -185,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   __shared__ __align__(16) uint8_t sf_smem[2048];
   __shared__ __align__(16) float red[RPP * D];
-  __shared__ float mean_s[D];
+  __shared__ __align__(16) float mean_s[D];
   const int t = threadIdx.x, c = t % CH, rl = t / CH;
   int bid = blockIdx.x;
   pdl_launch_dependents();                 // the K kernel may come in and fetch its tiles as SMs fall idle
@@ -200,7 +214,9 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   if (bid >= P.s_first && bid < P.s_first + P.s_blocks) {
     // ----------------------------------------------------------------------------- K channel-sum role
     bid -= P.s_first;
-    const int chunk = bid % P.chunks, bh = bid / P.chunks, b = bh / P.Hkv, h = bh % P.Hkv;
+    int chunk, bh, b, h;
+    P.by_chunks.split(bid, bh, chunk);
+    P.by_Hkv.split(bh, b, h);
     const int N = P.cu_k ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
     channel_partial<D, 8>(P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + h * P.k_sh, P.k_sn, N, chunk, P.chunk_tokens,
                        P.d_in, P.partial + (int64_t)bid * D, red);
@@ -212,9 +228,10 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     // ----------------------------------------------------------------------------- Q / K roles
     const bool is_q = bid < P.q_blocks;
     if (!is_q) bid -= P.q_blocks;
-    const int T = is_q ? P.Tq : P.Tk, H = is_q ? P.Hq : P.Hkv;
-    int N = is_q ? P.Nq : P.Nk;
-    const int tile = bid % T, bh = bid / T, b = bh / H, h = bh % H;
+    const int T = is_q ? P.Tq : P.Tk;
+    int N = is_q ? P.Nq : P.Nk, tile, bh, b, h;
+    (is_q ? P.by_Tq : P.by_Tk).split(bid, bh, tile);
+    (is_q ? P.by_Hq : P.by_Hkv).split(bh, b, h);
     const int64_t sn = is_q ? P.q_sn : P.k_sn;
     const int* cu = is_q ? P.cu_q : P.cu_k;
     const __nv_bfloat16* src = is_q ? P.q + b * P.q_sb + h * P.q_sh : P.k + b * P.k_sb + h * P.k_sh;
@@ -336,29 +353,33 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   constexpr int TPB = (kThreads / 32) / WPT;     // tiles per CTA (1 for D=128, 2 for D=64)
   const int warp = t >> 5, lane = t & 31;
   const int tl = warp / WPT;                     // tile slot inside this CTA
-  const int64_t gt = (int64_t)bid * TPB + tl;    // global tile index over (b, h, tile)
-  const int64_t total = (int64_t)P.B * P.Hkv * P.Tk;
+  const int gt = bid * TPB + tl;                 // global tile index over (b, h, tile)
+  const int total = P.B * P.Hkv * P.Tk;
   for (int i = t; i < 2048 / 16; i += kThreads) reinterpret_cast<uint4*>(sf_smem)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  const int tile = (int)(gt % P.Tk), bh = (int)(gt / P.Tk), b = bh / P.Hkv, h = bh % P.Hkv;
+  int tile, bh, b, h;
+  P.by_Tk.split(gt, bh, tile);
+  P.by_Hkv.split(bh, b, h);
   const int Nv = P.cu_k && gt < total ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
   if (gt < total && (P.pack || tile * kTile < Nv)) {      // (nothing reads a V tile beyond its sequence)
     const int c4 = (warp % WPT) * 4 + (lane >> 3);        // group of 4 channels
     const int blk = lane & 7;                              // 16-token block
-    const __nv_bfloat16* src = P.v + (P.cu_k ? (int64_t)P.cu_k[b] * P.v_sn : b * P.v_sb) + h * P.v_sh + c4 * 4;
     // K-packing mode: a block is a group, 15 tokens behind an empty slot
     const int n0 = P.pack ? (tile * 8 + blk) * kGroup - 1 : tile * kTile + blk * 16;
+    const __nv_bfloat16* src = P.v + (P.cu_k ? (int64_t)P.cu_k[b] * P.v_sn : b * P.v_sb) + h * P.v_sh + c4 * 4 + (int64_t)n0 * P.v_sn;
+    const int lim = c4 * 4 < P.d_in ? Nv - n0 : 0;         // slots of the block that there are
     uint2 x[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const int n = n0 + i;
-      x[i] = (n < Nv && c4 * 4 < P.d_in && !(P.pack && i == 0)) ? __ldcs(reinterpret_cast<const uint2*>(src + (int64_t)n * P.v_sn)) : make_uint2(0, 0);
+      x[i] = (i < lim && !(i == 0 && P.pack)) ? __ldcs(reinterpret_cast<const uint2*>(src)) : make_uint2(0, 0);
+      src += P.v_sn;
     }
-    uint8_t* codes = P.vt_codes + gt * (D * 64);
+    uint8_t* codes = P.vt_codes + (int64_t)gt * (D * 64);
     // largest magnitudes of the 4 channels, two at a time (bf16 comparisons are exact)
     uint32_t m01 = habsmax2(x[0].x, x[1].x), m23 = habsmax2(x[0].y, x[1].y);
 #pragma unroll
     for (int i = 2; i < 16; ++i) { m01 = habsmax2(m01, x[i].x); m23 = habsmax2(m23, x[i].y); }
+    m01 = abs2(m01); m23 = abs2(m23);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float f[16];
@@ -395,9 +416,9 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   // each tile's 1 KB of scales leaves as 64 x 16 bytes
   {
     const int slot = t / 64, vec = t % 64;
-    const int64_t g2 = (int64_t)bid * TPB + slot;
+    const int g2 = bid * TPB + slot;
     if (slot < TPB && g2 < total)
-      reinterpret_cast<uint4*>(P.vt_sf + g2 * 1024)[vec] = reinterpret_cast<const uint4*>(sf_smem + slot * 1024)[vec];
+      reinterpret_cast<uint4*>(P.vt_sf + (int64_t)g2 * 1024)[vec] = reinterpret_cast<const uint4*>(sf_smem + slot * 1024)[vec];
   }
 }
 
@@ -483,6 +504,7 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   const int64_t k_bytes = (int64_t)a.B * a.Hkv * a.Nk * a.D * 2;
   const bool fits = k_bytes <= 96 << 20 && k_bytes >= 8 << 20;
   P.s_first = fits ? P.q_blocks + P.k_blocks + P.v_blocks : 0;
+  P.by_Tq.set(P.Tq > 0 ? P.Tq : 1); P.by_Tk.set(P.Tk > 0 ? P.Tk : 1); P.by_Hq.set(a.Hq); P.by_Hkv.set(a.Hkv); P.by_chunks.set(P.chunks > 0 ? P.chunks : 1);
   P.order = a.order; P.n_order = a.n_order; P.causal = a.causal;
   P.o_blocks = a.order != nullptr ? 1 : 0;
   const int grid = P.o_blocks + P.s_blocks + P.q_blocks + P.k_blocks + P.v_blocks;

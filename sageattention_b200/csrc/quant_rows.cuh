@@ -58,10 +58,13 @@ __device__ __forceinline__ void quant_rows_store(const uint4 (&w)[kTile / (kThre
                                                  uint8_t* sf_smem) {
   constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
   const int t = threadIdx.x, c = t % CH, rl = t / CH;
+  // scale of block c / 2 in row p * RPP + rl: sf_atom_offset with what depends on p taken out as a constant (rl < RPP <= 32; written as
+  // such, the addresses were 15 % of the instructions)
+  uint8_t* const sf_row = sf_smem + (c >> 3) * 512 + ((c >> 1) & 3) + rl * 16;
+  uint8_t* const out = codes_tile + rl * (D / 2) + c * 4;
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
-    const int row = p * RPP + rl;
-    uint32_t m2 = habsmax2(habsmax2(w[p].x, w[p].y), habsmax2(w[p].z, w[p].w));
+    const uint32_t m2 = abs2(habsmax2(habsmax2(w[p].x, w[p].y), habsmax2(w[p].z, w[p].w)));
     float amax = fmaxf(bf16_lo(m2), bf16_hi(m2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));       // 16-element block = 2 threads
     uint32_t sfb; float inv;
@@ -70,11 +73,9 @@ __device__ __forceinline__ void quant_rows_store(const uint4 (&w)[kTile / (kThre
     const float2 f0 = mul2_ftz(bf16x2_to_f32(w[p].x), inv2), f1 = mul2_ftz(bf16x2_to_f32(w[p].y), inv2);
     const float2 f2 = mul2_ftz(bf16x2_to_f32(w[p].z), inv2), f3 = mul2_ftz(bf16x2_to_f32(w[p].w), inv2);
     const uint32_t code = f32x8_to_e2m1x8(f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y);
-    *reinterpret_cast<uint32_t*>(codes_tile + row * (D / 2) + c * 4) = code;
-    if ((c & 1) == 0) {
-      const int blk = c >> 1;                                        // 16-channel block index
-      sf_smem[(blk >> 2) * 512 + sf_atom_offset(row, blk & 3)] = (uint8_t)sfb;
-    }
+    *reinterpret_cast<uint32_t*>(out + p * (RPP * D / 2)) = code;
+    static_assert(RPP == 16 || RPP == 32, "rows of a pass");
+    if ((c & 1) == 0) sf_row[RPP == 16 ? (p & 1) * 256 + (p >> 1) * 4 : p * 4] = (uint8_t)sfb;
   }
   __syncthreads();
   constexpr int SFV = (D / 64) * 512 / 16;                           // 16-byte vectors of scales
