@@ -18,7 +18,7 @@
 // tensor map).  HBM-bound: the output ([Tq x 128] bf16 per CTA and query head) dominates the traffic, in a chain of
 // dependent steps per CTA.  So a CTA walks several key tiles of a head: tensor memory, barrier and K means are set up once, and
 // the next tile's rows are on their way (in the registers that the quantised tile leaves) during the MMAs and stores of the
-// present one (B4 H32 N4096 D64 52 -> 45 us, B1 H40 N9450 66 -> 57 us, B1 H40 N32760 327 -> 314 us; one tile per CTA with three
+// present one (B4 H32 N4096 D64 52 -> 45 us, B1 H40 N9450 66 -> 57 us, B1 H40 N32760 327 -> 314 us, by now 282; one tile per CTA with three
 // CTAs per SM was the best without that).  Up to 128 rows of A (kMulti = false) A is loaded once per CTA; with more, the next
 // 128 wait in registers during a round (390 us without).
 //
@@ -28,7 +28,7 @@
 //
 // Operand layout in shared memory (K-major, no swizzle): 8-row x 16-byte core matrices; the 16 row groups of one
 // 8-channel chunk are contiguous (128 B apart), chunks are kChunk bytes apart - 16 bytes more than their size so
-// that the 16 lanes which write one row's chunks hit different banks.
+// that the lanes which write one row's chunks hit different banks (A: 16 of them, K: as RowTile deals them out).
 #include <cuda.h>
 
 #include <atomic>
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   uint8_t* sA = dyn_smem + kDsStageBytes;              // 128 Q block means [CH][kChunk]
   uint8_t* sB = sA + kTileBytes;                       // smoothed K tile  [CH][kChunk]
   uint8_t* sf_smem = sB + kTileBytes;                  // 2048 B
-  uint8_t* misc = sf_smem + 2048;                      // mbarrier (8 B), tensor-memory slot (4 B)
+  uint8_t* misc = sf_smem + 2048;                      // mbarrier (8 B), tensor-memory slot (4 B), from byte 16 on the K means
   const uint32_t bar = smem_u32(misc), slot = smem_u32(misc + 8);
   const int first = blockIdx.x * P.run, bh = blockIdx.y, b = bh / P.Hkv, hkv = bh % P.Hkv;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, c = t % CH, rl = t / CH;
@@ -88,19 +88,28 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
       return;
     }
   }
-  const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + c * 8;
+  using R = RowTile<D>;
+  const int kc = R::block(t), krl = R::row(t);          // K rows: 16 channels a thread (A rows, c and rl: 8)
+  const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + kc * 16;
+  auto place = [&](const int p, const int i) {          // of channels 8 i ... of this thread's row p in sB
+    const int row = p * R::kRows + krl;
+    return reinterpret_cast<uint4*>(sB + (2 * kc + i) * kChunk + (row >> 3) * 128 + (row & 7) * 16);
+  };
   const int end = min(first + P.run, P.cu_k != nullptr ? (Nk + kTile - 1) / kTile : P.Tk);
   // token in slot `row` of a tile (kPack: 16 slots hold 15 tokens, none the first)
   auto token_of = [&](const int tile, const int row) {
     if (!kPack) return tile * kTile + row;
     return (row & 15) == 0 ? -1 : (tile * (kTile / 16) + (row >> 4)) * kGroup + (row & 15) - 1;
   };
-  uint4 w[NP];
+  uint4 w[R::kPasses][2];
   auto load = [&](const int tile) {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {                     // all loads in flight before the first use
-      const int n = token_of(tile, p * RPP + rl);
-      w[p] = (n >= 0 && n < Nk && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn) : make_uint4(0, 0, 0, 0);
+    for (int p = 0; p < R::kPasses; ++p) {             // all loads in flight before the first use
+      const int n = token_of(tile, p * R::kRows + krl);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        w[p][i] = (n >= 0 && n < Nk && kc * 16 + 8 * i < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn + 8 * i)
+                                                                 : make_uint4(0, 0, 0, 0);
     }
   };
   load(first);
@@ -134,15 +143,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   };
   if (!kMulti) load_a(0);
   const bool smooth = P.km != nullptr || P.partial != nullptr;
-  float2 neg[4];
-  if (smooth) {
+  float* const neg_s = reinterpret_cast<float*>(misc + 16) + kc * 16 + (kc >> 1) * 4;   // this thread's means, negative (four words further
+  if (smooth) {                                                                        // every 32 channels, for the banks)
     static_assert(kMaxChunks * D * 4 <= (int)kTileBytes, "partial rows of the K mean");
-    float mean[8];
+    float mean[16];
     k_mean<D>(P.km, P.partial + (int64_t)bh * P.chunks * D, P.chunks, (float)max(Nk, 1), bh, reinterpret_cast<float*>(sB),
               first == 0 ? P.km_out : nullptr, mean);
-    __syncthreads();                                   // every thread has its means: sB takes the K tile
+    if (krl == 0)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) neg[i] = make_float2(-mean[2 * i], -mean[2 * i + 1]);
+      for (int i = 0; i < 16; ++i) neg_s[i] = -mean[i];
+    __syncthreads();                                   // every thread has read the means from sB, which takes the K tile
   }
   bool ok = true;
   uint32_t done = 0;                                   // rounds so far, of all tiles
@@ -150,17 +160,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   for (int tile = first; tile < end && ok; ++tile) {
   if (smooth) {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      if (const int n = token_of(tile, p * RPP + rl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
-        w[p] = subtract_mean(w[p], neg);
-      }
+    for (int i = 0; i < 2; ++i) {
+      const float4 a = reinterpret_cast<const float4*>(neg_s)[2 * i], b4 = reinterpret_cast<const float4*>(neg_s)[2 * i + 1];
+      const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b4.x, b4.y}, {b4.z, b4.w}};
+#pragma unroll
+      for (int p = 0; p < R::kPasses; ++p)
+        if (const int n = token_of(tile, p * R::kRows + krl); n >= 0 && n < Nk)   // padding rows stay zero (the reference subtracts before padding)
+          w[p][i] = subtract_mean(w[p][i], neg);
     }
   }
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    const int row = p * RPP + rl;
-    *reinterpret_cast<uint4*>(sB + c * kChunk + (row >> 3) * 128 + (row & 7) * 16) = w[p];
-  }
+  for (int p = 0; p < R::kPasses; ++p) { *place(p, 0) = w[p][0]; *place(p, 1) = w[p][1]; }
   if constexpr (kPack) {
     // one warp per group: rows 16 warp ... +15 of the tile, lane l channels l*C ... (8-channel chunks of sB)
     constexpr int C = D / 32;
@@ -187,10 +197,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
     if (lane < 16) P.lam[((int64_t)bh * P.Tk + tile) * kTile + warp * 16 + lane] = my_lam;
     __syncthreads();
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int row = p * RPP + rl;
-      w[p] = *reinterpret_cast<const uint4*>(sB + c * kChunk + (row >> 3) * 128 + (row & 7) * 16);
-    }
+    for (int p = 0; p < R::kPasses; ++p) { w[p][0] = *place(p, 0); w[p][1] = *place(p, 1); }
   }
   if (P.k_codes != nullptr) {
     const int64_t kt = (int64_t)bh * P.Tk + tile;
@@ -314,7 +321,7 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const bool multi = P.rows > 128;
-  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + 1024;
+  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + (a.D + a.D / 8) * 4 + 1024;
   static std::atomic<unsigned long long> ready[8];      // per kernel: devices on which the shared memory was asked for
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

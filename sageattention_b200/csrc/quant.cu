@@ -13,10 +13,10 @@
 // (common.cuh: block_scale, f32x8_to_e2m1x8), so codes and scale bytes are bit-identical.
 //
 // Memory plan (HBM-bound): every thread issues all of its 128-bit loads for a 128-token tile
-// before the first use (a whole 32 KB tile in flight per CTA), pairs of threads combine their
-// 8-element absmax with one warp shuffle, codes leave as full 32-byte sectors and the scale
-// bytes are staged in shared memory so that they leave as 16-byte vectors in the exact order
-// the attention kernel's tcgen05.cp expects.
+// before the first use (a whole 32 KB tile in flight per CTA) and owns whole 16-element blocks, codes
+// leave as full 32-byte sectors and the scale bytes are staged in shared memory so that they leave as
+// 16-byte vectors in the exact order the attention kernel's tcgen05.cp expects.  What paces it is instructions
+// (about 60 % of the issue slots) as much as memory: 12 per element of Q, 12 of V with its share of the K sums.
 //
 // Output layouts (per batch b, head h; Np = tokens padded to a multiple of 128, T = Np/128):
 //   codes  Q,K : [T][128 rows][D/2] bytes            (row-major, element 2i in the low nibble)
@@ -196,11 +196,11 @@ __device__ __forceinline__ void varlen_order(const QuantLaunch& P, int* hist) {
 // 260 at three per SM)
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunch P) {
-  constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
+  using R = RowTile<D>;
   __shared__ __align__(16) uint8_t sf_smem[2048];
-  __shared__ __align__(16) float red[RPP * D];
-  __shared__ __align__(16) float mean_s[D];
-  const int t = threadIdx.x, c = t % CH, rl = t / CH;
+  __shared__ __align__(16) float red[kThreads / (D / 8) * D];    // (what the K channel sums need; the Q means less)
+  __shared__ __align__(16) float mean_s[D + D / 8];              // four words further every 32 channels, for the banks
+  const int t = threadIdx.x, c = R::block(t), rl = R::row(t);
   int bid = blockIdx.x;
   pdl_launch_dependents();                 // the K kernel may come in and fetch its tiles as SMs fall idle
   if (bid == 0 && t == 0 && P.zero_status != nullptr) *P.zero_status = 0;
@@ -239,90 +239,95 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       N = min(cu[b + 1] - cu[b], N);       // cut at max_seqlen, which sizes the output layouts
       src = (is_q ? P.q + h * P.q_sh : P.k + h * P.k_sh) + (int64_t)cu[b] * sn;
       if (is_q && tile * kTile >= N) {     // beyond the sequence: only the block mean is read (for delta_s rows that no
-        if (P.q_mean_mode == 1 && rl == 0) //   query uses), so it must at least be a number
-          *reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 8) = make_uint4(0, 0, 0, 0);
+        if (P.q_mean_mode == 1 && rl == 0)  //   query uses), so it must at least be a number
+          for (int i = 0; i < 2; ++i)
+            reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 16)[i] = make_uint4(0, 0, 0, 0);
         return;
       }
     }
-    uint4 w[NP];
+    uint4 w[R::kPasses][2];
+    src += (int64_t)(tile * kTile + rl) * sn + c * 16;
+    const int rows = N - tile * kTile - rl;      // this thread's rows are there below it
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int n = tile * kTile + p * RPP + rl;
-      w[p] = (n < N && c * 8 < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * sn + c * 8) : make_uint4(0, 0, 0, 0);
+    for (int p = 0; p < R::kPasses; ++p) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        w[p][i] = (p * R::kRows < rows && c * 16 + 8 * i < P.d_in) ? *reinterpret_cast<const uint4*>(src + 8 * i) : make_uint4(0, 0, 0, 0);
+      src += R::kRows * sn;
     }
+    float mean[16];
     if (is_q && P.q_dot_km != nullptr) {
       // q . km in fp32 from the raw rows: what K smoothing took out of every score of the row; the attention
       // kernel adds sm_scale times it to the log-sum-exp (the pattern of sageattention/core.py:993-994)
-      const int hkv = h / (P.Hq / P.Hkv);
-      const uint4 m = *reinterpret_cast<const uint4*>(P.km_for_q + ((int64_t)b * P.Hkv + hkv) * D + c * 8);
-      const float kmv[8] = {bf16_lo(m.x), bf16_hi(m.x), bf16_lo(m.y), bf16_hi(m.y),
-                            bf16_lo(m.z), bf16_hi(m.z), bf16_lo(m.w), bf16_hi(m.w)};
+      bf16x16_to_f32(P.km_for_q + ((int64_t)b * P.Hkv + h / (P.Hq / P.Hkv)) * D + c * 16, mean);
 #pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        float d = bf16_lo(w[p].x) * kmv[0];
-        d = fmaf(bf16_hi(w[p].x), kmv[1], d); d = fmaf(bf16_lo(w[p].y), kmv[2], d); d = fmaf(bf16_hi(w[p].y), kmv[3], d);
-        d = fmaf(bf16_lo(w[p].z), kmv[4], d); d = fmaf(bf16_hi(w[p].z), kmv[5], d); d = fmaf(bf16_lo(w[p].w), kmv[6], d);
-        d = fmaf(bf16_hi(w[p].w), kmv[7], d);
+      for (int p = 0; p < R::kPasses; ++p) {
+        float d = 0.f;
 #pragma unroll
-        for (int o = 1; o < CH; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        const int n = tile * kTile + p * RPP + rl;
-        if (c == 0 && n < N) P.q_dot_km[(int64_t)bh * P.Nq + n] = d;
+        for (int i = 0; i < 2; ++i) {
+          const uint4 x = w[p][i];
+          const float* m = mean + 8 * i;
+          d = fmaf(bf16_lo(x.x), m[0], d); d = fmaf(bf16_hi(x.x), m[1], d); d = fmaf(bf16_lo(x.y), m[2], d); d = fmaf(bf16_hi(x.y), m[3], d);
+          d = fmaf(bf16_lo(x.z), m[4], d); d = fmaf(bf16_hi(x.z), m[5], d); d = fmaf(bf16_lo(x.w), m[6], d); d = fmaf(bf16_hi(x.w), m[7], d);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+          if (o & R::kBlockBits) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (c == 0 && p * R::kRows < rows) P.q_dot_km[(int64_t)bh * P.Nq + tile * kTile + p * R::kRows + rl] = d;
       }
     }
-    float mean[8];
     bool subtract = true;
     if (is_q && P.q_mean_mode == 1) {
       if (P.qm_override != nullptr) {
-        const float* mp = P.qm_override + ((int64_t)bh * T + tile) * D + c * 8;
+        const float* mp = P.qm_override + ((int64_t)bh * T + tile) * D + c * 16;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mean[i] = mp[i];
+        for (int i = 0; i < 16; ++i) mean[i] = mp[i];
       } else {
-        // fp32 column sums over the tile's 128 rows (zero rows of the padding included), / 128
-        float2 acc2[4] = {};
+        // fp32 column sums over the tile's 128 rows (zero rows of the padding included), / 128: the thread's rows, the warp's (each
+        // step of the exchange leaves a lane half the channels), the CTA's
+        float2 acc2[2][4] = {};
 #pragma unroll
-        for (int p = 0; p < NP; ++p) add_channels(acc2, w[p]);
-        float acc[8];
+        for (int p = 0; p < R::kPasses; ++p) { add_channels(acc2[0], w[p][0]); add_channels(acc2[1], w[p][1]); }
+        float acc[16];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { acc[2 * i] = acc2[i].x; acc[2 * i + 1] = acc2[i].y; }
-        if (CH == 16) {
+        for (int i = 0; i < 8; ++i) { acc[2 * i] = acc2[i >> 2][i & 3].x; acc[2 * i + 1] = acc2[i >> 2][i & 3].y; }
+        int first = 0;                           // of the channels that this lane is left with
 #pragma unroll
-          for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
-        } else {
+        for (int step = 0; step < (D == 128 ? 2 : 3); ++step) {
+          const int o = step == 0 ? 16 : (D == 128 ? 4 : 16 >> step), n = 16 >> (step + 1);   // the lane's bits that are the row
+          const bool upper = (t & o) != 0;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 8);
-            acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+          for (int i = 0; i < n; ++i) {
+            const float give = upper ? acc[i] : acc[n + i], own = upper ? acc[n + i] : acc[i];
+            acc[i] = own + __shfl_xor_sync(0xffffffffu, give, o);
           }
+          if (upper) first += n;
         }
-        if ((t & 31) < CH) {
+        constexpr int kLeft = D == 128 ? 4 : 2;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) red[(t >> 5) * D + c * 8 + i] = acc[i];
-        }
+        for (int i = 0; i < kLeft; ++i) red[(t >> 5) * D + c * 16 + first + i] = acc[i];
         __syncthreads();
         if (t < D) {
           float s = 0.f;
 #pragma unroll
           for (int r = 0; r < kThreads / 32; ++r) s += red[r * D + t];
-          mean_s[t] = s * (1.0f / kTile);
+          mean_s[t + (t >> 5) * 4] = s * (1.0f / kTile);
         }
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mean[i] = mean_s[c * 8 + i];
+        for (int i = 0; i < 16; ++i) mean[i] = mean_s[c * 16 + (c >> 1) * 4 + i];
       }
       if (rl == 0) {   // bf16 block mean, consumed by the delta_s kernel
-        uint4 o;
-        o.x = pack_bf16(mean[0], mean[1]); o.y = pack_bf16(mean[2], mean[3]);
-        o.z = pack_bf16(mean[4], mean[5]); o.w = pack_bf16(mean[6], mean[7]);
-        *reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 8) = o;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 16)[i] =
+              make_uint4(pack_bf16(mean[8 * i], mean[8 * i + 1]), pack_bf16(mean[8 * i + 2], mean[8 * i + 3]),
+                         pack_bf16(mean[8 * i + 4], mean[8 * i + 5]), pack_bf16(mean[8 * i + 6], mean[8 * i + 7]));
       }
     } else if (is_q && P.q_mean_mode == 2) {
-      uint4 m = *reinterpret_cast<const uint4*>(P.q_mean_seq + (int64_t)bh * D + c * 8);
-      mean[0] = bf16_lo(m.x); mean[1] = bf16_hi(m.x); mean[2] = bf16_lo(m.y); mean[3] = bf16_hi(m.y);
-      mean[4] = bf16_lo(m.z); mean[5] = bf16_hi(m.z); mean[6] = bf16_lo(m.w); mean[7] = bf16_hi(m.w);
+      bf16x16_to_f32(P.q_mean_seq + (int64_t)bh * D + c * 16, mean);
     } else if (!is_q && P.km != nullptr) {
-      uint4 m = *reinterpret_cast<const uint4*>(P.km + (int64_t)bh * D + c * 8);
-      mean[0] = bf16_lo(m.x); mean[1] = bf16_hi(m.x); mean[2] = bf16_lo(m.y); mean[3] = bf16_hi(m.y);
-      mean[4] = bf16_lo(m.z); mean[5] = bf16_hi(m.z); mean[6] = bf16_lo(m.w); mean[7] = bf16_hi(m.w);
+      bf16x16_to_f32(P.km + (int64_t)bh * D + c * 16, mean);
     } else {
       subtract = false;
     }
@@ -330,11 +335,13 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       // x - mean in fp32, rounded to bf16 (what a bf16 tensor subtraction does).  Q: padding rows
       // become -mean like the reference (it pads before subtracting); K: padding rows stay zero
       // (the reference subtracts before padding).
-      const float2 neg[4] = {{-mean[0], -mean[1]}, {-mean[2], -mean[3]}, {-mean[4], -mean[5]}, {-mean[6], -mean[7]}};
 #pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const int n = tile * kTile + p * RPP + rl;
-        if (is_q || n < N) w[p] = subtract_mean(w[p], neg);
+      for (int i = 0; i < 2; ++i) {
+        const float2 neg[4] = {{-mean[8 * i], -mean[8 * i + 1]}, {-mean[8 * i + 2], -mean[8 * i + 3]},
+                               {-mean[8 * i + 4], -mean[8 * i + 5]}, {-mean[8 * i + 6], -mean[8 * i + 7]}};
+#pragma unroll
+        for (int p = 0; p < R::kPasses; ++p)
+          if (is_q || p * R::kRows < rows) w[p][i] = subtract_mean(w[p][i], neg);
       }
     }
     uint8_t* codes = (is_q ? P.q_codes : P.k_codes) + ((int64_t)bh * T + tile) * (kTile * D / 2);

@@ -9,7 +9,30 @@ namespace sage3 {
 constexpr int kTile = 128;
 constexpr int kThreads = 256;
 
-// The 8 channels of this thread (chunk threadIdx.x % (D/8)) of a head's K mean: from `km` where it is given, else from
+// Row-wise quantisation of one 128-token tile held in registers (Q and K roles).  Thread t owns the 16 channels 16 block(t) ... of
+// rows row(t), + kRows, ...: whole quantisation blocks, so that scales need no exchange and are worked out once.  (With 8 channels a
+// thread, two threads to a block: B1 H40 N32760 228 -> 219 us, K pass 321 -> 292.)
+// Which lane has which, D=128: bits 0, 1 and 3 are the block, 2 and 4 the row, so that 8 lanes' 16-byte stores of the K pass
+// (delta_s.cu), 4128 bytes from block to block and 16 from row to row, meet different banks.
+// ------------------------------------------------------------------------------------------------
+template <int D>
+struct RowTile {
+  static constexpr int kPerRow = D / 16, kRows = kThreads / kPerRow, kPasses = kTile / kRows;
+  static constexpr int kBlockBits = D == 128 ? 11 : 3;     // bits of the lane that are the block
+  static __device__ __forceinline__ int block(const int t) { return D == 128 ? (t & 3) | ((t >> 1) & 4) : t & 3; }
+  static __device__ __forceinline__ int row(const int t) { return D == 128 ? ((t >> 2) & 1) | ((t >> 4) << 1) : t >> 2; }
+  static_assert(kRows == 32 || kRows == 64, "rows of a pass");
+};
+__device__ __forceinline__ void bf16x16_to_f32(const __nv_bfloat16* p, float (&x)[16]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint4 m = reinterpret_cast<const uint4*>(p)[i];
+    x[8 * i] = bf16_lo(m.x); x[8 * i + 1] = bf16_hi(m.x); x[8 * i + 2] = bf16_lo(m.y); x[8 * i + 3] = bf16_hi(m.y);
+    x[8 * i + 4] = bf16_lo(m.z); x[8 * i + 5] = bf16_hi(m.z); x[8 * i + 6] = bf16_lo(m.w); x[8 * i + 7] = bf16_hi(m.w);
+  }
+}
+
+// The 16 channels of this thread (16 block(threadIdx.x) ...) of a head's K mean: from `km` where it is given, else from
 // the partial sums, by the whole CTA; also written to km_out if that is not null.  `stage`: shared memory for kMaxChunks
 // partial rows - they are fetched all at once, so that the CTA waits for memory once and not once per few rows (the K
 // kernel at B1 H40 N32760: 328 us, 356 with a chain of loads).
@@ -17,12 +40,10 @@ constexpr int kMaxChunks = 64;             // at most so many partial rows per h
 template <int D>
 __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, const float* __restrict__ partial, const int nchunks,
                                        const float divisor, const int64_t bh, float* stage, __nv_bfloat16* km_out,
-                                       float (&mean)[8]) {
-  const int t = threadIdx.x, c = t % (D / 8);
+                                       float (&mean)[16]) {
+  const int t = threadIdx.x, c = RowTile<D>::block(t);
   if (km != nullptr) {
-    const uint4 m = *reinterpret_cast<const uint4*>(km + bh * D + c * 8);
-    mean[0] = bf16_lo(m.x); mean[1] = bf16_hi(m.x); mean[2] = bf16_lo(m.y); mean[3] = bf16_hi(m.y);
-    mean[4] = bf16_lo(m.z); mean[5] = bf16_hi(m.z); mean[6] = bf16_lo(m.w); mean[7] = bf16_hi(m.w);
+    bf16x16_to_f32(km + bh * D + c * 16, mean);
     return;
   }
   constexpr int V = kMaxChunks * D / 4 / kThreads;
@@ -46,36 +67,34 @@ __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, con
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) mean[i] = stage[c * 8 + i];
+  for (int i = 0; i < 16; ++i) mean[i] = stage[c * 16 + i];
 }
 
-// Row-wise quantisation of one 128-token tile held in registers (Q and K roles).
-// Thread t owns 8 consecutive channels (chunk c) of rows rl, rl+RPP, ... ; w[p] = 4 packed bf16x2.
-// ------------------------------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void quant_rows_store(const uint4 (&w)[kTile / (kThreads / (D / 8))],
-                                                 uint8_t* __restrict__ codes_tile, uint8_t* __restrict__ sf_tile,
-                                                 uint8_t* sf_smem) {
-  constexpr int CH = D / 8, RPP = kThreads / CH, NP = kTile / RPP;
-  const int t = threadIdx.x, c = t % CH, rl = t / CH;
-  // scale of block c / 2 in row p * RPP + rl: sf_atom_offset with what depends on p taken out as a constant (rl < RPP <= 32; written as
-  // such, the addresses were 15 % of the instructions)
-  uint8_t* const sf_row = sf_smem + (c >> 3) * 512 + ((c >> 1) & 3) + rl * 16;
-  uint8_t* const out = codes_tile + rl * (D / 2) + c * 4;
+__device__ __forceinline__ void quant_rows_store(const uint4 (&w)[RowTile<D>::kPasses][2], uint8_t* __restrict__ codes_tile,
+                                                 uint8_t* __restrict__ sf_tile, uint8_t* sf_smem) {
+  using R = RowTile<D>;
+  const int t = threadIdx.x, c = R::block(t), rl = R::row(t);
+  // sf_atom_offset of row p * kRows + rl, with what depends on p taken out as a constant (left to the compiler, the addresses were
+  // 15 % of the instructions)
+  uint8_t* const sf_row = sf_smem + (c >> 2) * 512 + (c & 3) + (rl & 31) * 16 + (rl >> 5) * 4;
+  uint8_t* const out = codes_tile + rl * (D / 2) + c * 8;
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    const uint32_t m2 = abs2(habsmax2(habsmax2(w[p].x, w[p].y), habsmax2(w[p].z, w[p].w)));
-    float amax = fmaxf(bf16_lo(m2), bf16_hi(m2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));       // 16-element block = 2 threads
+  for (int p = 0; p < R::kPasses; ++p) {
+    uint32_t m2 = habsmax2(habsmax2(w[p][0].x, w[p][0].y), habsmax2(w[p][0].z, w[p][0].w));
+    m2 = abs2(habsmax2(m2, habsmax2(habsmax2(w[p][1].x, w[p][1].y), habsmax2(w[p][1].z, w[p][1].w))));
     uint32_t sfb; float inv;
-    block_scale(amax, sfb, inv);
+    block_scale(fmaxf(bf16_lo(m2), bf16_hi(m2)), sfb, inv);
     const float2 inv2 = make_float2(inv, inv);
-    const float2 f0 = mul2_ftz(bf16x2_to_f32(w[p].x), inv2), f1 = mul2_ftz(bf16x2_to_f32(w[p].y), inv2);
-    const float2 f2 = mul2_ftz(bf16x2_to_f32(w[p].z), inv2), f3 = mul2_ftz(bf16x2_to_f32(w[p].w), inv2);
-    const uint32_t code = f32x8_to_e2m1x8(f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y);
-    *reinterpret_cast<uint32_t*>(out + p * (RPP * D / 2)) = code;
-    static_assert(RPP == 16 || RPP == 32, "rows of a pass");
-    if ((c & 1) == 0) sf_row[RPP == 16 ? (p & 1) * 256 + (p >> 1) * 4 : p * 4] = (uint8_t)sfb;
+    uint32_t code[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 f0 = mul2_ftz(bf16x2_to_f32(w[p][i].x), inv2), f1 = mul2_ftz(bf16x2_to_f32(w[p][i].y), inv2);
+      const float2 f2 = mul2_ftz(bf16x2_to_f32(w[p][i].z), inv2), f3 = mul2_ftz(bf16x2_to_f32(w[p][i].w), inv2);
+      code[i] = f32x8_to_e2m1x8(f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y);
+    }
+    *reinterpret_cast<uint2*>(out + p * (R::kRows * D / 2)) = make_uint2(code[0], code[1]);
+    sf_row[p * (R::kRows / 32) * 4] = (uint8_t)sfb;
   }
   __syncthreads();
   constexpr int SFV = (D / 64) * 512 / 16;                           // 16-byte vectors of scales
