@@ -335,7 +335,11 @@ int sage3_attention(const sage3_fwd_args* a, void* stream) {
     cudaError_t e = cudaMemsetAsync(a->km_out, 0, z.km, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e);
   }
+  if (int st = check_tensor(a->v)) return st;
+  const bool v_later = decode && sage3::decode_takes_v(a->shape.B, a->shape.Hq, a->shape.Hkv, a->shape.Nq, a->shape.Nk, a->shape.D);
+  if (v_later) q.v.ptr = nullptr;                       // quantised beside the scores
   if (int st = quant_qkv_impl(&q, nullptr, nullptr, stream, status, nullptr, nullptr, 0, nullptr, 0, decode ? &decode_k : nullptr)) return st;
+  if (v_later) { decode_k.v = a->v.ptr; decode_k.v_sb = a->v.stride_b; decode_k.v_sh = a->v.stride_h; decode_k.v_sn = a->v.stride_n; }
   sage3_attn_args t{};
   t.shape = a->shape;
   t.q_codes = q.q_codes; t.q_sf = q.q_sf; t.k_codes = q.k_codes; t.k_sf = q.k_sf; t.vt_codes = q.vt_codes; t.vt_sf = q.vt_sf;

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "quant_v.cuh"
 
 namespace sage3 {
 
@@ -31,7 +32,10 @@ constexpr int kMaxChunks = 64;                           // CTAs of the output k
 constexpr int kMaxRows = 64;                             // query rows per kv head
 
 struct DecodeParams {
-  const uint8_t *q_codes, *q_sf, *vt_codes, *vt_sf;
+  const uint8_t *q_codes, *q_sf;
+  uint8_t *vt_codes, *vt_sf;
+  const __nv_bfloat16* v;                                // scores kernel with kV: V as it is
+  int64_t v_sb, v_sh, v_sn;
   const __nv_bfloat16 *k, *qm, *km;                      // km: the K mean, or
   const float* partial;                                  // its partial sums, [kv][mean_chunks][D], or neither
   __nv_bfloat16* km_out;
@@ -145,12 +149,19 @@ __device__ __forceinline__ constexpr int score_place(const int k) { return (k & 
 // works on the present one.  K is smoothed, quantised and multiplied where it was loaded, so neither its codes nor delta_s
 // exist in memory.  kOne: at most 8 query rows; the quantised rows then take the registers of the smoothed ones.
 // (One tile per CTA of four warps, 32 keys each: 47 us at B8 H32/8 Nk4096, now 26.)
-template <int D, bool kOne>
+// kV: V of the same key tile comes through shared memory meanwhile and is quantised behind the scores: the conversions of K leave most
+// of the memory's time unused, and K, of which the launch before has just taken the sums, is still in L2 where V has not been read in
+// between.
+// (D=128 only, see decode_takes_v.)
+constexpr int kVRowsBytes = kTile * 128 * 2 + 8 * 16;    // 16-token blocks 16 bytes further apart, for the banks
+template <int D, bool kOne, bool kV>
 __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores_kernel(const DecodeParams P) {
+  static_assert(!kV || D == 128, "8 warps of 16 channels each");
   constexpr int W = D / 8;                               // words of a lane's part of a row, as halves or bf16
   extern __shared__ __align__(16) uint32_t frag[];       // [groups of 8 query rows][W / 4][32 lanes][4]: Q^, then their Q means
   __shared__ __align__(16) float neg_mean[D + D / 8];    // four words further every 32 channels, for the banks
   __shared__ float tmax[2][8][kOne ? 8 : kMaxRows];
+  __shared__ __align__(16) uint8_t v_sf[kV ? 1024 : 16];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
   const int kv = blockIdx.y, groups = kOne ? 1 : (P.rows + 7) / 8;
   const int first = blockIdx.x * P.score_run, end = min(first + P.score_run, P.Tk);
@@ -169,6 +180,18 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
     }
   };
   load(first);
+  uint8_t* const v_rows = reinterpret_cast<uint8_t*>(frag) + groups * 2 * 32 * W * 4;
+  auto load_v = [&](const int tile) {                    // 16-byte pieces of whole rows; zeros beyond the keys and channels there are
+    constexpr int CH = D / 8, RPP = kScoreThreads / CH;
+    const __nv_bfloat16* v = P.v + kv / P.Hkv * P.v_sb + kv % P.Hkv * P.v_sh + t % CH * 8;
+#pragma unroll
+    for (int p = 0; p < kTile / RPP; ++p) {
+      const int row = p * RPP + t / CH, key = tile * kTile + row;
+      cp_async16(smem_u32(v_rows) + row * D * 2 + (row >> 4) * 16 + t % CH * 16, v + (int64_t)min(key, P.Nk - 1) * P.v_sn,
+                 key < P.Nk && t % CH * 8 < P.d_in);
+    }
+  };
+  if (kV) load_v(first);
   pdl_wait();
   if (blockIdx.x == 0 && t < P.rows) P.counter[kv * P.rows + t] = 0;
   for (int i = t; i < groups * 64; i += kScoreThreads) {
@@ -285,12 +308,24 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
         scores(s, kq, n);
       }
     }
+    if (kV) cp_async_wait_all();
     __syncthreads();                                     // (the other half of tmax is written next)
     if (t < P.rows) {
       float m = tmax[tile & 1][0][t];
 #pragma unroll
       for (int i = 1; i < 8; ++i) m = fmaxf(m, tmax[tile & 1][i][t]);
       P.tile_max[((int64_t)kv * P.rows + t) * P.Tk + tile] = m;
+    }
+    if constexpr (kV) {
+      const int64_t vt = (int64_t)kv * P.Tk + tile;
+      const int d = (warp * 4 + (lane >> 3)) * 4, blk = lane & 7;
+      uint2 x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = *reinterpret_cast<const uint2*>(v_rows + (blk * 16 + i) * D * 2 + blk * 16 + d * 2);
+      quant_v_block(x, d, blk, false, P.vt_codes + vt * (D * 64), v_sf);
+      __syncthreads();                                   // the rows have been read, the scales are complete
+      if (tile + 1 < end) load_v(tile + 1);
+      if (t < 64) reinterpret_cast<uint4*>(P.vt_sf + vt * 1024)[t] = reinterpret_cast<const uint4*>(v_sf)[t];
     }
   }
 }
@@ -511,8 +546,12 @@ cudaError_t launch(DecodeParams P, bool overlap, cudaStream_t stream) {
     if (cost < best) { best = cost; P.score_run = run; }
   }
   const dim3 grid((P.Tk + P.score_run - 1) / P.score_run, P.kvs);
-  e = launch_pdl(P.rows <= 8 ? decode_scores_kernel<D, true> : decode_scores_kernel<D, false>, grid, kScoreThreads, frag, stream,
-                             overlap, P);
+  constexpr bool kV = D == 128;
+  if (kV && P.v != nullptr)
+    e = launch_pdl(decode_scores_kernel<D, true, kV>, grid, kScoreThreads, frag + kVRowsBytes, stream, overlap, P);
+  else
+    e = launch_pdl(P.rows <= 8 ? decode_scores_kernel<D, true, false> : decode_scores_kernel<D, false, false>, grid, kScoreThreads, frag,
+                   stream, overlap, P);
   if (e != cudaSuccess) return e;
   return launch_pdl(decode_output_kernel<D, NT>, dim3((unsigned)(P.kvs * P.chunks), groups), kThreads, 0, stream, true, P);
 }
@@ -527,6 +566,13 @@ bool decode_fits(int Hq, int Hkv, int Nq, int Nk) {
   return Nk > 3 * kTile && rows <= kMaxRows && (Nq <= 8 || (Nq <= 16 && rows <= 32 && Nk > 1024));
 }
 
+// Only the kernels of one group of rows and D=128 (D=64 keeps half the warps busy with V: B8 H32 Nk2000 63.1 -> 64.1 us), and not where
+// a launch is a chain of latencies anyhow (device time without / with: 48 tiles 13.6 / 13.9 us; B1 H32/8 Nk4096, 256 tiles 17.4 / 16.4,
+// B8 58.2 / 55.6, B32 224 / 202, B16 H32 Nk8000 779 / 679).
+bool decode_takes_v(int B, int Hq, int Hkv, int Nq, int Nk, int D) {
+  return D == 128 && Hq / Hkv * Nq <= 8 && (int64_t)B * Hkv * ((Nk + kTile - 1) / kTile) >= 128;
+}
+
 size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D) {
   if (!decode_fits(Hq, Hkv, Nq, Nk)) return 0;
   const size_t Tk = (Nk + kTile - 1) / kTile, rows = (size_t)B * Hq * Nq, chunks = Tk < kMaxChunks ? Tk : kMaxChunks;
@@ -538,7 +584,9 @@ cudaError_t launch_attn_decode(const AttnArgs& a, const DeltaSArgs& k, void* scr
   if ((a.D != 128 && a.D != 64) || !decode_fits(a.Hq, a.Hkv, a.Nq, a.Nk)) return cudaErrorInvalidValue;
   DecodeParams P;
   P.q_codes = (const uint8_t*)a.q_codes; P.q_sf = (const uint8_t*)a.q_sf;
-  P.vt_codes = (const uint8_t*)a.vt_codes; P.vt_sf = (const uint8_t*)a.vt_sf;
+  P.vt_codes = (uint8_t*)a.vt_codes; P.vt_sf = (uint8_t*)a.vt_sf;
+  P.v = (const __nv_bfloat16*)k.v; P.v_sb = k.v_sb; P.v_sh = k.v_sh; P.v_sn = k.v_sn;
+  if ((P.v != nullptr) != decode_takes_v(a.B, a.Hq, a.Hkv, a.Nq, a.Nk, a.D)) return cudaErrorInvalidValue;
   P.k = (const __nv_bfloat16*)k.k; P.k_sb = k.k_sb; P.k_sh = k.k_sh; P.k_sn = k.k_sn;
   P.qm = (const __nv_bfloat16*)k.qm; P.km = (const __nv_bfloat16*)k.km; P.partial = (const float*)k.partial;
   P.km_out = (__nv_bfloat16*)k.km_out;

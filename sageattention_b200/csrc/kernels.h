@@ -93,6 +93,8 @@ struct DeltaSArgs {
   int* status = nullptr;                  // optional device status word for the kernel's bounded wait
   int d_in = 0;                           // as in QuantArgs
   float* k_lambda = nullptr;              // K-packing mode: K (Nk tokens) is packed on the way in, lambdas go here
+  const void* v = nullptr;                // launch_attn_decode where decode_takes_v: bf16 V, strides below
+  int64_t v_sb = 0, v_sh = 0, v_sn = 0;
   bool after_quant = false;               // launched right behind launch_quant_qkv on the same stream: may overlap its end
 };
 cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream);
@@ -125,7 +127,9 @@ cudaError_t launch_attn_fwd_varlen(const AttnArgs& a, cudaStream_t stream);   //
 // Attention of a few query rows per head (decode.cu); scratch of decode_scratch_bytes, 0 where decode_fits says no.
 bool decode_fits(int Hq, int Hkv, int Nq, int Nk);
 size_t decode_scratch_bytes(int B, int Hq, int Hkv, int Nq, int Nk, int D);
-// K is taken as it is, with the means and Q block means that launch_delta_s would get; no codes of K, no delta_s.
+// K is taken as it is, with the means and Q block means that launch_delta_s would get; no codes of K, no delta_s.  With decode_takes_v
+// V is taken as it is too (k.v) and its codes are written on the way; else they are there already.
+bool decode_takes_v(int B, int Hq, int Hkv, int Nq, int Nk, int D);
 cudaError_t launch_attn_decode(const AttnArgs& a, const DeltaSArgs& k, void* scratch, cudaStream_t stream);
 
 // Back-to-back block-scaled FP4 MMAs on resident operands, one CTA per SM (peak.cu); *ctas = CTAs launched.

@@ -28,6 +28,7 @@
 #include "kernels.h"
 #include "pack_group.cuh"
 #include "quant_rows.cuh"
+#include "quant_v.cuh"
 
 namespace sage3 {
 
@@ -382,42 +383,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       src += P.v_sn;
     }
     uint8_t* codes = P.vt_codes + (int64_t)gt * (D * 64);
-    // largest magnitudes of the 4 channels, two at a time (bf16 comparisons are exact)
-    uint32_t m01 = habsmax2(x[0].x, x[1].x), m23 = habsmax2(x[0].y, x[1].y);
-#pragma unroll
-    for (int i = 2; i < 16; ++i) { m01 = habsmax2(m01, x[i].x); m23 = habsmax2(m23, x[i].y); }
-    m01 = abs2(m01); m23 = abs2(m23);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float f[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        uint32_t wv = (j < 2) ? x[i].x : x[i].y;
-        f[i] = (j & 1) ? bf16_hi(wv) : bf16_lo(wv);
-      }
-      const uint32_t mv = j < 2 ? m01 : m23;
-      float amax = (j & 1) ? bf16_hi(mv) : bf16_lo(mv);
-      if (P.split_first) {
-        f[0] = __bfloat162float(__float2bfloat16_rn(split_first_value(f[1], amax)));
-        amax = fmaxf(fabsf(f[0]), fabsf(f[1]));
-#pragma unroll
-        for (int i = 2; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
-      }
-      uint32_t sfb; float inv;
-      block_scale(amax, sfb, inv);
-      const float2 inv2 = make_float2(inv, inv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float2 y = mul2_ftz(make_float2(f[2 * i], f[2 * i + 1]), inv2);
-        f[2 * i] = y.x; f[2 * i + 1] = y.y;
-      }
-      uint2 o;
-      o.x = f32x8_to_e2m1x8(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
-      o.y = f32x8_to_e2m1x8(f[8], f[9], f[10], f[11], f[12], f[13], f[14], f[15]);
-      const int d = c4 * 4 + j;
-      *reinterpret_cast<uint2*>(codes + d * 64 + blk * 8) = o;
-      sf_smem[tl * 1024 + (blk >> 2) * 512 + sf_atom_offset(d, blk & 3)] = (uint8_t)sfb;
-    }
+    quant_v_block(x, c4 * 4, blk, P.split_first, codes, sf_smem + tl * 1024);
   }
   __syncthreads();
   // each tile's 1 KB of scales leaves as 64 x 16 bytes

@@ -37,6 +37,20 @@ def test_few_query_rows(B, Hq, Hkv, Nq, Nk, D, causal):
     assert torch.allclose(lse, other_lse + term, atol=4e-3, rtol=1e-4)
 
 
+# V quantised beside the scores: from 128 key tiles of all kv heads on (one fewer: beside the K sums), a last tile of one key, narrow
+# rows, tokens strided; against the tile kernels on V quantised by its own launch, up to the order of fp32 sums (<= 1e-3, as above)
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,d,layout", [
+    (1, 1, 1, 1, 16256, 128, "HND"), (1, 1, 1, 1, 16257, 128, "HND"), (4, 8, 8, 1, 513, 72, "NHD"), (3, 32, 8, 2, 1000, 104, "HND"),
+    (16, 8, 8, 8, 640, 128, "NHD")])
+def test_v_quantised_beside_the_scores(B, Hq, Hkv, Nq, Nk, d, layout):
+    q, k, v = (t[..., :d] for t in U.make_qkv(B, Hq, Hkv, Nq, Nk, 128, seed=Nk + d, device=DEV, layout=layout))
+    v = v * torch.arange(1, Hkv + 1, device=DEV).view((1, -1, 1, 1) if layout == "HND" else (1, 1, -1, 1)).to(v.dtype)
+    out = sa.sageattn(q, k, v, tensor_layout=layout, is_causal=True, sm_scale=0.1, check_status=True)
+    q, k, v = (torch.nn.functional.pad(t, (0, 128 - d)) for t in (q, k, v))
+    want = sa.fp4_attention(sa.quantize_qkv(q, k, v, tensor_layout=layout), is_causal=True, sm_scale=0.1, tensor_layout=layout)
+    assert sage3.accuracy(out.float().cpu(), want[..., :d].float().cpu())[1] <= 1e-3
+
+
 def test_few_query_rows_in_other_layouts():
     q, k, v = U.make_qkv(2, 8, 2, 3, 1300, 128, seed=5, device=DEV)
     want = sa.sageattn(q, k, v, is_causal=True)
