@@ -108,6 +108,16 @@ __device__ __forceinline__ uint4 subtract_mean(const uint4& w, const float2 (&ne
   return make_uint4(pack_bf16(fadd2(bf16x2_to_f32(w.x), neg[0])), pack_bf16(fadd2(bf16x2_to_f32(w.y), neg[1])),
                     pack_bf16(fadd2(bf16x2_to_f32(w.z), neg[2])), pack_bf16(fadd2(bf16x2_to_f32(w.w), neg[3])));
 }
+// The same for a mean that is a bf16 value: the packed subtraction rounds the exact difference once, and no pair of bf16 values
+// exists for which rounding to fp32 first would change that (all 2^32 compared on the device, NaNs and subnormals included).
+__device__ __forceinline__ uint4 subtract_mean(const uint4& w, const uint4& mean) {
+  uint4 r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r.x) : "r"(w.x), "r"(mean.x));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r.y) : "r"(w.y), "r"(mean.y));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r.z) : "r"(w.z), "r"(mean.z));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r.w) : "r"(w.w), "r"(mean.w));
+  return r;
+}
 __device__ __forceinline__ void add_channels(float2 (&acc)[4], const uint4& w) {
   acc[0] = fadd2(acc[0], bf16x2_to_f32(w.x)); acc[1] = fadd2(acc[1], bf16x2_to_f32(w.y));
   acc[2] = fadd2(acc[2], bf16x2_to_f32(w.z)); acc[3] = fadd2(acc[3], bf16x2_to_f32(w.w));

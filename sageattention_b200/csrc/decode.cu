@@ -159,7 +159,7 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
   static_assert(!kV || D == 128, "8 warps of 16 channels each");
   constexpr int W = D / 8;                               // words of a lane's part of a row, as halves or bf16
   extern __shared__ __align__(16) uint32_t frag[];       // [groups of 8 query rows][W / 4][32 lanes][4]: Q^, then their Q means
-  __shared__ __align__(16) float neg_mean[D + D / 8];    // four words further every 32 channels, for the banks
+  __shared__ __align__(16) __nv_bfloat16 mean_s[D];
   __shared__ float tmax[2][8][kOne ? 8 : kMaxRows];
   __shared__ __align__(16) uint8_t v_sf[kV ? 1024 : 16];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
@@ -214,19 +214,18 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
   if (t >= kScoreThreads - D) {
     // the mean: given, or from the partial sums (same order and rounding as in the other K kernel), or none
     const int d = t - (kScoreThreads - D);
-    float m = 0.f;
+    __nv_bfloat16 m = __float2bfloat16_rn(0.f);
     if (P.km != nullptr) {
-      m = __bfloat162float(P.km[(int64_t)kv * D + d]);
+      m = P.km[(int64_t)kv * D + d];
     } else if (P.partial != nullptr) {
       const float* p = P.partial + (int64_t)kv * P.mean_chunks * D + d;
       float s = 0.f;
 #pragma unroll 16
       for (int i = 0; i < P.mean_chunks; ++i) s += __ldcg(p + i * D);
-      const __nv_bfloat16 b = __float2bfloat16_rn(s / (float)P.Nk);
-      if (blockIdx.x == 0 && P.km_out != nullptr) P.km_out[(int64_t)kv * D + d] = b;
-      m = __bfloat162float(b);
+      m = __float2bfloat16_rn(s / (float)P.Nk);
+      if (blockIdx.x == 0 && P.km_out != nullptr) P.km_out[(int64_t)kv * D + d] = m;
     }
-    neg_mean[d + d / 32 * 4] = -m;
+    mean_s[d] = m;
   }
   __syncthreads();
   const int64_t ld = (int64_t)P.Tk * kTile;
@@ -237,13 +236,11 @@ __global__ __launch_bounds__(kScoreThreads, D == 128 ? 2 : 3) void decode_scores
     const int key = tile * kTile + 16 * warp + g;
 #pragma unroll
     for (int j = 0; j < W / 4; ++j) {
-      const float* nm = &neg_mean[channel(tg, j) + channel(tg, j) / 32 * 4];
-      const float4 a = *reinterpret_cast<const float4*>(nm), b = *reinterpret_cast<const float4*>(nm + 4);
-      const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
+      const uint4 mean = *reinterpret_cast<const uint4*>(&mean_s[channel(tg, j)]);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         uint4 x = w[i][j];
-        if (P.smooth && key + 8 * i < P.Nk) x = subtract_mean(x, neg);     // padding rows stay zero
+        if (P.smooth && key + 8 * i < P.Nk) x = subtract_mean(x, mean);    // padding rows stay zero
         kb[i][4 * j] = x.x; kb[i][4 * j + 1] = x.y; kb[i][4 * j + 2] = x.z; kb[i][4 * j + 3] = x.w;
         amax[i][j] = habsmax2(habsmax2(x.x, x.y), habsmax2(x.z, x.w));
       }

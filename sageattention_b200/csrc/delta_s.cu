@@ -143,31 +143,28 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   };
   if (!kMulti) load_a(0);
   const bool smooth = P.km != nullptr || P.partial != nullptr;
-  float* const neg_s = reinterpret_cast<float*>(misc + 16) + kc * 16 + (kc >> 1) * 4;   // this thread's means, negative (four words further
-  if (smooth) {                                                                        // every 32 channels, for the banks)
+  // this thread's means: in registers, or (kMulti, where the waiting A rows take them) in shared memory
+  uint4 mean[2];
+  uint4* const mean_s = reinterpret_cast<uint4*>(misc + 16) + 2 * kc;
+  if (smooth) {
     static_assert(kMaxChunks * D * 4 <= (int)kTileBytes, "partial rows of the K mean");
-    float mean[16];
     k_mean<D>(P.km, P.partial + (int64_t)bh * P.chunks * D, P.chunks, (float)max(Nk, 1), bh, reinterpret_cast<float*>(sB),
               first == 0 ? P.km_out : nullptr, mean);
-    if (krl == 0)
-#pragma unroll
-      for (int i = 0; i < 16; ++i) neg_s[i] = -mean[i];
-    __syncthreads();                                   // every thread has read the means from sB, which takes the K tile
+    if (kMulti && krl == 0) { mean_s[0] = mean[0]; mean_s[1] = mean[1]; }
+    __syncthreads();                                   // every thread has its means: sB takes the K tile
   }
   bool ok = true;
   uint32_t done = 0;                                   // rounds so far, of all tiles
 #pragma unroll 1
   for (int tile = first; tile < end && ok; ++tile) {
   if (smooth) {
+    if (kMulti) { mean[0] = mean_s[0]; mean[1] = mean_s[1]; }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float4 a = reinterpret_cast<const float4*>(neg_s)[2 * i], b4 = reinterpret_cast<const float4*>(neg_s)[2 * i + 1];
-      const float2 neg[4] = {{a.x, a.y}, {a.z, a.w}, {b4.x, b4.y}, {b4.z, b4.w}};
-#pragma unroll
-      for (int p = 0; p < R::kPasses; ++p)
-        if (const int n = token_of(tile, p * R::kRows + krl); n >= 0 && n < Nk)   // padding rows stay zero (the reference subtracts before padding)
-          w[p][i] = subtract_mean(w[p][i], neg);
-    }
+    for (int p = 0; p < R::kPasses; ++p)
+      if (const int n = token_of(tile, p * R::kRows + krl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
+        w[p][0] = subtract_mean(w[p][0], mean[0]);
+        w[p][1] = subtract_mean(w[p][1], mean[1]);
+      }
   }
 #pragma unroll
   for (int p = 0; p < R::kPasses; ++p) { *place(p, 0) = w[p][0]; *place(p, 1) = w[p][1]; }
@@ -321,7 +318,7 @@ cudaError_t launch_delta_s(const DeltaSArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const bool multi = P.rows > 128;
-  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + (a.D + a.D / 8) * 4 + 1024;
+  const int smem = kDsStageBytes + 2 * (a.D / 8) * (int)kChunk + 2048 + 16 + a.D * 2 + 1024;
   static std::atomic<unsigned long long> ready[8];      // per kernel: devices on which the shared memory was asked for
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -40,10 +40,11 @@ constexpr int kMaxChunks = 64;             // at most so many partial rows per h
 template <int D>
 __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, const float* __restrict__ partial, const int nchunks,
                                        const float divisor, const int64_t bh, float* stage, __nv_bfloat16* km_out,
-                                       float (&mean)[16]) {
+                                       uint4 (&mean)[2]) {
   const int t = threadIdx.x, c = RowTile<D>::block(t);
   if (km != nullptr) {
-    bf16x16_to_f32(km + bh * D + c * 16, mean);
+    mean[0] = reinterpret_cast<const uint4*>(km + bh * D + c * 16)[0];
+    mean[1] = reinterpret_cast<const uint4*>(km + bh * D + c * 16)[1];
     return;
   }
   constexpr int V = kMaxChunks * D / 4 / kThreads;
@@ -62,12 +63,12 @@ __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, con
   __syncthreads();
   if (t < D) {
     const __nv_bfloat16 m = __float2bfloat16_rn(s / divisor);
-    stage[t] = __bfloat162float(m);
+    reinterpret_cast<__nv_bfloat16*>(stage)[t] = m;
     if (km_out != nullptr) km_out[bh * D + t] = m;
   }
   __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 16; ++i) mean[i] = stage[c * 16 + i];
+  mean[0] = reinterpret_cast<const uint4*>(stage)[2 * c];
+  mean[1] = reinterpret_cast<const uint4*>(stage)[2 * c + 1];
 }
 
 template <int D>
