@@ -72,8 +72,10 @@ __device__ __forceinline__ void channel_partial(const __nv_bfloat16* __restrict_
 // The sums and the mean in one launch: grid = (chunks, B*H), the last CTA of a (b,h) to finish adds the partial rows
 // and writes mean = sum / divisor as bf16.
 // scratch: partial[B*H][chunks][D] fp32 followed by counters[B*H] u32 (zeroed by the host).
+// Eight rows in flight per thread and four CTAs per SM: B1 H40 N9450 34.6 -> 27.2 us (four rows and eight CTAs before; sixteen and
+// three 30.0).
 template <int D>
-__global__ void __launch_bounds__(kThreads) channel_mean_kernel(
+__global__ void __launch_bounds__(kThreads, 4) channel_mean_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
     int chunk_tokens, float divisor, float* __restrict__ partial, unsigned int* __restrict__ counters,
     __nv_bfloat16* __restrict__ mean_out, const int* __restrict__ cu, int d_in) {
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(kThreads) channel_mean_kernel(
     N = min(cu[b + 1] - cu[b], N);         // never beyond the caller's max_seqlen (the grid covers no more)
     divisor = (float)max(N, 1);
   }
-  channel_partial<D, 4>(x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh, sn, N, chunk, chunk_tokens, d_in,
+  channel_partial<D, 8>(x + (cu ? (int64_t)cu[b] * sn : b * sb) + h * sh, sn, N, chunk, chunk_tokens, d_in,
                      partial + ((int64_t)bh * nchunks + chunk) * D, red);
   __threadfence();
   __syncthreads();
