@@ -132,6 +132,7 @@ struct QuantLaunch {
   __nv_bfloat16* qm;                     // [B,Hq,Tq,D] (mode 1)
   int q_blocks, k_blocks, v_blocks;      // CTAs per role
   Div by_Tq, by_Tk, by_Hq, by_Hkv, by_chunks;
+  int q_heads;                           // kVar: heads that a CTA of the Q role takes; by_Hq then divides by their groups
   const int *cu_q, *cu_k;                // variable-length batches (else null)
   int d_in;                              // channels the input rows really have (<= D, multiple of 8); the rest are zero
   int s_blocks, chunks, chunk_tokens;    // CTAs of the K channel-sum role (0: none), chunks per head, tokens per chunk
@@ -197,7 +198,11 @@ __device__ __forceinline__ void varlen_order(const QuantLaunch& P, int* hist) {
 
 // 64 registers: four CTAs per SM, each with a whole 32 KB tile in flight (B1 H40 N32760 D128, with the K sums: 240 us;
 // 260 at three per SM)
-template <int D>
+// kVar: variable-length batches, whose grid is sized for sequences of the greatest length.  A CTA of the Q role then takes its tile of
+// up to four heads, so that there are a quarter of the CTAs for tiles that no sequence has, and one of the V role leaves at once
+// (16 prompts of 187 to 3000 tokens, H32/8: 77.7 -> 66.5 us; operator with 31 prompts of 600 and 8000, D=64: 687 -> 650, with eight
+// of 2000 each: 304 -> 299).
+template <int D, bool kVar>
 __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunch P) {
   using R = RowTile<D>;
   __shared__ __align__(16) uint8_t sf_smem[2048];
@@ -232,9 +237,15 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     const bool is_q = bid < P.q_blocks;
     if (!is_q) bid -= P.q_blocks;
     const int T = is_q ? P.Tq : P.Tk;
-    int N = is_q ? P.Nq : P.Nk, tile, bh, b, h;
+    int tile, bh, b, h;
     (is_q ? P.by_Tq : P.by_Tk).split(bid, bh, tile);
     (is_q ? P.by_Hq : P.by_Hkv).split(bh, b, h);
+    const int heads = kVar && is_q ? P.q_heads : 1;
+    if (kVar && is_q) { h *= heads; bh = b * P.Hq + h; }
+#pragma unroll 1
+    for (int i_head = 0; i_head < (kVar ? heads : 1); ++i_head, ++h, ++bh) {
+    int N = is_q ? P.Nq : P.Nk;
+    if (kVar && i_head > 0) __syncthreads();   // shared memory of the head before has been read
     const int64_t sn = is_q ? P.q_sn : P.k_sn;
     const int* cu = is_q ? P.cu_q : P.cu_k;
     const __nv_bfloat16* src = is_q ? P.q + b * P.q_sb + h * P.q_sh : P.k + b * P.k_sb + h * P.k_sh;
@@ -245,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
         if (P.q_mean_mode == 1 && rl == 0)  //   query uses), so it must at least be a number
           for (int i = 0; i < 2; ++i)
             reinterpret_cast<uint4*>(P.qm + ((int64_t)bh * T + tile) * D + c * 16)[i] = make_uint4(0, 0, 0, 0);
-        return;
+        continue;
       }
     }
     uint4 w[R::kPasses][2];
@@ -350,6 +361,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     uint8_t* codes = (is_q ? P.q_codes : P.k_codes) + ((int64_t)bh * T + tile) * (kTile * D / 2);
     uint8_t* sf = (is_q ? P.q_sf : P.k_sf) + ((int64_t)bh * T + tile) * ((D / 64) * 512);
     quant_rows_store<D>(w, codes, sf, sf_smem);
+    }
     return;
   }
 
@@ -365,12 +377,13 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
   const int tl = warp / WPT;                     // tile slot inside this CTA
   const int gt = bid * TPB + tl;                 // global tile index over (b, h, tile)
   const int total = P.B * P.Hkv * P.Tk;
-  for (int i = t; i < 2048 / 16; i += kThreads) reinterpret_cast<uint4*>(sf_smem)[i] = make_uint4(0, 0, 0, 0);
-  __syncthreads();
   int tile, bh, b, h;
   P.by_Tk.split(gt, bh, tile);
   P.by_Hkv.split(bh, b, h);
   const int Nv = P.cu_k && gt < total ? min(P.cu_k[b + 1] - P.cu_k[b], P.Nk) : P.Nk;
+  if (kVar && TPB == 1 && tile * kTile >= Nv) return;     // (nothing reads a V tile beyond its sequence)
+  for (int i = t; i < 2048 / 16; i += kThreads) reinterpret_cast<uint4*>(sf_smem)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
   if (gt < total && (P.pack || tile * kTile < Nv)) {      // (nothing reads a V tile beyond its sequence)
     const int c4 = (warp % WPT) * 4 + (lane >> 3);        // group of 4 channels
     const int blk = lane & 7;                              // 16-token block
@@ -443,6 +456,10 @@ void quant_chunks(int BH, int N, int* chunks, int* chunk_tokens) {
   *chunks = (N + *chunk_tokens - 1) / *chunk_tokens;
 }
 
+// Fewest CTAs of the Q role of a variable-length batch that sharing one among heads may leave: two waves.  (Below, a chain of four
+// heads is what counts: two prompts of 64 and 30 tokens 15.7 us, 19.0 with four heads to a CTA.)
+constexpr int64_t kVarCtas = 1184;
+
 cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   QuantLaunch P;
   P.q = (const __nv_bfloat16*)a.q; P.k = (const __nv_bfloat16*)a.k; P.v = (const __nv_bfloat16*)a.v;
@@ -467,7 +484,10 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   P.s_blocks = a.partial != nullptr ? a.B * a.Hkv * P.chunks : 0;
   P.q_dot_km = (a.q_dot_km != nullptr && a.km != nullptr && a.cu_q == nullptr) ? (float*)a.q_dot_km : nullptr;
   P.km_for_q = (const __nv_bfloat16*)a.km;
-  P.q_blocks = a.q ? a.B * a.Hq * P.Tq : 0;
+  const bool var = a.cu_q != nullptr || a.cu_k != nullptr;
+  P.q_heads = !var ? 1 : (a.Hq % 4 == 0 ? 4 : (a.Hq % 2 == 0 ? 2 : 1));
+  while (P.q_heads > 1 && (int64_t)a.B * (a.Hq / P.q_heads) * P.Tq < kVarCtas) P.q_heads >>= 1;
+  P.q_blocks = a.q ? a.B * (a.Hq / P.q_heads) * P.Tq : 0;
   P.k_blocks = a.k && a.k_codes ? a.B * a.Hkv * P.Tk : 0;
   const int tpb = a.D == 128 ? 1 : 2;
   P.v_blocks = a.v ? (int)(((int64_t)a.B * a.Hkv * P.Tk + tpb - 1) / tpb) : 0;
@@ -479,13 +499,18 @@ cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
   const int64_t k_bytes = (int64_t)a.B * a.Hkv * a.Nk * a.D * 2;
   const bool fits = k_bytes <= 96 << 20 && k_bytes >= 8 << 20;
   P.s_first = fits ? P.q_blocks + P.k_blocks + P.v_blocks : 0;
-  P.by_Tq.set(P.Tq > 0 ? P.Tq : 1); P.by_Tk.set(P.Tk > 0 ? P.Tk : 1); P.by_Hq.set(a.Hq); P.by_Hkv.set(a.Hkv); P.by_chunks.set(P.chunks > 0 ? P.chunks : 1);
+  P.by_Tq.set(P.Tq > 0 ? P.Tq : 1); P.by_Tk.set(P.Tk > 0 ? P.Tk : 1); P.by_Hq.set(a.Hq / P.q_heads); P.by_Hkv.set(a.Hkv); P.by_chunks.set(P.chunks > 0 ? P.chunks : 1);
   P.order = a.order; P.n_order = a.n_order; P.causal = a.causal;
   P.o_blocks = a.order != nullptr ? 1 : 0;
   const int grid = P.o_blocks + P.s_blocks + P.q_blocks + P.k_blocks + P.v_blocks;
   if (grid == 0) return cudaSuccess;
-  if (a.D == 128) quant_qkv_kernel<128><<<grid, kThreads, 0, stream>>>(P);
-  else            quant_qkv_kernel<64><<<grid, kThreads, 0, stream>>>(P);
+  if (var) {
+    if (a.D == 128) quant_qkv_kernel<128, true><<<grid, kThreads, 0, stream>>>(P);
+    else            quant_qkv_kernel<64, true><<<grid, kThreads, 0, stream>>>(P);
+  } else {
+    if (a.D == 128) quant_qkv_kernel<128, false><<<grid, kThreads, 0, stream>>>(P);
+    else            quant_qkv_kernel<64, false><<<grid, kThreads, 0, stream>>>(P);
+  }
   return cudaGetLastError();
 }
 

@@ -255,6 +255,27 @@ def test_bounded_wait_gives_up_and_reports():
     assert torch.isfinite(out).all()
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,D,cap", [(40, 32, 8, 128, 700), (120, 6, 2, 64, 700), (300, 5, 5, 128, 129)])
+def test_varlen_batches_of_many_tiles(B, Hq, Hkv, D, cap):
+    """Enough tiles that a CTA of the quantisation kernel takes one of four, two or (odd head counts) one head; lengths 1 ... cap, one
+    sequence of length 1 and one of a multiple of 128.  Against calls on single kv heads, which are below that line (K channel sums are
+    cut into other chunks there: tolerance as above)."""
+    g = torch.Generator().manual_seed(B)
+    lens = torch.randint(1, cap + 1, (B,), generator=g).tolist()
+    lens[0], lens[1], lens[2] = 1, cap, 128
+    q = torch.randn(sum(lens), Hq, D, generator=g).to(torch.bfloat16).to(DEV)
+    k = (torch.randn(sum(lens), Hkv, D, generator=g) + torch.randn(1, Hkv, D, generator=g)).to(torch.bfloat16).to(DEV)
+    v = torch.randn(sum(lens), Hkv, D, generator=g).to(torch.bfloat16).to(DEV)
+    cu = torch.tensor([0] + np.cumsum(lens).tolist(), dtype=torch.int32, device=DEV)
+    out = sa.sageattn_varlen(q, k, v, cu, cu, cap, cap, is_causal=True, check_status=True)
+    G = Hq // Hkv
+    for h in range(Hkv):
+        one = sa.sageattn_varlen(q[:, h * G:(h + 1) * G].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(), cu, cu, cap,
+                                 cap, is_causal=True)
+        cos, l1 = sage3.accuracy(out[:, h * G:(h + 1) * G].float().cpu(), one.float().cpu())
+        assert cos >= 0.9995 and l1 <= 2e-2, (h, cos, l1)
+
+
 def test_varlen_sequences_longer_than_max_seqlen_are_cut_not_overrun():
     """A caller that passes max_seqlen smaller than its longest sequence gets that sequence cut at max_seqlen (the
     operand layouts and the workspace are sized by it): no tile index beyond the layouts is ever formed."""
