@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   const int kc = R::block(t), krl = R::row(t);          // K rows: 16 channels a thread (A rows, c and rl: 8)
   const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + kc * 16;
   auto place = [&](const int p, const int i) {          // of channels 8 i ... of this thread's row p in sB
-    const int row = p * R::kRows + krl;
+    const int row = p * R::kStep + krl;
     return reinterpret_cast<uint4*>(sB + (2 * kc + i) * kChunk + (row >> 3) * 128 + (row & 7) * 16);
   };
   const int end = min(first + P.run, P.cu_k != nullptr ? (Nk + kTile - 1) / kTile : P.Tk);
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   auto load = [&](const int tile) {
 #pragma unroll
     for (int p = 0; p < R::kPasses; ++p) {             // all loads in flight before the first use
-      const int n = token_of(tile, p * R::kRows + krl);
+      const int n = token_of(tile, p * R::kStep + krl);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
         w[p][i] = (n >= 0 && n < Nk && kc * 16 + 8 * i < P.d_in) ? *reinterpret_cast<const uint4*>(src + (int64_t)n * P.k_sn + 8 * i)
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
     if (kMulti) { mean[0] = mean_s[0]; mean[1] = mean_s[1]; }
 #pragma unroll
     for (int p = 0; p < R::kPasses; ++p)
-      if (const int n = token_of(tile, p * R::kRows + krl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
+      if (const int n = token_of(tile, p * R::kStep + krl); n >= 0 && n < Nk) {   // padding rows stay zero (the reference subtracts before padding)
         w[p][0] = subtract_mean(w[p][0], mean[0]);
         w[p][1] = subtract_mean(w[p][1], mean[1]);
       }

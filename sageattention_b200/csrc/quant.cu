@@ -107,6 +107,46 @@ __global__ void __launch_bounds__(kThreads, 4) channel_mean_kernel(
   }
 }
 
+// Channel sums of a Q tile: those of the warps' rows, red[warp][D].  The order is fixed - rows r, r + kStep, ... of the whole tile
+// one after another, then r and r + 1 (D=64: then the same of r + 2 and r + 3), the warps last, by the caller - because a block mean
+// that rounds the other way is seen in 128 rows of delta_s.  So a lane with rows 0 ... 63 hands its sums to the one that has the
+// other half of the same rows, which goes on from there; each later step leaves a lane half the channels.
+template <int D>
+__device__ __forceinline__ void tile_sums(const uint4 (&w)[RowTile<D>::kPasses][2], const int t, const int c, float* red) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {                  // 8 channels at a time, for the registers
+    float2 a[4] = {};
+#pragma unroll
+    for (int p = 0; p < RowTile<D>::kPasses; ++p) add_channels(a, w[p][i]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      a[j].x = __shfl_xor_sync(0xffffffffu, a[j].x, 16);
+      a[j].y = __shfl_xor_sync(0xffffffffu, a[j].y, 16);
+    }
+#pragma unroll
+    for (int p = 0; p < RowTile<D>::kPasses; ++p) add_channels(a, w[p][i]);
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { acc[2 * j] = a[j].x; acc[2 * j + 1] = a[j].y; }
+    int first = c * 16 + 8 * i;
+#pragma unroll
+    for (int step = 0; step < (D == 128 ? 1 : 2); ++step) {
+      const int o = 4 << step, n = 4 >> step;    // the lane's bits that are the row
+      const bool upper = (t & o) != 0;
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        const float give = upper ? acc[j] : acc[n + j], own = upper ? acc[n + j] : acc[j];
+        acc[j] = own + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      if (upper) first += n;
+    }
+    if (t & 16) {
+#pragma unroll
+      for (int j = 0; j < (D == 128 ? 4 : 2); ++j) red[(t >> 5) * D + first + j] = acc[j];
+    }
+  }
+}
+
 // Division by a number that the host knows, for 0 <= n < 2^31 (Granlund and Montgomery, "Division by invariant integers using
 // multiplication", 1994): the six of a CTA's index arithmetic were 10 % of the Q role's instructions.
 struct Div {
@@ -266,8 +306,8 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     for (int p = 0; p < R::kPasses; ++p) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        w[p][i] = (p * R::kRows < rows && c * 16 + 8 * i < P.d_in) ? *reinterpret_cast<const uint4*>(src + 8 * i) : make_uint4(0, 0, 0, 0);
-      src += R::kRows * sn;
+        w[p][i] = (p * R::kStep < rows && c * 16 + 8 * i < P.d_in) ? *reinterpret_cast<const uint4*>(src + 8 * i) : make_uint4(0, 0, 0, 0);
+      src += R::kStep * sn;
     }
     float mean[16];
     if (is_q && P.q_dot_km != nullptr) {
@@ -287,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
           if (o & R::kBlockBits) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (c == 0 && p * R::kRows < rows) P.q_dot_km[(int64_t)bh * P.Nq + tile * kTile + p * R::kRows + rl] = d;
+        if (c == 0 && p * R::kStep < rows) P.q_dot_km[(int64_t)bh * P.Nq + tile * kTile + p * R::kStep + rl] = d;
       }
     }
     bool subtract = true;
@@ -297,29 +337,8 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
 #pragma unroll
         for (int i = 0; i < 16; ++i) mean[i] = mp[i];
       } else {
-        // fp32 column sums over the tile's 128 rows (zero rows of the padding included), / 128: the thread's rows, the warp's (each
-        // step of the exchange leaves a lane half the channels), the CTA's
-        float2 acc2[2][4] = {};
-#pragma unroll
-        for (int p = 0; p < R::kPasses; ++p) { add_channels(acc2[0], w[p][0]); add_channels(acc2[1], w[p][1]); }
-        float acc[16];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { acc[2 * i] = acc2[i >> 2][i & 3].x; acc[2 * i + 1] = acc2[i >> 2][i & 3].y; }
-        int first = 0;                           // of the channels that this lane is left with
-#pragma unroll
-        for (int step = 0; step < (D == 128 ? 2 : 3); ++step) {
-          const int o = step == 0 ? 16 : (D == 128 ? 4 : 16 >> step), n = 16 >> (step + 1);   // the lane's bits that are the row
-          const bool upper = (t & o) != 0;
-#pragma unroll
-          for (int i = 0; i < n; ++i) {
-            const float give = upper ? acc[i] : acc[n + i], own = upper ? acc[n + i] : acc[i];
-            acc[i] = own + __shfl_xor_sync(0xffffffffu, give, o);
-          }
-          if (upper) first += n;
-        }
-        constexpr int kLeft = D == 128 ? 4 : 2;
-#pragma unroll
-        for (int i = 0; i < kLeft; ++i) red[(t >> 5) * D + c * 16 + first + i] = acc[i];
+        // fp32 column sums over the tile's 128 rows (zero rows of the padding included), / 128
+        tile_sums<D>(w, t, c, red);
         __syncthreads();
         if (t < D) {
           float s = 0.f;
@@ -355,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
                                {-mean[8 * i + 4], -mean[8 * i + 5]}, {-mean[8 * i + 6], -mean[8 * i + 7]}};
 #pragma unroll
         for (int p = 0; p < R::kPasses; ++p)
-          if (is_q || p * R::kRows < rows) w[p][i] = subtract_mean(w[p][i], neg);
+          if (is_q || p * R::kStep < rows) w[p][i] = subtract_mean(w[p][i], neg);
       }
     }
     uint8_t* codes = (is_q ? P.q_codes : P.k_codes) + ((int64_t)bh * T + tile) * (kTile * D / 2);

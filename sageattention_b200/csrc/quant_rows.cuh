@@ -10,18 +10,21 @@ constexpr int kTile = 128;
 constexpr int kThreads = 256;
 
 // Row-wise quantisation of one 128-token tile held in registers (Q and K roles).  Thread t owns the 16 channels 16 block(t) ... of
-// rows row(t), + kRows, ...: whole quantisation blocks, so that scales need no exchange and are worked out once.  (With 8 channels a
+// rows row(t), + kStep, ...: whole quantisation blocks, so that scales need no exchange and are worked out once.  (With 8 channels a
 // thread, two threads to a block: B1 H40 N32760 228 -> 219 us, K pass 321 -> 292.)
-// Which lane has which, D=128: bits 0, 1 and 3 are the block, 2 and 4 the row, so that 8 lanes' 16-byte stores of the K pass
-// (delta_s.cu), 4128 bytes from block to block and 16 from row to row, meet different banks.
+// Which lane has which: its bits kBlockBits are the block, bit 4 is the half of the tile (rows 0 ... 63 or 64 ... 127, see tile_sums in
+// quant.cu), the others and the warp are the row modulo kStep.  D=128: so that 8 lanes' 16-byte stores of the K pass (delta_s.cu),
+// 4128 bytes from block to block and 16 from row to row, meet different banks.
 // ------------------------------------------------------------------------------------------------
 template <int D>
 struct RowTile {
-  static constexpr int kPerRow = D / 16, kRows = kThreads / kPerRow, kPasses = kTile / kRows;
+  static constexpr int kPerRow = D / 16, kPasses = kTile * kPerRow / kThreads, kStep = kTile / 2 / kPasses;
   static constexpr int kBlockBits = D == 128 ? 11 : 3;     // bits of the lane that are the block
   static __device__ __forceinline__ int block(const int t) { return D == 128 ? (t & 3) | ((t >> 1) & 4) : t & 3; }
-  static __device__ __forceinline__ int row(const int t) { return D == 128 ? ((t >> 2) & 1) | ((t >> 4) << 1) : t >> 2; }
-  static_assert(kRows == 32 || kRows == 64, "rows of a pass");
+  static __device__ __forceinline__ int row(const int t) {
+    return (D == 128 ? ((t >> 2) & 1) | ((t >> 5) << 1) : ((t >> 2) & 3) | ((t >> 5) << 2)) + ((t >> 4) & 1) * (kTile / 2);
+  }
+  static_assert(kStep == kThreads / 32 * (D == 128 ? 2 : 4), "every row once");
 };
 __device__ __forceinline__ void bf16x16_to_f32(const __nv_bfloat16* p, float (&x)[16]) {
 #pragma unroll
@@ -76,9 +79,9 @@ __device__ __forceinline__ void quant_rows_store(const uint4 (&w)[RowTile<D>::kP
                                                  uint8_t* __restrict__ sf_tile, uint8_t* sf_smem) {
   using R = RowTile<D>;
   const int t = threadIdx.x, c = R::block(t), rl = R::row(t);
-  // sf_atom_offset of row p * kRows + rl, with what depends on p taken out as a constant (left to the compiler, the addresses were
+  // sf_atom_offset of row rl + p * kStep is the sum of both offsets, the second a constant (left to the compiler, the addresses were
   // 15 % of the instructions)
-  uint8_t* const sf_row = sf_smem + (c >> 2) * 512 + (c & 3) + (rl & 31) * 16 + (rl >> 5) * 4;
+  uint8_t* const sf_row = sf_smem + (c >> 2) * 512 + sf_atom_offset(rl, c & 3);
   uint8_t* const out = codes_tile + rl * (D / 2) + c * 8;
 #pragma unroll
   for (int p = 0; p < R::kPasses; ++p) {
@@ -94,8 +97,8 @@ __device__ __forceinline__ void quant_rows_store(const uint4 (&w)[RowTile<D>::kP
       const float2 f2 = mul2_ftz(bf16x2_to_f32(w[p][i].z), inv2), f3 = mul2_ftz(bf16x2_to_f32(w[p][i].w), inv2);
       code[i] = f32x8_to_e2m1x8(f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y);
     }
-    *reinterpret_cast<uint2*>(out + p * (R::kRows * D / 2)) = make_uint2(code[0], code[1]);
-    sf_row[p * (R::kRows / 32) * 4] = (uint8_t)sfb;
+    *reinterpret_cast<uint2*>(out + p * (R::kStep * D / 2)) = make_uint2(code[0], code[1]);
+    sf_row[sf_atom_offset(p * R::kStep, 0)] = (uint8_t)sfb;
   }
   __syncthreads();
   constexpr int SFV = (D / 64) * 512 / 16;                           // 16-byte vectors of scales

@@ -134,6 +134,39 @@ def test_self_computed_means_are_close_to_torch():
     assert ((z.k_codes != z2.k_codes).float().mean()) < 5e-3
 
 
+def _q_block_means(q):
+    """Means of 128-token blocks in the kernel's order of fp32 sums: rows r, r + 16 (D=64: r + 32), ... of the block, then the rows
+    of a warp in pairs, then the warps."""
+    B, H, N, D = q.shape
+    x = q.float().reshape(B, H, N // 128, -1, 16 if D == 128 else 32, D)
+    s = x[..., 0, :, :]
+    for p in range(1, x.shape[-3]):
+        s = s + x[..., p, :, :]
+    while s.shape[-2] > 8:
+        s = s[..., ::2, :] + s[..., 1::2, :]
+    total = s[..., 0, :]
+    for w in range(1, 8):
+        total = total + s[..., w, :]
+    return total * (1.0 / 128)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_order_of_q_block_sums(D):
+    """Magnitudes over 24 binary orders with much cancellation, so that another order of the sums gives other means; exact."""
+    g = torch.Generator().manual_seed(D)
+    q = (torch.randn(2, 3, 640, D, generator=g) * 2.0 ** torch.randint(0, 24, (2, 3, 640, D), generator=g)).to(torch.bfloat16)
+    want = _q_block_means(q)
+    q = q.to(DEV)
+    z = sa.quantize_qkv(q, q, q)
+    assert torch.equal(z.qm.cpu(), want.to(torch.bfloat16))
+    given = sa.quantize_qkv(q, q, q, qm_fp32=want.to(DEV))
+    assert torch.equal(z.q_codes, given.q_codes) and torch.equal(z.q_sf, given.q_sf)
+    # a last block that is partly padding
+    z = sa.quantize_qkv(q[:, :, :600], q, q)
+    q[:, :, 600:] = 0
+    assert torch.equal(z.qm.cpu(), _q_block_means(q.cpu()).to(torch.bfloat16))
+
+
 def test_whole_sequence_q_mean_mode():
     B, H, N, D = 1, 2, 300, 128
     q, k, v = U.make_qkv(B, H, H, N, N, D, seed=3, device=DEV)
