@@ -40,13 +40,6 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
   return d;
 }
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<uint64_t&>(d))
-      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-  return d;
-}
 __device__ __forceinline__ float2 mul2_ftz(float2 a, float2 b) {
   float2 d;
   asm("mul.rn.ftz.f32x2 %0, %1, %2;"

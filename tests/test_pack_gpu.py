@@ -39,6 +39,23 @@ def test_pack_kernel_matches_oracle(B, H, N, D):
     assert int(diff.max()) <= 1 and float((diff > 0).float().mean()) <= 5e-3
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_residuals_round_the_product_by_itself(D):
+    """Residual = x - lambda * mean with the product rounded to fp32 before the subtraction, then to bf16: exact, from the lambdas and means
+    that the kernel returns.  Tokens of a group are multiples of one vector, so that residuals are no more than those roundings
+    and a fused operation would give others almost everywhere."""
+    g = torch.Generator().manual_seed(D)
+    base = torch.tensor([0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])[torch.randint(0, 7, (1, 4, 20, 1, D), generator=g)]
+    base[..., ::16] = 6.0                                                       # the largest of every quantisation block
+    a = torch.randint(1, 64, (1, 4, 20, 15, 1), generator=g).float() / 16
+    for x in (a * base, torch.randn(1, 4, 20, 15, D, generator=g)):
+        k = x.to(torch.bfloat16).reshape(1, 4, 300, D)
+        kp, _, lam, _ = sa.pack_kv(k.to(DEV), k.to(DEV), smooth_k=False)
+        kp, lam = kp.cpu().reshape(1, 4, 20, 16, D), lam.cpu()[..., :320].reshape(1, 4, 20, 16, 1)
+        want = k.float().reshape(1, 4, 20, 15, D) - lam[..., 1:, :] * kp[..., :1, :].float()
+        assert torch.equal(kp[..., 1:, :], want.to(torch.bfloat16))
+
+
 def oracle_on_packed_operands(z, sm_scale, causal, mean_slot="mask"):
     B, Hq, Hkv, Nq, Nk, D = z.shape
     qc, qs = U.unpack_rows(z.q_codes, z.q_sf)
