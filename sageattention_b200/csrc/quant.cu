@@ -316,14 +316,17 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
       bf16x16_to_f32(P.km_for_q + ((int64_t)b * P.Hkv + h / (P.Hq / P.Hkv)) * D + c * 16, mean);
 #pragma unroll
       for (int p = 0; p < R::kPasses; ++p) {
-        float d = 0.f;
+        float d8[2];                             // of 8 channels each, then of more and more: an order that the LSE's last bits show
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const uint4 x = w[p][i];
           const float* m = mean + 8 * i;
-          d = fmaf(bf16_lo(x.x), m[0], d); d = fmaf(bf16_hi(x.x), m[1], d); d = fmaf(bf16_lo(x.y), m[2], d); d = fmaf(bf16_hi(x.y), m[3], d);
-          d = fmaf(bf16_lo(x.z), m[4], d); d = fmaf(bf16_hi(x.z), m[5], d); d = fmaf(bf16_lo(x.w), m[6], d); d = fmaf(bf16_hi(x.w), m[7], d);
+          float d = bf16_lo(x.x) * m[0];
+          d = fmaf(bf16_hi(x.x), m[1], d); d = fmaf(bf16_lo(x.y), m[2], d); d = fmaf(bf16_hi(x.y), m[3], d);
+          d = fmaf(bf16_lo(x.z), m[4], d); d = fmaf(bf16_hi(x.z), m[5], d); d = fmaf(bf16_lo(x.w), m[6], d);
+          d8[i] = fmaf(bf16_hi(x.w), m[7], d);
         }
+        float d = d8[0] + d8[1];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
           if (o & R::kBlockBits) d += __shfl_xor_sync(0xffffffffu, d, o);

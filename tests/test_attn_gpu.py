@@ -229,6 +229,25 @@ def test_operator_can_be_captured_in_a_cuda_graph():
     assert torch.equal(out, sa.sageattn(q2, k2, v2, is_causal=True))
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_order_of_the_sums_behind_the_lse_of_smoothed_keys(D):
+    """The K-mean term of the LSE: 8 channels one after another, then pairs of those sums.  With a single key everything else in the
+    LSE is 0; magnitudes over 30 binary orders with much cancellation, so that another order gives other sums."""
+    g = torch.Generator().manual_seed(D)
+    q = (torch.randn(1, 4, 256, D, generator=g) * 2.0 ** torch.randint(0, 30, (1, 4, 256, D), generator=g)).to(torch.bfloat16)
+    k = torch.randn(1, 4, 1, D, generator=g).to(torch.bfloat16)
+    _, lse = sa.sageattn(q.to(DEV), k.to(DEV), k.to(DEV), sm_scale=1.0, return_lse=True)
+    x = (q.float() * k.float()).reshape(1, 4, 256, D // 8, 8)                   # products of two bf16 are exact
+    s = x[..., 0]
+    for i in range(1, 8):
+        s = s + x[..., i]
+    while s.shape[-1] > 1:
+        s = s[..., ::2] + s[..., 1::2]
+    want = s[..., 0]
+    # sm_scale through log2(e) and back, the sum with log(1): three roundings
+    assert ((lse.cpu() - want).abs() <= want.abs() * 3 * 2.0 ** -24 + 1e-3).all()
+
+
 def test_bounded_wait_gives_up_and_reports():
     """A wait on a barrier nothing completes runs out after its (short) poll limit: the kernel returns normally, the
     status word carries its code, the host call maps it to SAGE3_ERR_DEVICE_WAIT and the context stays usable.  Warps beside
