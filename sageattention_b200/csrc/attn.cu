@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             const float m_loc = fmax3(fmax3(bm[0], bm[1], bm[2]), fmax3(bm[3], bm[4], bm[5]), fmaxf(bm[6], bm[7]));
             const float m_new = fmaxf(m_run, m_loc);
             const float alpha = ex2_approx((m_run - m_new) * c);
-            l = fmaf(nan_of_poly_columns(c6, c12), 0.f, l) * alpha;
+            l = fmaf(nan_of_poly_columns(c6, c12), 0.f, l);
             m_run = m_new;
             const float off = fmaf(m_new, c, kLog2Inv2688);       // P = 2^(s*c - off) in (0, 2688]
             float neg_e[8], sb[8];
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             exp_quantise<kPacked, 3>(s, c, neg_e, sb, P.slot_first, lsum, code);
             s_ready = mbar_test(bar_s, (sc + 1) & 1);
             tmem_st4(tm_Prow + 12, code[0], code[1], code[2], code[3]);
-            l += lsum;
+            l = fmaf(l, alpha, lsum);              // one rounding, whatever the compiler would make of a product and a sum
           }
           if (!ok) break;
           l_row[(items & 1) * 512] = l;

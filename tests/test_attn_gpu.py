@@ -248,6 +248,17 @@ def test_order_of_the_sums_behind_the_lse_of_smoothed_keys(D):
     assert ((lse.cpu() - want).abs() <= want.abs() * 3 * 2.0 ** -24 + 1e-3).all()
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_row_sums_keep_their_bits(D):
+    """LSE of 8 key tiles, bit for bit: row sums are carried from tile to tile by one fused multiply-add.  Recorded (golden/row_sums.npz,
+    first head) from the kernel of 12 + 4 warps as it first was on a B200; only a change that states another order of these sums
+    may record it anew."""
+    want = np.load(U.ROOT / "tests" / "golden" / "row_sums.npz")[f"lse{D}"]
+    q, k, v = U.make_qkv(1, 40, 8, 1024, 1024, D, seed=D, device=DEV)
+    lse = sa.sageattn(q, k, v, return_lse=True)[1][0, 0].cpu().numpy()
+    assert np.array_equal(lse, want)
+
+
 def test_bounded_wait_gives_up_and_reports():
     """A wait on a barrier nothing completes runs out after its (short) poll limit: the kernel returns normally, the
     status word carries its code, the host call maps it to SAGE3_ERR_DEVICE_WAIT and the context stays usable.  Warps beside
