@@ -258,7 +258,8 @@ SAGE3_API int sage3_attn_fwd_packed(const sage3_attn_args* args, const float* k_
 SAGE3_API int sage3_k_mean_static(const sage3_shape* shape, const sage3_tensor* k, void* km_out, void* stream);
 
 /* Synchronises `stream`, copies the device status word back and maps it to a status
- * (SAGE3_OK or SAGE3_ERR_DEVICE_WAIT); *code_out, if given, receives the raw word. */
+ * (SAGE3_OK or SAGE3_ERR_DEVICE_WAIT); *code_out, if given, receives the raw word: the code of the first wait that
+ * ran out (those of the attention kernel are listed at the head of csrc/attn.cu). */
 SAGE3_API int sage3_read_device_status(const int32_t* device_status, void* stream, int32_t* code_out);
 
 /* Self-test of the kernels' bounded waits: enqueues a one-CTA kernel that waits, with a short poll limit (a few

@@ -61,8 +61,11 @@
 // Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128) (D=64: one for each query tile, [2D,2D+256)); 56 columns of scale
 // factors, P^0 and P^1 (16 columns each: 128 FP4 codes per row).
 //
-// Every wait on an mbarrier is bounded; if one gives up the CTA records a code in *status, waits
-// (bounded) for its own copies and MMAs in flight, frees its tensor memory and returns.
+// Every wait on an mbarrier is bounded; if one gives up the CTA records its code in *status, waits
+// (bounded) for its own copies and MMAs in flight, frees its tensor memory and returns.  The codes, one for each wait:
+//   TMA producer 10 K stage free, 11 V stage free, 12 Q slot free; QK issuer 20 Q tile there, 21 K stage there, 23 score buffer
+//   free, 25 delta_s operand there; PV issuer 24 V stage there, 26 P^ there; softmax 30 scores there, 31 last P.V done;
+//   O 32 alpha there, 33 row sum there, 34 last P.V done; delta_s 40 K stage there
 #include <cuda.h>
 
 #include "common.cuh"
@@ -501,12 +504,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       if (warp == 12) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_o); }
-        bool ok = true;
+        int fail = 0;
         uint32_t g = 0;                       // K/V stages completely issued so far
         uint32_t gk = 0;                      // K stages issued so far (g or g + 1)
         uint32_t qn[2] = {0, 0};              // Q tiles loaded so far per slot
 #pragma unroll 1
-        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+        for (int r = 0, w; fail == 0 && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
           int64_t ds_row[2];
 #pragma unroll
@@ -514,9 +517,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             const int qt = (kList ? P.per_item : 2) * wk.pair + t;
             if (kList) ds_row[t] = ((int64_t)wk.b * P.Hq + head_of<kList>(P, wk, t)) * P.ds_rows + (P.ds_rows == 1 ? 0 : tile_of<kList>(P, wk, t));
             else ds_row[t] = ((int64_t)wk.b * P.Hq + wk.hq) * P.ds_rows + (P.ds_rows == 1 ? 0 : qt);
-            if (ok && wk.n_t[t] > 0) {
+            if (fail == 0 && wk.n_t[t] > 0) {
               // the slot's previous Q tile must have been read by its last QK MMA
-              if (qn[t] > 0 && !(ok = wait_bar<>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1))) break;
+              if (qn[t] > 0 && (fail = wait_bar<12>(bars + Bars::q_empty + 8 * t, (qn[t] - 1) & 1)) != 0) break;
               const int64_t qtile = ((int64_t)wk.b * P.Hq + wk.hq) * P.Tq + qt;
               const uint32_t qb = bars + Bars::q_full + 8 * t;
               if (lane == 0) {
@@ -530,10 +533,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           }
           const int64_t kvhead = ((int64_t)wk.b * P.Hkv + wk.hkv) * P.Tk;
 #pragma unroll 1
-          for (int it = 0; ok && it < wk.n_max; ++it, ++g) {
+          for (int it = 0; fail == 0 && it < wk.n_max; ++it, ++g) {
             const int j = wk.n_max - 1 - it, s = g % kStages;
             const uint32_t ph = ((g / kStages) & 1) ^ 1;
-            if (!(ok = wait_bar<>(bars + Bars::k_empty + 8 * s, ph))) break;
+            if ((fail = wait_bar<10>(bars + Bars::k_empty + 8 * s, ph)) != 0) break;
             const uint32_t kb = bars + Bars::k_full + 8 * s;
             const int nds = has_ds ? (int)(j < wk.n_t[0]) + (int)(j < wk.n_t[1]) : 0;
             if (lane == 0) {
@@ -550,7 +553,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             }
             __syncwarp();
             ++gk;
-            if (!(ok = wait_bar<>(bars + Bars::v_empty + 8 * s, ph))) break;
+            if ((fail = wait_bar<11>(bars + Bars::v_empty + 8 * s, ph)) != 0) break;
             const uint32_t vb = bars + Bars::v_full + 8 * s;
             if (lane == 0) {
               mbar_arrive_expect_tx(vb, L::kVBytes + L::kSfV);
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             __syncwarp();
           }
         }
-        if (!ok) give_up(abort_s, P.status, 10);
+        if (fail != 0) give_up(abort_s, P.status, fail);
         if (__any_sync(0xffffffffu, *abort_s != 0)) {
           // giving up: the copies this thread started must land before the CTA may exit
           for (int t = 0; t < 2; ++t)
@@ -574,14 +577,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         // ---------------------------------------------------------------- delta_s -> rank-1 B operand
         // B1 is a K-major [128 keys x 16] bf16 operand in 8x16-byte core matrices: key n's first
         // element sits at (n/8)*128 + (n%8)*16; everything else stays zero.
-        bool ok = true;
+        int fail = 0;
         uint32_t s = 0, ph = 0;
 #pragma unroll 1
-        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+        for (int r = 0, w; fail == 0 && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
           for (int j = wk.n_max - 1; j >= 0; --j) {
-            if (!(ok = wait_bar<>(bars + Bars::k_full + 8 * s, ph))) break;
+            if ((fail = wait_bar<40>(bars + Bars::k_full + 8 * s, ph)) != 0) break;
 #pragma unroll 1
             for (int t = 0; t < 2; ++t) {
               if (j < (t == 0 ? wk.n_t[0] : wk.n_t[1])) {
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
-        if (!ok) give_up(abort_s, P.status, 40);
+        if (fail != 0) give_up(abort_s, P.status, fail);
       } else if (warp == 13) {
         // ---------------------------------------------------------------- QK issuer
         // Its instruction stream is kept minimal: every shared-memory descriptor is a constant high word (stride /
@@ -612,19 +615,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         const uint32_t sfq_lo = (sbase + L::sfq) >> 4, sfk_lo = (sbase + L::sfk) >> 4;
         const uint32_t a1_lo = ((sbase + L::a1) >> 4) | (((uint32_t)(L::zero - L::a1) >> 4) << 16);
         const uint32_t b1_lo = ((sbase + L::b1) >> 4) | (((uint32_t)(L::zero - L::b1) >> 4) << 16);
-        bool ok = true;
+        int fail = 0;
         uint32_t s = 0, ph = 0;               // K stage and its parity
         uint32_t nqk = 0;                     // QK groups issued so far (= uses of the score buffer)
         uint32_t s_odd = 0;                   // K stages so far, odd or even
-        uint32_t s_par = 0;                   // bit t: the same, odd or even, for tile t's own buffer
+        uint32_t s_par = 0;                   // bit t: uses of tile t's own score buffer so far (kSBufs == 2), odd or even
         uint32_t q_par = 0;                   // bit t: parity of the Q tile to come in slot t
 #pragma unroll 1
-        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+        for (int r = 0, w; fail == 0 && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
-          for (int j = wk.n_max - 1; ok && j >= 0; --j) {
-            if (!(ok = wait_bar_uniform(bars + Bars::k_full + 8 * s, ph))) break;
-            if (has_ds && !(ok = wait_bar_uniform(bars + Bars::ds_ready + 8 * s, ph))) break;
+          for (int j = wk.n_max - 1; fail == 0 && j >= 0; --j) {
+            if ((fail = wait_bar_uniform<21>(bars + Bars::k_full + 8 * s, ph)) != 0) break;
+            if (has_ds && (fail = wait_bar_uniform<25>(bars + Bars::ds_ready + 8 * s, ph)) != 0) break;
             // its scale factors on their way before the score buffer is free, into the columns that the MMAs of the stage before do not
             // read (B1 H10 N32760 D128 3466 -> 3452 us)
             const uint32_t tm_sfk_s = tm_sfk + 8 * (s_odd & 1);
@@ -638,17 +641,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             for (int t = 0; t < 2; ++t) {
               const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
               if (j >= n_t) continue;
-              // the one score buffer must be free: the softmax warpgroup that got the previous Q.K^T (the other
-              // query tile, or this one in the previous key tile) has copied it into registers
-              if (kSBufs == 1) {
-                if (!(ok = wait_bar_uniform(bars + Bars::s_free, (nqk - 1) & 1))) break;      // (nothing to wait for: parity 1)
-              } else {
-                if (!(ok = wait_bar_uniform(bars + Bars::s_free + 8 * t, ((s_par >> t) & 1) ^ 1))) break;
-                s_par ^= 1u << t;
-              }
+              // the score buffer must be free: the softmax warpgroup that got its last Q.K^T (the one buffer: of the other
+              // query tile, or of this one in the previous key tile; a buffer for each: of this one) has copied it into
+              // registers.  (Nothing to wait for: parity 1.)
+              const uint32_t free_par = kSBufs == 1 ? (nqk - 1) & 1 : ((s_par >> t) & 1) ^ 1;
+              if ((fail = wait_bar_uniform<23>(bars + Bars::s_free + 8 * (kSBufs - 1) * t, free_par)) != 0) break;
+              if (kSBufs == 2) s_par ^= 1u << t;
               const uint32_t tm_S = tm_Sbuf + 128 * (kSBufs - 1) * t;
               if (j == n_t - 1) {                                  // first key tile of this query tile
-                if (!(ok = wait_bar_uniform(bars + Bars::q_full + 8 * t, (q_par >> t) & 1))) break;
+                if ((fail = wait_bar_uniform<20>(bars + Bars::q_full + 8 * t, (q_par >> t) & 1)) != 0) break;
                 q_par ^= 1u << t;
                 tc_fence_after();
                 if (elect_one())
@@ -672,12 +673,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               __syncwarp();
               ++nqk;
             }
-            if (ok && elect_one()) tc_commit(bars + Bars::k_empty + 8 * s);
+            if (fail == 0 && elect_one()) tc_commit(bars + Bars::k_empty + 8 * s);
             if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
-        if (!ok) {
-          give_up(abort_s, P.status, 20);
+        if (fail != 0) {
+          give_up(abort_s, P.status, fail);
           // giving up: let every MMA / scale copy already issued finish before tensor memory is freed
           if (elect_one()) tc_commit(bars + Bars::drain);
           mbar_wait<true>(bars + Bars::drain, 0, 1u << 16);
@@ -692,16 +693,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         constexpr uint32_t LBO1 = 1u << 16;
         const uint32_t v_lo = ((sbase + L::v) >> 4) | LBO1;
         const uint32_t sfv_lo = (sbase + L::sfv) >> 4, sfp_lo = (sbase + L::sfp) >> 4;
-        bool ok = true;
+        int fail = 0;
         uint32_t s = 0, ph = 0;               // V stage and its parity
         uint32_t p_par = 0;                   // bit t: parity of the P^ to come of tile t
 #pragma unroll 1
-        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+        for (int r = 0, w; fail == 0 && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
 #pragma unroll 1
-          for (int j = wk.n_max - 1; ok && j >= 0; --j) {
+          for (int j = wk.n_max - 1; fail == 0 && j >= 0; --j) {
             // the V stage and its scale factors do not depend on the softmax: fetch them before waiting for P
-            if (!(ok = wait_bar<>(bars + Bars::v_full + 8 * s, ph))) break;
+            if ((fail = wait_bar<24>(bars + Bars::v_full + 8 * s, ph)) != 0) break;
             tc_fence_after();
             if (elect_one())
 #pragma unroll
@@ -710,7 +711,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             for (int t = 0; t < 2; ++t) {
               const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
               if (j >= n_t) continue;
-              if (!(ok = wait_bar<>(bars + Bars::p_full + 8 * t, (p_par >> t) & 1))) break;
+              if ((fail = wait_bar<26>(bars + Bars::p_full + 8 * t, (p_par >> t) & 1)) != 0) break;
               p_par ^= 1u << t;
               tc_fence_after();
               if (elect_one()) {
@@ -724,12 +725,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               }
               __syncwarp();
             }
-            if (ok && elect_one()) tc_commit(bars + Bars::v_empty + 8 * s);
+            if (fail == 0 && elect_one()) tc_commit(bars + Bars::v_empty + 8 * s);
             if (++s == kStages) { s = 0; ph ^= 1; }
           }
         }
-        if (!ok) {
-          give_up(abort_s, P.status, 24);
+        if (fail != 0) {
+          give_up(abort_s, P.status, fail);
           if (elect_one()) tc_commit(bars + Bars::drain + 8);
           mbar_wait<true>(bars + Bars::drain + 8, 0, 1u << 16);
         }
@@ -742,7 +743,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       if (warp < 8) {
         // ---------------------------------------------------------------- softmax
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegSplit::softmax));
-        bool ok = true;
+        // (which wait ran out as a flag and not, as elsewhere, as its code: B1 H40 N32760 13.47 -> 13.30 ms, D64 H10 3.33 -> 3.28)
+        bool ok = true, late = false;
         const int t = warp >> 2;                                 // query tile slot of this warpgroup
         const uint32_t tm_S = tm_Sbuf + 128 * (kSBufs - 1) * t + lane_addr;
         const uint32_t bar_f = bars + Bars::s_free + 8 * (kSBufs - 1) * t;
@@ -792,7 +794,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             const bool ready = __all_sync(0xffffffffu, s_ready);
             if (!ready) {
               hand_over(it > 0);
-              if (!(ok = wait_bar<>(bar_s, sc & 1))) break;
+              if (!(ok = wait_bar<30>(bar_s, sc & 1) == 0)) break;
             }
             tc_fence_after();
             uint32_t s[128];
@@ -851,7 +853,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             uint32_t code[4];
             exp_quantise<kPacked, 0>(s, c, neg_e, sb, P.slot_first, lsum, code);
             // the P.V MMAs of the previous key tile are complete: P^ and its scales may be rewritten, O rescaled
-            if (!__all_sync(0xffffffffu, pv_ready) && !(ok = wait_bar<>(bar_pv, (sc - 1) & 1))) break;
+            if (!__all_sync(0xffffffffu, pv_ready) && !(ok = wait_bar<31>(bar_pv, (sc - 1) & 1) == 0)) {
+              late = true;
+              break;
+            }
             tc_fence_after();
             *alpha_row = alpha;
             __syncwarp();
@@ -874,26 +879,26 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           hand_over(true);
           ++items;
         }
-        if (!ok) give_up(abort_s, P.status, 30);
+        if (!ok) give_up(abort_s, P.status, late ? 31 : 30);
       } else {
         // ---------------------------------------------------------------- O: rescaling and output
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit::corr));
-        bool ok = true;
+        int fail = 0;
         uint32_t sc[2] = {0, 0}, items[2] = {0, 0};              // key tiles / work items so far per query tile slot
 #pragma unroll 1
-        for (int r = 0, w; ok && (w = work_at(r, total_work)) >= 0; ++r) {
+        for (int r = 0, w; fail == 0 && (w = work_at(r, total_work)) >= 0; ++r) {
           const Work wk = get_work<kCausal, kPacked, kList>(P, w);
           // O_t *= alpha for the rows whose maximum moved, in place in tensor memory, between the P.V of the previous
           // key tile and that of this one; warps in which no row's maximum moved skip it.  The first key tile of an
           // item overwrites O_t: this arrival then says that the previous item's output has been read.
 #pragma unroll 1
-          for (int it = 0; ok && it < wk.n_max; ++it) {
+          for (int it = 0; fail == 0 && it < wk.n_max; ++it) {
 #pragma unroll 1
             for (int t = 0; t < 2; ++t) {
               const int n_t = t == 0 ? wk.n_t[0] : wk.n_t[1];
               if (wk.n_max - 1 - it >= n_t) continue;
               uint32_t& cnt = t == 0 ? sc[0] : sc[1];
-              if (!(ok = wait_bar<>(bars + Bars::corr + 8 * (2 * quarter + t), cnt & 1))) break;
+              if ((fail = wait_bar<32>(bars + Bars::corr + 8 * (2 * quarter + t), cnt & 1)) != 0) break;
               ++cnt;
               const float alpha = *(reinterpret_cast<volatile float*>(smem + L::alpha) + t * 128 + row);
               if (it != wk.n_max - n_t && __any_sync(0xffffffffu, alpha != 1.0f)) {
@@ -922,7 +927,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               mbar_arrive_if(lane == 0, bars + Bars::p_full + 8 * t);
             }
           }
-          if (!ok) break;
+          if (fail != 0) break;
 
           // ---- output: O / l -> bf16 -> global.  D=128, dense batches: through a swizzled staging tile in shared
           // memory and two TMA stores per warp (32 rows x 64 columns) - a thread owns an output row, so direct
@@ -952,11 +957,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             const uint32_t last = (t == 0 ? sc[0] : sc[1]) - 1;
             uint32_t& ni = t == 0 ? items[0] : items[1];
             // the last key tile's row sum is there, and its P.V has landed
-            if (!(ok = wait_bar<>(bars + Bars::p_full + 8 * t, last & 1))) break;
+            if ((fail = wait_bar<33>(bars + Bars::p_full + 8 * t, last & 1)) != 0) break;
             const volatile float* l_row = reinterpret_cast<const volatile float*>(smem + L::lx) + t * 256 + row + (ni & 1) * 512;
             const float l = l_row[0], m = l_row[128];
             ++ni;
-            if (!(ok = wait_bar<>(bars + Bars::pv_done + 8 * t, last & 1))) break;
+            if ((fail = wait_bar<34>(bars + Bars::pv_done + 8 * t, last & 1)) != 0) break;
             tc_fence_after();
             const uint32_t tm_O = tmem + t * D + lane_addr;
             const bool keyless = m == kNoMax;                    // a row that has seen no key: zeros, LSE -inf
@@ -1015,7 +1020,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             }
           }
         }
-        if (!ok) give_up(abort_s, P.status, 32);
+        if (fail != 0) give_up(abort_s, P.status, fail);
         if (kTmaStore && lane == 0) bulk_wait_read0();   // the last output tiles have left shared memory before the CTA ends
       }
     }

@@ -509,7 +509,7 @@ int sage3_selftest_bounded_wait(int32_t* device_status, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   cudaError_t e = cudaMemsetAsync(device_status, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return cuda_fail(e);
-  e = sage3::launch_bounded_wait_selftest(device_status, 77, stream);
+  e = sage3::launch_bounded_wait_selftest(device_status, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   return SAGE3_OK;
 }

@@ -182,40 +182,48 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // block of a handful of instructions: left to the compiler it was unrolled at every one of the kernels' many waits,
 // and the instruction cache paid for it.  kWarp: by all 32 lanes of a warp, which leave it together and with the same answer,
 // each poll being a vote.
-template <bool kWarp = false>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
-  uint32_t ok;
+// Returns 0, or kCode where the limit is reached.
+template <bool kWarp, int kCode>
+__device__ __forceinline__ int mbar_wait_or(uint32_t bar, uint32_t parity, uint32_t limit) {
+  int fail;
 #define SAGE3_WAIT(VOTE)                                                                        \
   "{\n.reg .pred p;\n.reg .b32 n;\nmov.b32 n, %3;\nPOLL:\n"                                    \
   "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n" VOTE                                \
-  "@p bra DONE;\nadd.u32 n, n, -1;\nsetp.ne.u32 p, n, 0;\n@p bra POLL;\nDONE:\nmin.u32 %0, n, 1;\n}"
+  "@p bra DONE;\nadd.u32 n, n, -1;\nsetp.ne.u32 p, n, 0;\n@p bra POLL;\nDONE:\nselp.s32 %0, 0, %4, p;\n}"
   if constexpr (kWarp)
-    asm volatile(SAGE3_WAIT("vote.sync.all.pred p, p, 0xffffffff;\n") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+    asm volatile(SAGE3_WAIT("vote.sync.all.pred p, p, 0xffffffff;\n")
+                 : "=r"(fail) : "r"(bar), "r"(parity), "r"(limit), "n"(kCode) : "memory");
   else
-    asm volatile(SAGE3_WAIT("") : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
+    asm volatile(SAGE3_WAIT("") : "=r"(fail) : "r"(bar), "r"(parity), "r"(limit), "n"(kCode) : "memory");
 #undef SAGE3_WAIT
-  return ok != 0;
+  return fail;
+}
+template <bool kWarp = false>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
+  return mbar_wait_or<kWarp, 1>(bar, parity, limit) == 0;
 }
 
-// Bounded wait of a whole warp of one of the kernels' roles.  Where it returns false the caller leaves its loops, calls give_up
-// and unwinds instead of hanging the SM.
+// Bounded wait of a whole warp of one of the kernels' roles: 0, or kCode where it ran out.  Then the caller leaves its loops, calls
+// give_up with that code and unwinds instead of hanging the SM.  (The code comes out of the instruction that told success from
+// failure, so knowing which wait it was costs nothing.)
 //
 // The warp goes on to warp-wide instructions (tcgen05.ld / st, __syncwarp), so it must never split on a wait that ran out for
 // some of its lanes only: each poll is a vote.  That also lets the compiler treat the loops as uniform, without the code that
-// brings diverged lanes together again (16 prompts 484 -> 476 us; one vote behind a loop that is not uniform cost 6 %).
+// brings diverged lanes together again.
 //
 // The limit.  A failing poll takes 80 ns (a busy CTA) to 4 us (a parked warp): the default gives up after 0.02 to 1.05
 // seconds, where the longest wait of a working kernel is some 10 us.  A warp that waits does not look whether another
 // has given up: all of them wait for one another, so each runs out its own limit at about the same time, and that is why it
 // is not longer.
-template <uint32_t kPolls = (1u << 18)>
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity) {
-  return mbar_wait<true>(bar, parity, kPolls);
+template <int kCode, uint32_t kPolls = (1u << 18)>
+__device__ __forceinline__ int wait_bar(uint32_t bar, uint32_t parity) {
+  return mbar_wait_or<true, kCode>(bar, parity, kPolls);
 }
 
 // The same as a loop that the compiler sees, so that it knows the answer to be the warp's, and with a suspend-time hint: for
 // the QK issuer (all four forms measured for each role, within 1 % of one another; this one was the best over all shapes).
-__device__ __forceinline__ bool wait_bar_uniform(uint32_t bar, uint32_t parity) {
+template <int kCode>
+__device__ __forceinline__ int wait_bar_uniform(uint32_t bar, uint32_t parity) {
 #pragma unroll 1
   for (uint32_t n = 1u << 18; n != 0; --n) {
     uint32_t ok;
@@ -224,12 +232,12 @@ __device__ __forceinline__ bool wait_bar_uniform(uint32_t bar, uint32_t parity) 
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
         "selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
-    if (__all_sync(0xffffffffu, ok)) return true;
+    if (__all_sync(0xffffffffu, ok)) return 0;
   }
-  return false;
+  return kCode;
 }
 
-// A wait of this warp ran out: raises the CTA's abort flag and records `code` in *status (first writer wins).
+// A wait of this warp ran out: raises the CTA's abort flag and records its code in *status (first writer wins).
 __device__ __forceinline__ void give_up(volatile int* abort_s, int* status, int code) {
   *abort_s = 1;
   atomicCAS(status, 0, code);

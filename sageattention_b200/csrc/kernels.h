@@ -135,7 +135,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a, const DeltaSArgs& k, void* scr
 // Back-to-back block-scaled FP4 MMAs on resident operands, one CTA per SM (peak.cu); *ctas = CTAs launched.
 cudaError_t launch_fp4_mma_peak(int n_cols, int bursts, int* status, cudaStream_t stream, int* ctas);
 
-// One CTA runs a bounded wait that must give up (selftest.cu); *status receives `code`.
-cudaError_t launch_bounded_wait_selftest(int* status, int code, cudaStream_t stream);
+// One CTA runs a bounded wait that must give up (selftest.cu); *status receives 77.
+cudaError_t launch_bounded_wait_selftest(int* status, cudaStream_t stream);
 
 }  // namespace sage3

@@ -190,3 +190,11 @@ def test_workspace_of_few_query_rows_holds_only_what_their_kernels_use():
     assert packed == tiles() + up(8 * 8 * 13 * 128 * 4)
     assert lib.sage3_attention_workspace(None, 1, C.byref(n)) == _lib.ERR_ARGUMENT
     assert lib.sage3_attention_workspace(C.byref(_lib.Shape(1, 1, 1, 1, 1, 128)), 1, None) == _lib.ERR_ARGUMENT
+
+
+def test_every_wait_of_the_attention_kernel_has_a_code_of_its_own():
+    """The status word tells which hand-over stalled, not only in which warps."""
+    src = (ROOT / "sageattention_b200" / "csrc" / "attn.cu").read_text()
+    codes = [int(c) for c in re.findall(r"\bwait_bar(?:_uniform)?<(\d+)>\(", src)]
+    assert len(codes) == len(re.findall(r"\bwait_bar\w*\b *[<(]", src))
+    assert sorted(codes) == [10, 11, 12, 20, 21, 23, 24, 25, 26, 30, 31, 32, 33, 34, 40]
