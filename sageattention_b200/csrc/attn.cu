@@ -230,13 +230,6 @@ __device__ __forceinline__ void apply_lambda(uint32_t* r, const float* lam16) {
   r[0] = 0xff800000u;
 }
 
-// 128 score columns of this thread's tensor-memory lane -> registers
-__device__ __forceinline__ void load_scores(const uint32_t tm_S, uint32_t (&s)[128]) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) tmem_ld32(tm_S + 32 * q, *reinterpret_cast<uint32_t (*)[32]>(&s[32 * q]));
-  tmem_wait_ld();
-}
-
 // 2^x for two values on the FMA pipe (the special-function unit paces the softmax): x = n + r with n the nearest
 // integer, found by adding and subtracting 1.5 * 2^23, |r| <= 1/2; 2^r by a polynomial of degree 5, minimax in the
 // relative error (Remez exchange, computed for this file: 1.5e-7 with its coefficients rounded to fp32, 2.1e-7 = 2^-22.2 evaluated in
