@@ -253,7 +253,7 @@ __device__ __forceinline__ float2 ex2_poly(float2 x) {
 // Which of the 8 pairs of a 16-key block take it: 3 in 16.  Measured for 0 / 2 / 3 / 4 of 16 on rows of 256 key tiles
 // (B1 H10 N32760): D=128 3.98 / 3.75 / 3.65 / 3.72 ms, D=64 3.86 / 3.73 / 3.62 / 3.65 ms - more, and the 12
 // instructions per pair cost more issue slots than the unit's cycles they save.
-__device__ constexpr bool on_fma_pipe(const int blk, const int pair) {  return pair == 3 || (pair == 6 && (blk & 1)); }
+__device__ constexpr bool on_fma_pipe(const int blk, const int pair) { return pair == 3 || (pair == 6 && (blk & 1)); }
 // A NaN if one of the columns that take it has a NaN score, else a finite number or +inf, from the maxima that max16 leaves:
 // times 0 it goes into the row sum, so that such a row ends as one with a NaN in any other column does (its output zero, its
 // LSE NaN) whatever the place of the key.  (A row with a score of +inf has that sum anyhow: inf - inf.)  7 instructions per key
@@ -621,8 +621,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           for (int j = wk.n_max - 1; fail == 0 && j >= 0; --j) {
             if ((fail = wait_bar_uniform<21>(bars + Bars::k_full + 8 * s, ph)) != 0) break;
             if (has_ds && (fail = wait_bar_uniform<25>(bars + Bars::ds_ready + 8 * s, ph)) != 0) break;
-            // its scale factors on their way before the score buffer is free, into the columns that the MMAs of the stage before do not
-            // read (B1 H10 N32760 D128 3466 -> 3452 us)
+            // Its scale factors on their way before the score buffer is free, into the columns that the MMAs of the stage before do not
+            // read (B1 H10 N32760 D128 3466 -> 3452 us).  MMAs of two stages before have been seen complete by the waits for score
+            // buffers; but where an item of both tiles is followed by one of tile 0 only, at D=64, whose tile 0 does not wait for
+            // tile 1's buffer, it is the order in which the tensor pipe takes the copies and MMAs that one thread issues, as for
+            // the columns of V's scale factors.
             const uint32_t tm_sfk_s = tm_sfk + 8 * (s_odd & 1);
             s_odd ^= 1;
             tc_fence_after();

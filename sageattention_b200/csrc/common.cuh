@@ -108,8 +108,10 @@ __device__ __forceinline__ uint4 subtract_mean(const uint4& w, const float2 (&ne
   return make_uint4(pack_bf16(fadd2(bf16x2_to_f32(w.x), neg[0])), pack_bf16(fadd2(bf16x2_to_f32(w.y), neg[1])),
                     pack_bf16(fadd2(bf16x2_to_f32(w.z), neg[2])), pack_bf16(fadd2(bf16x2_to_f32(w.w), neg[3])));
 }
-// The same for a mean that is a bf16 value: the packed subtraction rounds the exact difference once, and no pair of bf16 values
-// exists for which rounding to fp32 first would change that (all 2^32 compared on the device, NaNs and subnormals included).
+// The same for a mean that is a bf16 value: the packed subtraction rounds the exact difference once.  Rounding to fp32 first, as above,
+// never changes that: 24 bits of significand are at least twice 8 and 2 more, so the second rounding is harmless (Figueroa, "When is
+// double rounding innocuous?", 1995); the formats share their exponents, so both overflow alike; and a difference below the
+// normal numbers is a multiple of the smallest bf16 value, hence exact in both.
 __device__ __forceinline__ uint4 subtract_mean(const uint4& w, const uint4& mean) {
   uint4 r;
   asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r.x) : "r"(w.x), "r"(mean.x));

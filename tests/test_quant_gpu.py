@@ -181,6 +181,49 @@ def test_whole_sequence_q_mean_mode():
     assert z.delta_s.shape == (B, H, 1, 384)
 
 
+def _bf16_of_bits(bits):
+    return bits.to(torch.int16).view(torch.bfloat16)
+
+
+def test_k_mean_subtracted_in_bf16_pairs():
+    """The K pass subtracts a given mean by packed bf16 instructions.  Its smoothed K is read back through delta_s with Q block means
+    that are unit vectors: equal to the fp32 difference rounded to bf16, for 16.8M pairs of any exponents (half of them with
+    a mean a few units in the last place away, subnormal values included), differences that overflow left out."""
+    g = torch.Generator().manual_seed(29)
+    B, H, N, D = 1, 8, 16384, 128
+    def bits(*shape):
+        return torch.randint(0, 2, shape, generator=g) * -32768 + torch.randint(0, 0x7E80, shape, generator=g)
+    km_bits = bits(B, H, D)
+    km_bits[0, 0] = km_bits[0, 0] % 0x100                                        # subnormals and the smallest normals
+    k_bits = bits(B, H, N, D)
+    near = km_bits[:, :, None] + torch.randint(-20, 21, (B, H, N, D), generator=g)
+    near = torch.where((near & 0x7FFF) < 0x7E80, near, km_bits[:, :, None])      # (no step below -0 or into larger ones)
+    k_bits[:, :, ::2] = near[:, :, ::2]
+    k, km = _bf16_of_bits(k_bits), _bf16_of_bits(km_bits)
+    want = (k.float() - km.float()[:, :, None]).to(torch.bfloat16)
+    assert torch.isfinite(want).all()
+    unit = torch.eye(D).expand(B, H, D, D).contiguous().to(DEV)
+    q = torch.zeros(B, H, D * 128, D, dtype=torch.bfloat16, device=DEV)
+    z = sa.quantize_qkv(q, k.to(DEV), q, km=km.to(DEV), qm_fp32=unit)
+    got = z.delta_s.cpu()                                                        # [B, H, block = channel, key]
+    assert torch.equal(got.float(), want.transpose(-1, -2).float())
+
+
+def test_k_mean_subtraction_of_values_that_are_not_finite():
+    """Infinities, NaN, overflow and cancelling infinities: codes and scales of the K pass (packed subtraction) equal those of the fused
+    quantiser (fp32 difference, rounded)."""
+    g = torch.Generator().manual_seed(31)
+    B, H, N, D = 2, 4, 1000, 128
+    bits = torch.randint(-32768, 32768, (B, H, N, D), generator=g)
+    bits[:, :, 1::2] = torch.where(torch.rand(B, H, N // 2, D, generator=g) < 0.05, bits[:, :, 1::2], bits[:, :, 1::2] & 0xBFFF)
+    odd = torch.tensor([0x7F80, -0x80, 0x7FC0, 0x7F7F, -0x81, 0x7F81, 0, -0x8000, 1, 0x80])
+    km_bits = odd[torch.randint(0, len(odd), (B, H, D), generator=g)]
+    k, km = _bf16_of_bits(bits).to(DEV), _bf16_of_bits(km_bits).to(DEV)
+    a = sa.quantize_qkv(k, k, k, km=km)
+    b = sa.quantize_qkv(k, k, k, km=km, with_delta_s=False)
+    assert torch.equal(a.k_codes, b.k_codes) and torch.equal(a.k_sf, b.k_sf)
+
+
 def test_bad_arguments_are_rejected():
     q, k, v = U.make_qkv(1, 2, 2, 128, 128, 128, device=DEV)
     with pytest.raises(AssertionError):
