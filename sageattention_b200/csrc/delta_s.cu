@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
       return;
     }
   }
-  using R = RowTile<D>;
+  using R = RowTile<D, false>;
   const int kc = R::block(t), krl = R::row(t);          // K rows: 16 channels a thread (A rows, c and rl: 8)
   const __nv_bfloat16* src = P.k + (P.cu_k ? (int64_t)P.cu_k[b] * P.k_sn : b * P.k_sb) + hkv * P.k_sh + kc * 16;
   auto place = [&](const int p, const int i) {          // of channels 8 i ... of this thread's row p in sB
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_quant_delta_s_kernel(const __gr
   }
   if (P.k_codes != nullptr) {
     const int64_t kt = (int64_t)bh * P.Tk + tile;
-    quant_rows_store<D>(w, P.k_codes + kt * (kTile * D / 2), P.k_sf + kt * ((D / 64) * 512), sf_smem);
+    quant_rows_store<D, false>(w, P.k_codes + kt * (kTile * D / 2), P.k_sf + kt * ((D / 64) * 512), sf_smem);
   }
   if (tile + 1 < end) load(tile + 1);
   // ---- delta_s: for the query blocks of all heads of the group, 128 at a time

@@ -109,42 +109,42 @@ __global__ void __launch_bounds__(kThreads, 4) channel_mean_kernel(
 
 // Channel sums of a Q tile: those of the warps' rows, red[warp][D].  The order is fixed - rows r, r + kStep, ... of the whole tile
 // one after another, then r and r + 1 (D=64: then the same of r + 2 and r + 3), the warps last, by the caller - because a block mean
-// that rounds the other way is seen in 128 rows of delta_s.  So a lane with rows 0 ... 63 hands its sums to the one that has the
-// other half of the same rows, which goes on from there; each later step leaves a lane half the channels.
+// that rounds the other way is seen in 128 rows of delta_s.  So the two lanes that have rows 0 ... 63 and 64 ... 127 of the same
+// kind swap half of their channels, and each adds all rows of 8.  (Launch of B1 H40 N32760 / B4 H32/8 N8192 / 16 prompts 218.8 / 96.8 /
+// 69.4 us; sums handed on, each lane adding twice: 223 / 99 / 72; swapped as sums are needed, twice the shuffles: 225 / 102 / 69; in
+// any order: 218.5 / 96.5 / 66.6.)
 template <int D>
-__device__ __forceinline__ void tile_sums(const uint4 (&w)[RowTile<D>::kPasses][2], const int t, const int c, float* red) {
+__device__ __forceinline__ void tile_sums(const uint4 (&w)[RowTile<D, true>::kPasses][2], const int t, const int c, float* red) {
+  constexpr int kPasses = RowTile<D, true>::kPasses;
+  const bool second = (t & 16) != 0;
+  float2 a[4] = {};
+  uint4 got[kPasses];                            // the first lane's channels 0 ... 7 of the other half, the second's 8 ... 15
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {                  // 8 channels at a time, for the registers
-    float2 a[4] = {};
-#pragma unroll
-    for (int p = 0; p < RowTile<D>::kPasses; ++p) add_channels(a, w[p][i]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      a[j].x = __shfl_xor_sync(0xffffffffu, a[j].x, 16);
-      a[j].y = __shfl_xor_sync(0xffffffffu, a[j].y, 16);
-    }
-#pragma unroll
-    for (int p = 0; p < RowTile<D>::kPasses; ++p) add_channels(a, w[p][i]);
-    float acc[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { acc[2 * j] = a[j].x; acc[2 * j + 1] = a[j].y; }
-    int first = c * 16 + 8 * i;
-#pragma unroll
-    for (int step = 0; step < (D == 128 ? 1 : 2); ++step) {
-      const int o = 4 << step, n = 4 >> step;    // the lane's bits that are the row
-      const bool upper = (t & o) != 0;
-#pragma unroll
-      for (int j = 0; j < n; ++j) {
-        const float give = upper ? acc[j] : acc[n + j], own = upper ? acc[n + j] : acc[j];
-        acc[j] = own + __shfl_xor_sync(0xffffffffu, give, o);
-      }
-      if (upper) first += n;
-    }
-    if (t & 16) {
-#pragma unroll
-      for (int j = 0; j < (D == 128 ? 4 : 2); ++j) red[(t >> 5) * D + first + j] = acc[j];
-    }
+  for (int p = 0; p < kPasses; ++p) {
+    const uint4 give = second ? w[p][0] : w[p][1];
+    got[p].x = __shfl_xor_sync(0xffffffffu, give.x, 16); got[p].y = __shfl_xor_sync(0xffffffffu, give.y, 16);
+    got[p].z = __shfl_xor_sync(0xffffffffu, give.z, 16); got[p].w = __shfl_xor_sync(0xffffffffu, give.w, 16);
+    add_channels(a, second ? got[p] : w[p][0]);
   }
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) add_channels(a, second ? w[p][1] : got[p]);
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { acc[2 * j] = a[j].x; acc[2 * j + 1] = a[j].y; }
+  int first = c * 16 + (second ? 8 : 0);
+#pragma unroll
+  for (int step = 0; step < (D == 128 ? 1 : 2); ++step) {        // each step of the exchange leaves a lane half its channels
+    const int o = 4 << step, n = 4 >> step;      // the lane's bits that are the row
+    const bool upper = (t & o) != 0;
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      const float give = upper ? acc[j] : acc[n + j], own = upper ? acc[n + j] : acc[j];
+      acc[j] = own + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+    if (upper) first += n;
+  }
+#pragma unroll
+  for (int j = 0; j < (D == 128 ? 4 : 2); ++j) red[(t >> 5) * D + first + j] = acc[j];
 }
 
 // Division by a number that the host knows, for 0 <= n < 2^31 (Granlund and Montgomery, "Division by invariant integers using
@@ -244,7 +244,7 @@ __device__ __forceinline__ void varlen_order(const QuantLaunch& P, int* hist) {
 // of 2000 each: 304 -> 299).
 template <int D, bool kVar>
 __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunch P) {
-  using R = RowTile<D>;
+  using R = RowTile<D, true>;
   __shared__ __align__(16) uint8_t sf_smem[2048];
   __shared__ __align__(16) float red[kThreads / (D / 8) * D];    // (what the K channel sums need; the Q means less)
   __shared__ __align__(16) float mean_s[D + D / 8];              // four words further every 32 channels, for the banks
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_qkv_kernel(const QuantLaunc
     }
     uint8_t* codes = (is_q ? P.q_codes : P.k_codes) + ((int64_t)bh * T + tile) * (kTile * D / 2);
     uint8_t* sf = (is_q ? P.q_sf : P.k_sf) + ((int64_t)bh * T + tile) * ((D / 64) * 512);
-    quant_rows_store<D>(w, codes, sf, sf_smem);
+    quant_rows_store<D, true>(w, codes, sf, sf_smem);
     }
     return;
   }

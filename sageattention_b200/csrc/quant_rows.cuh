@@ -12,19 +12,21 @@ constexpr int kThreads = 256;
 // Row-wise quantisation of one 128-token tile held in registers (Q and K roles).  Thread t owns the 16 channels 16 block(t) ... of
 // rows row(t), + kStep, ...: whole quantisation blocks, so that scales need no exchange and are worked out once.  (With 8 channels a
 // thread, two threads to a block: B1 H40 N32760 228 -> 219 us, K pass 321 -> 292.)
-// Which lane has which: its bits kBlockBits are the block, bit 4 is the half of the tile (rows 0 ... 63 or 64 ... 127, see tile_sums in
-// quant.cu), the others and the warp are the row modulo kStep.  D=128: so that 8 lanes' 16-byte stores of the K pass (delta_s.cu),
-// 4128 bytes from block to block and 16 from row to row, meet different banks.
+// Which lane has which: its bits kBlockBits are the block, the others the row.  D=128: so that 8 lanes' 16-byte stores of the K pass
+// (delta_s.cu), 4128 bytes from block to block and 16 from row to row, meet different banks.
+// kHalves (Q): bit 4 is the half of the tile (rows 0 ... 63 or 64 ... 127), which the order of the block sums asks for (tile_sums in
+// quant.cu); else a warp has rows next to one another (K pass of B1 H40 N32760 280 us, 299 with kHalves).
 // ------------------------------------------------------------------------------------------------
-template <int D>
+template <int D, bool kHalves>
 struct RowTile {
-  static constexpr int kPerRow = D / 16, kPasses = kTile * kPerRow / kThreads, kStep = kTile / 2 / kPasses;
+  static constexpr int kPerRow = D / 16, kPasses = kTile * kPerRow / kThreads, kStep = kTile / kPasses / (kHalves ? 2 : 1);
   static constexpr int kBlockBits = D == 128 ? 11 : 3;     // bits of the lane that are the block
   static __device__ __forceinline__ int block(const int t) { return D == 128 ? (t & 3) | ((t >> 1) & 4) : t & 3; }
   static __device__ __forceinline__ int row(const int t) {
+    if (!kHalves) return D == 128 ? ((t >> 2) & 1) | ((t >> 4) << 1) : t >> 2;
     return (D == 128 ? ((t >> 2) & 1) | ((t >> 5) << 1) : ((t >> 2) & 3) | ((t >> 5) << 2)) + ((t >> 4) & 1) * (kTile / 2);
   }
-  static_assert(kStep == kThreads / 32 * (D == 128 ? 2 : 4), "every row once");
+  static_assert(kStep == kThreads / (kHalves ? 2 : 1) / kPerRow, "every row once");
 };
 __device__ __forceinline__ void bf16x16_to_f32(const __nv_bfloat16* p, float (&x)[16]) {
 #pragma unroll
@@ -44,7 +46,7 @@ template <int D>
 __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, const float* __restrict__ partial, const int nchunks,
                                        const float divisor, const int64_t bh, float* stage, __nv_bfloat16* km_out,
                                        uint4 (&mean)[2]) {
-  const int t = threadIdx.x, c = RowTile<D>::block(t);
+  const int t = threadIdx.x, c = RowTile<D, false>::block(t);
   if (km != nullptr) {
     mean[0] = reinterpret_cast<const uint4*>(km + bh * D + c * 16)[0];
     mean[1] = reinterpret_cast<const uint4*>(km + bh * D + c * 16)[1];
@@ -74,10 +76,10 @@ __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, con
   mean[1] = reinterpret_cast<const uint4*>(stage)[2 * c + 1];
 }
 
-template <int D>
-__device__ __forceinline__ void quant_rows_store(const uint4 (&w)[RowTile<D>::kPasses][2], uint8_t* __restrict__ codes_tile,
+template <int D, bool kHalves>
+__device__ __forceinline__ void quant_rows_store(const uint4 (&w)[RowTile<D, kHalves>::kPasses][2], uint8_t* __restrict__ codes_tile,
                                                  uint8_t* __restrict__ sf_tile, uint8_t* sf_smem) {
-  using R = RowTile<D>;
+  using R = RowTile<D, kHalves>;
   const int t = threadIdx.x, c = R::block(t), rl = R::row(t);
   // sf_atom_offset of row rl + p * kStep is the sum of both offsets, the second a constant (left to the compiler, the addresses were
   // 15 % of the instructions)
