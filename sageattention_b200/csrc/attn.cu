@@ -54,9 +54,10 @@
 // exponentials, and so do the other hand-overs of a key tile (clock stamps).  So those of the softmax lie behind one another no
 // more than they must: the next scores' barrier is looked at in the last exponentials, that of the last P.V before the first
 // exponentials, whose codes wait in registers, and P^ is handed over while the next scores are on their way.  With it and with
-// loops that are not unrolled in the issuers: B1 H10 N32760 D128 3.67 -> 3.47 ms (whole operator), D64 3.59 -> 3.33, B4 H32/8 N8192
-// causal 1.66 -> 1.59, 16 prompts 435 -> 408 us.  The arithmetic of the softmax alone, two warps per sub-partition with every barrier
-// satisfied, takes 1200 to 1250 cycles per key tile and 128 query rows; here it is 1330, and was 1530.
+// loops that are not unrolled in the issuers: B1 H10 N32760 D128 3.67 -> 3.47 ms (whole operator; by now 3.41), D64 3.59 -> 3.33
+// (3.27), B4 H32/8 N8192 causal 1.66 -> 1.59 (1.56), 16 prompts 435 -> 408 us (376).  The arithmetic of the softmax alone, two warps
+// per sub-partition with every barrier satisfied, took 1170 to 1250 cycles per key tile and 128 query rows in two measurements;
+// the kernel takes 1410 (its time over the 35 rounds of B1 H40 N32760), and took 1530 before.
 //
 // Tensor memory (512 columns): O0 [0,D) O1 [D,2D) S [2D,2D+128) (D=64: one for each query tile, [2D,2D+256)); 56 columns of scale
 // factors, P^0 and P^1 (16 columns each: 128 FP4 codes per row).
@@ -250,8 +251,8 @@ __device__ __forceinline__ float2 ex2_poly(float2 x) {
   p.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
   return p;
 }
-// Which of the 8 pairs of a 16-key block take it: 3 in 16.  Measured for 0 / 2 / 3 / 4 of 16 on rows of 256 key tiles
-// (B1 H10 N32760): D=128 3.98 / 3.75 / 3.65 / 3.72 ms, D=64 3.86 / 3.73 / 3.62 / 3.65 ms - more, and the 12
+// Which of the 8 pairs of a 16-key block take it: 3 in 16.  Whole operator for 0 / 2 / 3 / 4 of 16 on rows of 256 key tiles
+// (B1 H10 N32760): D=128 3.55 / 3.42 / 3.41 / 3.45 ms, D=64 3.61 / 3.37 / 3.27 / 3.54 ms - more, and the 12
 // instructions per pair cost more issue slots than the unit's cycles they save.
 __device__ constexpr bool on_fma_pipe(const int blk, const int pair) { return pair == 3 || (pair == 6 && (blk & 1)); }
 // A NaN if one of the columns that take it has a NaN score, else a finite number or +inf, from the maxima that max16 leaves:
@@ -414,8 +415,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
                                                                    const __grid_constant__ CUtensorMap tm_o,
                                                                    const KParams P) {
   using L = Smem<D>;
-  // Score buffers in tensor memory: one for each query tile where there is room (D=64: B4 H32 N8192 causal 1553 -> 1543 us, longer rows
-  // gain nothing)
+  // Score buffers in tensor memory: one for each query tile where there is room (D=64, one buffer / two: B4 H32 N4096 753 / 739 us, B4
+  // H32/8 N8192 causal 1445 / 1408, B1 H10 N32760 3296 / 3273, B2 H16 N4100 Nk333 39.9 / 39.1, B8 H32 N1024 causal 115.5 / 113.0)
   constexpr int kSBufs = D == 64 ? 2 : 1;
   constexpr int kKB = D / 64;                              // K=64 blocks of the QK contraction
   constexpr uint32_t kSwzQK = (D == 128) ? 4u : 6u;        // 64-byte / 32-byte swizzle
@@ -622,7 +623,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
             if ((fail = wait_bar_uniform<21>(bars + Bars::k_full + 8 * s, ph)) != 0) break;
             if (has_ds && (fail = wait_bar_uniform<25>(bars + Bars::ds_ready + 8 * s, ph)) != 0) break;
             // Its scale factors on their way before the score buffer is free, into the columns that the MMAs of the stage before do not
-            // read (B1 H10 N32760 D128 3466 -> 3452 us).  MMAs of two stages before have been seen complete by the waits for score
+            // read (B1 H10 N32760 D128 3466 -> 3452 us; D=64 is within 0.3 % either way).  MMAs of two stages before have been seen complete by the waits for score
             // buffers; but where an item of both tiles is followed by one of tile 0 only, at D=64, whose tile 0 does not wait for
             // tile 1's buffer, it is the order in which the tensor pipe takes the copies and MMAs that one thread issues, as for
             // the columns of V's scale factors.

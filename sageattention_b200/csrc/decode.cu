@@ -148,7 +148,8 @@ __device__ __forceinline__ constexpr int score_place(const int k) { return (k & 
 // A CTA takes `score_run` key tiles one after another, each warp 16 keys of a tile, and fetches the rows of the next while it
 // works on the present one.  K is smoothed, quantised and multiplied where it was loaded, so neither its codes nor delta_s
 // exist in memory.  kOne: at most 8 query rows; the quantised rows then take the registers of the smoothed ones.
-// (One tile per CTA of four warps, 32 keys each: 47 us at B8 H32/8 Nk4096, now 26.)
+// (One tile per CTA of four warps, 32 keys each: 47 us at B8 H32/8 Nk4096, so 26; with V beside it 35, for 18 us less in the launch
+// before.)
 // kV: V of the same key tile comes through shared memory meanwhile and is quantised behind the scores: the conversions of K leave most
 // of the memory's time unused, and K, of which the launch before has just taken the sums, is still in L2 where V has not been read in
 // between.
@@ -564,8 +565,9 @@ bool decode_fits(int Hq, int Hkv, int Nq, int Nk) {
 }
 
 // Only the kernels of one group of rows and D=128 (D=64 keeps half the warps busy with V: B8 H32 Nk2000 63.1 -> 64.1 us), and not where
-// a launch is a chain of latencies anyhow (device time without / with: 48 tiles 13.6 / 13.9 us; B1 H32/8 Nk4096, 256 tiles 17.4 / 16.4,
-// B8 58.2 / 55.6, B32 224 / 202, B16 H32 Nk8000 779 / 679).
+// a launch is a chain of latencies anyhow (device time without / with, B1 H32/8: 32 tiles 11.3 / 11.7 us, 64 13.5 / 13.9, 96 16.6 / 15.8,
+// 128 17.3 / 17.4, 160 18.7 / 18.6, 192 21.7 / 19.5, 256 16.8 / 16.2; B2 and B4, 128 tiles 16.6 / 15.8 and 15.1 / 14.3; B8, 2048 tiles
+// 58.2 / 55.6; B32 224 / 202; B16 H32 Nk8000 779 / 679).
 bool decode_takes_v(int B, int Hq, int Hkv, int Nq, int Nk, int D) {
   return D == 128 && Hq / Hkv * Nq <= 8 && (int64_t)B * Hkv * ((Nk + kTile - 1) / kTile) >= 128;
 }

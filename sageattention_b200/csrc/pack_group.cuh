@@ -58,7 +58,7 @@ __device__ __forceinline__ float pack_group(const float (&x)[kGroup][C], const i
   for (int c = 0; c < C; ++c) dir[c] = nsq > 0.f ? __fdiv_rn(m[c], nsq) : 0.f;
   // ---- lambda of every token: 16 sums over the warp at once, each step of the exchange leaving a lane half of them - token
   // lane / 2 in the end.  The pairs of lanes that are added are those of an exchange of every sum on its own, and so are the bits.
-  // (On its own: 75 shuffles instead of 31.)
+  // (On its own, 75 shuffles instead of 31, K pass of B4 H32 N2048 D128 65.9 us; now 64.2.)
   float v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) {

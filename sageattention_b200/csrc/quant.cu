@@ -236,8 +236,8 @@ __device__ __forceinline__ void varlen_order(const QuantLaunch& P, int* hist) {
   }
 }
 
-// 64 registers: four CTAs per SM, each with a whole 32 KB tile in flight (B1 H40 N32760 D128, with the K sums: 240 us;
-// 260 at three per SM)
+// 64 registers: four CTAs per SM, each with a whole 32 KB tile in flight (B1 H40 N32760 D128, with the K sums: 219 us, 229 at three
+// per SM; B4 H32/8 N8192 96, 105)
 // kVar: variable-length batches, whose grid is sized for sequences of the greatest length.  A CTA of the Q role then takes its tile of
 // up to four heads, so that there are a quarter of the CTAs for tiles that no sequence has, and one of the V role leaves at once
 // (16 prompts of 187 to 3000 tokens, H32/8: 77.7 -> 66.5 us; operator with 31 prompts of 600 and 8000, D=64: 687 -> 650, with eight
@@ -478,7 +478,7 @@ void quant_chunks(int BH, int N, int* chunks, int* chunk_tokens) {
   *chunks = (N + *chunk_tokens - 1) / *chunk_tokens;
 }
 
-// Fewest CTAs of the Q role of a variable-length batch that sharing one among heads may leave: two waves.  (Below, a chain of four
+// Fewest CTAs of the Q role of a variable-length batch that sharing one among heads may leave: two waves of four CTAs on each of 148 SMs.  (Below, a chain of four
 // heads is what counts: two prompts of 64 and 30 tokens 15.7 us, 19.0 with four heads to a CTA.)
 constexpr int64_t kVarCtas = 1184;
 

@@ -40,7 +40,7 @@ __device__ __forceinline__ void bf16x16_to_f32(const __nv_bfloat16* p, float (&x
 // The 16 channels of this thread (16 block(threadIdx.x) ...) of a head's K mean: from `km` where it is given, else from
 // the partial sums, by the whole CTA; also written to km_out if that is not null.  `stage`: shared memory for kMaxChunks
 // partial rows - they are fetched all at once, so that the CTA waits for memory once and not once per few rows (the K
-// kernel at B1 H40 N32760: 328 us, 356 with a chain of loads).
+// kernel of that time at B1 H40 N32760: 328 us, 356 with a chain of loads; by now 281).
 constexpr int kMaxChunks = 64;             // at most so many partial rows per head (pick_chunk_tokens, quant.cu)
 template <int D>
 __device__ __forceinline__ void k_mean(const __nv_bfloat16* __restrict__ km, const float* __restrict__ partial, const int nchunks,
