@@ -478,8 +478,8 @@ void quant_chunks(int BH, int N, int* chunks, int* chunk_tokens) {
   *chunks = (N + *chunk_tokens - 1) / *chunk_tokens;
 }
 
-// Fewest CTAs of the Q role of a variable-length batch that sharing one among heads may leave: two waves of four CTAs on each of 148 SMs.  (Below, a chain of four
-// heads is what counts: two prompts of 64 and 30 tokens 15.7 us, 19.0 with four heads to a CTA.)
+// Fewest CTAs of the Q role of a variable-length batch that sharing one among heads may leave: two waves of four CTAs on each of 148
+// SMs.  (Below, a chain of four heads is what counts: two prompts of 64 and 30 tokens 15.7 us, 19.0 with four heads to a CTA.)
 constexpr int64_t kVarCtas = 1184;
 
 cudaError_t launch_quant_qkv(const QuantArgs& a, cudaStream_t stream) {
