@@ -16,7 +16,7 @@
 // before the first use (a whole 32 KB tile in flight per CTA) and owns whole 16-element blocks, codes
 // leave as full 32-byte sectors and the scale bytes are staged in shared memory so that they leave as
 // 16-byte vectors in the exact order the attention kernel's tcgen05.cp expects.  What paces it is instructions
-// (about half of the issue slots, at 4.6 TB/s) as much as memory: 12 per element of Q, 12 of V with its share of the K sums.
+// (about half of the issue slots, at 4.6 TB/s) as much as memory: 13 per element of Q, 12 of V with its share of the K sums.
 //
 // Output layouts (per batch b, head h; Np = tokens padded to a multiple of 128, T = Np/128):
 //   codes  Q,K : [T][128 rows][D/2] bytes            (row-major, element 2i in the low nibble)
